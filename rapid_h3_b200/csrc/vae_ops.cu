@@ -15,9 +15,16 @@
 // reference builds with approximate division, this kernel divides exactly, so the last code bit can differ
 // from that binary: parity is defined by the CPU oracle, oracle/vae_ops.py).
 //
-// One CTA per row at a time (persistent), K / 8 threads, a warp owns one 256-column group: lane l holds
-// columns 8l .. 8l+7, i.e. base-4 digits (d0 = j & 3, d1 = (j >> 2) + 2 (l & 1), d2 = (l >> 1) & 3, d3 = l >> 3).
-// HBM-bound: 3 bytes per element (2 in, 1 out).
+// One CTA per row at a time (persistent), K / 16 threads, the next row's loads in flight while a row is worked on. A
+// half-warp owns one 256-column group: thread t of it holds columns 16t .. 16t+15, i.e. the two low base-4 digits, so
+// stages 1 and 4 run inside the thread; one 16 x 16 exchange through shared memory (4-float rows padded to 20: no bank
+// conflicts, only the half-warp's own patch, so __syncwarp orders it) gives the thread columns t, t + 16, ... for
+// stages 16 and 64, and the codes go back through the same patch as bytes for 16-byte stores. No value crosses lanes by
+// shuffle: the form with eight columns per thread and shuffles for three of the four stages (9 shuffles per value, and
+// 1,024 threads per 8,192-wide row, one CTA per SM) took 131 us for 3,594 x 8,192 and 35 us for 3,594 x 2,048 with the
+// RMSNorm prologue, this one 40 and 16.
+// Algorithmic traffic: 3 bytes per element (2 in, 1 out), 13.5 and 3.4 us at those sizes and the measured copy rate; what
+// is left above it is instruction issue (about 25 per value).
 #include "common.cuh"
 #include "rapidh3_b200.h"
 
@@ -30,50 +37,22 @@ __device__ __forceinline__ float nan_to_num_h(__half h) {
   return __half2float(h);
 }
 
-// one stage: the value at position k (0..3) of the quadruple (e0, e1, e2, e3)
-__device__ __forceinline__ float fht_stage(float e0, float e1, float e2, float e3, int k) {
-  float r;
-  if (k == 0) r = __fsub_rn(__fadd_rn(__fadd_rn(e0, e1), e2), e3);
-  else if (k == 1) r = __fadd_rn(__fsub_rn(__fadd_rn(e0, e1), e2), e3);
-  else if (k == 2) r = __fadd_rn(__fadd_rn(__fsub_rn(e0, e1), e2), e3);
-  else r = __fadd_rn(__fadd_rn(__fsub_rn(e1, e0), e2), e3);  // -x0 + x1 == x1 - x0 exactly
-  return 0.5f * r;
+// One radix-4 stage without its factor 1/2 (an exact scaling, applied once as 1/16 after the four stages):
+// e0' = ((e0 + e1) + e2) - e3, e1' = ((e0 + e1) - e2) + e3, e2' = ((e0 - e1) + e2) + e3, e3' = ((e1 - e0) + e2) + e3
+__device__ __forceinline__ void fht_quad(float& e0, float& e1, float& e2, float& e3) {
+  const float s = __fadd_rn(e0, e1), d = __fsub_rn(e0, e1);  // e1 - e0 == -d exactly
+  e0 = __fsub_rn(__fadd_rn(s, e2), e3);
+  e1 = __fadd_rn(__fsub_rn(s, e2), e3);
+  const float t2 = __fadd_rn(__fadd_rn(d, e2), e3), t3 = __fadd_rn(__fsub_rn(e2, d), e3);
+  e2 = t2;
+  e3 = t3;
 }
-
-__device__ __forceinline__ void fht256(float* x, int lane) {
+// the two stages whose digits the thread's 16 values span
+__device__ __forceinline__ void fht16(float* x) {
 #pragma unroll
-  for (int b = 0; b < 8; b += 4) {  // stride 1
-    const float e0 = x[b], e1 = x[b + 1], e2 = x[b + 2], e3 = x[b + 3];
+  for (int b = 0; b < 16; b += 4) fht_quad(x[b], x[b + 1], x[b + 2], x[b + 3]);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) x[b + k] = fht_stage(e0, e1, e2, e3, k);
-  }
-  {  // stride 4: positions 0, 1 are x[j], x[j+4] of the even lane, 2, 3 those of the odd lane
-    const bool odd = lane & 1;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float u = x[j], w = x[j + 4];
-      const float pu = __shfl_xor_sync(0xffffffffu, u, 1), pw = __shfl_xor_sync(0xffffffffu, w, 1);
-      const float e0 = odd ? pu : u, e1 = odd ? pw : w, e2 = odd ? u : pu, e3 = odd ? w : pw;
-      x[j] = odd ? fht_stage(e0, e1, e2, e3, 2) : fht_stage(e0, e1, e2, e3, 0);
-      x[j + 4] = odd ? fht_stage(e0, e1, e2, e3, 3) : fht_stage(e0, e1, e2, e3, 1);
-    }
-  }
-#pragma unroll
-  for (int stage = 0; stage < 2; ++stage) {  // strides 16 and 64: one position per lane
-    const int shift = stage == 0 ? 1 : 3;
-    const int k = (lane >> shift) & 3;
-    const int base = lane & ~(3 << shift);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float e0 = __shfl_sync(0xffffffffu, x[j], base);
-      const float e1 = __shfl_sync(0xffffffffu, x[j], base | (1 << shift));
-      const float e2 = __shfl_sync(0xffffffffu, x[j], base | (2 << shift));
-      const float e3 = __shfl_sync(0xffffffffu, x[j], base | (3 << shift));
-      x[j] = k == 0 ? fht_stage(e0, e1, e2, e3, 0)
-                    : (k == 1 ? fht_stage(e0, e1, e2, e3, 1)
-                              : (k == 2 ? fht_stage(e0, e1, e2, e3, 2) : fht_stage(e0, e1, e2, e3, 3)));
-    }
-  }
+  for (int j = 0; j < 4; ++j) fht_quad(x[j], x[j + 4], x[j + 8], x[j + 12]);
 }
 
 enum { ACT_NONE = 0, ACT_RMS_NORM = 1, ACT_SWIGLU = 2 };
@@ -90,102 +69,198 @@ struct OutQuantParams {
   int64_t head_stride;    // elements between consecutive D-wide pieces of a row
   int64_t row_stride;     // elements between rows
   int64_t rows;
+  int wide;               // q is 16-byte aligned: 16-byte stores (8-byte ones otherwise)
 };
 
-template <int T>
-__global__ void __launch_bounds__(T) vae_out_quant_kernel(const OutQuantParams p) {
-  __shared__ float red[T / 32];
-  const int tid = threadIdx.x;
-  const int K = p.K;
-  const int col = tid << 3;
-  const bool active = col < K;
-  const int head = active ? col / p.D : 0;
-  const int d = col - head * p.D;
-  for (int64_t row = blockIdx.x; row < p.rows; row += gridDim.x) {
-    float v[8];
-    if (active) {
-      const uint4 raw = __ldg(reinterpret_cast<const uint4*>(p.o + head * p.head_stride + row * p.row_stride + d));
-      const __half* h = reinterpret_cast<const __half*>(&raw);
+constexpr int ROW_F = 20;               // floats per 16-value row of a half-warp's exchange patch (16 + 4 padding)
+constexpr int PATCH_F = 16 * ROW_F + 16;  // the two half-warps of a warp land on different banks
+
+__device__ __forceinline__ void unpack16h(const uint4* raw, float* v) {
+  const uint32_t w[8] = {raw[0].x, raw[0].y, raw[0].z, raw[0].w, raw[1].x, raw[1].y, raw[1].z, raw[1].w};
+  uint32_t special = 0;  // a half with all exponent bits set (NaN or infinity) carries into its sign bit
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = nan_to_num_h(h[j]);
-    } else {
+  for (int j = 0; j < 8; ++j) {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
+    v[2 * j] = f.x;
+    v[2 * j + 1] = f.y;
+    special |= (w[j] & 0x7FFF7FFFu) + 0x04000400u;
+  }
+  if (special & 0x80008000u) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = 0.f;
-    }
-    if (p.act == ACT_RMS_NORM) {
-      // y = (x * r) * w, r = 1 / sqrt(mean(x^2) + eps); the sum of squares in a fixed order: the 8 values of a
-      // thread in order, an xor butterfly over the warp, then the warps in order
-      float ss = 0.f;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) ss = __fadd_rn(ss, __fmul_rn(v[j], v[j]));
-      ss = warp_sum_xor(ss);
-      if ((tid & 31) == 0) red[tid >> 5] = ss;
-      __syncthreads();
-      ss = red[0];
-#pragma unroll
-      for (int w = 1; w < T / 32; ++w) ss = __fadd_rn(ss, red[w]);
-      __syncthreads();
-      const float r = __fdiv_rn(1.f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, static_cast<float>(K)), p.eps)));
-      if (active) {
-        float wv[8] = {1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f};
-        if (p.act_w) {
-          const uint4 raw = __ldg(reinterpret_cast<const uint4*>(p.act_w + col));
-          const __half* h = reinterpret_cast<const __half*>(&raw);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) wv[j] = __half2float(h[j]);
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = __fmul_rn(__fmul_rn(v[j], r), wv[j]);
-      }
-    } else if (p.act == ACT_SWIGLU) {
-      // y = silu(gate) * up with gate = this row's first K values, up = the K values up_offset further on
-      if (active) {
-        const uint4 raw = __ldg(reinterpret_cast<const uint4*>(p.o + head * p.head_stride + row * p.row_stride + d + p.up_offset));
-        const __half* h = reinterpret_cast<const __half*>(&raw);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float g = v[j], u = nan_to_num_h(h[j]);
-          v[j] = __fmul_rn(__fmul_rn(g, __fdiv_rn(1.f, __fadd_rn(1.f, expf(-g)))), u);
-        }
-      }
-    }
-    if (tid - (tid & 31) < (K >> 3)) fht256(v, tid & 31);  // warp-uniform: K is a multiple of 256
-    float am = 0.f;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) am = fmaxf(am, fabsf(v[j]));
-    am = warp_max(am);
-    if ((tid & 31) == 0) red[tid >> 5] = am;
-    __syncthreads();
-    am = red[0];
-#pragma unroll
-    for (int w = 1; w < T / 32; ++w) am = fmaxf(am, red[w]);
-    __syncthreads();
-    const float scale = fmaxf(__fmul_rn(fminf(am, 65504.f), 1.0f / 127.0f), 1.0e-30f);
-    const float scale_h = __half2float(__float2half_rn(scale));
-    if (tid == 0) p.scales[row] = scale;
-    if (active) {
-      uint32_t code[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float vh = __half2float(__float2half_rn(v[j]));
-        const float qf = __half2float(__float2half_rn(__fdiv_rn(vh, scale_h)));
-        code[j] = static_cast<uint32_t>(static_cast<int>(fminf(127.f, fmaxf(-128.f, rintf(qf)))));
-      }
-      const uint2 o = make_uint2(pack_low_bytes(code[0], code[1], code[2], code[3]),
-                                 pack_low_bytes(code[4], code[5], code[6], code[7]));
-      *reinterpret_cast<uint2*>(p.q + row * K + col) = o;
+    for (int j = 0; j < 8; ++j) {
+      const __half2 h = *reinterpret_cast<const __half2*>(&w[j]);
+      v[2 * j] = nan_to_num_h(__low2half(h));
+      v[2 * j + 1] = nan_to_num_h(__high2half(h));
     }
   }
 }
 
-template <int T>
+template <int T, int ACT>
+__global__ void __launch_bounds__(T) vae_out_quant_kernel(const OutQuantParams p) {
+  __shared__ __align__(16) float patch[T / 16][PATCH_F];
+  __shared__ float red[2][T / 16], red_ss[2][T / 16];  // two sets: one barrier per reduction and row is enough
+  const int tid = threadIdx.x, grp = tid >> 4, t = tid & 15;
+  const int K = p.K;
+  const int col = tid << 4;
+  const bool active = col < K;  // K is a multiple of 256: uniform over a half-warp
+  const int ngrp = K >> 8;
+  int64_t off[2] = {0, 0};      // the row's two 8-wide pieces may belong to different heads
+  if (active) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int c = col + 8 * i, head = c / p.D;
+      off[i] = head * p.head_stride + (c - head * p.D);
+    }
+  }
+  uint4 raw[2], up[2];
+  auto load = [&](int64_t row) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      raw[i] = make_uint4(0, 0, 0, 0);
+      if (ACT == ACT_SWIGLU) up[i] = make_uint4(0, 0, 0, 0);
+      if (active) {
+        const __half* src = p.o + off[i] + row * p.row_stride;
+        raw[i] = __ldg(reinterpret_cast<const uint4*>(src));
+        if (ACT == ACT_SWIGLU) up[i] = __ldg(reinterpret_cast<const uint4*>(src + p.up_offset));
+      }
+    }
+  };
+  int64_t row = blockIdx.x;
+  if (row < p.rows) load(row);
+  for (int par = 0; row < p.rows; row += gridDim.x, par ^= 1) {
+    float v[16];
+    unpack16h(raw, v);
+    if (ACT == ACT_SWIGLU) {
+      // y = silu(gate) * up with gate = this row's first K values, up = the K values up_offset further on
+      float u[16];
+      unpack16h(up, u);
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        v[j] = __fmul_rn(__fmul_rn(v[j], __fdiv_rn(1.f, __fadd_rn(1.f, expf(-v[j])))), u[j]);
+    }
+    if (row + gridDim.x < p.rows) load(row + gridDim.x);  // in flight under the rest of this row
+    if (ACT == ACT_RMS_NORM) {
+      // y = (x * r) * w, r = 1 / sqrt(mean(x^2) + eps); the sum of squares in a fixed order: runs of 8 columns in order,
+      // an xor butterfly (16, 8, 4, 2, 1) over the 32 runs of a group, then the groups in order. A thread holds the runs
+      // 2t and 2t + 1: run distance 16, 8, 4, 2 is lane distance 8, 4, 2, 1, the last step is inside the thread.
+      float sa = 0.f, sb = 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        sa = __fadd_rn(sa, __fmul_rn(v[j], v[j]));
+        sb = __fadd_rn(sb, __fmul_rn(v[8 + j], v[8 + j]));
+      }
+#pragma unroll
+      for (int o = 8; o; o >>= 1) {
+        sa = __fadd_rn(sa, __shfl_xor_sync(0xffffffffu, sa, o));
+        sb = __fadd_rn(sb, __shfl_xor_sync(0xffffffffu, sb, o));
+      }
+      if (t == 0) red_ss[par][grp] = __fadd_rn(sa, sb);
+      __syncthreads();
+      float ss = red_ss[par][0];
+      for (int w = 1; w < ngrp; ++w) ss = __fadd_rn(ss, red_ss[par][w]);
+      const float r = __fdiv_rn(1.f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, static_cast<float>(K)), p.eps)));
+      if (active) {
+        float wv[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) wv[j] = 1.f;
+        if (p.act_w) {
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const uint4 wr = __ldg(reinterpret_cast<const uint4*>(p.act_w + col + 8 * i));
+            const __half* h = reinterpret_cast<const __half*>(&wr);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) wv[8 * i + j] = __half2float(h[j]);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = __fmul_rn(__fmul_rn(v[j], r), wv[j]);
+      }
+    }
+    // stages 1 and 4, exchange, stages 16 and 64: v[i] becomes column t + 16 i of the group
+    float* mine = patch[grp];
+    fht16(v);
+#pragma unroll
+    for (int j = 0; j < 16; j += 4)
+      *reinterpret_cast<float4*>(mine + t * ROW_F + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = mine[i * ROW_F + t];
+    fht16(v);
+    float am = 0.f;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      v[j] = __fmul_rn(v[j], 0.0625f);
+      am = fmaxf(am, fabsf(v[j]));
+    }
+#pragma unroll
+    for (int o = 8; o; o >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
+    if (t == 0) red[par][grp] = am;
+    __syncthreads();
+    am = red[par][0];
+    for (int w = 1; w < ngrp; ++w) am = fmaxf(am, red[par][w]);
+    const float scale = fmaxf(__fmul_rn(fminf(am, 65504.f), 1.0f / 127.0f), 1.0e-30f);
+    const float scale_h = __half2float(__float2half_rn(scale));
+    if (tid == 0) p.scales[row] = scale;
+    // The quotient vh / scale_h is the correctly rounded one: with inv the rounded reciprocal, q0 = vh * inv and the exact
+    // remainder fma(-q0, scale_h, vh), q = fma(remainder, inv, q0) equals the IEEE quotient (Markstein) as long as nothing
+    // under- or overflows. vh and scale_h are fp16 values, so that holds whenever vh is finite and scale_h is not 0; a
+    // row with a value beyond fp16's range, or so small that its scale rounds to 0, divides (uniform over the row).
+    const bool exact_div = !(am <= 65504.f) || scale_h == 0.f;
+    const float inv = __fdiv_rn(1.f, scale_h);
+    uint8_t* bytes = reinterpret_cast<uint8_t*>(mine);
+    __syncwarp();  // the group's values have been read
+    const __half2 lo2 = __float2half2_rn(-128.f), hi2 = __float2half2_rn(127.f), magic2 = __float2half2_rn(1536.f);
+#pragma unroll
+    for (int i = 0; i < 16; i += 2) {
+      const float2 vh = __half22float2(__floats2half2_rn(v[i], v[i + 1]));
+      float q0, q1;
+      if (exact_div) {
+        q0 = __fdiv_rn(vh.x, scale_h);
+        q1 = __fdiv_rn(vh.y, scale_h);
+      } else {
+        q0 = __fmul_rn(vh.x, inv);
+        q1 = __fmul_rn(vh.y, inv);
+        q0 = fmaf(fmaf(-q0, scale_h, vh.x), inv, q0);
+        q1 = fmaf(fmaf(-q1, scale_h, vh.y), inv, q1);
+      }
+      // the quotient through fp16, clamped (a NaN quotient, 0 / 0, becomes -128), then rounded half to even by adding
+      // 1.5 * 2^10, whose last place is 1: the code is the low byte of the sum's bits
+      const __half2 c = __hadd2(__hmin2(__hmax2(__floats2half2_rn(q0, q1), lo2), hi2), magic2);
+      const uint32_t bits = *reinterpret_cast<const uint32_t*>(&c);
+      bytes[t + 16 * i] = static_cast<uint8_t>(bits);
+      bytes[t + 16 * i + 16] = static_cast<uint8_t>(bits >> 16);
+    }
+    __syncwarp();
+    if (active) {
+      const uint4 o = *reinterpret_cast<const uint4*>(bytes + 16 * t);
+      int8_t* dst = p.q + row * K + col;
+      if (p.wide) {
+        *reinterpret_cast<uint4*>(dst) = o;
+      } else {
+        *reinterpret_cast<uint2*>(dst) = make_uint2(o.x, o.y);
+        *reinterpret_cast<uint2*>(dst + 8) = make_uint2(o.z, o.w);
+      }
+    }
+    __syncwarp();  // before the next row's values overwrite the patch
+  }
+}
+
+template <int T, int ACT>
 int launch_out_quant(const OutQuantParams& p, cudaStream_t stream) {
-  auto kern = vae_out_quant_kernel<T>;
+  auto kern = vae_out_quant_kernel<T, ACT>;
   int occ = 1;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, T, 0) != cudaSuccess || occ < 1) occ = 1;
   const int64_t resident = static_cast<int64_t>(device_sm_count()) * occ;
   kern<<<static_cast<unsigned>(p.rows < resident ? p.rows : resident), T, 0, stream>>>(p);
   return check_cuda(cudaGetLastError(), "vae_out_quant launch");
+}
+template <int ACT>
+int launch_out_quant_act(const OutQuantParams& p, cudaStream_t stream) {
+  const int threads = p.K / 16;
+  if (threads <= 64) return launch_out_quant<64, ACT>(p, stream);
+  if (threads <= 128) return launch_out_quant<128, ACT>(p, stream);
+  if (threads <= 256) return launch_out_quant<256, ACT>(p, stream);
+  return launch_out_quant<512, ACT>(p, stream);
 }
 
 }  // namespace
@@ -194,12 +269,11 @@ int launch_out_quant(const OutQuantParams& p, cudaStream_t stream) {
 using namespace rh3;
 
 namespace {
-int out_quant_launch(const OutQuantParams& p, cudaStream_t stream) {
-  const int64_t threads = p.K / 8;
-  if (threads <= 128) return launch_out_quant<128>(p, stream);
-  if (threads <= 256) return launch_out_quant<256>(p, stream);
-  if (threads <= 512) return launch_out_quant<512>(p, stream);
-  return launch_out_quant<1024>(p, stream);
+int out_quant_launch(OutQuantParams p, cudaStream_t stream) {
+  p.wide = (reinterpret_cast<uintptr_t>(p.q) & 15) == 0;
+  if (p.act == ACT_RMS_NORM) return launch_out_quant_act<ACT_RMS_NORM>(p, stream);
+  if (p.act == ACT_SWIGLU) return launch_out_quant_act<ACT_SWIGLU>(p, stream);
+  return launch_out_quant_act<ACT_NONE>(p, stream);
 }
 }  // namespace
 

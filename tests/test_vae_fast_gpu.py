@@ -193,3 +193,38 @@ def test_vae_ff_forward(vf, epilogue):
     hh = torch.nn.functional.silu(hh[:, :f]) * hh[:, f:]
     full = (hh @ w2.float().t() + b2.float()) * rs.float() + resid.float()
     assert ((y.cpu().reshape(m, k).float() - full).norm() / full.norm()).item() < 2e-2
+
+
+@pytest.mark.parametrize("k", [256, 768, 1280, 2304, 4352])
+@pytest.mark.parametrize("act", ["none", "rms_norm"])
+def test_vae_quantizer_partial_blocks_and_extreme_rows(vf, k, act):
+    """Row widths that leave part of the block idle; rows that are zero, so small that their fp16 scale is 0 or
+    subnormal, beyond fp16's range after the rotation, or hold NaN / inf; more rows than resident blocks."""
+    vae_fast, lib = vf
+    g = inputs.gen(k)
+    x = torch.randn(2500, k, generator=g)
+    x[0] = 0
+    x[1] *= 1e-7
+    x[2] *= 3e-6
+    x[3] = 60000.0
+    x[4] *= 20000.0
+    x[5, ::17] = float("nan")
+    x[6, 3] = float("inf")
+    x[7, 250:255] = float("-inf")
+    x = x.half()
+    q, s = vae_fast._quantize(x.cuda(), act, None, 1e-6)
+    lib.check_status()
+    qr, sr = ov.quant_rows_f16(x, act, None, 1e-6)
+    assert torch.equal(s.cpu().reshape(-1), sr) and torch.equal(q.cpu(), qr)
+
+
+def test_vae_quantizer_eight_byte_aligned_codes(vf):
+    vae_fast, lib = vf
+    x = torch.randn(9, 512, generator=inputs.gen(2)).half()
+    buf = torch.zeros(9 * 512 + 8, dtype=torch.int8, device="cuda")
+    s = torch.empty(9, device="cuda")
+    xd = x.cuda()
+    lib.call("rh3_vae_quant_rows", xd.data_ptr(), 512, 9, 512, buf.data_ptr() + 8, s.data_ptr(), lib.stream())
+    lib.check_status()
+    qr, sr = ov.quant_rows_f16(x)
+    assert torch.equal(buf[8:].view(9, 512).cpu(), qr) and torch.equal(s.cpu(), sr) and not buf[:8].any()
