@@ -252,6 +252,10 @@ int rh3_gn_reduce(const float* gn_part, int64_t rows_per_sample, int64_t N, doub
 /* y = silu((x - mean[n, g]) * rstd[n, g] * gamma[c] + beta[c]); mean_rstd is fp32 [N, 32, 2]; 32 groups. */
 int rh3_gn_silu_apply(const void* x, const float* mean_rstd, const void* gamma, const void* beta, int64_t N,
                       int64_t sites_per_sample, int64_t C, void* y, cudaStream_t stream);
+/* The same from the fp64 sums [N, 32, 2] of rh3_gn_reduce: mean = s * (1/count), rstd = rsqrt(max(s2 * (1/count) - mean^2, 0)
+ * + eps), each operation rounded in fp64, both then rounded to fp32. count = values per (sample, group). */
+int rh3_gn_silu_from_sums(const void* x, const double* sums, double count, double eps, const void* gamma, const void* beta,
+                          int64_t N, int64_t sites_per_sample, int64_t C, void* y, cudaStream_t stream);
 /* y[N, 2T-1, 2H, 2W, C]: nearest-neighbour 2x in space, causal 2x in time (the first frame is not repeated). */
 int rh3_upsample_causal2x(const void* x, void* y, int64_t N, int64_t T, int64_t H, int64_t W, int64_t C,
                           cudaStream_t stream);

@@ -13,7 +13,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "librapidh3_b200.so")
 HEADER_PATH = os.path.join(os.path.dirname(HERE), "include", "rapidh3_b200.h")
 
-_P, _I64, _I, _F = ctypes.c_void_p, ctypes.c_int64, ctypes.c_int, ctypes.c_float
+_P, _I64, _I, _F, _D = ctypes.c_void_p, ctypes.c_int64, ctypes.c_int, ctypes.c_float, ctypes.c_double
 
 # argument types per entry point, in header order (every pointer / stream is a void*)
 SIGNATURES = {
@@ -65,6 +65,7 @@ SIGNATURES = {
     "rh3_conv3d_gn_part_rows": [_I64, _I64, _I64, _I64],
     "rh3_gn_reduce": [_P, _I64, _I64, _P, _P],
     "rh3_gn_silu_apply": [_P, _P, _P, _P, _I64, _I64, _I64, _P, _P],
+    "rh3_gn_silu_from_sums": [_P, _P, _D, _D, _P, _P, _I64, _I64, _I64, _P, _P],
     "rh3_upsample_causal2x": [_P, _P, _I64, _I64, _I64, _I64, _I64, _P],
 }
 # entry points that return a value instead of a status

@@ -603,11 +603,29 @@ __device__ __forceinline__ float silu_fast(float t) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
   return t * r;
 }
+// FROM_SUMS: mean and rstd are taken from the fp64 sums by the first warp of the block (a group per lane), in the order
+// a chain of elementwise kernels would compute them (s * (1/count), E[x^2] - mean^2, clamped, + eps, rsqrt, all rounded
+// one by one in fp64), so the bits are the same and the chain's eight launches of one tiny block each are gone: a decode
+// runs 13 of these norms, 104 launches of about 3 us, which bounded small decodes on the host side.
+template <bool FROM_SUMS>
 __global__ void __launch_bounds__(256) gn_silu_kernel(const __nv_bfloat16* __restrict__ x,
                                                       const float* __restrict__ mean_rstd,  // [N][32][2]
+                                                      const double* __restrict__ sums,      // [N][32][2]
+                                                      double inv_count, double eps,
                                                       const __nv_bfloat16* __restrict__ gamma,
                                                       const __nv_bfloat16* __restrict__ beta, int64_t sites_per_sample,
                                                       int C, __nv_bfloat16* __restrict__ y) {
+  __shared__ float2 mr_s[GN_GROUPS];
+  if (FROM_SUMS) {
+    if (threadIdx.x < GN_GROUPS) {
+      const double* sg = sums + (static_cast<int64_t>(blockIdx.y) * GN_GROUPS + threadIdx.x) * 2;
+      const double mean = __dmul_rn(sg[0], inv_count);
+      double var = __dsub_rn(__dmul_rn(sg[1], inv_count), __dmul_rn(mean, mean));
+      if (var < 0.0) var = 0.0;  // a NaN stays
+      mr_s[threadIdx.x] = make_float2(static_cast<float>(mean), static_cast<float>(rsqrt(__dadd_rn(var, eps))));
+    }
+    __syncthreads();
+  }
   const int vps = C >> 3;                       // 16-byte vectors per site
   const int lane_vec = threadIdx.x % vps;       // this thread's vector inside a site
   const int site_in_block = threadIdx.x / vps;
@@ -623,7 +641,8 @@ __global__ void __launch_bounds__(256) gn_silu_kernel(const __nv_bfloat16* __res
     const uint32_t gw[4] = {gr.x, gr.y, gr.z, gr.w}, bw[4] = {br.x, br.y, br.z, br.w};
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const float2 mr = *reinterpret_cast<const float2*>(mean_rstd + (static_cast<int64_t>(n) * GN_GROUPS + (c0 + j) / gs) * 2);
+      const float2 mr = FROM_SUMS ? mr_s[(c0 + j) / gs]
+                                  : *reinterpret_cast<const float2*>(mean_rstd + (static_cast<int64_t>(n) * GN_GROUPS + (c0 + j) / gs) * 2);
       const float gv = (j & 1) ? bf16_hi(gw[j >> 1]) : bf16_lo(gw[j >> 1]);
       const float bv = (j & 1) ? bf16_hi(bw[j >> 1]) : bf16_lo(bw[j >> 1]);
       a[j] = mr.y * gv;
@@ -813,9 +832,10 @@ extern "C" int rh3_gn_reduce(const float* gn_part, int64_t rows_per_sample, int6
   return check_cuda(cudaGetLastError(), "gn_reduce launch");
 }
 
-extern "C" int rh3_gn_silu_apply(const void* x, const float* mean_rstd, const void* gamma, const void* beta, int64_t N,
-                                 int64_t sites_per_sample, int64_t C, void* y, cudaStream_t stream) {
-  RH3_CHECK_ARG(x && mean_rstd && gamma && beta && y && a16(x) && a16(y) && a16(gamma) && a16(beta),
+namespace {
+int gn_silu_launch(const void* x, const float* mean_rstd, const double* sums, double count, double eps, const void* gamma,
+                   const void* beta, int64_t N, int64_t sites_per_sample, int64_t C, void* y, cudaStream_t stream) {
+  RH3_CHECK_ARG(x && (mean_rstd || sums) && gamma && beta && y && a16(x) && a16(y) && a16(gamma) && a16(beta),
                 "gn_silu_apply: null or misaligned pointer");
   RH3_CHECK_ARG(N > 0 && sites_per_sample > 0 && C > 0 && C % 8 == 0 && C % GN_GROUPS == 0, "gn_silu_apply: bad shape");
   RH3_CHECK_ARG(C / 8 <= 256, "gn_silu_apply: C=%lld is larger than 2048", (long long)C);
@@ -824,11 +844,25 @@ extern "C" int rh3_gn_silu_apply(const void* x, const float* mean_rstd, const vo
   const int64_t want = (sites_per_sample + sites_per_iter - 1) / sites_per_iter;
   const int64_t cap = static_cast<int64_t>(device_sm_count()) * 16;  // a few waves of resident blocks, grid-stride beyond
   const dim3 grid(static_cast<unsigned>(want < cap ? want : cap), static_cast<unsigned>(N));
-  gn_silu_kernel<<<grid, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(x), mean_rstd,
-                                          static_cast<const __nv_bfloat16*>(gamma),
-                                          static_cast<const __nv_bfloat16*>(beta), sites_per_sample, (int)C,
-                                          static_cast<__nv_bfloat16*>(y));
+  auto kern = sums ? gn_silu_kernel<true> : gn_silu_kernel<false>;
+  kern<<<grid, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(x), mean_rstd, sums, 1.0 / count, eps,
+                                 static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta),
+                                 sites_per_sample, (int)C, static_cast<__nv_bfloat16*>(y));
   return check_cuda(cudaGetLastError(), "gn_silu_apply launch");
+}
+}  // namespace
+
+extern "C" int rh3_gn_silu_apply(const void* x, const float* mean_rstd, const void* gamma, const void* beta, int64_t N,
+                                 int64_t sites_per_sample, int64_t C, void* y, cudaStream_t stream) {
+  RH3_CHECK_ARG(mean_rstd, "gn_silu_apply: null or misaligned pointer");
+  return gn_silu_launch(x, mean_rstd, nullptr, 1.0, 0.0, gamma, beta, N, sites_per_sample, C, y, stream);
+}
+
+extern "C" int rh3_gn_silu_from_sums(const void* x, const double* sums, double count, double eps, const void* gamma,
+                                     const void* beta, int64_t N, int64_t sites_per_sample, int64_t C, void* y,
+                                     cudaStream_t stream) {
+  RH3_CHECK_ARG(sums, "gn_silu_from_sums: null sums");
+  return gn_silu_launch(x, nullptr, sums, count, eps, gamma, beta, N, sites_per_sample, C, y, stream);
 }
 
 // Depth-to-space by 8 of the decoder head: y [N, T, H, W, 3*8*8] (channel = (ch*8 + dy)*8 + dx) ->

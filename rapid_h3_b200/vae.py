@@ -64,11 +64,15 @@ def gn_silu(x, sums, count, gamma, beta, out=None):
     """GroupNorm(32 groups) + SiLU of x [N,T,H,W,C] given its (sum, sum of squares) per (sample, group);
     `out` may be a contiguous buffer of x's shape (e.g. the data frames of a halo-padded buffer)."""
     n, c = x.shape[0], x.shape[-1]
+    y = torch.empty_like(x) if out is None else out
+    assert y.shape == x.shape and y.is_contiguous() and y.dtype == x.dtype
+    if sums.dtype == torch.float64 and sums.is_cuda and sums.shape == (n, GROUPS, 2) and sums.is_contiguous() and isinstance(count, (int, float)):
+        _lib.call("rh3_gn_silu_from_sums", x.data_ptr(), sums.data_ptr(), float(count), EPS, gamma.data_ptr(), beta.data_ptr(),
+                  n, x.numel() // (n * c), c, y.data_ptr(), _lib.stream())
+        return y
     mean = sums[..., 0] / count
     var = (sums[..., 1] / count - mean * mean).clamp_min(0.0)
     mr = torch.stack([mean, torch.rsqrt(var + EPS)], -1).float().contiguous()
-    y = torch.empty_like(x) if out is None else out
-    assert y.shape == x.shape and y.is_contiguous() and y.dtype == x.dtype
     _lib.call("rh3_gn_silu_apply", x.data_ptr(), mr.data_ptr(), gamma.data_ptr(), beta.data_ptr(), n,
               x.numel() // (n * c), c, y.data_ptr(), _lib.stream())
     return y

@@ -126,6 +126,28 @@ def test_gn_silu_and_upsample(vae):
     assert torch.equal(v.upsample(xd).cpu(), ov.upsample(x))
 
 
+@pytest.mark.parametrize("c", [32, 96, 128, 2048])
+@pytest.mark.parametrize("sites", [1, 37])
+def test_gn_silu_from_sums_equals_the_elementwise_chain(vae, c, sites):
+    v, lib = vae
+    g = torch.Generator().manual_seed(c + sites)
+    x = (torch.randn(3, 1, 1, sites, c, generator=g) * 2 + 0.5).to(torch.bfloat16)
+    x[1] = 1.5  # a constant sample: zero variance
+    x = x.cuda()
+    gamma = (1 + 0.1 * torch.randn(c, generator=g)).to(torch.bfloat16).cuda()
+    beta = (0.1 * torch.randn(c, generator=g)).to(torch.bfloat16).cuda()
+    sums, count = v.gn_sums_from_tensor(x), x.numel() // (3 * 32)
+    y = v.gn_silu(x, sums, count, gamma, beta)
+    mean = sums[..., 0] / count
+    var = (sums[..., 1] / count - mean * mean).clamp_min(0.0)
+    mr = torch.stack([mean, torch.rsqrt(var + v.EPS)], -1).float().contiguous()
+    ref = torch.empty_like(x)
+    lib.call("rh3_gn_silu_apply", x.data_ptr(), mr.data_ptr(), gamma.data_ptr(), beta.data_ptr(), 3, sites, c, ref.data_ptr(),
+             lib.stream())
+    lib.check_status()
+    assert torch.equal(y, ref)
+
+
 def test_decoder_matches_oracle(vae):
     v, lib = vae
     dec = v.VAEDecoder(seed=1, widths=(128, 64, 64), blocks_per_stage=1)
