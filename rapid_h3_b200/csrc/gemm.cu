@@ -9,11 +9,11 @@
 // (reference: custom_nodes/rapid_h3/csrc/fp8_rowwise.cu:294-304 plain epilogue, :333-336 gated
 //  residual, :74-93 SwiGLU store; PyTorch emulation custom_nodes/rapid_h3/kernels.py:129-137).
 //
-// Structure (one persistent CTA per SM, 192 threads):
+// Structure (one persistent CTA per SM, 320 threads):
 //   warp 0      TMA producer: 128x128-byte A tile + 256x128-byte B tile per stage, 4-stage ring
 //   warp 1      MMA issuer: 4 x tcgen05.mma (M128 N256 K32) per stage into a TMEM accumulator;
 //               two 256-column accumulators so the epilogue of tile i overlaps the main loop of i+1
-//   warps 2..5  epilogue: tcgen05.ld 32 columns at a time, dequantize, fused epilogue, 64-byte
+//   warps 2..9  epilogue: tcgen05.ld 32 columns at a time, dequantize, fused epilogue, 64-byte
 //               contiguous bf16 stores per thread-row
 // Tensor-core bound: 2*M*N*K operations per call.
 
@@ -32,7 +32,14 @@ constexpr int STAGES = 4;
 constexpr int A_BYTES = BM * BK;
 constexpr int B_BYTES = BN * BK;
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr int GEMM_THREADS = 192;
+// Two warps per TMEM lane quadrant, each draining half of the accumulator's columns: with one, the epilogue of a short K
+// outlasts the main loop of the next tile (w1 + SwiGLU in fp16, 3,594 x 16,384 x 2,048: 187 us with four warps and the
+// division routine, 85 with eight and silu_div; fp16 with residual, N = 2,048, K = 8,192: 61 -> 56; long-K bf16 shapes
+// measure the same).
+constexpr int EPI_WARPS = 8;
+constexpr int EPI_COLS = BN / (EPI_WARPS / 4);
+constexpr int EPI_THREADS = 32 * EPI_WARPS;
+constexpr int GEMM_THREADS = 64 + EPI_THREADS;
 #ifndef RH3_GEMM_GROUP_M
 #define RH3_GEMM_GROUP_M 16
 #endif
@@ -90,18 +97,18 @@ __device__ __forceinline__ void tile_coords(int tile, int num_m, int num_n, int&
 // while the tile's MMAs still run, so the epilogue's loads do not wait on HBM (the residual of a step is far
 // larger than L2 and cold by the time its tile comes up).
 template <int EPI>
-__device__ __forceinline__ void prefetch_residual(const GemmParams& p, int row, bool row_ok, int n0) {
+__device__ __forceinline__ void prefetch_residual(const GemmParams& p, int row, bool row_ok, int n0) {  // n0: first of EPI_COLS columns
   if (!row_ok) return;
   if (EPI == EPI_GATED) {
     const __nv_bfloat16* r = p.resid + static_cast<int64_t>(row) * p.ldr + n0;
 #pragma unroll
-    for (int c = 0; c < BN; c += 64)
+    for (int c = 0; c < EPI_COLS; c += 64)
       if (n0 + c < p.N) prefetch_l2(r + c);
   } else if (EPI == EPI_F16) {
     if (p.resid_h) {
       const __half* r = p.resid_h + static_cast<int64_t>(row) * p.ldr + n0;
 #pragma unroll
-      for (int c = 0; c < BN; c += 64)
+      for (int c = 0; c < EPI_COLS; c += 64)
         if (n0 + c < p.N) prefetch_l2(r + c);
     }
   }
@@ -139,9 +146,24 @@ __device__ __forceinline__ void load_gated_residual(const GemmParams& p, int row
   }
 }
 
+// g / (1 + e^-g) without the division routine: 1/d from the approximate reciprocal and one Newton step (to the last
+// bit or its neighbour), times g, one correction by the exact remainder g - q d. The exponent is held at 80: beyond it
+// d would leave the range the reciprocal works in, and g / e^80 is already far below fp16's smallest value (a NaN g
+// still gives NaN; an infinite one gives what the division would: g itself, or NaN for -inf / inf).
+__device__ __forceinline__ float silu_div(float g) {
+  const float d = 1.f + __expf(fminf(-g, 80.f));
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  r = fmaf(fmaf(-d, r, 1.f), r, r);
+  const float q = g * r;
+  const float rem = fmaf(-q, d, g);
+  return fabsf(g) <= 65504.f ? fmaf(rem, r, q) : (g > 0.f ? q : __int_as_float(0x7fffffff));
+}
+
 template <int KIND_F8, int EPI>
 __device__ __forceinline__ void epilogue_row(const GemmParams& p, const GemmSmemTail* tail, uint32_t t_row, int row,
-                                             bool row_ok, float xs, int n0, const uint4* res0) {
+                                             bool row_ok, float xs, int n0, int c_first, const uint4* res0) {
+  // `c_first`: first 32-column chunk of this warp's EPI_COLS columns
   // two 32-column chunks are loaded per wait, so a tile costs four TMEM round trips instead of eight; `old4` = the
   // chunk's residual values (gated residual only), loaded one round trip ahead
   auto chunk = [&](const uint32_t* r, int c, const uint4* old4) {
@@ -233,7 +255,7 @@ __device__ __forceinline__ void epilogue_row(const GemmParams& p, const GemmSmem
               for (int j = 0; j < 4; ++j) {
                 const float gv = __half2float(__float2half_rn(__fadd_rn(y[b + j], tail->aux[c * 32 + b + j])));
                 const float uv = __half2float(__float2half_rn(__fadd_rn(y[b + 4 + j], tail->aux[c * 32 + b + 4 + j])));
-                h[j] = gv / (1.f + __expf(-gv)) * uv;
+                h[j] = silu_div(gv) * uv;
               }
               const __half2 h01 = __floats2half2_rn(h[0], h[1]), h23 = __floats2half2_rn(h[2], h[3]);
               w[q * 2] = *reinterpret_cast<const uint32_t*>(&h01);
@@ -283,12 +305,12 @@ __device__ __forceinline__ void epilogue_row(const GemmParams& p, const GemmSmem
 #pragma unroll
     for (int i = 0; i < 8; ++i) res[0][i] = res0[i];
 #pragma unroll
-    for (int it = 0; it < BN / 64; ++it) {
-      const int c = it * 2;
+    for (int it = 0; it < EPI_COLS / 64; ++it) {
+      const int c = c_first + it * 2;
       uint32_t ra[32], rb[32];
       tmem_ld32(t_row + c * 32, ra);
       tmem_ld32(t_row + c * 32 + 32, rb);
-      if (it + 1 < BN / 64) load_res(res[(it + 1) & 1], c + 2);
+      if (it + 1 < EPI_COLS / 64) load_res(res[(it + 1) & 1], c + 2);
       tmem_ld_wait_regs(ra);
       tmem_ld_wait_regs(rb);
       chunk(ra, c, res[it & 1]);
@@ -297,7 +319,7 @@ __device__ __forceinline__ void epilogue_row(const GemmParams& p, const GemmSmem
     return;
   }
 #pragma unroll 1
-  for (int c = 0; c < BN / 32; c += 2) {
+  for (int c = c_first; c < c_first + EPI_COLS / 32; c += 2) {
     uint32_t ra[32], rb[32];
     tmem_ld32(t_row + c * 32, ra);
     tmem_ld32(t_row + c * 32 + 32, rb);
@@ -329,7 +351,7 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tail->acc_full[b], 1);
-      mbar_init(&tail->acc_empty[b], 4);  // one arrival per epilogue warp
+      mbar_init(&tail->acc_empty[b], EPI_WARPS);  // one arrival per epilogue warp
     }
     tail->abort_flag = 0;
     fence_barrier_init();
@@ -407,9 +429,10 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       if (++acc == 2) { acc = 0; acc_phase ^= 1; }
     }
   } else {
-    // ------------------------------ epilogue (warps 2..5) ------------------------------
+    // ------------------------------ epilogue (warps 2..9) ------------------------------
     const int quad = warp & 3;           // TMEM lane quadrant this warp may read
-    const int et = threadIdx.x - 64;     // 0..127
+    const int et = threadIdx.x - 64;     // 0 .. EPI_THREADS - 1
+    const int c_first = ((warp - 2) >> 2) * (EPI_COLS / 32);
     int acc = 0;
     uint32_t acc_phase = 0;
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
@@ -417,8 +440,8 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       tile_coords(tile, num_m, num_n, m_blk, n_blk);
       const int n0 = n_blk * BN;
       // stage the per-column scale (and bias / gate) of this tile in shared memory
-      asm volatile("bar.sync 1, 128;" ::: "memory");  // previous tile's readers are done
-      for (int c = et; c < BN; c += 128) {
+      asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory");  // previous tile's readers are done
+      for (int c = et; c < BN; c += EPI_THREADS) {
         const int n = n0 + c;
         tail->ws[c] = n < p.N ? p.ws[n] : 0.f;
         if (EPI == EPI_PLAIN) tail->aux[c] = (p.bias && n < p.N) ? __bfloat162float(p.bias[n]) : 0.f;
@@ -428,23 +451,23 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       }
       const int row = m_blk * BM + quad * 32 + lane;
       const bool row_ok = row < p.M;
-      if (tile == static_cast<int>(blockIdx.x)) prefetch_residual<EPI>(p, row, row_ok, n0);
+      if (tile == static_cast<int>(blockIdx.x)) prefetch_residual<EPI>(p, row, row_ok, n0 + c_first * 32);
       if (tile + static_cast<int>(gridDim.x) < num_tiles) {   // the next tile's residual, a whole epilogue ahead
         int m2, n2;
         tile_coords(tile + gridDim.x, num_m, num_n, m2, n2);
         const int row2 = m2 * BM + quad * 32 + lane;
-        prefetch_residual<EPI>(p, row2, row2 < p.M, n2 * BN);
+        prefetch_residual<EPI>(p, row2, row2 < p.M, n2 * BN + c_first * 32);
       }
       uint4 res0[8];
-      if (EPI == EPI_GATED) load_gated_residual(p, row, row_ok, n0, 0, res0);
+      if (EPI == EPI_GATED) load_gated_residual(p, row, row_ok, n0, c_first, res0);
       // the four warps leave together: a warp that gave up its wait takes the others with it at this barrier
       // (which also publishes the staged columns), so none of them waits at the next tile's barrier alone
       const bool got = mbar_wait(&tail->acc_full[acc], acc_phase, abort_flag, p.status, ST_TIMEOUT_ACC_FULL);
-      if (bar_sync_or(1, 128, !got)) break;
+      if (bar_sync_or(1, EPI_THREADS, !got)) break;
       tc_fence_after();
       const float xs = row_ok ? p.xs[row] : 0.f;
       const uint32_t t_row = tmem_base + acc * BN + (static_cast<uint32_t>(quad * 32) << 16);
-      epilogue_row<KIND_F8, EPI>(p, tail, t_row, row, row_ok, xs, n0, res0);
+      epilogue_row<KIND_F8, EPI>(p, tail, t_row, row, row_ok, xs, n0, c_first, res0);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tail->acc_empty[acc]);
@@ -515,7 +538,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tail->acc_full[b], 1);
-      mbar_init(&tail->acc_empty[b], 8);  // the even CTA's: one arrival per epilogue warp of both CTAs
+      mbar_init(&tail->acc_empty[b], 2 * EPI_WARPS);  // the even CTA's: one arrival per epilogue warp of both CTAs
     }
     tail->abort_flag = 0;
     fence_barrier_init();
@@ -599,9 +622,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       }
     }
   } else {
-    // ------------------------------ epilogue (warps 2..5 of both CTAs) ------------------------------
+    // ------------------------------ epilogue (warps 2..9 of both CTAs) ------------------------------
     const int quad = warp & 3;
     const int et = threadIdx.x - 64;
+    const int c_first = ((warp - 2) >> 2) * (EPI_COLS / 32);
     GemmSmemTail* cols = &tail->cols;
     int acc = 0;
     uint32_t acc_phase = 0;
@@ -609,8 +633,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       int m_blk, n_blk;
       tile_coords(tile, num_m, num_n, m_blk, n_blk);
       const int n0 = n_blk * BN;
-      asm volatile("bar.sync 1, 128;" ::: "memory");  // previous tile's readers are done
-      for (int c = et; c < BN; c += 128) {
+      asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory");  // previous tile's readers are done
+      for (int c = et; c < BN; c += EPI_THREADS) {
         const int n = n0 + c;
         cols->ws[c] = n < p.N ? p.ws[n] : 0.f;
         if (EPI == EPI_PLAIN) cols->aux[c] = (p.bias && n < p.N) ? __bfloat162float(p.bias[n]) : 0.f;
@@ -620,21 +644,21 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       }
       const int row = m_blk * 2 * BM + static_cast<int>(rank) * BM + quad * 32 + lane;
       const bool row_ok = row < p.M;
-      if (tile == pair) prefetch_residual<EPI>(p, row, row_ok, n0);
+      if (tile == pair) prefetch_residual<EPI>(p, row, row_ok, n0 + c_first * 32);
       if (tile + num_pairs < num_tiles) {   // the next tile's residual, a whole epilogue ahead
         int m2, n2;
         tile_coords(tile + num_pairs, num_m, num_n, m2, n2);
         const int row2 = m2 * 2 * BM + static_cast<int>(rank) * BM + quad * 32 + lane;
-        prefetch_residual<EPI>(p, row2, row2 < p.M, n2 * BN);
+        prefetch_residual<EPI>(p, row2, row2 < p.M, n2 * BN + c_first * 32);
       }
       uint4 res0[8];
-      if (EPI == EPI_GATED) load_gated_residual(p, row, row_ok, n0, 0, res0);
+      if (EPI == EPI_GATED) load_gated_residual(p, row, row_ok, n0, c_first, res0);
       const bool got = mbar_wait(&tail->acc_full[acc], acc_phase, abort_flag, p.status, ST_TIMEOUT_ACC_FULL);
-      if (bar_sync_or(1, 128, !got)) break;
+      if (bar_sync_or(1, EPI_THREADS, !got)) break;
       tc_fence_after();
       const float xs = row_ok ? p.xs[row] : 0.f;
       const uint32_t t_row = tmem_base + acc * BN + (static_cast<uint32_t>(quad * 32) << 16);
-      epilogue_row<KIND_F8, EPI>(p, cols, t_row, row, row_ok, xs, n0, res0);
+      epilogue_row<KIND_F8, EPI>(p, cols, t_row, row, row_ok, xs, n0, c_first, res0);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_remote(&tail->acc_empty[acc], 0);

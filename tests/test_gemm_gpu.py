@@ -219,3 +219,30 @@ def test_epilogues_on_rows_that_are_only_16_byte_aligned(ops):
     gemm.int8_gemm_swiglu(xq, xs, wq, ws, out=s_odd)
     lib.check_status()
     assert torch.equal(s_odd, s)
+
+
+@pytest.mark.parametrize("m", [100, 128, 129, 300])
+@pytest.mark.parametrize("n", [120, 128, 136, 392])
+def test_epilogue_column_split(ops, m, n):
+    """A tile's 256 columns are drained by two warps per row group: widths that end just before, at and just after the
+    border between them, alone and after a full tile, through the one-CTA and the pair kernel, every bf16 epilogue."""
+    gemm, kernels, lib = ops
+    k = 256
+    xq, wq, xs, ws = _rand_codes(m, n, k, seed=m * n)
+    acc = ol.int_mm(xq, wq)
+    dev = [t.cuda() for t in (xq, xs, wq, ws)]
+    assert torch.equal(gemm.int8_gemm(*dev).cpu(), ol.dequant(acc, xs, ws))
+    g = inputs.gen(m + n)
+    gate, res = torch.randn(n, generator=g).to(torch.bfloat16), torch.randn(m, n, generator=g).to(torch.bfloat16)
+    y = ol.dequant(acc, xs, ws).float()
+    want = torch.addcmul(res.double(), y.double(), gate.double()).float().to(torch.bfloat16)
+    got = gemm.int8_gemm_gated_residual(*dev, gate.cuda(), res.cuda())
+    lib.check_status()
+    assert (got.cpu() != want).float().mean() < 1e-4  # one fused rounding on the device, two here (fp64, then bf16)
+    if n % 16 == 0:
+        h = gemm.int8_gemm_swiglu(*dev)
+        lib.check_status()
+        assert h.shape == (m, n // 2)
+        gu = y.to(torch.bfloat16).float().view(m, n // 8, 2, 4)
+        ref = (gu[:, :, 0] / (1 + torch.exp(-gu[:, :, 0])) * gu[:, :, 1]).reshape(m, n // 2)
+        assert rel_l2(h.cpu(), ref) <= 3e-3  # bf16 rounding, 2^-9 at worst

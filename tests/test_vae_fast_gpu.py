@@ -228,3 +228,24 @@ def test_vae_quantizer_eight_byte_aligned_codes(vf):
     lib.check_status()
     qr, sr = ov.quant_rows_f16(x)
     assert torch.equal(buf[8:].view(9, 512).cpu(), qr) and torch.equal(s.cpu(), sr) and not buf[:8].any()
+
+
+def test_swiglu_epilogue_over_the_gate_range(vf):
+    """Gates from -inf to inf through the bias (codes are 0): the reciprocal form gives what the division would."""
+    vae_fast, lib = vf
+    inf, nan = float("inf"), float("nan")
+    gates = torch.cat([torch.tensor([0.0, -0.0, 6e-8, -6e-8, 80, -80, 81, -81, 88, -88.5, 100, -100, 65504, -65504, inf, -inf, nan, 1.0]),
+                       torch.linspace(-20, 20, 494)]).half()
+    up = torch.tensor([1.0, 3.0]).half().repeat(256)
+    n = 1024
+    bias = ov.interleave_rows(torch.cat([gates, up]), n).contiguous().cuda()
+    xq, wq = torch.zeros(3, 16, dtype=torch.int8, device="cuda"), torch.zeros(n, 16, dtype=torch.int8, device="cuda")
+    out = vae_fast.vae_gemm_swiglu(xq, wq, torch.ones(3, device="cuda"), torch.ones(n, device="cuda"), bias).cpu()
+    lib.check_status()
+    g = gates.float()
+    ref = (g / (1 + torch.exp(-g)) * up.float()).half()
+    for row in out:
+        assert torch.equal(row.isnan(), ref.isnan()) and torch.equal(row.isinf(), ref.isinf())
+        fin = ref.isfinite()
+        # the hardware e^-g: relative error 2^-22 + |g| 2^-24 in fp32, at most one place of the fp16 result
+        assert ((row[fin].float() - ref[fin].float()).abs() <= 1.01 * 2 ** -10 * ref[fin].float().abs() + 6e-8).all()
