@@ -124,6 +124,11 @@ int rh3_gemm_use_pairs(int on);
 int rh3_gemm_w8a8(const void* xq, int64_t lda, const void* wq, const float* xs, const float* ws, const void* bias,
                   int64_t M, int64_t N, int64_t K, int kind, void* out, int64_t ldo, int32_t* acc_dump,
                   cudaStream_t stream);
+/* out[M,N] bf16 = bf16(bf16((acc * xs[m]) * ws[n]) + bias[n]): the product rounded first, the bias (bf16 [N], required) added
+ * to the rounded value, i.e. the bits of rh3_gemm_w8a8 without a bias and a bf16 addition after it. Other arguments as above.
+ * Replaces the GEMM and the separate bias addition of _QuantLinear (custom_nodes/rapid_h3/__init__.py:132-167). */
+int rh3_gemm_w8a8_bias_after(const void* xq, int64_t lda, const void* wq, const float* xs, const float* ws, const void* bias,
+                             int64_t M, int64_t N, int64_t K, int kind, void* out, int64_t ldo, cudaStream_t stream);
 /* resid[M,N] = bf16(fma(bf16((acc*xs)*ws), gate[n], resid)) in place (row stride ldr). M == 0 is a no-op.
  * Replaces int8_gemm_gated_residual (fp8_rowwise.cu:333-389, :587-608). */
 int rh3_gemm_w8a8_gated_residual(const void* xq, int64_t lda, const void* wq, const float* xs, const float* ws,

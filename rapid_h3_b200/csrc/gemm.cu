@@ -3,6 +3,8 @@
 //   acc[m, n] = sum_k xq[m, k] * wq[n, k]          int8 x int8 -> int32 (tcgen05 kind::i8), or
 //                                                   e4m3 x e4m3 -> fp32 (tcgen05 kind::f8f6f4)
 //   EPI_PLAIN : out[m, n]   = bf16(((float(acc) * xs[m]) * ws[n]) + bias[n])
+//   EPI_BIAS2 : out[m, n]   = bf16(bf16((float(acc) * xs[m]) * ws[n]) + bias[n]): a product that is rounded first and
+//               gets its bias in bf16, as a separate addition would give it
 //   EPI_GATED : resid[m, n] = bf16(fma(bf16((float(acc) * xs[m]) * ws[n]), gate[n], resid[m, n]))   (in place)
 //   EPI_SWIGLU: columns come in groups of 8 = [g 4j..4j+3 | u 4j..4j+3];
 //               out[m, n/2] = bf16(silu(bf16(g)) * bf16(u)), half-width store
@@ -45,13 +47,13 @@ constexpr int GEMM_THREADS = 64 + EPI_THREADS;
 #endif
 constexpr int GROUP_M = RH3_GEMM_GROUP_M;  // tile rasterisation: GROUP_M row-tiles share each column-tile in L2
 
-enum { EPI_PLAIN = 0, EPI_GATED = 1, EPI_SWIGLU = 2, EPI_F16 = 3, EPI_SWIGLU_F16 = 4 };
+enum { EPI_PLAIN = 0, EPI_GATED = 1, EPI_SWIGLU = 2, EPI_F16 = 3, EPI_SWIGLU_F16 = 4, EPI_BIAS2 = 5 };
 
 struct GemmParams {
   int M, N, K;
   const float* xs;
   const float* ws;
-  const __nv_bfloat16* bias;  // EPI_PLAIN, optional
+  const __nv_bfloat16* bias;  // EPI_PLAIN (optional), EPI_BIAS2
   __nv_bfloat16* out;         // EPI_PLAIN / EPI_SWIGLU
   int64_t ldo;
   int32_t* acc_dump;          // optional raw accumulator dump [M, N] (int32, or fp32 bits for fp8)
@@ -181,7 +183,7 @@ __device__ __forceinline__ void epilogue_row(const GemmParams& p, const GemmSmem
         const float a = KIND_F8 ? __uint_as_float(r[j]) : __int2float_rn(static_cast<int>(r[j]));
         y[j] = __fmul_rn(__fmul_rn(a, xs), tail->ws[c * 32 + j]);
       }
-      if (EPI == EPI_PLAIN) {
+      if (EPI == EPI_PLAIN || EPI == EPI_BIAS2) {
         __nv_bfloat16* o = p.out + static_cast<int64_t>(row) * p.ldo + col0;
         uint4 w4[4];
 #pragma unroll
@@ -190,7 +192,8 @@ __device__ __forceinline__ void epilogue_row(const GemmParams& p, const GemmSmem
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const int e = g * 8 + 2 * j;
-            w[j] = pack_bf16x2(__fadd_rn(y[e], tail->aux[c * 32 + e]), __fadd_rn(y[e + 1], tail->aux[c * 32 + e + 1]));
+            const float y0 = EPI == EPI_BIAS2 ? bf16_round(y[e]) : y[e], y1 = EPI == EPI_BIAS2 ? bf16_round(y[e + 1]) : y[e + 1];
+            w[j] = pack_bf16x2(__fadd_rn(y0, tail->aux[c * 32 + e]), __fadd_rn(y1, tail->aux[c * 32 + e + 1]));
           }
           w4[g] = make_uint4(w[0], w[1], w[2], w[3]);
         }
@@ -444,7 +447,7 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       for (int c = et; c < BN; c += EPI_THREADS) {
         const int n = n0 + c;
         tail->ws[c] = n < p.N ? p.ws[n] : 0.f;
-        if (EPI == EPI_PLAIN) tail->aux[c] = (p.bias && n < p.N) ? __bfloat162float(p.bias[n]) : 0.f;
+        if (EPI == EPI_PLAIN || EPI == EPI_BIAS2) tail->aux[c] = (p.bias && n < p.N) ? __bfloat162float(p.bias[n]) : 0.f;
         if (EPI == EPI_GATED) tail->aux[c] = n < p.N ? __bfloat162float(p.gate[n]) : 0.f;
         if (EPI == EPI_F16 || EPI == EPI_SWIGLU_F16) tail->aux[c] = n < p.N ? __half2float(p.bias_h[n]) : 0.f;
         if (EPI == EPI_F16) tail->aux2[c] = (p.rscale_h && n < p.N) ? __half2float(p.rscale_h[n]) : 0.f;
@@ -637,7 +640,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       for (int c = et; c < BN; c += EPI_THREADS) {
         const int n = n0 + c;
         cols->ws[c] = n < p.N ? p.ws[n] : 0.f;
-        if (EPI == EPI_PLAIN) cols->aux[c] = (p.bias && n < p.N) ? __bfloat162float(p.bias[n]) : 0.f;
+        if (EPI == EPI_PLAIN || EPI == EPI_BIAS2) cols->aux[c] = (p.bias && n < p.N) ? __bfloat162float(p.bias[n]) : 0.f;
         if (EPI == EPI_GATED) cols->aux[c] = n < p.N ? __bfloat162float(p.gate[n]) : 0.f;
         if (EPI == EPI_F16 || EPI == EPI_SWIGLU_F16) cols->aux[c] = n < p.N ? __half2float(p.bias_h[n]) : 0.f;
         if (EPI == EPI_F16) cols->aux2[c] = (p.rscale_h && n < p.N) ? __half2float(p.rscale_h[n]) : 0.f;
@@ -776,6 +779,26 @@ extern "C" int rh3_gemm_w8a8(const void* xq, int64_t lda, const void* wq, const 
   p.out = static_cast<__nv_bfloat16*>(out); p.ldo = ldo; p.acc_dump = acc_dump; p.status = device_status_word();
   p.wide = (reinterpret_cast<uintptr_t>(out) & 31) == 0 && ldo % 16 == 0;
   return kind == RH3_KIND_F8 ? launch_gemm<1, EPI_PLAIN>(ta, tb, tbp, p, stream) : launch_gemm<0, EPI_PLAIN>(ta, tb, tbp, p, stream);
+}
+
+// The bias lands on the rounded product (two roundings), so the result is bit for bit that of rh3_gemm_w8a8 without a
+// bias followed by a bf16 addition; what it saves is that addition's pass over the output (read and written once more;
+// the host framework's broadcast kernel took 138 us for 5,003 x 12,288 beside 164 us for the GEMM itself).
+extern "C" int rh3_gemm_w8a8_bias_after(const void* xq, int64_t lda, const void* wq, const float* xs, const float* ws,
+                                        const void* bias, int64_t M, int64_t N, int64_t K, int kind, void* out,
+                                        int64_t ldo, cudaStream_t stream) {
+  CUtensorMap ta, tb, tbp;
+  if (int e = gemm_common(xq, lda, wq, xs, ws, M, N, K, kind, &ta, &tb, &tbp)) return e;
+  if (M == 0) return 0;
+  RH3_CHECK_ARG(bias, "gemm_w8a8_bias_after: bias is required");
+  RH3_CHECK_ARG(out && ldo >= N && ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0,
+                "gemm_w8a8_bias_after: out must be 16-byte aligned with a row stride >= N that is a multiple of 8");
+  GemmParams p{};
+  p.M = (int)M; p.N = (int)N; p.K = (int)K; p.xs = xs; p.ws = ws;
+  p.bias = static_cast<const __nv_bfloat16*>(bias);
+  p.out = static_cast<__nv_bfloat16*>(out); p.ldo = ldo; p.status = device_status_word();
+  p.wide = (reinterpret_cast<uintptr_t>(out) & 31) == 0 && ldo % 16 == 0;
+  return kind == RH3_KIND_F8 ? launch_gemm<1, EPI_BIAS2>(ta, tb, tbp, p, stream) : launch_gemm<0, EPI_BIAS2>(ta, tb, tbp, p, stream);
 }
 
 extern "C" int rh3_gemm_w8a8_gated_residual(const void* xq, int64_t lda, const void* wq, const float* xs,

@@ -38,6 +38,20 @@ def _gemm(xq, xs, wq, ws, bias, kind, dtype, acc_dump=None, out=None):
     return out
 
 
+def gemm_bias_after(xq, xs, wq, ws, bias):
+    """bf16(bf16((acc * xs[m]) * ws[n]) + bias[n]) in one kernel: the bits of `int8_gemm` / `fp8_gemm` (whichever the codes'
+    dtype asks for) followed by `+ bias` in bf16. `bias` is bf16 with N elements."""
+    f8 = xq.dtype == torch.float8_e4m3fn
+    m, n, k, xs, ws = _check(xq, xs, wq, ws, torch.float8_e4m3fn if f8 else torch.int8)
+    _lib.require_cuda(bias)
+    if bias.dtype != torch.bfloat16 or bias.numel() != n or not bias.is_contiguous():
+        raise RuntimeError("bias must be contiguous bf16 with N elements")
+    out = torch.empty((m, n), device=xq.device, dtype=torch.bfloat16)
+    _lib.call("rh3_gemm_w8a8_bias_after", xq.data_ptr(), xq.stride(0), wq.data_ptr(), xs.data_ptr(), ws.data_ptr(),
+              bias.data_ptr(), m, n, k, _lib.KIND_F8 if f8 else _lib.KIND_I8, out.data_ptr(), out.stride(0), _lib.stream())
+    return out
+
+
 def int8_gemm(xq, xs, wq, ws, bias=None, config=2, acc_dump=None, out=None):
     """W8A8 int8 GEMM with row-wise scales: bf16 [M, N] = ((acc * xs[m]) * ws[n]) + bias[n], acc the exact int32
     dot product of row m of xq [M, K] with row n of wq [N, K]. xs / ws are fp32 with M / N elements in any shape.

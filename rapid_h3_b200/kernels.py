@@ -73,11 +73,14 @@ def gemm_config(k, n):
     return 6
 
 
-def linear(x, qw, mode):
-    """y = x @ W^T for x [M, K] bf16 and a QWeight of W [N, K]; returns bf16."""
+def linear(x, qw, mode, bias=None):
+    """y = x @ W^T for x [M, K] bf16 and a QWeight of W [N, K]; returns bf16. `bias` (contiguous bf16 [N]) is added to the
+    rounded product, as a separate `y + bias` would."""
     if mode in _UNSUPPORTED:
         raise NotImplementedError(f"mode {mode!r} is not implemented in rapid_h3_b200")
     xq, sa = quantize_rows(x.contiguous(), mode)
+    if bias is not None:
+        return _cf.gemm_bias_after(xq, sa, qw.q, qw.scale, bias)
     if mode in _ROWWISE_F8 + _TENSOR_F8:
         return _cf.fp8_gemm(xq, sa, qw.q, qw.scale)
     return _cf.int8_gemm(xq, sa, qw.q, qw.scale)

@@ -66,6 +66,16 @@ def _stored_as_rotated_int8(w):
             and not getattr(meta, "transposed", False))
 
 
+def _plain_bias(b, n, device):
+    """True when adding `b` to a [M, n] product can be left to the GEMM's epilogue: a plain tensor of the product's own
+    device, and nothing that would have to see the addition as an operation of its own (a gradient for the bias, a
+    forward-mode tangent, a functional transform, a trace). Everything else is added by torch."""
+    return (type(b) in (torch.Tensor, torch.nn.Parameter) and b.device == device and b.shape == (n,)
+            and not (b.requires_grad and torch.is_grad_enabled())
+            and torch.autograd.forward_ad._current_level < 0 and torch._C._functorch.peek_interpreter_stack() is None
+            and not torch.jit.is_tracing())
+
+
 class _QuantLinear:
     """Replacement forward bound to one Linear: row quantizer + W8A8 GEMM, bias added afterwards in bf16
     (reference: __init__.py:132-167). The quantized weight is made on first use and kept until the weight it was
@@ -111,11 +121,16 @@ class _QuantLinear:
             raise NotImplementedError("_QuantLinear: only CUDA bf16 activations are supported (no fallback path)")
         shape = x.shape
         qw = self.qweight_for(x)
-        y = kernels.linear(x.reshape(-1, shape[-1]), qw, self.mode)
+        bias, n = self.module.bias, qw.q.shape[0]
+        if bias is not None and qw.layout == "rows" and _plain_bias(bias, n, x.device):
+            y = kernels.linear(x.reshape(-1, shape[-1]), qw, self.mode, bias.to(torch.bfloat16).contiguous())
+            bias = None
+        else:
+            y = kernels.linear(x.reshape(-1, shape[-1]), qw, self.mode)
         if qw.layout == "swiglu8":  # the fused block keeps fc1 in its epilogue's row order: put the columns back
             y = y.index_select(-1, torch.argsort(cf.swiglu_perm(y.shape[-1], y.device)))
-        if self.module.bias is not None:
-            y = y + self.module.bias.to(y.dtype)
+        if bias is not None:
+            y = y + bias.to(y.dtype)
         y = y.reshape(*shape[:-1], y.shape[-1])
         self.calls += 1
         if self.measure_every and self.calls % self.measure_every == 0 and self.module.weight.numel():

@@ -221,6 +221,21 @@ def test_epilogues_on_rows_that_are_only_16_byte_aligned(ops):
     assert torch.equal(s_odd, s)
 
 
+@pytest.mark.parametrize("shape", [(1, 8, 16), (37, 264, 1040), (128, 256, 128), (300, 264, 1040), (515, 4096, 512)])
+@pytest.mark.parametrize("kind", ["int8", "fp8"])
+def test_bias_after_equals_a_separate_addition(ops, shape, kind):
+    gemm, kernels, lib = ops
+    m, n, k = shape
+    xq, wq, xs, ws = (t.cuda() for t in _rand_codes(m, n, k, seed=m + k))
+    if kind == "fp8":
+        xq, wq = (xq.float() / 16).to(torch.float8_e4m3fn), (wq.float() / 16).to(torch.float8_e4m3fn)
+    bias = torch.randn(n, generator=inputs.gen(7)).to(torch.bfloat16).cuda()
+    y = gemm.gemm_bias_after(xq, xs, wq, ws, bias)
+    plain = (gemm.fp8_gemm if kind == "fp8" else gemm.int8_gemm)(xq, xs, wq, ws)
+    lib.check_status()
+    assert torch.equal(y, plain + bias)
+
+
 @pytest.mark.parametrize("m", [100, 128, 129, 300])
 @pytest.mark.parametrize("n", [120, 128, 136, 392])
 def test_epilogue_column_split(ops, m, n):
