@@ -110,6 +110,13 @@ int rh3_norm_mod_rot_quant_rows_i8(const void* x, int64_t ldx, const void* w, fl
                                    const float* shift, const float* scale, int64_t ld_tab, int64_t M, int64_t K,
                                    void* q, int64_t ldq, float* s, cudaStream_t stream);
 
+/* Input side of the text encoder's linear on x fp32 [M, K] (row stride ldx; K % 256 == 0, K <= 8192): q1 [M, K], s1 [M] = the
+ * int8 row quantizer on rotate(bf16(x)); flags [M] bytes = 1 where 127 s1 / max(rms(x), 1e-12) > ratio; those rows also get a
+ * slot i < *count (any order): rows[i], and q2[i], s2[i] = the int8 codes of rotate(x) - q1 s1. *count (int32) is set by the
+ * call; *total (uint64, may be NULL) grows by it. rows, q2 and s2 have room for M rows.
+ * Replaces te_quant.py:90-105 of the reference (custom_nodes/rapid_h3/te_quant.py). */
+int rh3_te_quant(const float* x, int64_t ldx, int64_t M, int64_t K, float ratio, void* q1, float* s1, void* flags,
+                 int32_t* count, int32_t* rows, void* q2, float* s2, void* total, cudaStream_t stream);
 /* ---- W8A8 row-wise-scaled GEMMs (tensor-core bound) ---------------------------------------- */
 /* Kernel choice of the GEMM entries below and of rh3_conv3d_causal (no reference counterpart): 0 = one CTA per tile, 1 (the
  * default) = CTA pairs (clusters of two, tcgen05 cta_group::2): 256 x 256 GEMM tiles with each CTA loading its own half of
@@ -138,6 +145,13 @@ int rh3_gemm_w8a8_gated_residual(const void* xq, int64_t lda, const void* wq, co
  * Replaces int8_gemm_swiglu (fp8_rowwise.cu:29-107, :611-629; row order cutlass_fp8.py:55-62). */
 int rh3_gemm_w8a8_swiglu(const void* xq, int64_t lda, const void* wq, const float* xs, const float* ws, int64_t M,
                          int64_t N, int64_t K, int kind, void* out, int64_t ldo, cudaStream_t stream);
+
+/* The products of the text encoder's linear (int8, contiguous codes): out fp32 [M, N] = float(bf16((acc1 s1) ws)) + bias;
+ * for the rows listed in rows[0 .. *count) the second product's float(bf16((acc2 s2) ws)) is added before the bias. bias may
+ * be NULL; rows NULL: no second product. count stays on the device. Replaces te_quant.py:95-112 of the reference. */
+int rh3_te_gemm(const void* q1, const float* s1, const void* wq, const float* ws, const float* bias, int64_t M, int64_t N,
+                int64_t K, const void* flags, const int32_t* count, const int32_t* rows, const void* q2, const float* s2,
+                float* out, int64_t ldo, cudaStream_t stream);
 
 /* ---- attention pre-pass (HBM-bound) and INT8 flash attention (tensor-core bound) ----------- */
 /* y = per-(token, head) RMSNorm over 128 channels (weight bf16[128]) followed, when rope_table is

@@ -5,6 +5,8 @@
 //   EPI_PLAIN : out[m, n]   = bf16(((float(acc) * xs[m]) * ws[n]) + bias[n])
 //   EPI_BIAS2 : out[m, n]   = bf16(bf16((float(acc) * xs[m]) * ws[n]) + bias[n]): a product that is rounded first and
 //               gets its bias in bf16, as a separate addition would give it
+//   EPI_F32   : out[m, n]   = float(bf16(...)) + bias[n] in fp32; rows flagged for a second pass leave the bias to it
+//   EPI_F32_ADD: out[rows[m], n] = (out[rows[m], n] + float(bf16(...))) + bias[n]; the number of rows is read on the device
 //   EPI_GATED : resid[m, n] = bf16(fma(bf16((float(acc) * xs[m]) * ws[n]), gate[n], resid[m, n]))   (in place)
 //   EPI_SWIGLU: columns come in groups of 8 = [g 4j..4j+3 | u 4j..4j+3];
 //               out[m, n/2] = bf16(silu(bf16(g)) * bf16(u)), half-width store
@@ -47,7 +49,7 @@ constexpr int GEMM_THREADS = 64 + EPI_THREADS;
 #endif
 constexpr int GROUP_M = RH3_GEMM_GROUP_M;  // tile rasterisation: GROUP_M row-tiles share each column-tile in L2
 
-enum { EPI_PLAIN = 0, EPI_GATED = 1, EPI_SWIGLU = 2, EPI_F16 = 3, EPI_SWIGLU_F16 = 4, EPI_BIAS2 = 5 };
+enum { EPI_PLAIN = 0, EPI_GATED = 1, EPI_SWIGLU = 2, EPI_F16 = 3, EPI_SWIGLU_F16 = 4, EPI_BIAS2 = 5, EPI_F32 = 6, EPI_F32_ADD = 7 };
 
 struct GemmParams {
   int M, N, K;
@@ -65,6 +67,12 @@ struct GemmParams {
   const __half* rscale_h;  // [N] or null (EPI_F16 with residual)
   const __half* resid_h;   // [M, N] row stride ldr, or null
   __half* out_h;           // row stride ldo
+  // fp32 epilogues of the text encoder's linears (EPI_F32 / EPI_F32_ADD)
+  float* out_f;            // row stride ldo
+  const float* bias_f;     // [N] or null
+  const uint8_t* flags;    // EPI_F32: rows whose bias the second pass adds, or null
+  const int32_t* rows;     // EPI_F32_ADD: output row of every row of xq
+  const int32_t* m_dev;    // EPI_F32_ADD: number of rows, at most M
   int wide;                // bf16 output (and gated residual) rows are 32-byte aligned: 32-byte accesses in the epilogue
   int* status;
 };
@@ -162,6 +170,12 @@ __device__ __forceinline__ float silu_div(float g) {
   return fabsf(g) <= 65504.f ? fmaf(rem, r, q) : (g > 0.f ? q : __int_as_float(0x7fffffff));
 }
 
+// rows of this call: the second pass reads its number from the device (the host never sees it)
+template <int EPI>
+__device__ __forceinline__ int gemm_rows(const GemmParams& p) {
+  return EPI == EPI_F32_ADD ? min(p.M, *p.m_dev) : p.M;
+}
+
 template <int KIND_F8, int EPI>
 __device__ __forceinline__ void epilogue_row(const GemmParams& p, const GemmSmemTail* tail, uint32_t t_row, int row,
                                              bool row_ok, float xs, int n0, int c_first, const uint4* res0) {
@@ -216,6 +230,27 @@ __device__ __forceinline__ void epilogue_row(const GemmParams& p, const GemmSmem
           w4[g] = make_uint4(w[0], w[1], w[2], w[3]);
         }
         store_chunk_bf16(o, w4, col0, p.N, p.wide);
+      } else if (EPI == EPI_F32 || EPI == EPI_F32_ADD) {
+        // aux holds the bias (-0 without one: adding it changes nothing)
+        float* o = p.out_f + static_cast<int64_t>(EPI == EPI_F32_ADD ? p.rows[row] : row) * p.ldo + col0;
+        const bool with_bias = EPI == EPI_F32_ADD || !(p.flags && p.flags[row]);
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          if (col0 + g * 8 + 8 <= p.N) {
+            uint4 old[2] = {};
+            if (EPI == EPI_F32_ADD) ld_global_32(o + g * 8, old[0], old[1]);
+            const uint32_t ow[8] = {old[0].x, old[0].y, old[0].z, old[0].w, old[1].x, old[1].y, old[1].z, old[1].w};
+            uint32_t w[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              float v = bf16_round(y[g * 8 + j]);
+              if (EPI == EPI_F32_ADD) v = __fadd_rn(__uint_as_float(ow[j]), v);
+              if (with_bias) v = __fadd_rn(v, tail->aux[c * 32 + g * 8 + j]);
+              w[j] = __float_as_uint(v);
+            }
+            st_global_32(o + g * 8, make_uint4(w[0], w[1], w[2], w[3]), make_uint4(w[4], w[5], w[6], w[7]));
+          }
+        }
       } else if (EPI == EPI_F16) {
         // y1 = fp16(y + bias); with a residual: out = fp16(float(y1) * rscale + resid), two separate roundings
         __half* o = p.out_h + static_cast<int64_t>(row) * p.ldo + col0;
@@ -343,7 +378,8 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   volatile int* abort_flag = &tail->abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int num_m = (p.M + BM - 1) / BM, num_n = (p.N + BN - 1) / BN;
+  const int M = gemm_rows<EPI>(p);
+  const int num_m = (M + BM - 1) / BM, num_n = (p.N + BN - 1) / BN;
   const int num_tiles = num_m * num_n;
   const int num_kb = (p.K + BK - 1) / BK;
 
@@ -448,18 +484,19 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         const int n = n0 + c;
         tail->ws[c] = n < p.N ? p.ws[n] : 0.f;
         if (EPI == EPI_PLAIN || EPI == EPI_BIAS2) tail->aux[c] = (p.bias && n < p.N) ? __bfloat162float(p.bias[n]) : 0.f;
+        if (EPI == EPI_F32 || EPI == EPI_F32_ADD) tail->aux[c] = (p.bias_f && n < p.N) ? p.bias_f[n] : -0.f;
         if (EPI == EPI_GATED) tail->aux[c] = n < p.N ? __bfloat162float(p.gate[n]) : 0.f;
         if (EPI == EPI_F16 || EPI == EPI_SWIGLU_F16) tail->aux[c] = n < p.N ? __half2float(p.bias_h[n]) : 0.f;
         if (EPI == EPI_F16) tail->aux2[c] = (p.rscale_h && n < p.N) ? __half2float(p.rscale_h[n]) : 0.f;
       }
       const int row = m_blk * BM + quad * 32 + lane;
-      const bool row_ok = row < p.M;
+      const bool row_ok = row < M;
       if (tile == static_cast<int>(blockIdx.x)) prefetch_residual<EPI>(p, row, row_ok, n0 + c_first * 32);
       if (tile + static_cast<int>(gridDim.x) < num_tiles) {   // the next tile's residual, a whole epilogue ahead
         int m2, n2;
         tile_coords(tile + gridDim.x, num_m, num_n, m2, n2);
         const int row2 = m2 * BM + quad * 32 + lane;
-        prefetch_residual<EPI>(p, row2, row2 < p.M, n2 * BN + c_first * 32);
+        prefetch_residual<EPI>(p, row2, row2 < M, n2 * BN + c_first * 32);
       }
       uint4 res0[8];
       if (EPI == EPI_GATED) load_gated_residual(p, row, row_ok, n0, c_first, res0);
@@ -530,7 +567,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_cta_rank();          // 0 = the even CTA of the pair: it issues the MMAs
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
-  const int num_m = (p.M + 2 * BM - 1) / (2 * BM), num_n = (p.N + BN - 1) / BN;
+  const int M = gemm_rows<EPI>(p);
+  const int num_m = (M + 2 * BM - 1) / (2 * BM), num_n = (p.N + BN - 1) / BN;
   const int num_tiles = num_m * num_n;
   const int num_kb = (p.K + BK - 1) / BK;
 
@@ -641,18 +679,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         const int n = n0 + c;
         cols->ws[c] = n < p.N ? p.ws[n] : 0.f;
         if (EPI == EPI_PLAIN || EPI == EPI_BIAS2) cols->aux[c] = (p.bias && n < p.N) ? __bfloat162float(p.bias[n]) : 0.f;
+        if (EPI == EPI_F32 || EPI == EPI_F32_ADD) cols->aux[c] = (p.bias_f && n < p.N) ? p.bias_f[n] : -0.f;
         if (EPI == EPI_GATED) cols->aux[c] = n < p.N ? __bfloat162float(p.gate[n]) : 0.f;
         if (EPI == EPI_F16 || EPI == EPI_SWIGLU_F16) cols->aux[c] = n < p.N ? __half2float(p.bias_h[n]) : 0.f;
         if (EPI == EPI_F16) cols->aux2[c] = (p.rscale_h && n < p.N) ? __half2float(p.rscale_h[n]) : 0.f;
       }
       const int row = m_blk * 2 * BM + static_cast<int>(rank) * BM + quad * 32 + lane;
-      const bool row_ok = row < p.M;
+      const bool row_ok = row < M;
       if (tile == pair) prefetch_residual<EPI>(p, row, row_ok, n0 + c_first * 32);
       if (tile + num_pairs < num_tiles) {   // the next tile's residual, a whole epilogue ahead
         int m2, n2;
         tile_coords(tile + num_pairs, num_m, num_n, m2, n2);
         const int row2 = m2 * 2 * BM + static_cast<int>(rank) * BM + quad * 32 + lane;
-        prefetch_residual<EPI>(p, row2, row2 < p.M, n2 * BN + c_first * 32);
+        prefetch_residual<EPI>(p, row2, row2 < M, n2 * BN + c_first * 32);
       }
       uint4 res0[8];
       if (EPI == EPI_GATED) load_gated_residual(p, row, row_ok, n0, c_first, res0);
@@ -831,6 +870,30 @@ extern "C" int rh3_gemm_w8a8_swiglu(const void* xq, int64_t lda, const void* wq,
   p.out = static_cast<__nv_bfloat16*>(out); p.ldo = ldo; p.status = device_status_word();
   p.wide = (reinterpret_cast<uintptr_t>(out) & 31) == 0 && ldo % 16 == 0;
   return kind == RH3_KIND_F8 ? launch_gemm<1, EPI_SWIGLU>(ta, tb, tbp, p, stream) : launch_gemm<0, EPI_SWIGLU>(ta, tb, tbp, p, stream);
+}
+
+// ---- fp32 epilogues: the text encoder's linears (fp32 in and out, custom_nodes/rapid_h3/te_quant.py:90-115) ----
+// First product: out = float(bf16(y)) + bias, the bias left out of the rows that `flags` marks. Second product over the
+// rows in `rows` (their number is *count, at most M): out[rows[m]] = (out[rows[m]] + float(bf16(y2))) + bias. One call
+// launches both; without `rows` only the first.
+extern "C" int rh3_te_gemm(const void* q1, const float* s1, const void* wq, const float* ws, const float* bias, int64_t M,
+                           int64_t N, int64_t K, const void* flags, const int32_t* count, const int32_t* rows,
+                           const void* q2, const float* s2, float* out, int64_t ldo, cudaStream_t stream) {
+  CUtensorMap ta, tb, tbp;
+  if (int e = gemm_common(q1, K, wq, s1, ws, M, N, K, RH3_KIND_I8, &ta, &tb, &tbp)) return e;
+  if (M == 0) return 0;
+  RH3_CHECK_ARG(out && ldo >= N && ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(out) & 31) == 0,
+                "te_gemm: out must be 32-byte aligned with a row stride >= N that is a multiple of 8");
+  RH3_CHECK_ARG(!rows || (count && q2 && s2 && flags), "te_gemm: the second product needs its count, codes, scales and flags");
+  GemmParams p{};
+  p.M = (int)M; p.N = (int)N; p.K = (int)K; p.xs = s1; p.ws = ws; p.bias_f = bias;
+  p.out_f = out; p.ldo = ldo; p.status = device_status_word();
+  p.flags = rows ? static_cast<const uint8_t*>(flags) : nullptr;
+  if (int e = launch_gemm<0, EPI_F32>(ta, tb, tbp, p, stream)) return e;
+  if (!rows) return 0;
+  if (int e = gemm_common(q2, K, wq, s2, ws, M, N, K, RH3_KIND_I8, &ta, &tb, &tbp)) return e;
+  p.xs = s2; p.flags = nullptr; p.rows = rows; p.m_dev = count;
+  return launch_gemm<0, EPI_F32_ADD>(ta, tb, tbp, p, stream);
 }
 
 // ---- fp16 epilogues: the reference's VAE transformer-decoder GEMMs (custom_nodes/rapid_h3/csrc/vae_ops.cu:150-227

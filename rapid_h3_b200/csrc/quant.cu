@@ -287,6 +287,86 @@ __global__ void __launch_bounds__(T) rot_residual_quant_kernel(const float* __re
   }
 }
 
+// Everything the text encoder's linear does to its input before the first product, one CTA of K/8 threads per row, the row
+// read once and held in registers:
+//   q1, s1   the int8 row quantizer on rotate(bf16(x)) (the codes of rot_quant_rows on the bf16 copy of x)
+//   outlier  127 s1 / max(rms(x), 1e-12) > ratio: H256 is orthonormal, so the rotated row has x's rms, and its abs-max is
+//            127 s1 by construction of the scale
+//   an outlier row takes the next free slot i of the second pass: rows[i] = row, and q2[i], s2[i] are the int8 codes of
+//   rotate(x) - q1 s1 (the arithmetic of rot_residual_quant_kernel). Slots are handed out by one atomic per outlier row, in
+//   any order: a slot's content does not depend on its number. `count` is what the second product reads its row number
+//   from, so the host never waits for it.
+// Bound by HBM in principle (4 bytes in, 1 out per value), by launches in practice: as separate steps (bf16 copy,
+// quantizer, square, mean, sqrt, clamp, compare, three kernels and a host round trip of the index list, residual
+// quantizer) this took 14 launches and 55 us of device time for 512 x 4,096.
+template <int T>
+__global__ void __launch_bounds__(T) te_quant_kernel(const float* __restrict__ x, int64_t ldx, int64_t M, int K, float ratio,
+                                                     int8_t* __restrict__ q1, float* __restrict__ s1,
+                                                     uint8_t* __restrict__ flags, int* __restrict__ count,
+                                                     int32_t* __restrict__ rows, int8_t* __restrict__ q2,
+                                                     float* __restrict__ s2, unsigned long long* __restrict__ total) {
+  __shared__ float red[T / 32];
+  __shared__ int slot_s;
+  const int tid = threadIdx.x;
+  const int col = tid << 3;
+  const bool active = col < K;
+  const bool whole = tid - (tid & 31) < (K >> 3);  // K is a multiple of 256: uniform over a warp
+  for (int64_t row = blockIdx.x; row < M; row += gridDim.x) {
+    float v[8], y[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = 0.f;
+    if (active) {
+      const float4 a = __ldg(reinterpret_cast<const float4*>(x + row * ldx + col));
+      const float4 b = __ldg(reinterpret_cast<const float4*>(x + row * ldx + col + 4));
+      v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      ss = fmaf(v[j], v[j], ss);
+      y[j] = bf16_round(v[j]);
+    }
+    if (whole) rotate256(y, tid & 31);
+    float am = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) am = fmaxf(am, fabsf(y[j]));
+    am = block_max<T>(am, red);
+    const float s = fmaxf(__fdiv_rn(am, 127.f), 1e-12f);
+    const uint2 code = quant8_i8(y, s, __fdiv_rn(1.f, s));
+    if (active) *reinterpret_cast<uint2*>(q1 + row * K + col) = code;
+    ss = block_sum_fixed<T>(ss, red);
+    float rms = __fsqrt_rn(__fdiv_rn(ss, static_cast<float>(K)));
+    if (rms < 1e-12f) rms = 1e-12f;                                   // a NaN stays: no comparison with it is true
+    const bool outlier = __fdiv_rn(__fmul_rn(127.f, s), rms) > ratio;  // the same value in every thread
+    if (tid == 0) {
+      s1[row] = s;
+      flags[row] = outlier;
+    }
+    if (!outlier) continue;
+    if (tid == 0) {
+      slot_s = atomicAdd(count, 1);
+      rows[slot_s] = static_cast<int32_t>(row);
+      if (total) atomicAdd(total, 1ull);
+    }
+    if (whole) rotate256(v, tid & 31);
+    am = 0.f;
+    if (active) {
+      const int8_t* cb = reinterpret_cast<const int8_t*>(&code);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        v[j] = __fsub_rn(v[j], __fmul_rn(static_cast<float>(cb[j]), s));
+        am = fmaxf(am, fabsf(v[j]));
+      }
+    }
+    am = block_max<T>(am, red);  // its barriers also publish the slot
+    const int64_t slot = slot_s;
+    const float sr = fmaxf(__fdiv_rn(am, 127.f), 1e-12f);
+    if (tid == 0) s2[slot] = sr;
+    if (active) *reinterpret_cast<uint2*>(q2 + slot * K + col) = quant8_i8(v, sr, __fdiv_rn(1.f, sr));
+    __syncthreads();  // the slot has been read by all before the next outlier row of this CTA replaces it
+  }
+}
+
 // max |x| over a whole [M, K] bf16 tensor into *out (which the caller zeroed): |x| >= 0, so the float order is the
 // order of the bit patterns and one atomicMax on the bits per CTA finishes the reduction, in any order.
 __global__ void __launch_bounds__(256) tensor_absmax_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, int64_t M,
@@ -501,4 +581,29 @@ extern "C" int rh3_rot_residual_quant_rows_i8(const float* x, int64_t ldx, const
   else RH3_RR(1024);
 #undef RH3_RR
   return check_cuda(cudaGetLastError(), "rot_residual_quant launch");
+}
+
+extern "C" int rh3_te_quant(const float* x, int64_t ldx, int64_t M, int64_t K, float ratio, void* q1, float* s1, void* flags,
+                            int32_t* count, int32_t* rows, void* q2, float* s2, void* total, cudaStream_t stream) {
+  RH3_CHECK_ARG(M >= 0 && M < (1ll << 31) && K > 0 && K % 256 == 0 && K <= 8192,
+                "te_quant: K=%lld must be a multiple of 256, <= 8192", (long long)K);
+  RH3_CHECK_ARG(ldx >= K && ldx % 4 == 0, "te_quant: bad row stride");
+  if (M == 0) return 0;
+  RH3_CHECK_ARG(x && q1 && s1 && flags && count && rows && q2 && s2, "te_quant: null pointer");
+  RH3_CHECK_ARG((reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(q1) & 7) == 0 &&
+                    (reinterpret_cast<uintptr_t>(q2) & 7) == 0 && (reinterpret_cast<uintptr_t>(total) & 7) == 0,
+                "te_quant: x must be 16-byte aligned, q1, q2 and total 8-byte aligned");
+  if (int e = check_cuda(cudaMemsetAsync(count, 0, sizeof(int32_t), stream), "te_quant count")) return e;
+  const int64_t threads = K / 8;
+  const unsigned grid = static_cast<unsigned>(M < 8 * device_sm_count() ? M : 8 * device_sm_count());
+#define RH3_TE(T_)                                                                                                       \
+  te_quant_kernel<T_><<<grid, T_, 0, stream>>>(x, ldx, M, (int)K, ratio, static_cast<int8_t*>(q1), s1,                   \
+                                               static_cast<uint8_t*>(flags), count, rows, static_cast<int8_t*>(q2), s2, \
+                                               static_cast<unsigned long long*>(total))
+  if (threads <= 128) RH3_TE(128);
+  else if (threads <= 256) RH3_TE(256);
+  else if (threads <= 512) RH3_TE(512);
+  else RH3_TE(1024);
+#undef RH3_TE
+  return check_cuda(cudaGetLastError(), "te_quant launch");
 }

@@ -9,15 +9,27 @@ are outside this path. CPU tensors raise: there is no fallback.
 """
 import torch
 
-from . import _lib, gemm, kernels, quantizers
+from . import _lib, gemm, kernels, nodes, quantizers
 
-# how often the second pass ran: [rows that took it, rows seen]; `residual_share()` reads it
+# how often the second pass ran: [rows that took it, rows seen]; `residual_share()` reads it. The fused route counts its
+# outlier rows on the device (one uint64 per device): the host does not wait for them.
 _ROWS = [0, 0]
+_TAKEN = {}
 
 
 def residual_share():
     """Fraction of the rows seen so far that were given the residual pass (0.0 before any call)."""
-    return _ROWS[0] / _ROWS[1] if _ROWS[1] else 0.0
+    taken = _ROWS[0] + sum(int(t.item()) for t in list(_TAKEN.values()))
+    return taken / _ROWS[1] if _ROWS[1] else 0.0
+
+
+def _taken(device):
+    """This device's counter (None while a graph is being captured before it exists: it must not live in the graph's pool)."""
+    t = _TAKEN.get(device)
+    if t is None and not torch.cuda.is_current_stream_capturing():
+        t = _TAKEN.setdefault(device, torch.zeros(1, dtype=torch.int64, device=device))
+        torch.cuda.current_stream(device).synchronize()  # once: its fill is done before any other stream adds to it
+    return t
 
 
 def rot_residual_quant_rows_i8(x, q1, s1, rows):
@@ -71,11 +83,54 @@ class _TELinear:
         _ROWS[0] += rows.numel()
         return y
 
+    def _fused(self, x2):
+        """Both passes for fp32 x2 [M, K] in three kernels: the input side (te_quant_kernel) and the two products, whose
+        epilogues write fp32 and add the bias. The number of outlier rows stays on the device."""
+        qw, dev = self.qweight, x2.device
+        m, k = x2.shape
+        n = qw.q.shape[0]
+        second = self.mode == "int8_rot"
+        ws = qw.scale.reshape(-1)
+        bias = self.bias
+        if bias is not None:
+            bias = bias.to(torch.float32).contiguous()
+        out = torch.empty((m, n), device=dev, dtype=torch.float32)
+        # one workspace: q1 | q2 | s1 | s2 | rows | count | flags (every piece starts on a 16-byte boundary: K % 256 == 0)
+        m4 = (m + 3) // 4 * 4
+        work = torch.empty(2 * m * k + 3 * 4 * m4 + 16 + m, device=dev, dtype=torch.uint8)
+        q1 = work.data_ptr()
+        q2 = q1 + m * k
+        s1 = q2 + m * k
+        s2, rows, count = s1 + 4 * m4, s1 + 8 * m4, s1 + 12 * m4
+        flags = count + 16
+        ratio = float(self.outlier_ratio) if second else float("inf")
+        _lib.call("rh3_te_quant", x2.data_ptr(), x2.stride(0), m, k, ratio, q1, s1, flags, count, rows, q2, s2,
+                  _lib.ptr(_taken(dev)) if second else None, _lib.stream())
+        if second:
+            _ROWS[1] += m
+        _lib.call("rh3_te_gemm", q1, s1, qw.q.data_ptr(), ws.data_ptr(), _lib.ptr(bias), m, n, k, flags, count,
+                  rows if second else None, q2, s2, out.data_ptr(), n, _lib.stream())
+        return out
+
+    def _can_fuse(self, x2):
+        """What the fused route takes: fp32 rows the kernel can read in place, a plain row-ordered int8 weight and a bias
+        torch need not see being added. Everything else goes through the separate steps."""
+        qw, k = self.qweight, x2.shape[1]
+        return (type(x2) is torch.Tensor and x2.dtype == torch.float32 and x2.shape[0] > 0 and k % 256 == 0 and k <= 8192
+                and x2.stride(1) == 1 and x2.stride(0) % 4 == 0 and x2.stride(0) >= k and x2.data_ptr() % 16 == 0
+                and qw.q.device == x2.device and qw.q.dtype == torch.int8 and qw.q.is_contiguous() and qw.q.shape[1] == k
+                and qw.q.shape[0] % 8 == 0 and qw.scale.device == x2.device and qw.scale.dtype == torch.float32
+                and qw.scale.numel() == qw.q.shape[0] and qw.scale.is_contiguous()
+                and (self.bias is None or nodes._plain_bias(self.bias, qw.q.shape[0], x2.device)))
+
     def __call__(self, x):
         if x.device.type != "cuda":
             raise NotImplementedError("_TELinear: CUDA tensors only (no fallback path)")
         lead, k = x.shape[:-1], x.shape[-1]
-        y = self._matmul(x.reshape(-1, k)).to(x.dtype)
+        x2 = x.reshape(-1, k)
+        if self._can_fuse(x2):
+            return self._fused(x2).reshape(*lead, self.qweight.q.shape[0])
+        y = self._matmul(x2).to(x.dtype)
         if self.bias is not None:
             y = y + self.bias.to(y.dtype)
         return y.reshape(*lead, y.shape[-1])

@@ -68,3 +68,34 @@ def test_te_linear_matches_oracle_and_helps_outlier_rows(te, mode):
     print(mode, "rows with residual pass:", n_out, "median / max row error:", err.median().item(), err.max().item())
     if mode == "int8_rot":
         assert err.max().item() < 0.02
+
+
+@pytest.mark.parametrize("shape", [(1, 256, 8), (130, 256, 264), (37, 2304, 512), (300, 8192, 128), (1500, 1024, 256)])
+@pytest.mark.parametrize("rows", ["some", "none", "all"])
+def test_fused_route_equals_the_separate_steps(te, shape, rows):
+    """The three-kernel route against quantizer, product, row selection, residual quantizer and second product as separate
+    calls: the same bits (row widths with idle threads, one row, more rows than blocks; no, some and only outlier rows)."""
+    te_quant, kernels, lib = te
+    m, k, n = shape
+    x, w = _case(m, max(k, 512), n, m + k)
+    x, w = x[:, :k].contiguous(), w[:, :k].contiguous()
+    qw = kernels.quantize_weight(w.cuda(), "int8_rot")
+    ratio = {"some": 8.0, "none": 1e9, "all": 0.0}[rows]
+    for bias in (None, 0.1 * torch.randn(n, generator=inputs.gen(3)).cuda()):
+        lin = te_quant._TELinear(qw, bias, "int8_rot", outlier_ratio=ratio)
+        xd = torch.cat([x, torch.full((m, 4), 1e30)], 1).cuda()[:, :k]  # a strided view
+        assert lin._can_fuse(xd)
+        seen = te_quant._ROWS[1]
+        taken = te_quant.residual_share() * seen
+        y = lin(xd)
+        if rows != "some":
+            assert round(te_quant.residual_share() * te_quant._ROWS[1] - taken) == (m if rows == "all" else 0)
+        assert te_quant._ROWS[1] == seen + m
+        lib.check_status()
+        xc = x.cuda()
+        ref = lin._matmul(xc).float()
+        ref = ref if bias is None else ref + bias
+        assert torch.equal(y, ref)
+        plain = te_quant._TELinear(qw, bias, "int8_rot_plain")(xd)
+        p = kernels.linear(xc.to(torch.bfloat16), qw, "int8_rot").float()
+        assert torch.equal(plain, p if bias is None else p + bias)
