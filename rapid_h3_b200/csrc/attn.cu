@@ -16,19 +16,28 @@
 // epilogue O/l*vscale+vmean) with the per-key-block scale structure of :1781-1889 (attn_fwd6) and
 // the operand definitions of bench/attn_emulate.py:10-23,88,101-103.
 //
-// One CTA = TWO 128-query tiles of one head (256 rows), 384 threads = three warp groups, one CTA per
+// One CTA = TWO 128-query tiles of one head (256 rows), 512 threads = four warp groups, one CTA per
 // SM. The two tiles share every K / V^T tile that TMA brings in (3-stage ring) and run as two
 // independent softmax pipelines:
 //   warp group 0  service: warp 0 = TMA producer (Q once, then K tile 128 keys x 128 B + V^T tile 128
 //                 channels x 128 keys per step), warp 1 = MMA issuer (for both query tiles, Q.K^T of
 //                 key tile j+1 is issued before P.V of tile j); gives its registers away (setmaxnreg)
-//   warp groups 1, 2  softmax of query tile 0 / 1, one query row per thread, 232 registers each so a
+//   warp groups 1, 2  softmax of query tile 0 / 1, one query row per thread, 208 registers each so a
 //                 whole row of S (128 values) lives in registers: the accumulator is pre-biased with
 //                 1.5*2^23 so its int32 bits are a float (no conversion); the row is read from TMEM
 //                 ONCE and S is handed straight back, so the next Q.K^T runs under the whole softmax;
 //                 3-input max over the raw values, then t = fma(bits, c, off) in packed f32x2, exp2,
 //                 e4m3 pack; P goes to shared memory in the 128-byte-swizzled K-major layout the MMA
-//                 reads; O and l are rescaled by an exact power of two when the integer maximum grows
+//                 reads (two buffers per tile: P of step j+1 is written while P.V of step j may still run)
+//   warp group 3  rescales O by an exact power of two in the steps where a row's integer maximum grows: a
+//                 softmax thread only writes its row's factor to shared memory and goes on with its
+//                 exponentials; P.V of the step waits for both. (Some row of a warp grows in a fifth of the
+//                 steps at 36,436 keys and in half of them at 4,500; done by the softmax threads the 128
+//                 columns cost them over 1,000 cycles each time.)
+// What bounds it: the serial chain of a softmax thread's step (wait, TMEM load, re-bias, maximum, exponentials,
+// hand-over) at two such warps per scheduler. Measured with H = 32: 16.8 ms at L = 36,436 and 0.340 ms at
+// L = 4,500 before the P buffers and the rescaling warps, 16.0 and 0.315 with them; timing-only builds without
+// any MMA run 15.0 / 0.283, without the exponentials 14.2 / 0.276, with the barriers alone 7.3 / 0.155.
 // TMEM (512 columns): S0 | S1 | O0 | O1, 128 columns each.
 // Tensor-core bound: 4 * Lq * Lk * 128 operations per head.
 #include <limits.h>
@@ -43,7 +52,7 @@ constexpr int BQ = 128, BKV = 128, HD = 128;
 constexpr int QG = 2;                  // query tiles per CTA
 constexpr int TILE_BYTES = 128 * 128;  // every operand tile is 128 rows x 128 bytes
 constexpr int KV_STAGES = 3;
-constexpr int ATTN_THREADS = 384;      // service warp group + two softmax warp groups
+constexpr int ATTN_THREADS = 512;      // service, two softmax and one rescaling warp group
 
 struct AttnParams {
   const float* qs;      // [H][Lq_pad/64]
@@ -69,13 +78,17 @@ struct __align__(8) AttnSmemTail {
   uint64_t q_full;
   uint64_t kv_full[KV_STAGES];
   uint64_t kv_empty[KV_STAGES];
-  uint64_t s_full[QG], s_empty[QG], p_full[QG], pv_done[QG];
+  uint64_t s_full[QG], s_empty[QG];
+  // one barrier per step parity: a softmax warp may be a step ahead of another one of its tile, and its arrival must
+  // not complete the phase the slower one still owes
+  uint64_t p_full[QG][2], pv_done[QG][2], f_full[QG][2];
   uint32_t tmem_base;
   int abort_flag;
+  float factor[QG][2][BQ];   // by how much O of a row is rescaled before P.V of the step (1 mostly)
 };
 
-// Q (2 tiles) | P (2 tiles) | KV ring (K + V^T per stage)
-constexpr int ATTN_SMEM_BYTES = (2 * QG + 2 * KV_STAGES) * TILE_BYTES + sizeof(AttnSmemTail) + 1024;
+// Q (2 tiles) | P (2 tiles x 2) | KV ring (K + V^T per stage)
+constexpr int ATTN_SMEM_BYTES = (3 * QG + 2 * KV_STAGES) * TILE_BYTES + sizeof(AttnSmemTail) + 1024;
 
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
@@ -202,13 +215,15 @@ __device__ __forceinline__ void exp_chunk(const uint32_t* r, int k, float cc, fl
 }
 
 // Register reallocation between warp groups (one instruction per warp, all four warps of the group).
-// The kernel is compiled for 168 registers per thread (384 threads, one CTA per SM); the service group
-// drops to 40 and each softmax thread rises to 232: 128 * 40 + 256 * 232 = 384 * 168 exactly. The two numbers
-// must keep that equality: a request for more registers than the CTA's pool holds never returns.
-constexpr int REGS_COMPILED = 168, REGS_SERVICE = 40, REGS_SOFTMAX = 232;  // 65536 / 384 rounded down to 8
-static_assert(128 * REGS_SERVICE + 256 * REGS_SOFTMAX == ATTN_THREADS * REGS_COMPILED, "register pool must balance");
+// The kernel is compiled for 128 registers per thread (512 threads, one CTA per SM); the service group drops to 40, the
+// rescaling group to 56 (32 columns of O at a time) and each softmax thread rises to 208: together exactly 512 * 128. The
+// numbers must keep that equality: a request for more registers than the CTA's pool holds never returns.
+constexpr int REGS_COMPILED = 128, REGS_SERVICE = 40, REGS_RESCALE = 56, REGS_SOFTMAX = 208;
+static_assert(128 * REGS_SERVICE + 128 * REGS_RESCALE + 256 * REGS_SOFTMAX == ATTN_THREADS * REGS_COMPILED,
+              "register pool must balance");
 __device__ __forceinline__ void reg_release_service() { asm volatile("setmaxnreg.dec.sync.aligned.u32 40;"); }
-__device__ __forceinline__ void reg_take_softmax() { asm volatile("setmaxnreg.inc.sync.aligned.u32 232;"); }
+__device__ __forceinline__ void reg_release_rescale() { asm volatile("setmaxnreg.dec.sync.aligned.u32 56;"); }
+__device__ __forceinline__ void reg_take_softmax() { asm volatile("setmaxnreg.inc.sync.aligned.u32 208;"); }
 
 template <bool DUMP>
 __global__ void __launch_bounds__(ATTN_THREADS, 1)
@@ -217,9 +232,9 @@ attn_int8_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;                            // [QG] tiles
-  uint8_t* sP = smem + QG * TILE_BYTES;          // [QG] tiles
-  uint8_t* sKV = smem + 2 * QG * TILE_BYTES;     // stage s: K at +s*2*TILE, V^T at +s*2*TILE + TILE
-  AttnSmemTail* tail = reinterpret_cast<AttnSmemTail*>(smem + (2 * QG + 2 * KV_STAGES) * TILE_BYTES);
+  uint8_t* sP = smem + QG * TILE_BYTES;          // [QG][2] tiles
+  uint8_t* sKV = smem + 3 * QG * TILE_BYTES;     // stage s: K at +s*2*TILE, V^T at +s*2*TILE + TILE
+  AttnSmemTail* tail = reinterpret_cast<AttnSmemTail*>(smem + (3 * QG + 2 * KV_STAGES) * TILE_BYTES);
   volatile int* abort_flag = &tail->abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -235,8 +250,11 @@ attn_int8_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
     for (int g = 0; g < QG; ++g) {
       mbar_init(&tail->s_full[g], 1);
       mbar_init(&tail->s_empty[g], 4);  // one arrival per softmax warp (128 separate arrivals on one
-      mbar_init(&tail->p_full[g], 4);   // barrier word serialise and cost more than the MMAs they gate)
-      mbar_init(&tail->pv_done[g], 1);
+      for (int b = 0; b < 2; ++b) {       // barrier word serialise and cost more than the MMAs they gate)
+        mbar_init(&tail->p_full[g][b], 8);   // four softmax warps (P is written), four rescaling warps (O is ready)
+        mbar_init(&tail->pv_done[g][b], 1);
+        mbar_init(&tail->f_full[g][b], 4);
+      }
     }
     tail->abort_flag = 0;
     fence_barrier_init();
@@ -310,13 +328,13 @@ attn_int8_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
         const int stage = j % KV_STAGES;
         const uint32_t v_addr = smem_u32(sKV + stage * 2 * TILE_BYTES + TILE_BYTES);
         for (int g = 0; g < QG && ok; ++g) {
-          ok = all_ok(mbar_wait_relaxed(&tail->p_full[g], j & 1, abort_flag, p.status, ST_TIMEOUT_P_READY, 64));
+          ok = all_ok(mbar_wait_relaxed(&tail->p_full[g][j & 1], (j >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_P_READY, 64));
           if (!ok) break;
           tc_fence_after();
-          const uint32_t p_addr = smem_u32(sP + g * TILE_BYTES);
+          const uint32_t p_addr = smem_u32(sP + (2 * g + (j & 1)) * TILE_BYTES);
           if (elect_one()) {
             mma4_f8_ss(tmem_base + 256 + g * 128, make_desc_k128(p_addr), make_desc_k128(v_addr), idesc_pv, j != 0);
-            mma_commit(&tail->pv_done[g]);
+            mma_commit(&tail->pv_done[g][j & 1]);
           }
           __syncwarp();
         }
@@ -324,6 +342,40 @@ attn_int8_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
           if (elect_one()) mma_commit(&tail->kv_empty[stage]);  // both query tiles have read this K / V^T stage
           __syncwarp();
         }
+      }
+    }
+  } else if (warp >= 12) {
+    // ============================ rescaling warp group ============================
+    reg_release_rescale();
+    const int quad = warp & 3;
+    const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
+    bool ok = true;
+    for (int j = 0; j < n_kv && ok; ++j) {
+      for (int g = 0; g < QG && ok; ++g) {
+        ok = __all_sync(0xffffffffu, mbar_wait_relaxed(&tail->f_full[g][j & 1], (j >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_P_READY, 32));
+        if (!ok) break;
+        const float f = tail->factor[g][j & 1][quad * 32 + lane];
+        if (__any_sync(0xffffffffu, f != 1.f)) {   // never in step 0: its factors are all 1
+          // O is complete up to step j - 1 once that step's P.V has finished
+          ok = __all_sync(0xffffffffu, mbar_wait_relaxed(&tail->pv_done[g][(j - 1) & 1], ((j - 1) >> 1) & 1, abort_flag, p.status,
+                                                         ST_TIMEOUT_PV_DONE, 32));
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t o_row = tmem_base + 256 + g * 128 + lane_off;
+#pragma unroll 1
+          for (int c = 0; c < 4; ++c) {
+            uint32_t r[32];
+            tmem_ld32(o_row + c * 32, r);
+            tmem_ld_wait_regs(r);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * f);
+            tmem_st32(o_row + c * 32, r);
+          }
+          tmem_st_wait();
+          tc_fence_before();
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tail->p_full[g][j & 1]);
       }
     }
   } else {
@@ -342,12 +394,10 @@ attn_int8_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
     const int64_t q_row = static_cast<int64_t>(q_pair) * (QG * BQ) + g * BQ + row;
     const float c_row = __fmul_rn(p.qs[static_cast<int64_t>(h) * (p.Lq_pad / 64) + (q_row >> 6)], p.sl2);
     const float* ks_h = p.ks + static_cast<int64_t>(h) * (p.Lk_pad / 64);
-    uint8_t* p_row = sP + g * TILE_BYTES + row * 128;
+    uint8_t* p_row0 = sP + 2 * g * TILE_BYTES + row * 128;
     const int sw = row & 7;
     uint64_t* s_full = &tail->s_full[g];
     uint64_t* s_empty = &tail->s_empty[g];
-    uint64_t* p_full = &tail->p_full[g];
-    uint64_t* pv_done = &tail->pv_done[g];
     float M = 0.f, l = 0.f;
     bool ok = true;
 
@@ -370,7 +420,9 @@ attn_int8_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
       }
       const float b0 = __fmul_rn(kMagic, c0), b1 = __fmul_rn(kMagic, c1);
       const int valid = min(BKV, p.Lk - j * BKV);
-      if (!mbar_wait_relaxed(s_full, j & 1, abort_flag, p.status, ST_TIMEOUT_ACC_FULL, 32)) { ok = false; break; }
+      // this phase also says that P.V of step j - 2 is done (the commit behind it covers every MMA issued before), so that
+      // step's P buffer is free
+      if (!mbar_wait(s_full, j & 1, abort_flag, p.status, ST_TIMEOUT_ACC_FULL)) { ok = false; break; }
       tc_fence_after();
       // ---- the whole row of S (128 raw values) into registers, once ----
       uint32_t r0[32], r1[32], r2[32], r3[32];
@@ -414,29 +466,17 @@ attn_int8_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
       const float mx0 = fmaxf(chunk_max(r0), chunk_max(r1)), mx1 = fmaxf(chunk_max(r2), chunk_max(r3));
       const float m = fmaxf(mx0 > 0.f ? fmaf(mx0, c0, -b0) : -INFINITY, mx1 > 0.f ? fmaf(mx1, c1, -b1) : -INFINITY);
       const float M_new = j == 0 ? ceilf(m) : fmaxf(M, ceilf(m));
-      const bool grow = j > 0 && M_new > M;
-      if (j > 0) {
-        // P.V of the previous tile has finished: O is complete up to tile j-1 and the P buffer is free
-        if (!mbar_wait_relaxed(pv_done, (j - 1) & 1, abort_flag, p.status, ST_TIMEOUT_PV_DONE, 32)) { ok = false; break; }
-        if (__any_sync(0xffffffffu, grow)) {
-          tc_fence_after();
-          const float f = grow ? ex2_approx(M - M_new) : 1.f;  // exact power of two
-#pragma unroll 1
-          for (int c = 0; c < 16; ++c) {  // 8 columns at a time: this path is rare and must stay small
-            uint32_t r[8];
-            tmem_ld8(o_row + c * 8, r);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * f);
-            tmem_st8(o_row + c * 8, r);
-          }
-          tmem_st_wait();
-          l *= f;
-        }
-      }
+      // what O and l of the rows before are worth against the new maximum: an exact power of two
+      const float f = j > 0 && M_new > M ? ex2_approx(M - M_new) : 1.f;
+      tail->factor[g][j & 1][row] = f;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tail->f_full[g][j & 1]);
+      l *= f;
       M = M_new;
       const float off0 = __fsub_rn(__fsub_rn(8.f, M), b0), off1 = __fsub_rn(__fsub_rn(8.f, M), b1);
       // ---- P = e4m3(2^t) into shared memory, l += p ----
       uint64_t lsum2 = pack2(0.f, 0.f);
+      uint8_t* p_row = p_row0 + (j & 1) * TILE_BYTES;
       exp_chunk(r0, 0, c0, off0, p_row, sw, lsum2);
       exp_chunk(r1, 1, c0, off0, p_row, sw, lsum2);
       exp_chunk(r2, 2, c1, off1, p_row, sw, lsum2);
@@ -447,10 +487,10 @@ attn_int8_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
       fence_proxy_async_smem();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(p_full);
+      if (lane == 0) mbar_arrive(&tail->p_full[g][j & 1]);
     }
     // ---- epilogue ----
-    if (ok && mbar_wait(pv_done, (n_kv - 1) & 1, abort_flag, p.status, ST_TIMEOUT_PV_DONE)) {
+    if (ok && mbar_wait(&tail->pv_done[g][(n_kv - 1) & 1], ((n_kv - 1) >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_PV_DONE)) {
       tc_fence_after();
       const float inv_l = __fdiv_rn(1.f, l);
       const float* vs = p.vscale + h * HD;

@@ -200,3 +200,19 @@ def test_prepass_operands_match_the_reference_emulation_fixture(ops):
         assert torch.equal(pre.k8[h, :l].cpu().float() * pre.ks[h].cpu()[blk][:, None], ref["k_fq"])
         vdec = pre.vt[h, :, :l].cpu().float().t() * pre.vscale[h].cpu()[None]
         assert torch.equal(vdec, ref["v_fq"])
+
+
+@pytest.mark.parametrize("lk", [64, 128, 129, 300, 900])
+@pytest.mark.parametrize("step", [0.02, 6.0])
+def test_row_maximum_that_grows_in_every_key_tile(ops, lk, step):
+    """Scores that rise with the key index, so every row's integer maximum grows in each step (by 1 or by many) and the
+    accumulated output is rescaled each time; one to eight key tiles, ragged last ones, a ragged query tile."""
+    attn, lib = ops
+    lq, h = 333, 2
+    q, _, _ = inputs.attention_case(lq, h, seed=31)
+    _, k, v = inputs.attention_case(lk, h, seed=32)
+    q[..., 0] = 8.0
+    k[..., 0] = (step * torch.arange(lk) / 8.0)[:, None].to(k.dtype)
+    out = attn.attention(q.cuda(), k.cuda(), v.cuda())
+    lib.check_status()
+    assert rel_l2(out.cpu(), oa.attention(q, k, v)) <= TOL
