@@ -108,7 +108,7 @@ def _int8_prepass(q, k, v, tab, qw, kw, eps, q_roped, k_roped):
         tab = tab.contiguous()
     lqp, lkp = _pad256(lq), _pad128(lk)
     f32 = dict(device=dev, dtype=torch.float32)
-    kmean, vmean, vscale = (torch.empty((h, D), **f32) for _ in range(3))
+    kmean, vmean, vscale = torch.empty((3, h, D), **f32).unbind(0)
     nbytes = _lib.lib().rh3_attn_kv_stats_scratch_bytes(lk, h)
     scratch = torch.empty(nbytes, device=dev, dtype=torch.uint8)
     q8 = torch.empty((h, lqp, D), device=dev, dtype=torch.int8)
@@ -199,7 +199,7 @@ def tok_prepass(q, k, v, tab=None, qw=None, kw=None, eps=1e-5, q_roped=None, k_r
         tab = tab.contiguous()
     lqp, lkp = _pad256(lq), _pad128(lk)
     f32 = dict(device=dev, dtype=torch.float32)
-    kmean, vmean, vscale = (torch.empty((h, D), **f32) for _ in range(3))
+    kmean, vmean, vscale = torch.empty((3, h, D), **f32).unbind(0)
     nbytes = _lib.lib().rh3_attn_kv_stats_scratch_bytes(lk, h)
     scratch = torch.empty(nbytes, device=dev, dtype=torch.uint8)
     q8 = torch.empty((h, lqp, D), device=dev, dtype=torch.int8)

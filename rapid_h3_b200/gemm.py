@@ -18,10 +18,9 @@ def _check(xq, xs, wq, ws, dtype):
         raise RuntimeError("xq needs unit column stride and wq must be contiguous")
     m, k = xq.shape
     n = wq.shape[0]
-    xs, ws = xs.reshape(-1), ws.reshape(-1)
     if xs.numel() != m or ws.numel() != n or xs.dtype != torch.float32 or ws.dtype != torch.float32:
         raise RuntimeError("xs / ws must be fp32 with M / N elements")
-    return m, n, k, xs.contiguous(), ws.contiguous()
+    return m, n, k, xs.contiguous(), ws.contiguous()   # in any shape: only their elements in order are read
 
 
 def _gemm(xq, xs, wq, ws, bias, kind, dtype, acc_dump=None, out=None):
