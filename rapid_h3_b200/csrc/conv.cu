@@ -745,9 +745,24 @@ extern "C" int rh3_conv3d_causal(const void* x, const void* w, const void* bias,
   // output channels per tile: the whole width when it fits one accumulator, else an even split. The epilogue walks
   // a tile in 32-column chunks, so a split tile is a multiple of 32 wide: a chunk must never reach into the columns
   // of the next tile (weight rows past Cout are zero-filled by TMA and their stores are skipped).
-  const int splits = (p.Cout + 255) / 256;
-  p.BN = ((p.Cout + splits - 1) / splits + 15) / 16 * 16;
-  if (splits > 1) p.BN = (p.BN + 31) / 32 * 32;
+  int splits = (p.Cout + 255) / 256;
+  auto tile_width = [&](int n) {
+    const int bn = ((p.Cout + n - 1) / n + 15) / 16 * 16;
+    return n > 1 ? (bn + 31) / 32 * 32 : bn;
+  };
+  // Few sites leave most of the chip idle at full width (a 3 x 12 x 21 latent has 6 site tiles: 12 CTAs at 512 channels,
+  // 79 us a layer), so the channels are split further while that lowers waves x time of a tile. A pair's tile takes as
+  // long as an SM needs to take in its K chunks, 16 KB of sites and 64 B per channel each, so a split is not free: half
+  // the width costs 3/4 of the time, and with enough site tiles for a whole wave full width stays the better one.
+  {
+    const int64_t pairs = (N * T * p.tiles_h * p.tiles_w + 1) / 2, resident = device_sm_count() / 2;
+    auto cost = [&](int n) {
+      const int bn = tile_width(n);
+      return ((pairs * ((p.Cout + bn - 1) / bn) + resident - 1) / resident) * (16384 + 64ll * bn);
+    };
+    for (int n = splits * 2; tile_width(n) >= 64 && cost(n) < cost(splits); n *= 2) splits = n;
+  }
+  p.BN = tile_width(splits);
   p.bias = static_cast<const __nv_bfloat16*>(bias);
   p.residual = static_cast<const __nv_bfloat16*>(residual);
   p.out = static_cast<__nv_bfloat16*>(out);

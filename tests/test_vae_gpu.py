@@ -75,6 +75,27 @@ def test_cta_pair_kernel_equals_the_single_cta_kernel(vae, shape):
         assert torch.equal(part_pair, part_one)
 
 
+@pytest.mark.parametrize("cin,cout", [(64, 512), (64, 256), (64, 128), (64, 288), (128, 192)])
+def test_channel_split_of_small_calls_changes_nothing(vae, cin, cout):
+    """A call with few sites splits its channels over more tiles; the same sample in a batch that fills the chip does not:
+    same outputs and GroupNorm sums bit for bit."""
+    v, lib = vae
+    g = torch.Generator().manual_seed(cout)
+    x = torch.randn(1, 2, 9, 13, cin, generator=g).to(torch.bfloat16).cuda()
+    wt = (0.05 * torch.randn(cout, 27, cin, generator=g)).to(torch.bfloat16).cuda()
+    b = (0.1 * torch.randn(cout, generator=g)).to(torch.bfloat16).cuda()
+    res = torch.randn(1, 2, 9, 13, cout, generator=g).to(torch.bfloat16).cuda()
+    stats = 32 % (cout // 32) == 0
+    y, part = v.conv3d_causal(x, wt, b, res, want_stats=stats)
+    n = 150  # 150 x 2 site tiles: more than a wave of pairs at full width
+    yb, part_b = v.conv3d_causal(x.expand(n, -1, -1, -1, -1).contiguous(), wt, b, res.expand(n, -1, -1, -1, -1).contiguous(),
+                                 want_stats=stats)
+    lib.check_status()
+    assert torch.equal(yb, y.expand(n, -1, -1, -1, -1))
+    if stats:
+        assert torch.equal(part_b.view(n, *part.shape), part.expand(n, *part.shape))
+
+
 def test_causality(vae):
     """Changing frame t must leave every output frame before t untouched."""
     v, lib = vae
