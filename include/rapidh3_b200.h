@@ -110,6 +110,10 @@ int rh3_norm_mod_rot_quant_rows_i8(const void* x, int64_t ldx, const void* w, fl
                                    const float* shift, const float* scale, int64_t ld_tab, int64_t M, int64_t K,
                                    void* q, int64_t ldq, float* s, cudaStream_t stream);
 
+/* out[M,K] bf16 = bf16((x * r) * w), r = rsqrt(mean(x^2) + eps) per row; x, out bf16 with row strides ldx, ldo, w bf16 [K];
+ * K % 8 == 0, K <= 16384. The transformer's final norm (no entry of its own in the reference: a host-framework RMSNorm). */
+int rh3_rms_norm_rows(const void* x, int64_t ldx, const void* w, float eps, int64_t M, int64_t K, void* out, int64_t ldo,
+                      cudaStream_t stream);
 /* Input side of the text encoder's linear on x fp32 [M, K] (row stride ldx; K % 256 == 0, K <= 8192): q1 [M, K], s1 [M] = the
  * int8 row quantizer on rotate(bf16(x)); flags [M] bytes = 1 where 127 s1 / max(rms(x), 1e-12) > ratio; those rows also get a
  * slot i < *count (any order): rows[i], and q2[i], s2[i] = the int8 codes of rotate(x) - q1 s1. *count (int32) is set by the

@@ -180,9 +180,10 @@ class H3Transformer(nn.Module):
             return v
         return torch.cat([v, self.audio_embed(audio.to(torch.bfloat16))], 0)
 
-    def untokens(self, x, latent_shape):
+    def untokens(self, x, latent_shape, norm=None):
+        """`norm` takes the place of the final norm's own forward (the quantized runtime's one-pass kernel)."""
         n_video = latent_shape[1] * latent_shape[2] * latent_shape[3]
-        h = self.final_norm(x)
+        h = (norm or self.final_norm)(x)
         video = self.unembed(h[:n_video]).t().reshape(latent_shape)
         audio = self.audio_unembed(h[n_video:])
         return video, audio

@@ -57,6 +57,19 @@ def quant_tensor(x):
     return q, s
 
 
+def rms_norm_rows(x, weight, eps):
+    """bf16((x * rsqrt(mean(x^2) + eps)) * weight) of bf16 rows x [M, K] in one pass; weight bf16 [K]."""
+    _check_rows(x)
+    m, k = x.shape
+    _lib.require_cuda(weight)
+    if weight.dtype != torch.bfloat16 or weight.numel() != k or not weight.is_contiguous():
+        raise RuntimeError("weight must be contiguous bf16 [K]")
+    out = torch.empty((m, k), device=x.device, dtype=torch.bfloat16)
+    _lib.call("rh3_rms_norm_rows", x.data_ptr(), x.stride(0), weight.data_ptr(), float(eps), m, k, out.data_ptr(), k,
+              _lib.stream())
+    return out
+
+
 def _rot_width(k):
     if k % ROT_GROUP:
         raise RuntimeError(f"the rotated width {k} must be a multiple of {ROT_GROUP}")

@@ -239,3 +239,26 @@ def test_rotated_codes_match_the_reference_convrot_fixture(ops):
         d = (q.cpu().int() - want_q.int()).abs()
         assert (d > 0).float().mean().item() < 1e-3 and int(d.max()) <= 1
         assert ((s.cpu().reshape(-1) - want_s.reshape(-1)).abs() / want_s.reshape(-1)).max() < 1e-6
+
+
+@pytest.mark.parametrize("shape", [(1, 8), (37, 264), (3000, 4096), (5, 8200), (9, 16384)])
+def test_rms_norm_rows(shape):
+    """Against 64-bit arithmetic: the fp32 chain (sum of K squares, reciprocal root, two products) is good to a few 2^-24
+    of the value, so the bf16 result is the nearest one or, next to a tie, its neighbour."""
+    from rapid_h3_b200 import _lib, model, quantizers
+    m, k = shape
+    g = torch.Generator().manual_seed(k)
+    x = (torch.randn(m, k, generator=g) * (0.1 + torch.rand(m, 1, generator=g))).to(torch.bfloat16)
+    x[0] = 0
+    w = (1 + 0.1 * torch.randn(k, generator=g)).to(torch.bfloat16)
+    wide = torch.cat([x, x[:, :8]], 1).cuda()[:, :k]  # a row stride of its own
+    y = quantizers.rms_norm_rows(wide, w.cuda(), 1e-6)
+    _lib.check_status()
+    xd = x.double()
+    ref = xd / (xd.pow(2).mean(-1, keepdim=True) + 1e-6).sqrt() * w.double()
+    assert ((y.cpu().double() - ref).abs() <= (2 ** -9 + 2 ** -20) * ref.abs() * 2).all()
+    norm = model.RMSNorm(k, 1e-6).cuda()
+    norm.weight.copy_(w)
+    assert (y != norm(x.cuda())).float().mean() < 2e-3
+    with pytest.raises(RuntimeError):
+        quantizers.rms_norm_rows(x, w, 1e-6)  # CPU tensors: no CPU path
