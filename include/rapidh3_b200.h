@@ -145,6 +145,11 @@ int rh3_gemm_w8a8_bias_after(const void* xq, int64_t lda, const void* wq, const 
 int rh3_gemm_w8a8_gated_residual(const void* xq, int64_t lda, const void* wq, const float* xs, const float* ws,
                                  const void* gate, void* resid, int64_t ldr, int64_t M, int64_t N, int64_t K,
                                  int kind, cudaStream_t stream);
+/* The same with two gate rows in fp32 [N], rounded to bf16 on the way: rows below `split` take gate0, the others gate1 (the
+ * video and audio rows of a packed sequence; reference: one addcmul per mod segment, __init__.py:189-200). */
+int rh3_gemm_w8a8_gated_residual2(const void* xq, int64_t lda, const void* wq, const float* xs, const float* ws,
+                                  const float* gate0, const float* gate1, int64_t split, void* resid, int64_t ldr, int64_t M,
+                                  int64_t N, int64_t K, int kind, cudaStream_t stream);
 /* wq rows interleaved [g 4j..4j+3 | u 4j..4j+3]; out[M, N/2] = bf16(silu(bf16 g) * bf16 u).
  * Replaces int8_gemm_swiglu (fp8_rowwise.cu:29-107, :611-629; row order cutlass_fp8.py:55-62). */
 int rh3_gemm_w8a8_swiglu(const void* xq, int64_t lda, const void* wq, const float* xs, const float* ws, int64_t M,

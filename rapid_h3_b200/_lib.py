@@ -49,6 +49,7 @@ SIGNATURES = {
     "rh3_gemm_w8a8": [_P, _I64, _P, _P, _P, _P, _I64, _I64, _I64, _I, _P, _I64, _P, _P],
     "rh3_gemm_w8a8_bias_after": [_P, _I64, _P, _P, _P, _P, _I64, _I64, _I64, _I, _P, _I64, _P],
     "rh3_gemm_w8a8_gated_residual": [_P, _I64, _P, _P, _P, _P, _P, _I64, _I64, _I64, _I64, _I, _P],
+    "rh3_gemm_w8a8_gated_residual2": [_P, _I64, _P, _P, _P, _P, _P, _I64, _P, _I64, _I64, _I64, _I64, _I, _P],
     "rh3_gemm_w8a8_swiglu": [_P, _I64, _P, _P, _P, _I64, _I64, _I64, _I, _P, _I64, _P],
     "rh3_rmsnorm_rope3d": [_P, _I64, _I64, _P, _I64, _I64, _I64, _I64, _P, _F, _P, _P],
     "rh3_attn_kv_stats_scratch_bytes": [_I64, _I64],

@@ -8,6 +8,7 @@
 //   EPI_F32   : out[m, n]   = float(bf16(...)) + bias[n] in fp32; rows flagged for a second pass leave the bias to it
 //   EPI_F32_ADD: out[rows[m], n] = (out[rows[m], n] + float(bf16(...))) + bias[n]; the number of rows is read on the device
 //   EPI_GATED : resid[m, n] = bf16(fma(bf16((float(acc) * xs[m]) * ws[n]), gate[n], resid[m, n]))   (in place)
+//   EPI_GATED2: the same with two fp32 gate rows, rounded to bf16 here: rows below gate_split take the first, the rest the second
 //   EPI_SWIGLU: columns come in groups of 8 = [g 4j..4j+3 | u 4j..4j+3];
 //               out[m, n/2] = bf16(silu(bf16(g)) * bf16(u)), half-width store
 // (reference: custom_nodes/rapid_h3/csrc/fp8_rowwise.cu:294-304 plain epilogue, :333-336 gated
@@ -49,7 +50,8 @@ constexpr int GEMM_THREADS = 64 + EPI_THREADS;
 #endif
 constexpr int GROUP_M = RH3_GEMM_GROUP_M;  // tile rasterisation: GROUP_M row-tiles share each column-tile in L2
 
-enum { EPI_PLAIN = 0, EPI_GATED = 1, EPI_SWIGLU = 2, EPI_F16 = 3, EPI_SWIGLU_F16 = 4, EPI_BIAS2 = 5, EPI_F32 = 6, EPI_F32_ADD = 7 };
+enum { EPI_PLAIN = 0, EPI_GATED = 1, EPI_SWIGLU = 2, EPI_F16 = 3, EPI_SWIGLU_F16 = 4, EPI_BIAS2 = 5, EPI_F32 = 6, EPI_F32_ADD = 7, EPI_GATED2 = 8 };
+__host__ __device__ constexpr bool is_gated(int epi) { return epi == EPI_GATED || epi == EPI_GATED2; }
 
 struct GemmParams {
   int M, N, K;
@@ -60,6 +62,8 @@ struct GemmParams {
   int64_t ldo;
   int32_t* acc_dump;          // optional raw accumulator dump [M, N] (int32, or fp32 bits for fp8)
   const __nv_bfloat16* gate;  // EPI_GATED
+  const float* gate_f[2];     // EPI_GATED2
+  int gate_split;
   __nv_bfloat16* resid;       // EPI_GATED
   int64_t ldr;
   // fp16 epilogues of the VAE transformer decoder (EPI_F16 / EPI_SWIGLU_F16)
@@ -109,7 +113,7 @@ __device__ __forceinline__ void tile_coords(int tile, int num_m, int num_n, int&
 template <int EPI>
 __device__ __forceinline__ void prefetch_residual(const GemmParams& p, int row, bool row_ok, int n0) {  // n0: first of EPI_COLS columns
   if (!row_ok) return;
-  if (EPI == EPI_GATED) {
+  if (is_gated(EPI)) {
     const __nv_bfloat16* r = p.resid + static_cast<int64_t>(row) * p.ldr + n0;
 #pragma unroll
     for (int c = 0; c < EPI_COLS; c += 64)
@@ -212,7 +216,8 @@ __device__ __forceinline__ void epilogue_row(const GemmParams& p, const GemmSmem
           w4[g] = make_uint4(w[0], w[1], w[2], w[3]);
         }
         store_chunk_bf16(o, w4, col0, p.N, p.wide);
-      } else if (EPI == EPI_GATED) {
+      } else if (is_gated(EPI)) {
+        const float* gate = EPI == EPI_GATED2 && row >= p.gate_split ? tail->aux2 : tail->aux;
         __nv_bfloat16* o = p.resid + static_cast<int64_t>(row) * p.ldr + col0;
         uint4 w4[4];
 #pragma unroll
@@ -223,8 +228,8 @@ __device__ __forceinline__ void epilogue_row(const GemmParams& p, const GemmSmem
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const int e = g * 8 + 2 * j;
-            const float v0 = fmaf(bf16_round(y[e]), tail->aux[c * 32 + e], bf16_lo(ow[j]));
-            const float v1 = fmaf(bf16_round(y[e + 1]), tail->aux[c * 32 + e + 1], bf16_hi(ow[j]));
+            const float v0 = fmaf(bf16_round(y[e]), gate[c * 32 + e], bf16_lo(ow[j]));
+            const float v1 = fmaf(bf16_round(y[e + 1]), gate[c * 32 + e + 1], bf16_hi(ow[j]));
             w[j] = pack_bf16x2(v0, v1);
           }
           w4[g] = make_uint4(w[0], w[1], w[2], w[3]);
@@ -334,7 +339,7 @@ __device__ __forceinline__ void epilogue_row(const GemmParams& p, const GemmSmem
       }
     }
   };
-  if (EPI == EPI_GATED) {
+  if (is_gated(EPI)) {
     // the residual of the next two chunks is fetched while the current two are computed (the loads of a row are
     // 16 bytes each from a cold 8 KB-strided row: waiting for them chunk by chunk was most of this epilogue's time)
     // (the first two chunks' values, `res0`, were fetched by the caller before it waited for the accumulator)
@@ -485,6 +490,10 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         tail->ws[c] = n < p.N ? p.ws[n] : 0.f;
         if (EPI == EPI_PLAIN || EPI == EPI_BIAS2) tail->aux[c] = (p.bias && n < p.N) ? __bfloat162float(p.bias[n]) : 0.f;
         if (EPI == EPI_F32 || EPI == EPI_F32_ADD) tail->aux[c] = (p.bias_f && n < p.N) ? p.bias_f[n] : -0.f;
+        if (EPI == EPI_GATED2) {
+          tail->aux[c] = n < p.N ? bf16_round(p.gate_f[0][n]) : 0.f;
+          tail->aux2[c] = n < p.N ? bf16_round(p.gate_f[1][n]) : 0.f;
+        }
         if (EPI == EPI_GATED) tail->aux[c] = n < p.N ? __bfloat162float(p.gate[n]) : 0.f;
         if (EPI == EPI_F16 || EPI == EPI_SWIGLU_F16) tail->aux[c] = n < p.N ? __half2float(p.bias_h[n]) : 0.f;
         if (EPI == EPI_F16) tail->aux2[c] = (p.rscale_h && n < p.N) ? __half2float(p.rscale_h[n]) : 0.f;
@@ -499,7 +508,7 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         prefetch_residual<EPI>(p, row2, row2 < M, n2 * BN + c_first * 32);
       }
       uint4 res0[8];
-      if (EPI == EPI_GATED) load_gated_residual(p, row, row_ok, n0, c_first, res0);
+      if (is_gated(EPI)) load_gated_residual(p, row, row_ok, n0, c_first, res0);
       // the four warps leave together: a warp that gave up its wait takes the others with it at this barrier
       // (which also publishes the staged columns), so none of them waits at the next tile's barrier alone
       const bool got = mbar_wait(&tail->acc_full[acc], acc_phase, abort_flag, p.status, ST_TIMEOUT_ACC_FULL);
@@ -680,6 +689,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         cols->ws[c] = n < p.N ? p.ws[n] : 0.f;
         if (EPI == EPI_PLAIN || EPI == EPI_BIAS2) cols->aux[c] = (p.bias && n < p.N) ? __bfloat162float(p.bias[n]) : 0.f;
         if (EPI == EPI_F32 || EPI == EPI_F32_ADD) cols->aux[c] = (p.bias_f && n < p.N) ? p.bias_f[n] : -0.f;
+        if (EPI == EPI_GATED2) {
+          cols->aux[c] = n < p.N ? bf16_round(p.gate_f[0][n]) : 0.f;
+          cols->aux2[c] = n < p.N ? bf16_round(p.gate_f[1][n]) : 0.f;
+        }
         if (EPI == EPI_GATED) cols->aux[c] = n < p.N ? __bfloat162float(p.gate[n]) : 0.f;
         if (EPI == EPI_F16 || EPI == EPI_SWIGLU_F16) cols->aux[c] = n < p.N ? __half2float(p.bias_h[n]) : 0.f;
         if (EPI == EPI_F16) cols->aux2[c] = (p.rscale_h && n < p.N) ? __half2float(p.rscale_h[n]) : 0.f;
@@ -694,7 +707,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         prefetch_residual<EPI>(p, row2, row2 < M, n2 * BN + c_first * 32);
       }
       uint4 res0[8];
-      if (EPI == EPI_GATED) load_gated_residual(p, row, row_ok, n0, c_first, res0);
+      if (is_gated(EPI)) load_gated_residual(p, row, row_ok, n0, c_first, res0);
       const bool got = mbar_wait(&tail->acc_full[acc], acc_phase, abort_flag, p.status, ST_TIMEOUT_ACC_FULL);
       if (bar_sync_or(1, EPI_THREADS, !got)) break;
       tc_fence_after();
@@ -854,6 +867,25 @@ extern "C" int rh3_gemm_w8a8_gated_residual(const void* xq, int64_t lda, const v
   p.resid = static_cast<__nv_bfloat16*>(resid); p.ldr = ldr; p.status = device_status_word();
   p.wide = (reinterpret_cast<uintptr_t>(resid) & 31) == 0 && ldr % 16 == 0;
   return kind == RH3_KIND_F8 ? launch_gemm<1, EPI_GATED>(ta, tb, tbp, p, stream) : launch_gemm<0, EPI_GATED>(ta, tb, tbp, p, stream);
+}
+
+// The gated residual over a packed sequence of two modalities in one launch: a launch per modality ran the 148 audio rows
+// through the whole K loop on 32 SMs (20 us at K = 4,096, 54 us at K = 16,384) and needed the gate table converted first.
+extern "C" int rh3_gemm_w8a8_gated_residual2(const void* xq, int64_t lda, const void* wq, const float* xs, const float* ws,
+                                             const float* gate0, const float* gate1, int64_t split, void* resid,
+                                             int64_t ldr, int64_t M, int64_t N, int64_t K, int kind, cudaStream_t stream) {
+  CUtensorMap ta, tb, tbp;
+  if (int e = gemm_common(xq, lda, wq, xs, ws, M, N, K, kind, &ta, &tb, &tbp)) return e;
+  if (M == 0) return 0;
+  RH3_CHECK_ARG(gate0 && gate1 && split >= 0, "gemm_w8a8_gated_residual2: two gate rows and a split >= 0 are required");
+  RH3_CHECK_ARG(resid && ldr >= N && ldr % 8 == 0 && (reinterpret_cast<uintptr_t>(resid) & 15) == 0,
+                "gemm_w8a8_gated_residual2: resid must be 16-byte aligned with a row stride >= N, multiple of 8");
+  GemmParams p{};
+  p.M = (int)M; p.N = (int)N; p.K = (int)K; p.xs = xs; p.ws = ws;
+  p.gate_f[0] = gate0; p.gate_f[1] = gate1; p.gate_split = (int)(split < M ? split : M);
+  p.resid = static_cast<__nv_bfloat16*>(resid); p.ldr = ldr; p.status = device_status_word();
+  p.wide = (reinterpret_cast<uintptr_t>(resid) & 31) == 0 && ldr % 16 == 0;
+  return kind == RH3_KIND_F8 ? launch_gemm<1, EPI_GATED2>(ta, tb, tbp, p, stream) : launch_gemm<0, EPI_GATED2>(ta, tb, tbp, p, stream);
 }
 
 extern "C" int rh3_gemm_w8a8_swiglu(const void* xq, int64_t lda, const void* wq, const float* xs, const float* ws,

@@ -81,6 +81,22 @@ def int8_gemm_gated_residual(xq, xs, wq, ws, gate, resid, config=6):
     return resid
 
 
+def int8_gemm_gated_residual2(xq, xs, wq, ws, gate0, gate1, split, resid):
+    """int8_gemm_gated_residual with gate bf16(gate0) for the rows below `split` and bf16(gate1) for the others; the gates
+    are contiguous fp32 [N]. Returns `resid`."""
+    m, n, k, xs, ws = _check(xq, xs, wq, ws, torch.int8)
+    _lib.require_cuda(gate0, gate1, resid)
+    for g in (gate0, gate1):
+        if g.dtype != torch.float32 or g.numel() != n or not g.is_contiguous():
+            raise RuntimeError("gates must be contiguous fp32 with N elements")
+    if resid.dtype != torch.bfloat16 or resid.shape != (m, n) or resid.stride(1) != 1:
+        raise RuntimeError("resid must be bf16 [M,N] with unit column stride")
+    _lib.call("rh3_gemm_w8a8_gated_residual2", xq.data_ptr(), xq.stride(0), wq.data_ptr(), xs.data_ptr(), ws.data_ptr(),
+              gate0.data_ptr(), gate1.data_ptr(), split, resid.data_ptr(), resid.stride(0) if m else n, m, n, k,
+              _lib.KIND_I8, _lib.stream())
+    return resid
+
+
 def swiglu_perm(n2, device):
     """Index tensor [n2] that re-orders the rows of an fc1 weight stored as F gate rows followed by F up rows
     (n2 = 2F, F a multiple of 4) into runs of eight: four gate rows, then the four up rows they multiply. The

@@ -202,10 +202,31 @@ class FusedBlock:
         return gate_tab.to(torch.bfloat16).contiguous()
 
     @staticmethod
+    def _two_gates(segments, s, gate_tab):
+        """(row of the first span, row of the second, first row of the second) when the packed sequence is one or two
+        spans with one gate row of the fp32 table each, which is one GEMM with both gates; None for anything else
+        (per-token rows, gaps, more spans, other tables), which takes a GEMM per span."""
+        spans = [(a, b, r) for a, b, r in segments if b > a]
+        if not 1 <= len(spans) <= 2 or any(torch.is_tensor(r) for _, _, r in spans):
+            return None
+        (a0, b0, r0), (a1, b1, r1) = spans[0], spans[-1]
+        rows = gate_tab.shape[0]
+        if a0 != 0 or b1 != s or (len(spans) == 2 and a1 != b0) or not (0 <= int(r0) < rows and 0 <= int(r1) < rows):
+            return None
+        if gate_tab.dtype != torch.float32 or gate_tab.ndim != 2 or gate_tab.stride(1) != 1 or not gate_tab.is_cuda:
+            return None
+        return int(r0), int(r1), b0
+
+    @staticmethod
     def _gemm_gated(xq, xs, q, x, gates, segments):
-        """x += gate * (xq @ W^T), one GEMM per modality segment, each with its own gate row of `gates` [R, d] bf16;
-        a segment whose row is a per-token tensor is split into runs of equal rows."""
+        """x += bf16(gate) * (xq @ W^T) with the gate row of `gates` [R, d] that each modality segment names: one GEMM
+        when there are one or two plain segments, else one per segment; a segment whose row is a per-token tensor is
+        split into runs of equal rows."""
         qw = q.qweight_for()
+        two = FusedBlock._two_gates(segments, x.shape[0], gates)
+        if two is not None:
+            return cf.int8_gemm_gated_residual2(xq, xs, qw.q, qw.scale, gates[two[0]], gates[two[1]], two[2], x)
+        gates = FusedBlock._gate_rows(gates)
         for a, b, row in segments:
             if b <= a:
                 continue
@@ -234,7 +255,6 @@ class FusedBlock:
             shift_msa, scale_msa, gate_msa, shift_mlp, scale_mlp, gate_mlp = blk.adaln_proj(t_emb)
             idx = _row_index(mod_segments, s, x.device)
             tab = rope_freqs.reshape(s, 48, 2, 2).contiguous()
-            gates_msa, gates_mlp = self._gate_rows(gate_msa), self._gate_rows(gate_mlp)
         rot = self.rotate
         qbytes = lambda k: s * k * 3 + 4 * s  # noqa: E731  (row quantizer: 2 bytes in, 1 out per element, a scale per row)
 
@@ -291,14 +311,17 @@ class FusedBlock:
                     oq, os_ = tq.quant_groups_i8(o, rotate=rot)
         del qkv, q, k, v
         with _phase("gemm_out_proj", 2 * s * d * hd):
-            x = self._gemm_gated(oq, os_, self.out_q, x, gates_msa, mod_segments)
+            x = self._gemm_gated(oq, os_, self.out_q, x, gate_msa, mod_segments)
         rec("x_attn", x)
 
         # ---- cross-attention to text ----
         if self.cq_q is not None:
             c = blk.cross
             zeros, ones = self._zeros_tab(d, x.device)
-            idx0 = self._const.setdefault(("idx0", s, str(x.device)), torch.zeros(s, dtype=torch.int32, device=x.device))
+            key0 = ("idx0", s, str(x.device))
+            idx0 = self._const.get(key0)
+            if idx0 is None:
+                idx0 = self._const.setdefault(key0, torch.zeros(s, dtype=torch.int32, device=x.device))
             with _phase("quant_norm_mod", qbytes(d)):
                 xq, xs = tq.norm_mod_rot_quant_rows_i8(x, self._norm_w(blk.norm_c), self._eps(blk.norm_c), idx0, zeros, zeros, rotate=rot)
             rec("cross_in_q", xq), rec("cross_in_s", xs)
@@ -337,7 +360,7 @@ class FusedBlock:
         rec("fc2_in_q", hq), rec("fc2_in_s", hs)
         del h
         with _phase("gemm_fc2", 2 * s * d * f):
-            out = self._gemm_gated(hq, hs, self.fc2_q, x, gates_mlp, mod_segments)
+            out = self._gemm_gated(hq, hs, self.fc2_q, x, gate_mlp, mod_segments)
         rec("x_out", out)
         return out
 

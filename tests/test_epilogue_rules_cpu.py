@@ -1,4 +1,4 @@
-"""Which biases a quantized linear may leave to the GEMM's epilogue, and which must stay an operation of torch's own."""
+"""Which biases and gates a GEMM's epilogue takes over, and which stay with the general path."""
 import torch
 
 from rapid_h3_b200 import nodes
@@ -25,3 +25,20 @@ def test_only_inert_plain_tensors_go_to_the_epilogue():
         pass
 
     assert not nodes._plain_bias(b.as_subclass(Sub), 8, cpu)
+
+
+def test_two_gates_takes_one_or_two_plain_spans_only():
+    two, tab = nodes.FusedBlock._two_gates, torch.zeros(2, 8)
+
+    class OnGpu(torch.Tensor):  # the rule asks for a device tensor; nothing is computed here
+        is_cuda = True
+
+    gpu = tab.as_subclass(OnGpu)
+    assert two([(0, 10, 0)], 10, gpu) == (0, 0, 10)
+    assert two([(0, 7, 1), (7, 10, 0)], 10, gpu) == (1, 0, 7)
+    assert two([(0, 7, 1), (7, 7, 0), (7, 10, 0)], 10, gpu) == (1, 0, 7)   # an empty span
+    for segs in ([], [(0, 7, 0)], [(1, 10, 0)], [(0, 6, 0), (7, 10, 1)], [(7, 10, 1), (0, 7, 0)], [(0, 3, 0), (3, 6, 1), (6, 10, 0)],
+                 [(0, 10, torch.zeros(10))], [(0, 10, 2)], [(0, 10, -1)]):
+        assert two(segs, 10, gpu) is None
+    assert two([(0, 10, 0)], 10, tab) is None and two([(0, 10, 0)], 10, gpu.to(torch.bfloat16)) is None
+    assert two([(0, 10, 0)], 10, torch.zeros(8, 2).t().as_subclass(OnGpu)) is None

@@ -261,3 +261,23 @@ def test_epilogue_column_split(ops, m, n):
         gu = y.to(torch.bfloat16).float().view(m, n // 8, 2, 4)
         ref = (gu[:, :, 0] / (1 + torch.exp(-gu[:, :, 0])) * gu[:, :, 1]).reshape(m, n // 2)
         assert rel_l2(h.cpu(), ref) <= 3e-3  # bf16 rounding, 2^-9 at worst
+
+
+@pytest.mark.parametrize("m,split", [(5, 0), (5, 2), (5, 5), (128, 100), (300, 255), (300, 256), (515, 400)])
+@pytest.mark.parametrize("n", [136, 512])
+def test_gated_residual_with_two_gates(ops, m, split, n):
+    """One launch over both modalities against one per modality with the bf16 gate rows: the same bits."""
+    gemm, kernels, lib = ops
+    k = 384
+    xq, wq, xs, ws = _rand_codes(m, n, k, seed=m + split)
+    dev = [t.cuda() for t in (xq, xs, wq, ws)]
+    g = inputs.gen(m + n)
+    gates = torch.randn(3, n, generator=g).cuda()
+    res = torch.randn(m, n, generator=g).to(torch.bfloat16).cuda()
+    want = res.clone()
+    for a, b, row in ((0, split, 2), (split, m, 0)):
+        if b > a:
+            gemm.int8_gemm_gated_residual(dev[0][a:b], dev[1][a:b], dev[2], dev[3], gates[row].to(torch.bfloat16), want[a:b])
+    got = gemm.int8_gemm_gated_residual2(*dev, gates[2], gates[0], split, res)
+    lib.check_status()
+    assert torch.equal(got, want)
