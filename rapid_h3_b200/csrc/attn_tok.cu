@@ -25,8 +25,15 @@
 // key scales / biases per step, 3-stage ring), warp 1 = MMA issuer, warps 4..11 = softmax, one query row per
 // thread with its 128 fp32 output values in registers (232 registers per softmax thread after the register
 // re-split). The scores are read from TMEM twice, 16 columns at a time (maximum, then exponentials), so that the
-// output row fits beside them. TMEM (512 columns): S0 | S1 | A0 | A1.
+// output row fits beside them. P has two buffers, so the exponentials of a tile do not wait for the previous tile's
+// P.V: its fold comes after them. TMEM (512 columns): S0 | S1 | A0 | A1.
+// What bounds it: issue slots and the serial chain of a softmax thread at two warps per scheduler. H = 32: 13.4 ms at
+// L = 22,332 and 0.614 ms at L = 4,500 with a test for the last tile's biases at every four scores and the fold ahead of
+// the exponentials; 11.6 and 0.523 with the test once per pass, the three-input maximum and the two P buffers. Rolled
+// passes (a quarter of the code) are slower: 11.8 with one, 12.2-12.4 with both.
 #include <limits.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "rapidh3_b200.h"
@@ -63,7 +70,7 @@ struct __align__(8) TokSmemTail {
   int abort_flag;
 };
 
-constexpr int TOK_SMEM_BYTES = 2 * QG * TILE_BYTES + KV_STAGES * STAGE_BYTES + sizeof(TokSmemTail) + 1024;
+constexpr int TOK_SMEM_BYTES = 3 * QG * TILE_BYTES + KV_STAGES * STAGE_BYTES + sizeof(TokSmemTail) + 1024;
 
 constexpr float kMagic = 12582912.f;          // 1.5 * 2^23
 constexpr uint32_t kMagicBits = 0x4B400000u;
@@ -119,15 +126,15 @@ static_assert(128 * REGS_SERVICE + 256 * REGS_SOFTMAX == TOK_THREADS * REGS_COMP
 __device__ __forceinline__ void reg_release_service() { asm volatile("setmaxnreg.dec.sync.aligned.u32 40;"); }
 __device__ __forceinline__ void reg_take_softmax() { asm volatile("setmaxnreg.inc.sync.aligned.u32 232;"); }
 
-// t = x * kscale for four columns; on the last key tile (`bias`, uniform over the CTA) the bias is added, which is 0
+// t = x * kscale for four columns; on the last key tile (BIAS: chosen once per pass) the bias is added, which is 0
 // for real keys and -inf for the padding keys. rn(x * s) + 0 is the same number as fma(x, s, 0).
-__device__ __forceinline__ void scores4(const uint32_t* r, uint32_t ks_addr, uint32_t kb_addr, bool bias, uint64_t& t01,
-                                        uint64_t& t23) {
+template <bool BIAS>
+__device__ __forceinline__ void scores4(const uint32_t* r, uint32_t ks_addr, uint32_t kb_addr, uint64_t& t01, uint64_t& t23) {
   uint64_t s01, s23;
   lds4x2(ks_addr, s01, s23);
   t01 = mul2(unbias2(r[0], r[1]), s01);
   t23 = mul2(unbias2(r[2], r[3]), s23);
-  if (bias) {
+  if (BIAS) {
     uint64_t b01, b23;
     lds4x2(kb_addr, b01, b23);
     t01 = add2(t01, b01);
@@ -135,30 +142,40 @@ __device__ __forceinline__ void scores4(const uint32_t* r, uint32_t ks_addr, uin
   }
 }
 
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
 // Maximum over one 16-column chunk of t.
-__device__ __forceinline__ float chunk_tmax(const uint32_t* r, uint32_t ks_addr, uint32_t kb_addr, bool bias, float tm) {
+template <bool BIAS>
+__device__ __forceinline__ float chunk_tmax(const uint32_t* r, uint32_t ks_addr, uint32_t kb_addr, float tm) {
+  float tn = -INFINITY;  // a second chain
 #pragma unroll
   for (int i = 0; i < 16; i += 4) {
     uint64_t t01, t23;
-    scores4(r + i, ks_addr + i * 4, kb_addr + i * 4, bias, t01, t23);
+    scores4<BIAS>(r + i, ks_addr + i * 4, kb_addr + i * 4, t01, t23);
     float t0, t1, t2, t3;
     unpack2(t01, t0, t1);
     unpack2(t23, t2, t3);
-    tm = fmaxf(fmaxf(tm, fmaxf(t0, t1)), fmaxf(t2, t3));
+    tm = max3(tm, t0, t1);
+    tn = max3(tn, t2, t3);
   }
-  return tm;
+  return fmaxf(tm, tn);
 }
 
 // One 16-column chunk: P = u8(rint(2^(t * c + off))) written to 16-byte chunk k of the row of P in shared memory
 // (XOR-swizzled like the TMA tiles), the integer codes added to `rs`.
-__device__ __forceinline__ void chunk_p(const uint32_t* r, uint32_t ks_addr, uint32_t kb_addr, bool bias, float c, float off,
-                                        int k, uint8_t* p_row, int sw, uint32_t& rs) {
+template <bool BIAS>
+__device__ __forceinline__ void chunk_p(const uint32_t* r, uint32_t ks_addr, uint32_t kb_addr, float c, float off, int k,
+                                        uint8_t* p_row, int sw, uint32_t& rs) {
   const uint64_t c2 = pack2(c, c), off2 = pack2(off, off), magic2 = pack2(kMagic, kMagic);
   uint32_t w[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     uint64_t t01, t23;
-    scores4(r + 4 * i, ks_addr + i * 16, kb_addr + i * 16, bias, t01, t23);
+    scores4<BIAS>(r + 4 * i, ks_addr + i * 16, kb_addr + i * 16, t01, t23);
     float e0, e1, e2, e3;
     unpack2(fma2(t01, c2, off2), e0, e1);
     unpack2(fma2(t23, c2, off2), e2, e3);
@@ -178,8 +195,8 @@ attn_tok_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;
-  uint8_t* sP = smem + QG * TILE_BYTES;
-  uint8_t* sKV = smem + 2 * QG * TILE_BYTES;  // stage s at +s*STAGE_BYTES: K, V^T, scales + biases
+  uint8_t* sP = smem + QG * TILE_BYTES;       // [QG][2] tiles
+  uint8_t* sKV = smem + 3 * QG * TILE_BYTES;  // stage s at +s*STAGE_BYTES: K, V^T, scales + biases
   TokSmemTail* tail = reinterpret_cast<TokSmemTail*>(sKV + KV_STAGES * STAGE_BYTES);
   volatile int* abort_flag = &tail->abort_flag;
 
@@ -275,11 +292,11 @@ attn_tok_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
         const int stage = j % KV_STAGES;
         const uint32_t v_addr = smem_u32(sKV + stage * STAGE_BYTES + TILE_BYTES);
         for (int g = 0; g < QG && ok; ++g) {
-          // P of tile j is in shared memory, and the same threads have folded the accumulator of tile j-1 before
+          // P of tile j is in shared memory, and the same threads have folded the accumulator of tile j-1
           ok = all_ok(mbar_wait_relaxed(&tail->p_full[g], j & 1, abort_flag, p.status, ST_TIMEOUT_P_READY, 64));
           if (!ok) break;
           tc_fence_after();
-          const uint32_t p_addr = smem_u32(sP + g * TILE_BYTES);
+          const uint32_t p_addr = smem_u32(sP + (2 * g + (j & 1)) * TILE_BYTES);
           if (elect_one()) {
             mma4_i8_ss(tmem_base + 256 + g * 128, make_desc_k128(p_addr), make_desc_k128(v_addr), idesc_pv, 1);  // onto the bias
             mma_commit(&tail->pv_done[g]);
@@ -303,7 +320,7 @@ attn_tok_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
     const uint32_t a_row = tmem_base + 256 + g * 128 + lane_off;
     const int64_t q_row = static_cast<int64_t>(q_pair) * (QG * BQ) + g * BQ + row;
     const float c_row = __fmul_rn(p.qs[static_cast<int64_t>(h) * p.Lq_pad + q_row], p.sl2);
-    uint8_t* p_row = sP + g * TILE_BYTES + row * 128;
+    uint8_t* p_row0 = sP + 2 * g * TILE_BYTES + row * 128;
     const int sw = row & 7;
     uint64_t* s_full = &tail->s_full[g];
     uint64_t* s_empty = &tail->s_empty[g];
@@ -342,6 +359,33 @@ attn_tok_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       }
     };
 
+    // two register sets: the load of the next 16 columns is in flight while these are worked on
+    auto pass1 = [&](auto bias, uint32_t ks_addr, uint32_t kb_addr) {
+      constexpr bool BIAS = decltype(bias)::value;
+      float tm = -INFINITY;
+      uint32_t ra[16], rb[16];
+      tmem_ld16_async(t_row, ra);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        uint32_t* r = (c & 1) ? rb : ra;
+        tmem_ld_wait16(r);
+        if (c + 1 < 8) tmem_ld16_async(t_row + (c + 1) * 16, (c & 1) ? ra : rb);
+        tm = chunk_tmax<BIAS>(r, ks_addr + c * 64, kb_addr + c * 64, tm);
+      }
+      return tm;
+    };
+    auto pass2 = [&](auto bias, uint32_t ks_addr, uint32_t kb_addr, float off, uint8_t* p_row, uint32_t& rs) {
+      constexpr bool BIAS = decltype(bias)::value;
+      uint32_t ra[16], rb[16];
+      tmem_ld16_async(t_row, ra);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        uint32_t* r = (c & 1) ? rb : ra;
+        tmem_ld_wait16(r);
+        if (c + 1 < 8) tmem_ld16_async(t_row + (c + 1) * 16, (c & 1) ? ra : rb);
+        chunk_p<BIAS>(r, ks_addr + c * 64, kb_addr + c * 64, c_row, off, c, p_row, sw, rs);
+      }
+    };
     // bias both accumulators of this query tile for key tile 0
     splat4(t_row);
     splat4(a_row);
@@ -359,46 +403,28 @@ attn_tok_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       if (!mbar_wait_relaxed(s_full, j & 1, abort_flag, p.status, ST_TIMEOUT_ACC_FULL, 32)) { ok = false; break; }
       tc_fence_after();
       // ---- pass 1: the tile's row maximum ----
-      float tm = -INFINITY;
-      {
-        uint32_t ra[16], rb[16];
-        tmem_ld16_async(t_row, ra);
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          uint32_t* r = (c & 1) ? rb : ra;
-          tmem_ld_wait16(r);
-          if (c + 1 < 8) tmem_ld16_async(t_row + (c + 1) * 16, (c & 1) ? ra : rb);
-          tm = chunk_tmax(r, ks_addr + c * 64, kb_addr + c * 64, last, tm);
-        }
-      }
+      const float tm = last ? pass1(std::true_type{}, ks_addr, kb_addr) : pass1(std::false_type{}, ks_addr, kb_addr);
       const float tmc = __fmul_rn(tm, c_row);
       const float m_new = fmaxf(m, tmc);
       const float a = ex2_approx(__fsub_rn(m, m_new)), ts = ex2_approx(__fsub_rn(tmc, m_new));
       const float off = __fsub_rn(kLog2_255, tmc);
       m = m_new;
+      // ---- pass 2: P into shared memory, integer row sum ----
+      // (this buffer was last read by P.V of tile j - 2, whose fold in the previous round waited for it)
+      uint8_t* p_row = p_row0 + (j & 1) * TILE_BYTES;
+      uint32_t rs = 0;
+      if (last) pass2(std::true_type{}, ks_addr, kb_addr, off, p_row, rs);
+      else pass2(std::false_type{}, ks_addr, kb_addr, off, p_row, rs);
+      // the scores have been read for the last time: bias the accumulator for the next Q.K^T and hand it back
+      splat4(t_row);
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(s_empty);
       if (j > 0) {
-        // P.V of the previous tile has finished: fold its accumulator; the P buffer is free again
+        // P.V of the previous tile has finished: fold its accumulator
         if (!mbar_wait_relaxed(pv_done, (j - 1) & 1, abort_flag, p.status, ST_TIMEOUT_PV_DONE, 32)) { ok = false; break; }
         fold(a_prev, ts_prev, true);
-      }
-      // ---- pass 2: P into shared memory, integer row sum ----
-      uint32_t rs = 0;
-      uint32_t ra[16], rb[16];
-      tmem_ld16_async(t_row, ra);
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        uint32_t* r = (c & 1) ? rb : ra;
-        tmem_ld_wait16(r);
-        if (c + 1 < 8) tmem_ld16_async(t_row + (c + 1) * 16, (c & 1) ? ra : rb);
-        if (c == 7) {
-          // the scores have been read for the last time: bias the accumulator for the next Q.K^T and hand it back
-          splat4(t_row);
-          tmem_st_wait();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(s_empty);
-        }
-        chunk_p(r, ks_addr + c * 64, kb_addr + c * 64, last, c_row, off, c, p_row, sw, rs);
       }
       l = fmaf(ts, static_cast<float>(rs), __fmul_rn(l, a));
       a_prev = a;
