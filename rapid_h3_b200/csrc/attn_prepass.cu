@@ -51,9 +51,6 @@ __device__ __forceinline__ void unpack8(const uint4 raw, float* x) {
   x[0] = bf16_lo(raw.x); x[1] = bf16_hi(raw.x); x[2] = bf16_lo(raw.y); x[3] = bf16_hi(raw.y);
   x[4] = bf16_lo(raw.z); x[5] = bf16_hi(raw.z); x[6] = bf16_lo(raw.w); x[7] = bf16_hi(raw.w);
 }
-__device__ __forceinline__ uint4 pack8(const float* x) {
-  return make_uint4(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]), pack_bf16x2(x[6], x[7]));
-}
 __device__ __forceinline__ uint4 load_row16(const __nv_bfloat16* row, int l16) {
   return __ldg(reinterpret_cast<const uint4*>(row + l16 * 8));
 }
@@ -69,53 +66,89 @@ __device__ __forceinline__ float half_warp_max(float v) {
   return v;
 }
 
-// What a lane needs of the norm weight and of one token's rope table row.
+// A row of 128 channels is shared by LANES lanes (16, or 8 in the per-token quantizer), 128 / LANES consecutive channels
+// each. These kernels are bound by their arithmetic, above all by what is done once per row (square root, reciprocals,
+// reductions): every lane of a row repeats it, so eight lanes per row halve it; where a lane also carries per-channel
+// statistics of 16 rows, sixteen lanes are what the registers allow.
+//
+// What a lane needs of the norm weight and of one token's rope table row: per channel the two factors (of the channel
+// itself, of its partner in the rotary pair) as a bf16 pair.
+template <int CH>
 struct NormRope {
-  float w[8];        // norm weight of this lane's channels
-  uint32_t t[16];    // rope words of this lane's 8 pairs: t[2j] = (t00, t01), t[2j+1] = (t10, t11) of pair j
+  float w[CH];      // norm weight of this lane's channels
+  uint32_t t[CH];   // low half: factor of the own channel, high half: factor of the partner's
 };
-__device__ __forceinline__ void load_norm_weight(const __nv_bfloat16* __restrict__ w, int l16, NormRope& nr) {
-  unpack8(load_row16(w, l16), nr.w);
-}
-// Lanes 0..5 hold the first halves of the rotary pairs (channels 0..47), lanes 6..11 the second halves (48..95);
-// both read the 64 bytes of the table row that describe their 8 pairs. Lanes 12..15 only normalise.
-__device__ __forceinline__ void load_rope_row(const __nv_bfloat16* __restrict__ tab_row, int l16, NormRope& nr) {
-  if (l16 < 12) {
-    const uint4* p = reinterpret_cast<const uint4*>(tab_row + (l16 < 6 ? l16 : l16 - 6) * 32);
+template <int CH>
+__device__ __forceinline__ void load_norm_weight(const __nv_bfloat16* __restrict__ w, int l, NormRope<CH>& nr) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < CH; i += 8) unpack8(__ldg(reinterpret_cast<const uint4*>(w + l * CH + i)), nr.w + i);
+}
+// Channels 0..47 hold the first halves of the rotary pairs, 48..95 the second halves (channel c pairs with c + 48); the
+// lanes of both halves read the words (t00, t01), (t10, t11) of their pairs and keep (t00, t01) or (t11, t10). Lanes of
+// channels 96..127 only normalise.
+template <int CH>
+__device__ __forceinline__ void load_rope_row(const __nv_bfloat16* __restrict__ tab_row, int l, NormRope<CH>& nr) {
+  constexpr int HALF = 48 / CH;  // lanes per half
+  if (l < 2 * HALF) {
+    const uint4* p = reinterpret_cast<const uint4*>(tab_row + (l < HALF ? l : l - HALF) * CH * 4);
+    const uint32_t pick = l < HALF ? 0x3210u : 0x5476u;  // the first word, or the second one with its halves swapped
+#pragma unroll
+    for (int i = 0; i < CH / 2; ++i) {
       const uint4 q = __ldg(p + i);
-      nr.t[4 * i] = q.x, nr.t[4 * i + 1] = q.y, nr.t[4 * i + 2] = q.z, nr.t[4 * i + 3] = q.w;
+      nr.t[2 * i] = __byte_perm(q.x, q.y, pick);
+      nr.t[2 * i + 1] = __byte_perm(q.z, q.w, pick);
     }
   }
 }
-// RMSNorm (+ RoPE when `rope`) of one row held as 8 floats per lane; the result is the bf16-rounded row, as floats.
-__device__ __forceinline__ void norm_rope_row(float* v, const NormRope& nr, float eps, bool rope, int lane) {
-  const int l16 = lane & 15;
-  float ss = 0.f;
+// Sum over the row of CH values per lane in a fixed order: runs of 8 channels in order, then an xor butterfly
+// (8, 4, 2, 1) over the 16 runs; a lane that holds two neighbouring runs does the last step by itself.
+template <int CH>
+__device__ __forceinline__ float row_sumsq(const float* v) {
+  float ss[CH / 8];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) ss = __fadd_rn(ss, __fmul_rn(v[j], v[j]));
-  ss = half_warp_sum(ss);
-  const float r = __fdiv_rn(1.f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, 128.f), eps)));
+  for (int r = 0; r < CH / 8; ++r) {
+    ss[r] = 0.f;
 #pragma unroll
-  for (int j = 0; j < 8; ++j) v[j] = bf16_round(__fmul_rn(__fmul_rn(r, v[j]), nr.w[j]));
+    for (int j = 0; j < 8; ++j) ss[r] = __fadd_rn(ss[r], __fmul_rn(v[8 * r + j], v[8 * r + j]));
+  }
+#pragma unroll
+  for (int o = 64 / CH; o; o >>= 1)
+#pragma unroll
+    for (int r = 0; r < CH / 8; ++r) ss[r] = __fadd_rn(ss[r], __shfl_xor_sync(0xffffffffu, ss[r], o));
+  return CH == 8 ? ss[0] : __fadd_rn(ss[0], ss[CH / 8 - 1]);
+}
+// RMSNorm (+ RoPE when `rope`) of one row held as CH floats per lane; the result is the bf16-rounded row, as floats in v
+// and packed in `out` (two channels per word). The rounded values travel between lanes two to a shuffle.
+template <int CH>
+__device__ __forceinline__ void norm_rope_row(float* v, const NormRope<CH>& nr, float eps, bool rope, int lane, uint32_t* out) {
+  static_assert(CH == 8 || CH == 16, "a row is shared by 16 or 8 lanes");
+  constexpr int HALF = 48 / CH, LANES = 128 / CH;
+  const int l = lane & (LANES - 1);
+  // dividing by 128 is the exact product with 2^-7
+  const float r = __fdiv_rn(1.f, __fsqrt_rn(__fadd_rn(__fmul_rn(row_sumsq<CH>(v), 0.0078125f), eps)));
+#pragma unroll
+  for (int j = 0; j < CH / 2; ++j)
+    out[j] = pack_bf16x2(__fmul_rn(__fmul_rn(r, v[2 * j]), nr.w[2 * j]), __fmul_rn(__fmul_rn(r, v[2 * j + 1]), nr.w[2 * j + 1]));
   if (rope) {
-    // the other half of every pair lives 6 lanes away (48 channels) in the same half-warp
-    const int partner = (lane & 16) | (l16 < 6 ? l16 + 6 : (l16 < 12 ? l16 - 6 : l16));
-    float other[8];
+    // the other half of every pair lives HALF lanes away (48 channels) in the same row
+    const int partner = (lane & ~(LANES - 1)) | (l < HALF ? l + HALF : (l < 2 * HALF ? l - HALF : l));
+    uint32_t other[CH / 2];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) other[j] = __shfl_sync(0xffffffffu, v[j], partner);
-    if (l16 < 12) {
-      const bool first = l16 < 6;
+    for (int j = 0; j < CH / 2; ++j) other[j] = __shfl_sync(0xffffffffu, out[j], partner);
+    if (l < 2 * HALF) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const uint32_t tw = first ? nr.t[2 * j] : nr.t[2 * j + 1];
-        const float a = first ? v[j] : other[j], b = first ? other[j] : v[j];
-        v[j] = bf16_round(__fadd_rn(__fmul_rn(a, bf16_lo(tw)), __fmul_rn(b, bf16_hi(tw))));
+      for (int j = 0; j < CH / 2; ++j) {
+        const uint32_t t0 = nr.t[2 * j], t1 = nr.t[2 * j + 1];
+        const float a = __fadd_rn(__fmul_rn(bf16_lo(out[j]), bf16_lo(t0)), __fmul_rn(bf16_lo(other[j]), bf16_hi(t0)));
+        const float b = __fadd_rn(__fmul_rn(bf16_hi(out[j]), bf16_lo(t1)), __fmul_rn(bf16_hi(other[j]), bf16_hi(t1)));
+        out[j] = pack_bf16x2(a, b);
       }
     }
   }
+#pragma unroll
+  for (int j = 0; j < CH / 2; ++j) v[2 * j] = bf16_lo(out[j]), v[2 * j + 1] = bf16_hi(out[j]);
 }
+__device__ __forceinline__ uint4 words4(const uint32_t* w) { return make_uint4(w[0], w[1], w[2], w[3]); }
 
 // ---------------------------------------------------------------------------------------------
 // RMSNorm + RoPE alone: a half-warp per (token, head) row
@@ -129,13 +162,14 @@ __global__ void __launch_bounds__(256) rmsnorm_rope_kernel(const __nv_bfloat16* 
   const bool live = row < S * H;
   const int64_t s = live ? row / H : 0;
   const int h = live ? static_cast<int>(row - s * H) : 0;
-  NormRope nr;
+  NormRope<8> nr;
   load_norm_weight(w, l16, nr);
   if (tab) load_rope_row(tab + s * 48 * 4, l16, nr);
   float v[8];
+  uint32_t o[4];
   unpack8(load_row16(x + s * x_ss + h * x_sh, l16), v);
-  norm_rope_row(v, nr, eps, tab != nullptr, lane);   // both half-warps take part in the shuffles
-  if (live) *reinterpret_cast<uint4*>(y + s * y_ss + h * y_sh + l16 * 8) = pack8(v);
+  norm_rope_row(v, nr, eps, tab != nullptr, lane, o);   // both half-warps take part in the shuffles
+  if (live) *reinterpret_cast<uint4*>(y + s * y_ss + h * y_sh + l16 * 8) = words4(o);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -162,26 +196,27 @@ __global__ void __launch_bounds__(256) rope_scatter_kernel(const __nv_bfloat16* 
   const int h = live ? static_cast<int>(id - s * H) : 0;
   const int64_t hd = static_cast<int64_t>(H) * D;
   const __nv_bfloat16* row = qkv + s * ld + h * D;
-  NormRope nq, nk;
+  NormRope<8> nq, nk;
   load_norm_weight(qw, l16, nq);
   load_norm_weight(kw, l16, nk);
   if (tab) {
     load_rope_row(tab + s * 48 * 4, l16, nq);   // q and k of a token share its rope words
 #pragma unroll
-    for (int i = 0; i < 16; ++i) nk.t[i] = nq.t[i];
+    for (int i = 0; i < 8; ++i) nk.t[i] = nq.t[i];
   }
   float q[8], k[8];
   unpack8(load_row16(row, l16), q);
   unpack8(load_row16(row + hd, l16), k);
   const uint4 v = load_row16(row + 2 * hd, l16);
-  norm_rope_row(q, nq, eps, tab != nullptr, lane);
-  norm_rope_row(k, nk, eps, tab != nullptr, lane);
+  uint32_t qo[4], ko[4];
+  norm_rope_row(q, nq, eps, tab != nullptr, lane, qo);
+  norm_rope_row(k, nk, eps, tab != nullptr, lane, ko);
   if (live) {
     const int r = h / heads_per_rank, hh = h - r * heads_per_rank;
     const int64_t w = static_cast<int64_t>(heads_per_rank) * D;
     __nv_bfloat16* out = dst.ptr[r] + (row0 + s) * 3 * w + hh * D + l16 * 8;
-    *reinterpret_cast<uint4*>(out) = pack8(q);
-    *reinterpret_cast<uint4*>(out + w) = pack8(k);
+    *reinterpret_cast<uint4*>(out) = words4(qo);
+    *reinterpret_cast<uint4*>(out + w) = words4(ko);
     *reinterpret_cast<uint4*>(out + 2 * w) = v;
   }
 }
@@ -220,7 +255,7 @@ __global__ void __launch_bounds__(256, 2) rope_stats_kernel(const RopeStatsParam
   const bool q_side = static_cast<int>(blockIdx.x) < p.q_ctas;
   const int idx = q_side ? blockIdx.x : blockIdx.x - p.q_ctas;
   const int chunk = idx / p.H, h = idx - chunk * p.H;
-  NormRope nr;
+  NormRope<8> nr;
 
   if (q_side) {
     // ---- Q: (norm + rope) -> rows kept as packed bf16 -> block-64 abs-max -> int8 codes ----
@@ -241,9 +276,10 @@ __global__ void __launch_bounds__(256, 2) rope_stats_kernel(const RopeStatsParam
       unpack8(kept[i], v);
       if (p.q_w) {
         if (p.tab) load_rope_row(p.tab + (live ? s : 0) * 48 * 4, l16, nr);
-        norm_rope_row(v, nr, p.eps, p.tab != nullptr, lane);
-        if (p.q_out && live) *reinterpret_cast<uint4*>(p.q_out + s * p.qo_ss + h * p.qo_sh + l16 * 8) = pack8(v);
-        kept[i] = pack8(v);
+        uint32_t o[4];
+        norm_rope_row(v, nr, p.eps, p.tab != nullptr, lane, o);
+        kept[i] = words4(o);
+        if (p.q_out && live) *reinterpret_cast<uint4*>(p.q_out + s * p.qo_ss + h * p.qo_sh + l16 * 8) = kept[i];
       }
       if (live) {
 #pragma unroll
@@ -295,8 +331,9 @@ __global__ void __launch_bounds__(256, 2) rope_stats_kernel(const RopeStatsParam
       unpack8(vraw[u], vv);
       if (p.k_w) {
         if (p.tab) load_rope_row(p.tab + (live ? s : 0) * 48 * 4, l16, nr);
-        norm_rope_row(kv, nr, p.eps, p.tab != nullptr, lane);
-        if (live) *reinterpret_cast<uint4*>(p.k_out + s * p.ko_ss + h * p.ko_sh + l16 * 8) = pack8(kv);
+        uint32_t o[4];
+        norm_rope_row(kv, nr, p.eps, p.tab != nullptr, lane, o);
+        if (live) *reinterpret_cast<uint4*>(p.k_out + s * p.ko_ss + h * p.ko_sh + l16 * 8) = words4(o);
       }
       if (live) {
 #pragma unroll
@@ -480,11 +517,12 @@ __global__ void __launch_bounds__(256, 3) quant_kv_kernel(const __nv_bfloat16* _
 // Reference: the per-token Q/K quantizer with `hadamard128` of custom_nodes/rapid_h3/csrc/README.md ("Q, K -> int8,
 // per token"), kernels attn_int8.cu:130-170.
 // ---------------------------------------------------------------------------------------------
+// (16 channels per lane, 8 lanes per row: strides 1, 2, 4, 8 inside the lane, 16, 32, 64 across lanes)
 __device__ __forceinline__ void hadamard128(float* v, int lane) {
 #pragma unroll
-  for (int d = 1; d < 8; d <<= 1) {
+  for (int d = 1; d < 16; d <<= 1) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < 16; ++j) {
       if ((j & d) == 0) {
         const float a = v[j], b = v[j + d];
         v[j] = __fadd_rn(a, b);
@@ -493,16 +531,19 @@ __device__ __forceinline__ void hadamard128(float* v, int lane) {
     }
   }
 #pragma unroll
-  for (int o = 1; o < 16; o <<= 1) {
-    const bool upper = (lane & o) != 0;
+  for (int o = 1; o < 8; o <<= 1) {
+    const float sign = (lane & o) != 0 ? -1.f : 1.f;  // the upper lane of a pair takes other - own, the lower own + other
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float other = __shfl_xor_sync(0xffffffffu, v[j], o);
-      v[j] = upper ? __fsub_rn(other, v[j]) : __fadd_rn(v[j], other);
-    }
+    for (int j = 0; j < 16; ++j) v[j] = fmaf(v[j], sign, __shfl_xor_sync(0xffffffffu, v[j], o));
   }
 }
 
+constexpr int TOK_ROWS = 32;  // rows of a 256-thread CTA, eight lanes each
+
+// Eight lanes per row, 16 channels each. With sixteen lanes per row (and 64-bit index divisions) this took, with the norm
+// and the rotation, 70 us for the Q rows of 6,196 tokens x 32 heads and 47 us for their K rows without them, now 60 and 40
+// (38 for 55 where Q is normalised but not rotated); 11 us is what their bytes take. A persistent form with the next
+// row's loads in flight measures the same: instruction issue is the bound.
 template <bool IS_K>
 __global__ void __launch_bounds__(256) quant_tok_kernel(const __nv_bfloat16* __restrict__ x, int64_t x_ss, int64_t x_sh,
                                                         int64_t L, int64_t Lpad, int H,
@@ -511,42 +552,65 @@ __global__ void __launch_bounds__(256) quant_tok_kernel(const __nv_bfloat16* __r
                                                         __nv_bfloat16* __restrict__ x_out, int64_t xo_ss, int64_t xo_sh,
                                                         const float* __restrict__ mean, int8_t* __restrict__ q8,
                                                         float* __restrict__ scales) {
-  const int lane = threadIdx.x & 31, l16 = lane & 15;
-  const int64_t row = static_cast<int64_t>(blockIdx.x) * HW_PER_CTA + (threadIdx.x >> 4);
+  const int lane = threadIdx.x & 31, l = lane & 7;
+  const int64_t row = static_cast<int64_t>(blockIdx.x) * TOK_ROWS + (threadIdx.x >> 3);
   const bool in_grid = row < Lpad * H;
-  const int64_t s = in_grid ? row / H : 0;
-  const int h = in_grid ? static_cast<int>(row - s * H) : 0;
+  int64_t s = 0;
+  int h = 0;
+  if (in_grid) {
+    if (Lpad * H <= 0xffffffffll) {
+      const uint32_t si = static_cast<uint32_t>(row) / static_cast<uint32_t>(H);
+      s = si;
+      h = static_cast<int>(static_cast<uint32_t>(row) - si * static_cast<uint32_t>(H));
+    } else {
+      s = row / H;
+      h = static_cast<int>(row - s * H);
+    }
+  }
   const bool live = in_grid && s < L;
-  float v[8];
-  unpack8(load_row16(x + (live ? s : 0) * x_ss + h * x_sh, l16), v);
+  const __nv_bfloat16* src = x + (live ? s : 0) * x_ss + h * x_sh + l * 16;
+  const uint4 r0 = __ldg(reinterpret_cast<const uint4*>(src)), r1 = __ldg(reinterpret_cast<const uint4*>(src + 8));
+  float v[16];
+  unpack8(r0, v);
+  unpack8(r1, v + 8);
   if (!live) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = 0.f;   // padding rows: zero codes and the smallest scale
+    for (int j = 0; j < 16; ++j) v[j] = 0.f;   // padding rows: zero codes and the smallest scale
   }
   if (w) {
-    NormRope nr;
-    load_norm_weight(w, l16, nr);
-    if (tab) load_rope_row(tab + (live ? s : 0) * 48 * 4, l16, nr);
-    norm_rope_row(v, nr, eps, tab != nullptr, lane);
-    if (x_out && live) *reinterpret_cast<uint4*>(x_out + s * xo_ss + h * xo_sh + l16 * 8) = pack8(v);
+    NormRope<16> nr;
+    uint32_t o[8];
+    load_norm_weight(w, l, nr);
+    if (tab) load_rope_row(tab + (live ? s : 0) * 48 * 4, l, nr);
+    norm_rope_row(v, nr, eps, tab != nullptr, lane, o);
+    if (x_out && live) {
+      __nv_bfloat16* dst = x_out + s * xo_ss + h * xo_sh + l * 16;
+      *reinterpret_cast<uint4*>(dst) = words4(o);
+      *reinterpret_cast<uint4*>(dst + 8) = words4(o + 4);
+    }
   }
   if (IS_K && mean) {
-    const float4 m0 = *reinterpret_cast<const float4*>(mean + h * D + l16 * 8);
-    const float4 m1 = *reinterpret_cast<const float4*>(mean + h * D + l16 * 8 + 4);
-    const float mm[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = __fsub_rn(v[j], mm[j]);
+    for (int j = 0; j < 16; j += 4) {
+      const float4 m = *reinterpret_cast<const float4*>(mean + h * D + l * 16 + j);
+      v[j] = __fsub_rn(v[j], m.x);
+      v[j + 1] = __fsub_rn(v[j + 1], m.y);
+      v[j + 2] = __fsub_rn(v[j + 2], m.z);
+      v[j + 3] = __fsub_rn(v[j + 3], m.w);
+    }
   }
-  hadamard128(v, lane);   // both half-warps take part in the shuffles
+  hadamard128(v, lane);   // all four rows of the warp take part in the shuffles
   float am = 0.f;
 #pragma unroll
-  for (int j = 0; j < 8; ++j) am = fmaxf(am, fabsf(v[j]));
-  am = half_warp_max(am);
+  for (int j = 0; j < 16; ++j) am = fmaxf(am, fabsf(v[j]));
+#pragma unroll
+  for (int o = 4; o; o >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
   const float scale = __fdiv_rn(fmaxf(am, 1e-8f), 127.f), inv = __fdiv_rn(1.f, scale);
   if (!in_grid) return;
-  *reinterpret_cast<uint2*>(q8 + (static_cast<int64_t>(h) * Lpad + s) * D + l16 * 8) =
-      live ? quant8_i8(v, scale, inv) : make_uint2(0, 0);
-  if (l16 == 0) {
+  uint2 c0 = make_uint2(0, 0), c1 = c0;
+  if (live) c0 = quant8_i8(v, scale, inv), c1 = quant8_i8(v + 8, scale, inv);
+  *reinterpret_cast<uint4*>(q8 + (static_cast<int64_t>(h) * Lpad + s) * D + l * 16) = make_uint4(c0.x, c0.y, c1.x, c1.y);
+  if (l == 0) {
     if (IS_K) {
       float* t = scales + (static_cast<int64_t>(h) * (Lpad / 128) + s / 128) * 256 + (s & 127);
       t[0] = live ? __fmul_rn(scale, 0.0078125f) : 0.f;
@@ -817,8 +881,10 @@ extern "C" int rh3_attn_tok_prepass(const void* q, int64_t q_ss, int64_t q_sh, i
   RH3_CHECK_ARG(scratch_bytes >= rh3_attn_kv_stats_scratch_bytes(Lk, H), "attn_tok_prepass: scratch too small (%lld < %lld)",
                 (long long)scratch_bytes, (long long)rh3_attn_kv_stats_scratch_bytes(Lk, H));
   const int64_t nchunk_k = (Lk + CHUNK - 1) / CHUNK;
-  const int64_t q_ctas = (Lq_pad * H + HW_PER_CTA - 1) / HW_PER_CTA, k_ctas = (Lk_pad * H + HW_PER_CTA - 1) / HW_PER_CTA;
-  RH3_CHECK_ARG(nchunk_k * H < (1ll << 31) && q_ctas < (1ll << 31) && k_ctas < (1ll << 31), "attn_tok_prepass: L x H too large");
+  RH3_CHECK_ARG(nchunk_k * H < (1ll << 31) && (Lq_pad * H + HW_PER_CTA - 1) / HW_PER_CTA < (1ll << 31) &&
+                    (Lk_pad * H + HW_PER_CTA - 1) / HW_PER_CTA < (1ll << 31),
+                "attn_tok_prepass: L x H too large");
+  const int64_t q_ctas = (Lq_pad * H + TOK_ROWS - 1) / TOK_ROWS, k_ctas = (Lk_pad * H + TOK_ROWS - 1) / TOK_ROWS;
   // 1 + 2: K (norm + rope, stored) and V chunk partials -> means and the int8 V scale
   RopeStatsParams p{};
   p.k = static_cast<const __nv_bfloat16*>(k); p.k_ss = k_ss; p.k_sh = k_sh;
