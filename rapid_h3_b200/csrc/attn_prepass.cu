@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(256) rope_scatter_kernel(const __nv_bfloat16* 
 }
 
 // ---------------------------------------------------------------------------------------------
-// Launch 1 of the pre-pass. CTAs [0, q_ctas) quantize Q: one CTA = 128 tokens (two 64-token blocks) of one head, a
+// Launch 1 of the pre-pass. CTAs [kv_ctas, kv_ctas + q_ctas) quantize Q: one CTA = 128 tokens (two 64-token blocks) of one head, a
 // half-warp owns 8 of them, loads all 8 rows before it touches the first and keeps them as packed bf16 until the
 // block maximum is known. The other CTAs prepare K and V: one CTA = one 256-token statistics chunk of one head, a
 // half-warp owns 16 tokens and works through them four at a time (eight 16-byte loads in flight per lane). Heads
@@ -246,14 +246,14 @@ struct RopeStatsParams {
   const __nv_bfloat16* tab;           // rope table [L][48][2][2] or null
   float eps;
   int H;
-  int q_ctas;
+  int q_ctas, kv_ctas;   // the K / V CTAs come first: they take about twice as long as the Q ones
 };
 
 __global__ void __launch_bounds__(256, 2) rope_stats_kernel(const RopeStatsParams p) {
   __shared__ float sh[HW_PER_CTA * 4 * D];  // Q side: 16 block maxima; K/V side: per half-warp partials [hw][4][128]
   const int lane = threadIdx.x & 31, l16 = lane & 15, hw = threadIdx.x >> 4;
-  const bool q_side = static_cast<int>(blockIdx.x) < p.q_ctas;
-  const int idx = q_side ? blockIdx.x : blockIdx.x - p.q_ctas;
+  const bool q_side = static_cast<int>(blockIdx.x) >= p.kv_ctas;
+  const int idx = q_side ? blockIdx.x - p.kv_ctas : blockIdx.x;
   const int chunk = idx / p.H, h = idx - chunk * p.H;
   NormRope<8> nr;
 
@@ -624,7 +624,8 @@ __global__ void __launch_bounds__(256) quant_tok_kernel(const __nv_bfloat16* __r
 bool aligned(const void* p, uintptr_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }
 bool strides16(int64_t a, int64_t b) { return a % 8 == 0 && b % 8 == 0; }  // rows start on 16-byte boundaries
 
-int launch_rope_stats(const RopeStatsParams& p, int kv_ctas, cudaStream_t stream) {
+int launch_rope_stats(RopeStatsParams p, int kv_ctas, cudaStream_t stream) {
+  p.kv_ctas = kv_ctas;
   const int64_t ctas = static_cast<int64_t>(p.q_ctas) + kv_ctas;
   if (ctas == 0) return 0;
   RH3_CHECK_ARG(ctas < (1ll << 31), "attention pre-pass: too many tokens x heads");
