@@ -36,7 +36,7 @@
 //                 columns cost them over 1,000 cycles each time.)
 // What bounds it: the serial chain of a softmax thread's step (wait, TMEM load, re-bias, maximum, exponentials,
 // hand-over) at two such warps per scheduler. Measured with H = 32: 16.8 ms at L = 36,436 and 0.340 ms at
-// L = 4,500 before the P buffers and the rescaling warps, 16.0 and 0.315 with them; timing-only builds without
+// L = 4,500 before the P buffers and the rescaling warps, 16.0 and 0.315 with them (0.306 with the wide epilogue); timing-only builds without
 // any MMA run 15.0 / 0.283, without the exponentials 14.2 / 0.276, with the barriers alone 7.3 / 0.155.
 // TMEM (512 columns): S0 | S1 | O0 | O1, 128 columns each.
 // Tensor-core bound: 4 * Lq * Lk * 128 operations per head.
@@ -63,6 +63,7 @@ struct AttnParams {
   int64_t o_ss, o_sh;
   int Lq, Lk, Lq_pad, Lk_pad, H;
   float sl2;  // softmax_scale * log2(e)
+  int vec_scales;  // vscale and vmean are 16-byte aligned
   int* status;
   // sequence-parallel output: query rows [dst_start[r], dst_start[r+1]) go to dst_ptr[r] (this GPU's or a peer's
   // memory), addressed relative to the start of the range; n_dst == 0 selects the single buffer `out`
@@ -503,20 +504,39 @@ attn_int8_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
         while (r + 1 < p.n_dst && q_row >= p.dst_start[r + 1]) ++r;
         o = p.dst_ptr[r] + (q_row - p.dst_start[r]) * p.o_ss + static_cast<int64_t>(h) * p.o_sh;
       }
+      // 32 channels per TMEM round trip; a head's 128 scales and means are the same for every row (vector loads where
+      // the caller's arrays are aligned for them, L1). Eight channels at a time with scalar loads and 16-byte stores cost
+      // a cross-attention CTA as much as one of its four key tiles: 36,436 x 512 keys 0.547 ms then, 0.474 now.
+      auto load4 = [&](const float* q) {
+        return p.vec_scales ? __ldg(reinterpret_cast<const float4*>(q)) : make_float4(q[0], q[1], q[2], q[3]);
+      };
+      const bool wide = (reinterpret_cast<uintptr_t>(o) & 31) == 0;
 #pragma unroll 1
-      for (int c = 0; c < 16; ++c) {
-        uint32_t r[8];
-        tmem_ld8(o_row + c * 8, r);
+      for (int c = 0; c < 4; ++c) {
+        uint32_t r[32];
+        tmem_ld32(o_row + c * 32, r);
+        tmem_ld_wait_regs(r);
         if (q_row < p.Lq) {
-          uint32_t w[4];
+          uint4 w[4];
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            const int d = c * 8 + 2 * i;
-            const float a = fmaf(__uint_as_float(r[2 * i]) * inv_l, vs[d], vm[d]);
-            const float b = fmaf(__uint_as_float(r[2 * i + 1]) * inv_l, vs[d + 1], vm[d + 1]);
-            w[i] = pack_bf16x2(a, b);
+            uint32_t u[4];
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+              const int e = i * 8 + k * 4;
+              const float4 sc = load4(vs + c * 32 + e), mn = load4(vm + c * 32 + e);
+              u[2 * k] = pack_bf16x2(fmaf(__uint_as_float(r[e]) * inv_l, sc.x, mn.x), fmaf(__uint_as_float(r[e + 1]) * inv_l, sc.y, mn.y));
+              u[2 * k + 1] = pack_bf16x2(fmaf(__uint_as_float(r[e + 2]) * inv_l, sc.z, mn.z), fmaf(__uint_as_float(r[e + 3]) * inv_l, sc.w, mn.w));
+            }
+            w[i] = make_uint4(u[0], u[1], u[2], u[3]);
           }
-          *reinterpret_cast<uint4*>(o + c * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+          if (wide) {
+            st_global_32(o + c * 32, w[0], w[1]);
+            st_global_32(o + c * 32 + 16, w[2], w[3]);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(o + c * 32 + i * 8) = w[i];
+          }
         }
       }
     }
@@ -584,6 +604,7 @@ int attn_launch(const void* q8, const float* qs, const void* k8, const float* ks
                            CU_TENSOR_MAP_SWIZZLE_128B))
     return e;
   p.qs = qs; p.ks = ks; p.vscale = vscale; p.vmean = vmean;
+  p.vec_scales = aligned16(vscale) && aligned16(vmean);
   p.o_ss = o_ss; p.o_sh = o_sh;
   p.Lq = (int)Lq; p.Lk = (int)Lk; p.Lq_pad = (int)Lq_pad; p.Lk_pad = (int)Lk_pad; p.H = (int)H;
   p.sl2 = static_cast<float>(static_cast<double>(softmax_scale) * 1.4426950408889634);
