@@ -198,6 +198,10 @@ class H3Transformer(nn.Module):
         return self.untokens(x, latent.shape)
 
 
+# what the quantized runtime's one-pass final norm stands for: a model whose method is another one is called as it is
+UNTOKENS = H3Transformer.untokens
+
+
 def init_weights(module, seed, device=None):
     """Random init of the benchmark configurations: Linear weights ~ N(0, 0.02), biases ~ N(0, 0.01),
     d-wide norm weights 1 + 0.1 N(0,1), per-head q/k norm weights 1 + 0.3 N(0,1). Generated on CPU so the

@@ -14,9 +14,13 @@ from . import nodes, quantizers
 from .sp import Ulysses, shard_segments
 
 
-def _final_norm(norm, x):
-    """The one-pass kernel for a plain model.RMSNorm on rows it takes, None (the module's own forward) for anything
-    else: another module, hooks, a gradient or tangent that has to pass through, a trace."""
+def _final_norm(m, x):
+    """The one-pass kernel for the final norm of an H3Transformer as model.py writes it, on rows the kernel takes. None
+    for anything else, which goes through `m.untokens(x, latent_shape)`: a model with an `untokens` of its own or
+    without a `final_norm`, another norm module, a gradient or tangent that has to pass through, a trace."""
+    if "untokens" in vars(m) or getattr(type(m), "untokens", None) is not M.UNTOKENS:
+        return None
+    norm = getattr(m, "final_norm", None)
     w = getattr(norm, "weight", None)
     if (type(norm) is not M.RMSNorm or "forward" in vars(norm) or norm._forward_hooks or norm._forward_pre_hooks
             or type(x) is not torch.Tensor or x.ndim != 2 or x.dtype != torch.bfloat16 or not x.is_cuda
@@ -131,7 +135,8 @@ class H3Runtime:
         vids, auds = [], []
         for i in range(b):
             x = xs[i] if sps[i] is None else sps[i].gather_tokens(xs[i])
-            v, a = m.untokens(x, latent.shape[1:], _final_norm(m.final_norm, x))
+            norm = _final_norm(m, x)
+            v, a = m.untokens(x, latent.shape[1:]) if norm is None else m.untokens(x, latent.shape[1:], norm)
             vids.append(v), auds.append(a)
         return torch.stack(vids), torch.stack(auds)
 
