@@ -198,8 +198,8 @@ class H3Transformer(nn.Module):
         return self.untokens(x, latent.shape)
 
 
-# what the quantized runtime's one-pass final norm stands for: a model whose method is another one is called as it is
-UNTOKENS = H3Transformer.untokens
+# what the quantized runtime's one-pass final norm stands for: a model whose methods are other ones is called as it is
+UNTOKENS, RMSNORM_FORWARD = H3Transformer.untokens, RMSNorm.forward
 
 
 def init_weights(module, seed, device=None):

@@ -95,6 +95,24 @@ def test_step_matches_manual_chain_and_bf16_noise_floor(pkg, mode):
     assert err <= 4.0 * floor
 
 
+def test_hooks_on_all_modules_see_the_final_norm(pkg):
+    r = pkg
+    cfg = r.model.H3Config.tiny(n_blocks=1)
+    model = r.model.init_weights(r.model.H3Transformer(cfg), seed=2).cuda()
+    rt = r.step.H3Runtime(model)
+    args = [t.cuda() for t in r.step.make_inputs(cfg, (2, 3, 4), 5, 1, 16, seed=3)]
+    seen = []
+    handle = torch.nn.modules.module.register_module_forward_hook(lambda mod, i, o: seen.append(mod))
+    try:
+        vid, aud = rt.step(*args)
+    finally:
+        handle.remove()
+    assert any(mod is model.final_norm for mod in seen)
+    vid2, aud2 = rt.step(*args)  # the one-pass kernel: bf16 rounding of the same norm
+    r._lib.check_status()
+    assert rel_l2(vid2, vid) <= 1e-2 and rel_l2(aud2, aud) <= 1e-2
+
+
 @pytest.mark.parametrize("mode", ["int8_rowwise", "int8_rot"])
 @pytest.mark.parametrize("attn", ["fast", "token"])
 def test_fused_block_at_the_benchmark_width_matches_oracle(pkg, mode, attn):

@@ -47,3 +47,28 @@ def test_the_models_own_untokens_runs(make):
     for i in range(2):
         v, a = m.untokens(m.tokens(latent[i], audio[i]), latent.shape[1:])
         assert torch.equal(vid[i], v) and torch.equal(aud[i], a)
+
+
+def test_a_norm_somebody_watches_is_called(monkeypatch):
+    """Hooks of the module or on all modules, and a replaced forward or __call__, keep the module's own call."""
+    norm = model.RMSNorm(8, 1e-6)
+    plain = step._plain_final_norm
+    assert plain(norm) and not plain(torch.nn.LayerNorm(8))
+
+    class Sub(model.RMSNorm):
+        pass
+
+    assert not plain(Sub(8, 1e-6))
+    hooks = torch.nn.modules.module
+    for register in (norm.register_forward_hook, norm.register_forward_pre_hook, hooks.register_module_forward_hook,
+                     hooks.register_module_forward_pre_hook, hooks.register_module_full_backward_hook):
+        handle = register(lambda *a: None)
+        assert not plain(norm)
+        handle.remove()
+        assert plain(norm)
+    forward, call = model.RMSNorm.forward, torch.nn.Module.__call__
+    for owner, name, was in ((model.RMSNorm, "forward", forward), (torch.nn.Module, "__call__", call)):
+        with monkeypatch.context() as patch:
+            patch.setattr(owner, name, lambda self, x: was(self, x))
+            assert not plain(norm)
+    assert plain(norm)
