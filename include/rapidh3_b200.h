@@ -121,6 +121,10 @@ int rh3_rms_norm_rows(const void* x, int64_t ldx, const void* w, float eps, int6
  * Replaces te_quant.py:90-105 of the reference (custom_nodes/rapid_h3/te_quant.py). */
 int rh3_te_quant(const float* x, int64_t ldx, int64_t M, int64_t K, float ratio, void* q1, float* s1, void* flags,
                  int32_t* count, int32_t* rows, void* q2, float* s2, void* total, cudaStream_t stream);
+/* The same; *seen (uint64, may be NULL) also grows by M when the kernel runs, so that `total` and `seen` keep step in a graph
+ * that is replayed. */
+int rh3_te_quant_counted(const float* x, int64_t ldx, int64_t M, int64_t K, float ratio, void* q1, float* s1, void* flags,
+                         int32_t* count, int32_t* rows, void* q2, float* s2, void* total, void* seen, cudaStream_t stream);
 /* ---- W8A8 row-wise-scaled GEMMs (tensor-core bound) ---------------------------------------- */
 /* Kernel choice of the GEMM entries below and of rh3_conv3d_causal (no reference counterpart): 0 = one CTA per tile, 1 (the
  * default) = CTA pairs (clusters of two, tcgen05 cta_group::2): 256 x 256 GEMM tiles with each CTA loading its own half of

@@ -39,6 +39,7 @@ SIGNATURES = {
     "rh3_rope_scatter_heads": [_P, _I64, _I64, _I64, _I64, _I64, _P, _P, _F, _P, _P, _P],
     "rh3_rms_norm_rows": [_P, _I64, _P, _F, _I64, _I64, _P, _I64, _P],
     "rh3_te_quant": [_P, _I64, _I64, _I64, _F, _P, _P, _P, _P, _P, _P, _P, _P, _P],
+    "rh3_te_quant_counted": [_P, _I64, _I64, _I64, _F, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P],
     "rh3_te_gemm": [_P, _P, _P, _P, _P, _I64, _I64, _I64, _P, _P, _P, _P, _P, _P, _I64, _P],
     "rh3_attn_int8_scatter": [_P, _P, _P, _P, _P, _P, _P, _I64, _I64, _I64, _I64, _I64, _F, _P, _P, _I64, _I64, _I64, _P],
     "rh3_vae_out_quant": [_P, _I64, _I64, _I64, _I64, _P, _P, _P],

@@ -347,10 +347,12 @@ __global__ void __launch_bounds__(T) te_quant_kernel(const float* __restrict__ x
                                                      int8_t* __restrict__ q1, float* __restrict__ s1,
                                                      uint8_t* __restrict__ flags, int* __restrict__ count,
                                                      int32_t* __restrict__ rows, int8_t* __restrict__ q2,
-                                                     float* __restrict__ s2, unsigned long long* __restrict__ total) {
+                                                     float* __restrict__ s2, unsigned long long* __restrict__ total,
+                                                     unsigned long long* __restrict__ seen) {
   __shared__ float red[T / 32];
   __shared__ int slot_s;
   const int tid = threadIdx.x;
+  if (seen && blockIdx.x == 0 && tid == 0) atomicAdd(seen, static_cast<unsigned long long>(M));
   const int col = tid << 3;
   const bool active = col < K;
   const bool whole = tid - (tid & 31) < (K >> 3);  // K is a multiple of 256: uniform over a warp
@@ -652,27 +654,35 @@ extern "C" int rh3_rms_norm_rows(const void* x, int64_t ldx, const void* w, floa
   return check_cuda(cudaGetLastError(), "rms_norm_rows launch");
 }
 
-extern "C" int rh3_te_quant(const float* x, int64_t ldx, int64_t M, int64_t K, float ratio, void* q1, float* s1, void* flags,
-                            int32_t* count, int32_t* rows, void* q2, float* s2, void* total, cudaStream_t stream) {
+extern "C" int rh3_te_quant_counted(const float* x, int64_t ldx, int64_t M, int64_t K, float ratio, void* q1, float* s1,
+                                    void* flags, int32_t* count, int32_t* rows, void* q2, float* s2, void* total,
+                                    void* seen, cudaStream_t stream) {
   RH3_CHECK_ARG(M >= 0 && M < (1ll << 31) && K > 0 && K % 256 == 0 && K <= 8192,
                 "te_quant: K=%lld must be a multiple of 256, <= 8192", (long long)K);
   RH3_CHECK_ARG(ldx >= K && ldx % 4 == 0, "te_quant: bad row stride");
   if (M == 0) return 0;
   RH3_CHECK_ARG(x && q1 && s1 && flags && count && rows && q2 && s2, "te_quant: null pointer");
   RH3_CHECK_ARG((reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(q1) & 7) == 0 &&
-                    (reinterpret_cast<uintptr_t>(q2) & 7) == 0 && (reinterpret_cast<uintptr_t>(total) & 7) == 0,
-                "te_quant: x must be 16-byte aligned, q1, q2 and total 8-byte aligned");
+                    (reinterpret_cast<uintptr_t>(q2) & 7) == 0 && (reinterpret_cast<uintptr_t>(total) & 7) == 0 &&
+                    (reinterpret_cast<uintptr_t>(seen) & 7) == 0,
+                "te_quant: x must be 16-byte aligned, q1, q2, total and seen 8-byte aligned");
   if (int e = check_cuda(cudaMemsetAsync(count, 0, sizeof(int32_t), stream), "te_quant count")) return e;
   const int64_t threads = K / 8;
   const unsigned grid = static_cast<unsigned>(M < 8 * device_sm_count() ? M : 8 * device_sm_count());
 #define RH3_TE(T_)                                                                                                       \
   te_quant_kernel<T_><<<grid, T_, 0, stream>>>(x, ldx, M, (int)K, ratio, static_cast<int8_t*>(q1), s1,                   \
                                                static_cast<uint8_t*>(flags), count, rows, static_cast<int8_t*>(q2), s2, \
-                                               static_cast<unsigned long long*>(total))
+                                               static_cast<unsigned long long*>(total),                                 \
+                                               static_cast<unsigned long long*>(seen))
   if (threads <= 128) RH3_TE(128);
   else if (threads <= 256) RH3_TE(256);
   else if (threads <= 512) RH3_TE(512);
   else RH3_TE(1024);
 #undef RH3_TE
   return check_cuda(cudaGetLastError(), "te_quant launch");
+}
+
+extern "C" int rh3_te_quant(const float* x, int64_t ldx, int64_t M, int64_t K, float ratio, void* q1, float* s1, void* flags,
+                            int32_t* count, int32_t* rows, void* q2, float* s2, void* total, cudaStream_t stream) {
+  return rh3_te_quant_counted(x, ldx, M, K, ratio, q1, s1, flags, count, rows, q2, s2, total, nullptr, stream);
 }

@@ -12,24 +12,33 @@ import torch
 from . import _lib, gemm, kernels, nodes, quantizers
 
 # how often the second pass ran: [rows that took it, rows seen]; `residual_share()` reads it. The fused route counts its
-# outlier rows on the device (one uint64 per device): the host does not wait for them.
+# outlier rows on the device, where the host need not wait for them: an int64 pair per device, [rows that took the pass,
+# rows seen by graph launches]. A call outside a capture runs once, so its rows are counted as seen here, on the host; a
+# captured call runs whenever its graph is replayed, so there the kernel counts both.
 _ROWS = [0, 0]
-_TAKEN = {}
+_DEVICE_ROWS = {}
 
 
 def residual_share():
-    """Fraction of the rows seen so far that were given the residual pass (0.0 before any call)."""
-    taken = _ROWS[0] + sum(int(t.item()) for t in list(_TAKEN.values()))
-    return taken / _ROWS[1] if _ROWS[1] else 0.0
+    """Fraction of the rows seen so far that were given the residual pass (0.0 before any call). Waits for the devices
+    that ran the fused route, so that calls still queued on any stream are in it."""
+    taken, seen = _ROWS
+    for device, pair in list(_DEVICE_ROWS.items()):
+        torch.cuda.synchronize(device)
+        t, s = pair.tolist()
+        taken, seen = taken + t, seen + s
+    return taken / seen if seen else 0.0
 
 
-def _taken(device):
-    """This device's counter (None while a graph is being captured before it exists: it must not live in the graph's pool)."""
-    t = _TAKEN.get(device)
-    if t is None and not torch.cuda.is_current_stream_capturing():
-        t = _TAKEN.setdefault(device, torch.zeros(1, dtype=torch.int64, device=device))
-        torch.cuda.current_stream(device).synchronize()  # once: its fill is done before any other stream adds to it
-    return t
+def _device_rows(device, capturing):
+    """This device's pair. None in a capture that comes before the first linear of the device was made or called: a
+    tensor made there would belong to the graph's pool, and such a graph's rows are counted nowhere."""
+    pair = _DEVICE_ROWS.get(device)
+    if pair is None and not capturing:
+        pair = torch.zeros(2, dtype=torch.int64, device=device)
+        torch.cuda.current_stream(device).synchronize()  # the zeros are there before another thread or stream can add
+        pair = _DEVICE_ROWS.setdefault(device, pair)
+    return pair
 
 
 def rot_residual_quant_rows_i8(x, q1, s1, rows):
@@ -53,6 +62,8 @@ class _TELinear:
         if mode not in ("int8_rot", "int8_rot_plain"):
             raise NotImplementedError(f"text-encoder mode {mode!r} is not implemented")
         self.qweight, self.bias, self.mode, self.outlier_ratio = qweight, bias, mode, outlier_ratio
+        if mode == "int8_rot" and qweight.q.is_cuda:  # here, so that a first call under capture finds it
+            _device_rows(qweight.q.device, torch.cuda.is_current_stream_capturing())
 
     def _outlier_rows(self, x32, s1):
         """Indices of the rows whose rotated peak is more than `outlier_ratio` times their rms. H256 is orthonormal,
@@ -95,19 +106,27 @@ class _TELinear:
         if bias is not None:
             bias = bias.to(torch.float32).contiguous()
         out = torch.empty((m, n), device=dev, dtype=torch.float32)
-        # one workspace: q1 | q2 | s1 | s2 | rows | count | flags (every piece starts on a 16-byte boundary: K % 256 == 0)
+        # one workspace: q1 | q2 | s1 | s2 | rows | count | flags (every piece starts on a 16-byte boundary: K % 256 == 0).
+        # Without a second pass no row is an outlier, and q2 is never written: it gets no room of its own.
         m4 = (m + 3) // 4 * 4
-        work = torch.empty(2 * m * k + 3 * 4 * m4 + 16 + m, device=dev, dtype=torch.uint8)
+        codes = m * k * (2 if second else 1)
+        work = torch.empty(codes + 3 * 4 * m4 + 16 + m, device=dev, dtype=torch.uint8)
         q1 = work.data_ptr()
-        q2 = q1 + m * k
-        s1 = q2 + m * k
+        q2, s1 = q1 + codes - m * k, q1 + codes
         s2, rows, count = s1 + 4 * m4, s1 + 8 * m4, s1 + 12 * m4
         flags = count + 16
-        ratio = float(self.outlier_ratio) if second else float("inf")
-        _lib.call("rh3_te_quant", x2.data_ptr(), x2.stride(0), m, k, ratio, q1, s1, flags, count, rows, q2, s2,
-                  _lib.ptr(_taken(dev)) if second else None, _lib.stream())
+        ratio, taken, seen = float("inf"), None, None
         if second:
-            _ROWS[1] += m
+            ratio = float(self.outlier_ratio)
+            capturing = torch.cuda.is_current_stream_capturing()
+            pair = _device_rows(dev, capturing)
+            if pair is not None:
+                taken = pair.data_ptr()
+                seen = taken + 8 if capturing else None
+            if not capturing:
+                _ROWS[1] += m
+        _lib.call("rh3_te_quant_counted", x2.data_ptr(), x2.stride(0), m, k, ratio, q1, s1, flags, count, rows, q2, s2,
+                  taken, seen, _lib.stream())
         _lib.call("rh3_te_gemm", q1, s1, qw.q.data_ptr(), ws.data_ptr(), _lib.ptr(bias), m, n, k, flags, count,
                   rows if second else None, q2, s2, out.data_ptr(), n, _lib.stream())
         return out

@@ -99,3 +99,46 @@ def test_fused_route_equals_the_separate_steps(te, shape, rows):
         plain = te_quant._TELinear(qw, bias, "int8_rot_plain")(xd)
         p = kernels.linear(xc.to(torch.bfloat16), qw, "int8_rot").float()
         assert torch.equal(plain, p if bias is None else p + bias)
+
+
+def _row_scales(x):
+    from rapid_h3_b200 import quantizers
+    return quantizers.rot_quant_rows_i8(x.to(torch.bfloat16))[1]
+
+
+def test_residual_share_counts_what_ran(te, monkeypatch):
+    """Rows seen and rows that took the residual pass stay in step: calls, replays of a captured call (which are not the
+    captures), a call on another stream that nobody waited for, a graph whose capture is the linear's first call."""
+    te_quant, kernels, lib = te
+    monkeypatch.setattr(te_quant, "_ROWS", [0, 0])
+    monkeypatch.setattr(te_quant, "_DEVICE_ROWS", {})
+    m, k, n = 50, 512, 64
+    x, w = _case(m, k, n, 8)
+    x = x.cuda()
+    qw = kernels.quantize_weight(w.cuda(), "int8_rot")
+    lin = te_quant._TELinear(qw, None, "int8_rot", outlier_ratio=8.0)
+    out = lin._outlier_rows(x, _row_scales(x)).numel()
+    assert 0 < out < m
+    assert te_quant.residual_share() == 0.0
+
+    def totals():
+        te_quant.residual_share()  # waits
+        t, s = te_quant._DEVICE_ROWS[x.device].tolist()
+        return te_quant._ROWS[0] + t, te_quant._ROWS[1] + s
+
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = lin(x)
+    assert totals() == (0, 0)  # captured, not run
+    for _ in range(5):
+        graph.replay()
+    assert totals() == (5 * out, 5 * m) and te_quant.residual_share() == out / m
+    assert torch.equal(lin(x), y)
+    assert totals() == (6 * out, 6 * m)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(20_000_000)
+        lin(x)
+    assert totals() == (7 * out, 7 * m)
+    lib.check_status()
