@@ -117,7 +117,7 @@ int rh3_rms_norm_rows(const void* x, int64_t ldx, const void* w, float eps, int6
 /* Input side of the text encoder's linear on x fp32 [M, K] (row stride ldx; K % 256 == 0, K <= 8192): q1 [M, K], s1 [M] = the
  * int8 row quantizer on rotate(bf16(x)); flags [M] bytes = 1 where 127 s1 / max(rms(x), 1e-12) > ratio; those rows also get a
  * slot i < *count (any order): rows[i], and q2[i], s2[i] = the int8 codes of rotate(x) - q1 s1. *count (int32) is set by the
- * call; *total (uint64, may be NULL) grows by it. rows, q2 and s2 have room for M rows.
+ * call, to 0 when M == 0 (count may be NULL then); *total (uint64, may be NULL) grows by it. rows, q2 and s2 have room for M rows.
  * Replaces te_quant.py:90-105 of the reference (custom_nodes/rapid_h3/te_quant.py). */
 int rh3_te_quant(const float* x, int64_t ldx, int64_t M, int64_t K, float ratio, void* q1, float* s1, void* flags,
                  int32_t* count, int32_t* rows, void* q2, float* s2, void* total, cudaStream_t stream);
@@ -161,7 +161,7 @@ int rh3_gemm_w8a8_swiglu(const void* xq, int64_t lda, const void* wq, const floa
 
 /* The products of the text encoder's linear (int8, contiguous codes): out fp32 [M, N] = float(bf16((acc1 s1) ws)) + bias;
  * for the rows listed in rows[0 .. *count) the second product's float(bf16((acc2 s2) ws)) is added before the bias. bias may
- * be NULL; rows NULL: no second product. count stays on the device. Replaces te_quant.py:95-112 of the reference. */
+ * be NULL; rows NULL: no second product. count stays on the device. out starts on a 32-byte boundary; ldo >= N is a multiple of 8. Replaces te_quant.py:95-112 of the reference. */
 int rh3_te_gemm(const void* q1, const float* s1, const void* wq, const float* ws, const float* bias, int64_t M, int64_t N,
                 int64_t K, const void* flags, const int32_t* count, const int32_t* rows, const void* q2, const float* s2,
                 float* out, int64_t ldo, cudaStream_t stream);
@@ -285,7 +285,7 @@ int rh3_gn_reduce(const float* gn_part, int64_t rows_per_sample, int64_t N, doub
 int rh3_gn_silu_apply(const void* x, const float* mean_rstd, const void* gamma, const void* beta, int64_t N,
                       int64_t sites_per_sample, int64_t C, void* y, cudaStream_t stream);
 /* The same from the fp64 sums [N, 32, 2] of rh3_gn_reduce: mean = s * (1/count), rstd = rsqrt(max(s2 * (1/count) - mean^2, 0)
- * + eps), each operation rounded in fp64, both then rounded to fp32. count = values per (sample, group). */
+ * + eps), each operation rounded in fp64, both then rounded to fp32. count = values per (sample, group), > 0. */
 int rh3_gn_silu_from_sums(const void* x, const double* sums, double count, double eps, const void* gamma, const void* beta,
                           int64_t N, int64_t sites_per_sample, int64_t C, void* y, cudaStream_t stream);
 /* y[N, 2T-1, 2H, 2W, C]: nearest-neighbour 2x in space, causal 2x in time (the first frame is not repeated). */

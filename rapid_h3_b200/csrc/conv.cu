@@ -877,6 +877,7 @@ extern "C" int rh3_gn_silu_from_sums(const void* x, const double* sums, double c
                                      const void* beta, int64_t N, int64_t sites_per_sample, int64_t C, void* y,
                                      cudaStream_t stream) {
   RH3_CHECK_ARG(sums, "gn_silu_from_sums: null sums");
+  RH3_CHECK_ARG(count > 0.0, "gn_silu_from_sums: count must be greater than 0");
   return gn_silu_launch(x, nullptr, sums, count, eps, gamma, beta, N, sites_per_sample, C, y, stream);
 }
 

@@ -660,7 +660,7 @@ extern "C" int rh3_te_quant_counted(const float* x, int64_t ldx, int64_t M, int6
   RH3_CHECK_ARG(M >= 0 && M < (1ll << 31) && K > 0 && K % 256 == 0 && K <= 8192,
                 "te_quant: K=%lld must be a multiple of 256, <= 8192", (long long)K);
   RH3_CHECK_ARG(ldx >= K && ldx % 4 == 0, "te_quant: bad row stride");
-  if (M == 0) return 0;
+  if (M == 0) return count ? check_cuda(cudaMemsetAsync(count, 0, sizeof(int32_t), stream), "te_quant count") : 0;
   RH3_CHECK_ARG(x && q1 && s1 && flags && count && rows && q2 && s2, "te_quant: null pointer");
   RH3_CHECK_ARG((reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(q1) & 7) == 0 &&
                     (reinterpret_cast<uintptr_t>(q2) & 7) == 0 && (reinterpret_cast<uintptr_t>(total) & 7) == 0 &&

@@ -66,7 +66,7 @@ def gn_silu(x, sums, count, gamma, beta, out=None):
     n, c = x.shape[0], x.shape[-1]
     y = torch.empty_like(x) if out is None else out
     assert y.shape == x.shape and y.is_contiguous() and y.dtype == x.dtype
-    if sums.dtype == torch.float64 and sums.is_cuda and sums.shape == (n, GROUPS, 2) and sums.is_contiguous() and isinstance(count, (int, float)):
+    if sums.dtype == torch.float64 and sums.is_cuda and sums.shape == (n, GROUPS, 2) and sums.is_contiguous() and isinstance(count, (int, float)) and count > 0:
         _lib.call("rh3_gn_silu_from_sums", x.data_ptr(), sums.data_ptr(), float(count), EPS, gamma.data_ptr(), beta.data_ptr(),
                   n, x.numel() // (n * c), c, y.data_ptr(), _lib.stream())
         return y

@@ -48,3 +48,14 @@ def test_argument_errors_of_the_later_entry_points():
     assert lib.rh3_rot_residual_quant_rows_i8(None, 100, None, 100, None, None, 2, 100, None, None, None) < 0
     # the no-allocation statistics entry refuses what its built-in scratch cannot hold
     assert lib.rh3_attn_kv_stats_noalloc(None, 128, 128, None, 128, 128, 1 << 22, 64, None, None, None, None) < 0
+
+
+def test_argument_errors_at_the_edges_of_the_fused_entries():
+    lib = _lib.lib()
+    err = lib.rh3_last_error_string
+    p = ctypes.c_void_p(4096)  # an address that is never touched: the argument checks come first
+    for count in (0.0, -1.0, float("nan")):
+        assert lib.rh3_gn_silu_from_sums(p, p, count, 1e-5, p, p, 1, 8, 256, p, None) < 0 and b"count" in err()
+    # no rows: nothing to do, and no count to set
+    for fn, extra in ((lib.rh3_te_quant, ()), (lib.rh3_te_quant_counted, (None,))):
+        assert fn(None, 256, 0, 256, 8.0, None, None, None, None, None, None, None, None, *extra, None) == 0

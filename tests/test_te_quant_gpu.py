@@ -142,3 +142,21 @@ def test_residual_share_counts_what_ran(te, monkeypatch):
         lin(x)
     assert totals() == (7 * out, 7 * m)
     lib.check_status()
+
+
+def test_no_rows_set_the_count_to_zero(te):
+    te_quant, kernels, lib = te
+    count = torch.full((1,), 77, dtype=torch.int32, device="cuda")
+    lib.call("rh3_te_quant", None, 256, 0, 256, 8.0, None, None, None, count.data_ptr(), None, None, None, None, lib.stream())
+    lib.check_status()
+    assert count.item() == 0
+
+
+def test_products_refuse_rows_their_stores_cannot_write(te):
+    te_quant, kernels, lib = te
+    q, f = torch.zeros(4, 256, dtype=torch.int8, device="cuda"), torch.ones(64, device="cuda")
+    w, out = torch.zeros(64, 256, dtype=torch.int8, device="cuda"), torch.zeros(4 * 72 + 4, device="cuda")
+    for offset, ldo in ((4, 64), (0, 68), (0, 56)):
+        with pytest.raises(RuntimeError, match="32-byte"):
+            lib.call("rh3_te_gemm", q.data_ptr(), f.data_ptr(), w.data_ptr(), f.data_ptr(), None, 4, 64, 256, None, None, None, None,
+                     None, out.data_ptr() + 4 * offset, ldo, lib.stream())

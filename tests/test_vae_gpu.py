@@ -169,6 +169,13 @@ def test_gn_silu_from_sums_equals_the_elementwise_chain(vae, c, sites):
     assert torch.equal(y, ref)
 
 
+def test_gn_silu_of_a_count_that_is_no_count(vae):
+    """Sums of no values: NaN, as the elementwise chain gives, and not an argument error."""
+    v, lib = vae
+    x, one = torch.ones(1, 1, 1, 4, 32, dtype=torch.bfloat16, device="cuda"), torch.ones(32, dtype=torch.bfloat16, device="cuda")
+    assert v.gn_silu(x, torch.zeros(1, 32, 2, dtype=torch.float64, device="cuda"), 0, one, one).isnan().all()
+
+
 def test_decoder_matches_oracle(vae):
     v, lib = vae
     dec = v.VAEDecoder(seed=1, widths=(128, 64, 64), blocks_per_stage=1)
