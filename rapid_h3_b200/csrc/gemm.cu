@@ -40,7 +40,7 @@ constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
 // Two warps per TMEM lane quadrant, each draining half of the accumulator's columns: with one, the epilogue of a short K
 // outlasts the main loop of the next tile (w1 + SwiGLU in fp16, 3,594 x 16,384 x 2,048: 187 us with four warps and the
 // division routine, 85 with eight and silu_div; fp16 with residual, N = 2,048, K = 8,192: 61 -> 56; long-K bf16 shapes
-// measure the same).
+// measure the same). The price is registers: 168 a thread at 320 threads, which every epilogue has to fit.
 constexpr int EPI_WARPS = 8;
 constexpr int EPI_COLS = BN / (EPI_WARPS / 4);
 constexpr int EPI_THREADS = 32 * EPI_WARPS;
@@ -142,20 +142,17 @@ __device__ __forceinline__ void store_chunk_bf16(__nv_bfloat16* o, const uint4* 
   }
 }
 
-// The gated residual's values of chunks c and c + 1 of a row (eight 16-byte pieces; zeros off the edge).
+// The gated residual's values of chunk c of a row (four 16-byte pieces; zeros off the edge).
 __device__ __forceinline__ void load_gated_residual(const GemmParams& p, int row, bool row_ok, int n0, int c, uint4* dst) {
+  const int col0 = n0 + c * 32;
+  const __nv_bfloat16* o = p.resid + static_cast<int64_t>(row) * p.ldr + col0;
 #pragma unroll
-  for (int q = 0; q < 2; ++q) {
-    const int col0 = n0 + (c + q) * 32;
-    const __nv_bfloat16* o = p.resid + static_cast<int64_t>(row) * p.ldr + col0;
-#pragma unroll
-    for (int g = 0; g < 4; g += 2) {
-      if (p.wide && row_ok && col0 + g * 8 + 16 <= p.N) {
-        ld_global_32(o + g * 8, dst[q * 4 + g], dst[q * 4 + g + 1]);
-      } else {
-        dst[q * 4 + g] = (row_ok && col0 + g * 8 + 8 <= p.N) ? *reinterpret_cast<const uint4*>(o + g * 8) : make_uint4(0, 0, 0, 0);
-        dst[q * 4 + g + 1] = (row_ok && col0 + g * 8 + 16 <= p.N) ? *reinterpret_cast<const uint4*>(o + g * 8 + 8) : make_uint4(0, 0, 0, 0);
-      }
+  for (int g = 0; g < 4; g += 2) {
+    if (p.wide && row_ok && col0 + g * 8 + 16 <= p.N) {
+      ld_global_32(o + g * 8, dst[g], dst[g + 1]);
+    } else {
+      dst[g] = (row_ok && col0 + g * 8 + 8 <= p.N) ? *reinterpret_cast<const uint4*>(o + g * 8) : make_uint4(0, 0, 0, 0);
+      dst[g + 1] = (row_ok && col0 + g * 8 + 16 <= p.N) ? *reinterpret_cast<const uint4*>(o + g * 8 + 8) : make_uint4(0, 0, 0, 0);
     }
   }
 }
@@ -184,8 +181,8 @@ template <int KIND_F8, int EPI>
 __device__ __forceinline__ void epilogue_row(const GemmParams& p, const GemmSmemTail* tail, uint32_t t_row, int row,
                                              bool row_ok, float xs, int n0, int c_first, const uint4* res0) {
   // `c_first`: first 32-column chunk of this warp's EPI_COLS columns
-  // two 32-column chunks are loaded per wait, so a tile costs four TMEM round trips instead of eight; `old4` = the
-  // chunk's residual values (gated residual only), loaded one round trip ahead
+  // Two 32-column chunks are loaded per wait where no residual has to be held beside them, so a warp's half of a tile costs
+  // two TMEM round trips instead of four; `old4` = the chunk's residual values (gated residual only), loaded one chunk ahead
   auto chunk = [&](const uint32_t* r, int c, const uint4* old4) {
     const int col0 = n0 + c * 32;
     if (row_ok && col0 < p.N) {
@@ -340,24 +337,24 @@ __device__ __forceinline__ void epilogue_row(const GemmParams& p, const GemmSmem
     }
   };
   if (is_gated(EPI)) {
-    // the residual of the next two chunks is fetched while the current two are computed (the loads of a row are
-    // 16 bytes each from a cold 8 KB-strided row: waiting for them chunk by chunk was most of this epilogue's time)
-    // (the first two chunks' values, `res0`, were fetched by the caller before it waited for the accumulator)
-    uint4 res[2][8];
-    auto load_res = [&](uint4* dst, int c) { load_gated_residual(p, row, row_ok, n0, c, dst); };
+    // The residual of the next chunk is fetched while the current one is computed (the loads of a row come from a cold
+    // 8 KB-strided row: waiting for them chunk by chunk was most of this epilogue's time); the first chunk's, `res0`, was
+    // fetched by the caller before it waited for the accumulator. One chunk per TMEM wait and one ahead is what 168
+    // registers hold: two and two spilled 40-72 bytes a thread. With two gates, N = K = 4,096: 36,436 rows 549 -> 481 us,
+    // 17,896 rows 278 -> 245, 6,196 rows 101 -> 88, 1,008 rows 23.1 -> 21.0 (four epilogue warps with two and two, which
+    // do not spill either: no better than the spilling form at the first two sizes); K = 16,384 hides the epilogue and
+    // measures the same within 2 %.
+    uint4 res[2][4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) res[0][i] = res0[i];
+    for (int i = 0; i < 4; ++i) res[0][i] = res0[i];
 #pragma unroll
-    for (int it = 0; it < EPI_COLS / 64; ++it) {
-      const int c = c_first + it * 2;
-      uint32_t ra[32], rb[32];
-      tmem_ld32(t_row + c * 32, ra);
-      tmem_ld32(t_row + c * 32 + 32, rb);
-      if (it + 1 < EPI_COLS / 64) load_res(res[(it + 1) & 1], c + 2);
-      tmem_ld_wait_regs(ra);
-      tmem_ld_wait_regs(rb);
-      chunk(ra, c, res[it & 1]);
-      chunk(rb, c + 1, res[it & 1] + 4);
+    for (int it = 0; it < EPI_COLS / 32; ++it) {
+      const int c = c_first + it;
+      uint32_t r[32];
+      tmem_ld32(t_row + c * 32, r);
+      if (it + 1 < EPI_COLS / 32) load_gated_residual(p, row, row_ok, n0, c + 1, res[(it + 1) & 1]);
+      tmem_ld_wait_regs(r);
+      chunk(r, c, res[it & 1]);
     }
     return;
   }
@@ -507,7 +504,7 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         const int row2 = m2 * BM + quad * 32 + lane;
         prefetch_residual<EPI>(p, row2, row2 < M, n2 * BN + c_first * 32);
       }
-      uint4 res0[8];
+      uint4 res0[4];
       if (is_gated(EPI)) load_gated_residual(p, row, row_ok, n0, c_first, res0);
       // the four warps leave together: a warp that gave up its wait takes the others with it at this barrier
       // (which also publishes the staged columns), so none of them waits at the next tile's barrier alone
@@ -706,7 +703,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         const int row2 = m2 * 2 * BM + static_cast<int>(rank) * BM + quad * 32 + lane;
         prefetch_residual<EPI>(p, row2, row2 < M, n2 * BN + c_first * 32);
       }
-      uint4 res0[8];
+      uint4 res0[4];
       if (is_gated(EPI)) load_gated_residual(p, row, row_ok, n0, c_first, res0);
       const bool got = mbar_wait(&tail->acc_full[acc], acc_phase, abort_flag, p.status, ST_TIMEOUT_ACC_FULL);
       if (bar_sync_or(1, EPI_THREADS, !got)) break;
