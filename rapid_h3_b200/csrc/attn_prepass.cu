@@ -71,23 +71,30 @@ __device__ __forceinline__ float half_warp_max(float v) {
 // reductions): every lane of a row repeats it, so eight lanes per row halve it; where a lane also carries per-channel
 // statistics of 16 rows, sixteen lanes are what the registers allow.
 //
-// What a lane needs of the norm weight and of one token's rope table row: per channel the two factors (of the channel
-// itself, of its partner in the rotary pair) as a bf16 pair.
-template <int CH>
+// What a lane needs of the norm weight and of one token's rope table row. PACKED: per channel the two factors (of the
+// channel itself, of its partner in the rotary pair) as a bf16 pair, and rounded values travel between lanes two to a
+// shuffle. Otherwise the table words stay as they were loaded and the values stay fp32. The same bits. Packed is fewer
+// instructions and the better one almost everywhere (rmsnorm_rope at 36,436 x 32 rows 252 -> 241 us, rope_scatter 411 ->
+// 399); launch 1 with a rotation, which has a row's loads and the kept rows or the statistics in registers beside the table
+// words, is better off unpacked (126 registers against 128, the most it may use): the three launches take 838 us against
+// 886 for 36,436 tokens x 32 heads, 425 against 449 for 17,896, 230 against 240 for 9,000, 164 against 172 for 6,196, and
+// the same below 2,000.
+template <int CH, bool PACKED = true>
 struct NormRope {
-  float w[CH];      // norm weight of this lane's channels
-  uint32_t t[CH];   // low half: factor of the own channel, high half: factor of the partner's
+  float w[CH];                          // norm weight of this lane's channels
+  uint32_t t[PACKED ? CH : 2 * CH];     // PACKED: low half: factor of the own channel, high half: factor of the partner's;
+                                        // else t[2j] = (t00, t01), t[2j + 1] = (t10, t11) of pair j
 };
-template <int CH>
-__device__ __forceinline__ void load_norm_weight(const __nv_bfloat16* __restrict__ w, int l, NormRope<CH>& nr) {
+template <int CH, bool PACKED>
+__device__ __forceinline__ void load_norm_weight(const __nv_bfloat16* __restrict__ w, int l, NormRope<CH, PACKED>& nr) {
 #pragma unroll
   for (int i = 0; i < CH; i += 8) unpack8(__ldg(reinterpret_cast<const uint4*>(w + l * CH + i)), nr.w + i);
 }
 // Channels 0..47 hold the first halves of the rotary pairs, 48..95 the second halves (channel c pairs with c + 48); the
-// lanes of both halves read the words (t00, t01), (t10, t11) of their pairs and keep (t00, t01) or (t11, t10). Lanes of
-// channels 96..127 only normalise.
-template <int CH>
-__device__ __forceinline__ void load_rope_row(const __nv_bfloat16* __restrict__ tab_row, int l, NormRope<CH>& nr) {
+// lanes of both halves read the words (t00, t01), (t10, t11) of their pairs and keep (t00, t01) or (t11, t10), or both
+// words where they are not PACKED. Lanes of channels 96..127 only normalise.
+template <int CH, bool PACKED>
+__device__ __forceinline__ void load_rope_row(const __nv_bfloat16* __restrict__ tab_row, int l, NormRope<CH, PACKED>& nr) {
   constexpr int HALF = 48 / CH;  // lanes per half
   if (l < 2 * HALF) {
     const uint4* p = reinterpret_cast<const uint4*>(tab_row + (l < HALF ? l : l - HALF) * CH * 4);
@@ -95,8 +102,12 @@ __device__ __forceinline__ void load_rope_row(const __nv_bfloat16* __restrict__ 
 #pragma unroll
     for (int i = 0; i < CH / 2; ++i) {
       const uint4 q = __ldg(p + i);
-      nr.t[2 * i] = __byte_perm(q.x, q.y, pick);
-      nr.t[2 * i + 1] = __byte_perm(q.z, q.w, pick);
+      if constexpr (PACKED) {
+        nr.t[2 * i] = __byte_perm(q.x, q.y, pick);
+        nr.t[2 * i + 1] = __byte_perm(q.z, q.w, pick);
+      } else {
+        nr.t[4 * i] = q.x, nr.t[4 * i + 1] = q.y, nr.t[4 * i + 2] = q.z, nr.t[4 * i + 3] = q.w;
+      }
     }
   }
 }
@@ -118,35 +129,57 @@ __device__ __forceinline__ float row_sumsq(const float* v) {
   return CH == 8 ? ss[0] : __fadd_rn(ss[0], ss[CH / 8 - 1]);
 }
 // RMSNorm (+ RoPE when `rope`) of one row held as CH floats per lane; the result is the bf16-rounded row, as floats in v
-// and packed in `out` (two channels per word). The rounded values travel between lanes two to a shuffle.
-template <int CH>
-__device__ __forceinline__ void norm_rope_row(float* v, const NormRope<CH>& nr, float eps, bool rope, int lane, uint32_t* out) {
+// and packed in `out` (two channels per word).
+template <int CH, bool PACKED>
+__device__ __forceinline__ void norm_rope_row(float* v, const NormRope<CH, PACKED>& nr, float eps, bool rope, int lane,
+                                              uint32_t* out) {
   static_assert(CH == 8 || CH == 16, "a row is shared by 16 or 8 lanes");
   constexpr int HALF = 48 / CH, LANES = 128 / CH;
   const int l = lane & (LANES - 1);
   // dividing by 128 is the exact product with 2^-7
   const float r = __fdiv_rn(1.f, __fsqrt_rn(__fadd_rn(__fmul_rn(row_sumsq<CH>(v), 0.0078125f), eps)));
+  // the other half of every pair lives HALF lanes away (48 channels) in the same row
+  const int partner = (lane & ~(LANES - 1)) | (l < HALF ? l + HALF : (l < 2 * HALF ? l - HALF : l));
+  if constexpr (PACKED) {
 #pragma unroll
-  for (int j = 0; j < CH / 2; ++j)
-    out[j] = pack_bf16x2(__fmul_rn(__fmul_rn(r, v[2 * j]), nr.w[2 * j]), __fmul_rn(__fmul_rn(r, v[2 * j + 1]), nr.w[2 * j + 1]));
-  if (rope) {
-    // the other half of every pair lives HALF lanes away (48 channels) in the same row
-    const int partner = (lane & ~(LANES - 1)) | (l < HALF ? l + HALF : (l < 2 * HALF ? l - HALF : l));
-    uint32_t other[CH / 2];
+    for (int j = 0; j < CH / 2; ++j)
+      out[j] = pack_bf16x2(__fmul_rn(__fmul_rn(r, v[2 * j]), nr.w[2 * j]), __fmul_rn(__fmul_rn(r, v[2 * j + 1]), nr.w[2 * j + 1]));
+    if (rope) {
+      uint32_t other[CH / 2];
 #pragma unroll
-    for (int j = 0; j < CH / 2; ++j) other[j] = __shfl_sync(0xffffffffu, out[j], partner);
-    if (l < 2 * HALF) {
+      for (int j = 0; j < CH / 2; ++j) other[j] = __shfl_sync(0xffffffffu, out[j], partner);
+      if (l < 2 * HALF) {
 #pragma unroll
-      for (int j = 0; j < CH / 2; ++j) {
-        const uint32_t t0 = nr.t[2 * j], t1 = nr.t[2 * j + 1];
-        const float a = __fadd_rn(__fmul_rn(bf16_lo(out[j]), bf16_lo(t0)), __fmul_rn(bf16_lo(other[j]), bf16_hi(t0)));
-        const float b = __fadd_rn(__fmul_rn(bf16_hi(out[j]), bf16_lo(t1)), __fmul_rn(bf16_hi(other[j]), bf16_hi(t1)));
-        out[j] = pack_bf16x2(a, b);
+        for (int j = 0; j < CH / 2; ++j) {
+          const uint32_t t0 = nr.t[2 * j], t1 = nr.t[2 * j + 1];
+          const float a = __fadd_rn(__fmul_rn(bf16_lo(out[j]), bf16_lo(t0)), __fmul_rn(bf16_lo(other[j]), bf16_hi(t0)));
+          const float b = __fadd_rn(__fmul_rn(bf16_hi(out[j]), bf16_lo(t1)), __fmul_rn(bf16_hi(other[j]), bf16_hi(t1)));
+          out[j] = pack_bf16x2(a, b);
+        }
       }
     }
-  }
 #pragma unroll
-  for (int j = 0; j < CH / 2; ++j) v[2 * j] = bf16_lo(out[j]), v[2 * j + 1] = bf16_hi(out[j]);
+    for (int j = 0; j < CH / 2; ++j) v[2 * j] = bf16_lo(out[j]), v[2 * j + 1] = bf16_hi(out[j]);
+  } else {
+#pragma unroll
+    for (int j = 0; j < CH; ++j) v[j] = bf16_round(__fmul_rn(__fmul_rn(r, v[j]), nr.w[j]));
+    if (rope) {
+      float other[CH];
+#pragma unroll
+      for (int j = 0; j < CH; ++j) other[j] = __shfl_sync(0xffffffffu, v[j], partner);
+      if (l < 2 * HALF) {
+        const bool first = l < HALF;
+#pragma unroll
+        for (int j = 0; j < CH; ++j) {
+          const uint32_t tw = first ? nr.t[2 * j] : nr.t[2 * j + 1];
+          const float a = first ? v[j] : other[j], b = first ? other[j] : v[j];
+          v[j] = bf16_round(__fadd_rn(__fmul_rn(a, bf16_lo(tw)), __fmul_rn(b, bf16_hi(tw))));
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < CH / 2; ++j) out[j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
+  }
 }
 __device__ __forceinline__ uint4 words4(const uint32_t* w) { return make_uint4(w[0], w[1], w[2], w[3]); }
 
@@ -249,13 +282,17 @@ struct RopeStatsParams {
   int q_ctas, kv_ctas;   // the K / V CTAs come first: they take about twice as long as the Q ones
 };
 
+// ROPE: calls with a rope table; the others (text keys, no norm at all) have nothing to shuffle and keep the packed form
+// (36,436 queries against 512 text keys, three launches: 228 us with one kernel for both, packed; 248 unpacked; 202 with a
+// kernel of its own, 114 registers)
+template <bool ROPE>
 __global__ void __launch_bounds__(256, 2) rope_stats_kernel(const RopeStatsParams p) {
   __shared__ float sh[HW_PER_CTA * 4 * D];  // Q side: 16 block maxima; K/V side: per half-warp partials [hw][4][128]
   const int lane = threadIdx.x & 31, l16 = lane & 15, hw = threadIdx.x >> 4;
   const bool q_side = static_cast<int>(blockIdx.x) >= p.kv_ctas;
   const int idx = q_side ? blockIdx.x - p.kv_ctas : blockIdx.x;
   const int chunk = idx / p.H, h = idx - chunk * p.H;
-  NormRope<8> nr;
+  NormRope<8, !ROPE> nr;
 
   if (q_side) {
     // ---- Q: (norm + rope) -> rows kept as packed bf16 -> block-64 abs-max -> int8 codes ----
@@ -275,9 +312,9 @@ __global__ void __launch_bounds__(256, 2) rope_stats_kernel(const RopeStatsParam
       float v[8];
       unpack8(kept[i], v);
       if (p.q_w) {
-        if (p.tab) load_rope_row(p.tab + (live ? s : 0) * 48 * 4, l16, nr);
+        if (ROPE) load_rope_row(p.tab + (live ? s : 0) * 48 * 4, l16, nr);
         uint32_t o[4];
-        norm_rope_row(v, nr, p.eps, p.tab != nullptr, lane, o);
+        norm_rope_row(v, nr, p.eps, ROPE, lane, o);
         kept[i] = words4(o);
         if (p.q_out && live) *reinterpret_cast<uint4*>(p.q_out + s * p.qo_ss + h * p.qo_sh + l16 * 8) = kept[i];
       }
@@ -330,9 +367,9 @@ __global__ void __launch_bounds__(256, 2) rope_stats_kernel(const RopeStatsParam
       unpack8(kraw[u], kv);
       unpack8(vraw[u], vv);
       if (p.k_w) {
-        if (p.tab) load_rope_row(p.tab + (live ? s : 0) * 48 * 4, l16, nr);
+        if (ROPE) load_rope_row(p.tab + (live ? s : 0) * 48 * 4, l16, nr);
         uint32_t o[4];
-        norm_rope_row(kv, nr, p.eps, p.tab != nullptr, lane, o);
+        norm_rope_row(kv, nr, p.eps, ROPE, lane, o);
         if (live) *reinterpret_cast<uint4*>(p.k_out + s * p.ko_ss + h * p.ko_sh + l16 * 8) = words4(o);
       }
       if (live) {
@@ -629,7 +666,8 @@ int launch_rope_stats(RopeStatsParams p, int kv_ctas, cudaStream_t stream) {
   const int64_t ctas = static_cast<int64_t>(p.q_ctas) + kv_ctas;
   if (ctas == 0) return 0;
   RH3_CHECK_ARG(ctas < (1ll << 31), "attention pre-pass: too many tokens x heads");
-  rope_stats_kernel<<<static_cast<unsigned>(ctas), 256, 0, stream>>>(p);
+  auto kern = p.tab ? rope_stats_kernel<true> : rope_stats_kernel<false>;
+  kern<<<static_cast<unsigned>(ctas), 256, 0, stream>>>(p);
   return check_cuda(cudaGetLastError(), "attention pre-pass (rope / statistics) launch");
 }
 
