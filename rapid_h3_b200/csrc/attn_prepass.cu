@@ -255,8 +255,8 @@ __global__ void __launch_bounds__(256) rope_scatter_kernel(const __nv_bfloat16* 
 }
 
 // ---------------------------------------------------------------------------------------------
-// Launch 1 of the pre-pass. CTAs [kv_ctas, kv_ctas + q_ctas) quantize Q: one CTA = 128 tokens (two 64-token blocks) of one head, a
-// half-warp owns 8 of them, loads all 8 rows before it touches the first and keeps them as packed bf16 until the
+// Launch 1 of the pre-pass. q_ctas CTAs quantize Q: one CTA = 128 tokens (two 64-token blocks) of one head, a half-warp
+// owns 8 of them, loads all 8 rows before it touches the first and keeps them as packed bf16 until the
 // block maximum is known. The other CTAs prepare K and V: one CTA = one 256-token statistics chunk of one head, a
 // half-warp owns 16 tokens and works through them four at a time (eight 16-byte loads in flight per lane). Heads
 // vary fastest, so the CTAs that share a token's rope table row run together and find it in L2.
@@ -279,7 +279,8 @@ struct RopeStatsParams {
   const __nv_bfloat16* tab;           // rope table [L][48][2][2] or null
   float eps;
   int H;
-  int q_ctas, kv_ctas;   // the K / V CTAs come first: they take about twice as long as the Q ones
+  int q_ctas, kv_ctas;
+  int kv_first;          // which of the two come first (launch_rope_stats)
 };
 
 // ROPE: calls with a rope table; the others (text keys, no norm at all) have nothing to shuffle and keep the packed form
@@ -289,8 +290,10 @@ template <bool ROPE>
 __global__ void __launch_bounds__(256, 2) rope_stats_kernel(const RopeStatsParams p) {
   __shared__ float sh[HW_PER_CTA * 4 * D];  // Q side: 16 block maxima; K/V side: per half-warp partials [hw][4][128]
   const int lane = threadIdx.x & 31, l16 = lane & 15, hw = threadIdx.x >> 4;
-  const bool q_side = static_cast<int>(blockIdx.x) >= p.kv_ctas;
-  const int idx = q_side ? blockIdx.x - p.kv_ctas : blockIdx.x;
+  const int n_first = p.kv_first ? p.kv_ctas : p.q_ctas;
+  const bool in_first = static_cast<int>(blockIdx.x) < n_first;
+  const bool q_side = in_first != (p.kv_first != 0);
+  const int idx = in_first ? blockIdx.x : blockIdx.x - n_first;
   const int chunk = idx / p.H, h = idx - chunk * p.H;
   NormRope<8, !ROPE> nr;
 
@@ -666,6 +669,14 @@ int launch_rope_stats(RopeStatsParams p, int kv_ctas, cudaStream_t stream) {
   const int64_t ctas = static_cast<int64_t>(p.q_ctas) + kv_ctas;
   if (ctas == 0) return 0;
   RH3_CHECK_ARG(ctas < (1ll << 31), "attention pre-pass: too many tokens x heads");
+  // A K / V CTA takes about twice as long as a Q CTA. While the K / V ones take at most four fifths of the resident slots
+  // (two per SM) they come first: all of them start at once, and the Q ones fill what is left, instead of the long ones
+  // running on alone at the end. Beyond that Q comes first, and launch 3 finds more of K and V in L2. The three launches,
+  // us, Q first -> K / V first, 32 heads with norm and rotation: 512 tokens 31.5 -> 28.5, 1,008: 39.3 -> 34.9, 1,280:
+  // 45.3 -> 43.1, 1,792 (224 CTAs): 57.8 -> 56.5, 2,048 (256): 57.5 -> 61.5, 4,500: 113 -> 121, 9,000: 220 -> 230, 36,436:
+  // 831 -> 838 (2,560 alone is better the other way: 78.8 -> 75.4); 8 heads, 8,192 tokens (256): 59.4 -> 63.7; 512 text
+  // keys (64) for 6,196 queries: 67.1 -> 58.6, for 36,436: 264 -> 258.
+  p.kv_first = 5ll * kv_ctas <= 4ll * 2 * device_sm_count();
   auto kern = p.tab ? rope_stats_kernel<true> : rope_stats_kernel<false>;
   kern<<<static_cast<unsigned>(ctas), 256, 0, stream>>>(p);
   return check_cuda(cudaGetLastError(), "attention pre-pass (rope / statistics) launch");

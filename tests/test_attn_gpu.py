@@ -216,3 +216,22 @@ def test_row_maximum_that_grows_in_every_key_tile(ops, lk, step):
     out = attn.attention(q.cuda(), k.cuda(), v.cuda())
     lib.check_status()
     assert rel_l2(out.cpu(), oa.attention(q, k, v)) <= TOL
+
+
+@pytest.mark.parametrize("h", [29, 30])
+def test_block_order_of_the_prepass_changes_nothing(ops, h):
+    """Which blocks of launch 1 come first depends on how many there are (232 and 240 K / V blocks lie on either side of
+    four fifths of 296 slots); a head's operands do not: the last heads alone are a call of 24 K / V blocks."""
+    attn, lib = ops
+    s, tail = 1900, 3
+    g = torch.Generator(device="cuda").manual_seed(h)
+    buf = torch.randn(s, 3 * h * 128, device="cuda", generator=g).to(torch.bfloat16)
+    tab = inputs.rope_table(inputs.random_positions(s, seed=2)).cuda()
+    qw, kw = (w.cuda() for w in inputs.norm_weights())
+    q, k, v = views(buf, h)
+    pre = attn.int8_prepass(q, k, v, tab, qw, kw)
+    few = attn.int8_prepass(q[:, -tail:], k[:, -tail:], v[:, -tail:], tab, qw, kw)
+    lib.check_status()
+    for name in ("q8", "qs", "k8", "ks", "kmean", "vmean", "vscale"):
+        assert torch.equal(getattr(pre, name)[-tail:], getattr(few, name)), name
+    assert torch.equal(pre.vt[-tail:].view(torch.uint8), few.vt.view(torch.uint8))
