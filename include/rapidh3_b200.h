@@ -116,8 +116,10 @@ int rh3_rms_norm_rows(const void* x, int64_t ldx, const void* w, float eps, int6
                       cudaStream_t stream);
 /* Input side of the text encoder's linear on x fp32 [M, K] (row stride ldx; K % 256 == 0, K <= 8192): q1 [M, K], s1 [M] = the
  * int8 row quantizer on rotate(bf16(x)); flags [M] bytes = 1 where 127 s1 / max(rms(x), 1e-12) > ratio; those rows also get a
- * slot i < *count (any order): rows[i], and q2[i], s2[i] = the int8 codes of rotate(x) - q1 s1. *count (int32) is set by the
- * call, to 0 when M == 0 (count may be NULL then); *total (uint64, may be NULL) grows by it. rows, q2 and s2 have room for M rows.
+ * slot i < *count (any order): rows[i], and q2[i], s2[i] = the int8 codes of rotate(x) - q1 s1. A row whose quotient lies
+ * within rounding of `ratio` may fall on either side, depending on the order its squares are summed in. With ratio = +inf no
+ * row is flagged, and rows, q2 and s2 are not written. *count (int32) is set by the call, to 0 when M == 0 (count may be NULL
+ * then); *total (uint64, may be NULL) grows by it. rows, q2 and s2 have room for M rows.
  * Replaces te_quant.py:90-105 of the reference (custom_nodes/rapid_h3/te_quant.py). */
 int rh3_te_quant(const float* x, int64_t ldx, int64_t M, int64_t K, float ratio, void* q1, float* s1, void* flags,
                  int32_t* count, int32_t* rows, void* q2, float* s2, void* total, cudaStream_t stream);

@@ -55,11 +55,6 @@ __device__ __forceinline__ uint4 load_row16(const __nv_bfloat16* row, int l16) {
   return __ldg(reinterpret_cast<const uint4*>(row + l16 * 8));
 }
 // sum over the 16 lanes of a half-warp, same value in every lane, fixed order (xor 8, 4, 2, 1)
-__device__ __forceinline__ float half_warp_sum(float v) {
-#pragma unroll
-  for (int o = 8; o; o >>= 1) v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
 __device__ __forceinline__ float half_warp_max(float v) {
 #pragma unroll
   for (int o = 8; o; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));

@@ -90,7 +90,7 @@ struct __align__(8) GemmSmemTail {
   int abort_flag;
   float ws[BN];
   float aux[BN];   // bias or gate as fp32
-  float aux2[BN];  // residual scale as fp32 (EPI_F16)
+  float aux2[BN];  // residual scale (EPI_F16) or second gate (EPI_GATED2) as fp32
 };
 
 constexpr int GEMM_SMEM_BYTES = STAGES * STAGE_BYTES + sizeof(GemmSmemTail) + 1024;  // +1024 alignment slack
@@ -105,9 +105,10 @@ __device__ __forceinline__ void tile_coords(int tile, int num_m, int num_n, int&
   n_blk = t / gsize;
 }
 
-// The epilogue of one accumulator row: 256 columns, 32 at a time from TMEM, dequantized and stored through the fused
-// epilogue EPI. `t_row` = TMEM address of this thread's row (lane) at the accumulator's first column.
-// The residual row of an epilogue that adds one (gated residual, fp16 residual): its BN columns are asked into L2
+// The epilogue of one accumulator row (epilogue_row below): EPI_COLS columns, 32 at a time from TMEM, dequantized and
+// stored through the fused epilogue EPI. `t_row` = TMEM address of this thread's row (lane) at the accumulator's first
+// column.
+// The residual row of an epilogue that adds one (gated residual, fp16 residual): its EPI_COLS columns are asked into L2
 // while the tile's MMAs still run, so the epilogue's loads do not wait on HBM (the residual of a step is far
 // larger than L2 and cold by the time its tile comes up).
 template <int EPI>
@@ -158,7 +159,8 @@ __device__ __forceinline__ void load_gated_residual(const GemmParams& p, int row
 }
 
 // g / (1 + e^-g) without the division routine: 1/d from the approximate reciprocal and one Newton step (to the last
-// bit or its neighbour), times g, one correction by the exact remainder g - q d. The exponent is held at 80: beyond it
+// bit or its neighbour), times g, one correction by the exact remainder g - q d (Markstein's division: the remainder is
+// exact in one fused multiply-add, and adding it times the reciprocal rounds the quotient once). The exponent is held at 80: beyond it
 // d would leave the range the reciprocal works in, and g / e^80 is already far below fp16's smallest value (a NaN g
 // still gives NaN; an infinite one gives what the division would: g itself, or NaN for -inf / inf).
 __device__ __forceinline__ float silu_div(float g) {
@@ -506,7 +508,7 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       }
       uint4 res0[4];
       if (is_gated(EPI)) load_gated_residual(p, row, row_ok, n0, c_first, res0);
-      // the four warps leave together: a warp that gave up its wait takes the others with it at this barrier
+      // the epilogue warps leave together: a warp that gave up its wait takes the others with it at this barrier
       // (which also publishes the staged columns), so none of them waits at the next tile's barrier alone
       const bool got = mbar_wait(&tail->acc_full[acc], acc_phase, abort_flag, p.status, ST_TIMEOUT_ACC_FULL);
       if (bar_sync_or(1, EPI_THREADS, !got)) break;

@@ -246,8 +246,8 @@ __global__ void __launch_bounds__(T) quant_rows_kernel(const QuantParams p) {
 
 // RMSNorm of bf16 rows to bf16, out = bf16((x * r) * w) with r = rsqrt(mean(x^2) + eps): one read, one write. The loop of
 // quant_rows_kernel: a row in registers, the next row's loads in flight. HBM-bound, 4 bytes per element; as a chain of
-// elementwise kernels (fp32 copy, square, mean, rsqrt, two products, two copies) the same rows cost 18 bytes per element:
-// 80 us for 1,008 x 4,096, 5.9 us here; 6,196 x 4,096 take 16 us (6.3 TB/s).
+// elementwise kernels (fp32 copy, square, mean, rsqrt, two products, copy back) the same rows cost about 40 bytes per
+// element (2 + 4, 4 + 4, 4, 4 + 4, 4 + 4, 4 + 2), in part out of L2: 80 us for 1,008 x 4,096, 5.9 us here; 6,196 x 4,096 take 16 us (6.3 TB/s).
 template <int T, int CPT>
 __global__ void __launch_bounds__(T) rms_norm_rows_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx,
                                                           const __nv_bfloat16* __restrict__ w, float eps, int64_t M, int K,
@@ -334,7 +334,9 @@ __global__ void __launch_bounds__(T) rot_residual_quant_kernel(const float* __re
 // read once and held in registers:
 //   q1, s1   the int8 row quantizer on rotate(bf16(x)) (the codes of rot_quant_rows on the bf16 copy of x)
 //   outlier  127 s1 / max(rms(x), 1e-12) > ratio: H256 is orthonormal, so the rotated row has x's rms, and its abs-max is
-//            127 s1 by construction of the scale
+//            127 s1 by construction of the scale. The squares are summed by fused multiply-adds in a fixed order; a sum in
+//            another order (torch's mean, in the separate steps) can differ in its last places, so a row whose quotient is
+//            within about 1e-6 of the ratio can fall on the other side there
 //   an outlier row takes the next free slot i of the second pass: rows[i] = row, and q2[i], s2[i] are the int8 codes of
 //   rotate(x) - q1 s1 (the arithmetic of rot_residual_quant_kernel). Slots are handed out by one atomic per outlier row, in
 //   any order: a slot's content does not depend on its number. `count` is what the second product reads its row number

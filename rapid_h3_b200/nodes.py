@@ -198,7 +198,7 @@ class FusedBlock:
 
     @staticmethod
     def _gate_rows(gate_tab):
-        """The gate table [R, d] as bf16 rows, converted once per forward (one row per modality)."""
+        """The gate table [R, d] as bf16 rows (one row per modality), for the calls that take a GEMM per span."""
         return gate_tab.to(torch.bfloat16).contiguous()
 
     @staticmethod

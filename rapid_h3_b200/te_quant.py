@@ -96,7 +96,9 @@ class _TELinear:
 
     def _fused(self, x2):
         """Both passes for fp32 x2 [M, K] in three kernels: the input side (te_quant_kernel) and the two products, whose
-        epilogues write fp32 and add the bias. The number of outlier rows stays on the device."""
+        epilogues write fp32 and add the bias. The number of outlier rows stays on the device. The bits of the separate
+        steps (_matmul), except for a row whose peak-over-rms lies within rounding of `outlier_ratio`: the two sum its
+        squares in different orders, and it may take the second pass on one route only."""
         qw, dev = self.qweight, x2.device
         m, k = x2.shape
         n = qw.q.shape[0]

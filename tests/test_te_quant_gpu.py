@@ -74,7 +74,9 @@ def test_te_linear_matches_oracle_and_helps_outlier_rows(te, mode):
 @pytest.mark.parametrize("rows", ["some", "none", "all"])
 def test_fused_route_equals_the_separate_steps(te, shape, rows):
     """The three-kernel route against quantizer, product, row selection, residual quantizer and second product as separate
-    calls: the same bits (row widths with idle threads, one row, more rows than blocks; no, some and only outlier rows)."""
+    calls: the same bits (row widths with idle threads, one row, more rows than blocks; no, some and only outlier rows).
+    The rows here lie far from the ratio: one next to it may be an outlier on one route only (its squares are summed in
+    another order)."""
     te_quant, kernels, lib = te
     m, k, n = shape
     x, w = _case(m, max(k, 512), n, m + k)
