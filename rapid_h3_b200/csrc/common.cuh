@@ -86,8 +86,12 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint64_t* bar, uint32_t parity
 // waiter polls it so the whole CTA drains instead of hanging. Returns true when the phase
 // completed, false when the wait was abandoned (the caller must then leave its loop).
 // The limit is generous (seconds): a healthy wait finishes in microseconds.
+// The poll loops stay rolled: unrolled by the compiler they were 60 % of the attention kernels' code (5,840 instructions
+// against 2,700), and warps of different roles then miss the 32 KB instruction cache. H = 32, ms before and after:
+// attn_int8 L = 4,500 0.305 / 0.298, 36,436 x 512 keys 0.473 / 0.465; attn_tok L = 22,332 11.58 / 11.28.
 __device__ __forceinline__ bool mbar_wait_polls(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                                 int* status, int code, uint32_t max_polls) {
+#pragma unroll 1
   for (uint32_t it = 0; it < max_polls; ++it) {
     if (mbar_try_wait(bar, parity)) return true;
     if (it > 64) {
@@ -108,6 +112,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
 // between polls the thread sleeps `ns` nanoseconds, so its polling does not take issue slots from those warps.
 __device__ __forceinline__ bool mbar_wait_relaxed(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status,
                                                   int code, unsigned ns) {
+#pragma unroll 1
   for (uint32_t it = 0; it < (1u << 24); ++it) {
     if (mbar_try_wait(bar, parity)) return true;
     __nanosleep(ns);
