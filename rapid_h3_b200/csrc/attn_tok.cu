@@ -16,21 +16,25 @@
 //   O = ts * A + a * O        the per-tile fold, fp32, in registers
 //   out = bf16((O / l) * vscale + vmean)
 //
-// Integers become floats without a conversion instruction: both accumulators are pre-biased with 0x4B400000 (the
-// softmax warps store it into TMEM before each tile's MMAs, which then accumulate onto it), so for |x| < 2^22 their
-// bits are the float 1.5*2^23 + x, and subtracting 1.5*2^23 from that float is exact. The per-score arithmetic runs
-// two values per instruction (fma/add/mul.rn.f32x2).
+// Every integer is below 2^24, so its conversion to fp32 is exact. The per-score arithmetic runs two values per
+// instruction (fma/add/mul.rn.f32x2).
 //
-// One CTA = two 128-query tiles of one head, 384 threads: warp 0 = TMA producer (K tile, V^T tile and the 1 KB of
-// key scales / biases per step, 3-stage ring), warp 1 = MMA issuer, warps 4..11 = softmax, one query row per
-// thread with its 128 fp32 output values in registers (232 registers per softmax thread after the register
-// re-split). The scores are read from TMEM twice, 16 columns at a time (maximum, then exponentials), so that the
-// output row fits beside them. P has two buffers, so the exponentials of a tile do not wait for the previous tile's
-// P.V: its fold comes after them. TMEM (512 columns): S0 | S1 | A0 | A1.
-// What bounds it: issue slots and the serial chain of a softmax thread at two warps per scheduler. H = 32: 13.4 ms at
-// L = 22,332 and 0.614 ms at L = 4,500 with a test for the last tile's biases at every four scores and the fold ahead of
-// the exponentials; 11.6 and 0.523 with the test once per pass, the three-input maximum and the two P buffers. Rolled
-// passes (a quarter of the code) are slower: 11.8 with one, 12.2-12.4 with both.
+// One CTA = two 128-query tiles of one head, 640 threads, one CTA per SM:
+//   warp group 0     service (32 registers): warp 0 = TMA producer (K tile, V^T tile and the 1 KB of key scales / biases per
+//                    step, 3-stage ring), warps 1 and 2 = MMA issuers of query tile 0 / 1
+//   warp groups 1, 2 softmax of query tile 0 / 1 (72 registers), one query row per thread, 16 columns of the tile at a time
+//                    with the next load in flight: the first pass turns the scores into t in place (back into TMEM) and takes
+//                    their maximum, the second turns t into P in shared memory (two buffers) and the integer row sum
+//   warp groups 3, 4 fold of query tile 0 / 1 (152 registers), one query row per thread with its 128 fp32 outputs in
+//                    registers: O = ts * A + a * O, from the factors the softmax threads leave in shared memory; where no
+//                    row of a warp has a new maximum (a = 1) the multiplication by a is left out
+// TMEM (512 columns): S0 | S1 | A0 | A1. 96 registers a thread are launched; the warp groups' shares add up to them.
+// What bounds it: issue slots (2,850 per scheduler and step of 4,880 cycles; an f32x2 instruction takes two) and the chain
+// scores -> first pass -> second pass -> next scores, which the fold warps and the other query tile run under. H = 32, ms at
+// L = 22,332 / 6,196 / 1,000: 11.28 / 0.997 / 0.037 with the fold, the scores' second conversion and scaling, and a bias
+// stored into both accumulators in the softmax threads' own chain (384 threads); 10.20 / 0.910 / 0.036 with the fold in warp
+// groups of its own and conversions in place of the bias; 8.99 / 0.811 / 0.035 with t kept in TMEM; 8.75 / 0.813 / 0.034
+// without the multiplication by a = 1. Spinning instead of sleeping waits 8.77-8.91, an 80 / 144 register split 8.96.
 #include <limits.h>
 
 #include <type_traits>
@@ -47,7 +51,7 @@ constexpr int TILE_BYTES = 128 * 128;
 constexpr int KSB_BYTES = 2 * BKV * 4;                   // per key tile: 128 scales, then 128 biases
 constexpr int STAGE_BYTES = 2 * TILE_BYTES + KSB_BYTES;  // K | V^T | scales, biases
 constexpr int KV_STAGES = 3;
-constexpr int TOK_THREADS = 384;
+constexpr int TOK_THREADS = 640;   // service, two softmax and two fold warp groups
 
 struct TokParams {
   const float* qs;      // [H][Lq_pad]  one scale per query token
@@ -65,15 +69,19 @@ struct __align__(8) TokSmemTail {
   uint64_t q_full;
   uint64_t kv_full[KV_STAGES];
   uint64_t kv_empty[KV_STAGES];
-  uint64_t s_full[QG], s_empty[QG], p_full[QG], pv_done[QG];
+  uint64_t s_full[QG], s_empty[QG], pv_done[QG], l_full[QG];
+  // one barrier per step parity: a softmax warp may be a step ahead of another one of its tile (or of the fold), and its
+  // arrival must not complete the phase the slower one still owes
+  uint64_t p_full[QG][2], a_empty[QG][2];
   uint32_t tmem_base;
   int abort_flag;
+  float2 fold[QG][2][BQ];   // {a, ts} of the row: O = ts * A + a * O
+  float row_sum[QG][BQ];
 };
 
 constexpr int TOK_SMEM_BYTES = 3 * QG * TILE_BYTES + KV_STAGES * STAGE_BYTES + sizeof(TokSmemTail) + 1024;
 
 constexpr float kMagic = 12582912.f;          // 1.5 * 2^23
-constexpr uint32_t kMagicBits = 0x4B400000u;
 constexpr float kLog2_255 = 7.99435343685886f;
 
 __device__ __forceinline__ float ex2_approx(float x) {
@@ -105,10 +113,8 @@ __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
-// The accumulators are pre-biased with 1.5*2^23 (see the kernel), so their bits ARE the float 1.5*2^23 + x; for
-// |x| < 2^22 subtracting the bias is exact: two exact integer values per instruction.
-__device__ __forceinline__ uint64_t unbias2(uint32_t lo, uint32_t hi) {
-  return add2(pack2(__uint_as_float(lo), __uint_as_float(hi)), pack2(-kMagic, -kMagic));
+__device__ __forceinline__ uint64_t int2(uint32_t lo, uint32_t hi) {
+  return pack2(static_cast<float>(static_cast<int>(lo)), static_cast<float>(static_cast<int>(hi)));
 }
 __device__ __forceinline__ void lds4x2(uint32_t addr, uint64_t& a, uint64_t& b) {
   asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(addr));
@@ -121,10 +127,14 @@ __device__ __forceinline__ void bulk_load(void* smem_dst, const void* gsrc, uint
                : "memory");
 }
 
-constexpr int REGS_COMPILED = 168, REGS_SERVICE = 40, REGS_SOFTMAX = 232;
-static_assert(128 * REGS_SERVICE + 256 * REGS_SOFTMAX == TOK_THREADS * REGS_COMPILED, "register pool must balance");
-__device__ __forceinline__ void reg_release_service() { asm volatile("setmaxnreg.dec.sync.aligned.u32 40;"); }
-__device__ __forceinline__ void reg_take_softmax() { asm volatile("setmaxnreg.inc.sync.aligned.u32 232;"); }
+constexpr int REGS_COMPILED = 96, REGS_SERVICE = 32, REGS_SOFTMAX = 72, REGS_FOLD = 152;
+static_assert(128 * REGS_SERVICE + 256 * REGS_SOFTMAX + 256 * REGS_FOLD == TOK_THREADS * REGS_COMPILED,
+              "register pool must balance");
+__device__ __forceinline__ void reg_release_service() { asm volatile("setmaxnreg.dec.sync.aligned.u32 32;"); }
+__device__ __forceinline__ void reg_release_softmax() { asm volatile("setmaxnreg.dec.sync.aligned.u32 72;"); }
+__device__ __forceinline__ void reg_take_fold() { asm volatile("setmaxnreg.inc.sync.aligned.u32 152;"); }
+
+__device__ __forceinline__ bool warp_all(bool ok) { return __all_sync(0xffffffffu, ok) != 0; }
 
 // t = x * kscale for four columns; on the last key tile (BIAS: chosen once per pass) the bias is added, which is 0
 // for real keys and -inf for the padding keys. rn(x * s) + 0 is the same number as fma(x, s, 0).
@@ -132,8 +142,8 @@ template <bool BIAS>
 __device__ __forceinline__ void scores4(const uint32_t* r, uint32_t ks_addr, uint32_t kb_addr, uint64_t& t01, uint64_t& t23) {
   uint64_t s01, s23;
   lds4x2(ks_addr, s01, s23);
-  t01 = mul2(unbias2(r[0], r[1]), s01);
-  t23 = mul2(unbias2(r[2], r[3]), s23);
+  t01 = mul2(int2(r[0], r[1]), s01);
+  t23 = mul2(int2(r[2], r[3]), s23);
   if (BIAS) {
     uint64_t b01, b23;
     lds4x2(kb_addr, b01, b23);
@@ -148,9 +158,9 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   return d;
 }
 
-// Maximum over one 16-column chunk of t.
+// t of one 16-column chunk in place of its scores, and the maximum over them.
 template <bool BIAS>
-__device__ __forceinline__ float chunk_tmax(const uint32_t* r, uint32_t ks_addr, uint32_t kb_addr, float tm) {
+__device__ __forceinline__ float chunk_tmax(uint32_t* r, uint32_t ks_addr, uint32_t kb_addr, float tm) {
   float tn = -INFINITY;  // a second chain
 #pragma unroll
   for (int i = 0; i < 16; i += 4) {
@@ -161,24 +171,21 @@ __device__ __forceinline__ float chunk_tmax(const uint32_t* r, uint32_t ks_addr,
     unpack2(t23, t2, t3);
     tm = max3(tm, t0, t1);
     tn = max3(tn, t2, t3);
+    r[i] = __float_as_uint(t0), r[i + 1] = __float_as_uint(t1), r[i + 2] = __float_as_uint(t2), r[i + 3] = __float_as_uint(t3);
   }
   return fmaxf(tm, tn);
 }
 
-// One 16-column chunk: P = u8(rint(2^(t * c + off))) written to 16-byte chunk k of the row of P in shared memory
+// One 16-column chunk of t: P = u8(rint(2^(t * c + off))) written to 16-byte chunk k of the row of P in shared memory
 // (XOR-swizzled like the TMA tiles), the integer codes added to `rs`.
-template <bool BIAS>
-__device__ __forceinline__ void chunk_p(const uint32_t* r, uint32_t ks_addr, uint32_t kb_addr, float c, float off, int k,
-                                        uint8_t* p_row, int sw, uint32_t& rs) {
+__device__ __forceinline__ void chunk_p(const uint32_t* r, float c, float off, int k, uint8_t* p_row, int sw, uint32_t& rs) {
   const uint64_t c2 = pack2(c, c), off2 = pack2(off, off), magic2 = pack2(kMagic, kMagic);
   uint32_t w[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    uint64_t t01, t23;
-    scores4<BIAS>(r + 4 * i, ks_addr + i * 16, kb_addr + i * 16, t01, t23);
     float e0, e1, e2, e3;
-    unpack2(fma2(t01, c2, off2), e0, e1);
-    unpack2(fma2(t23, c2, off2), e2, e3);
+    unpack2(fma2(pack2(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1])), c2, off2), e0, e1);
+    unpack2(fma2(pack2(__uint_as_float(r[4 * i + 2]), __uint_as_float(r[4 * i + 3])), c2, off2), e2, e3);
     // p <= 255 * (1 + 2^-20): adding 1.5*2^23 leaves rint(p) (ties to even) in the low byte
     float p0, p1, p2, p3;
     unpack2(add2(pack2(ex2_approx(e0), ex2_approx(e1)), magic2), p0, p1);
@@ -208,13 +215,17 @@ attn_tok_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
     mbar_init(&tail->q_full, 1);
     for (int s = 0; s < KV_STAGES; ++s) {
       mbar_init(&tail->kv_full[s], 1);
-      mbar_init(&tail->kv_empty[s], 1);
+      mbar_init(&tail->kv_empty[s], QG);  // P.V of both query tiles
     }
     for (int g = 0; g < QG; ++g) {
       mbar_init(&tail->s_full[g], 1);
       mbar_init(&tail->s_empty[g], 4);  // one arrival per softmax warp
-      mbar_init(&tail->p_full[g], 4);
       mbar_init(&tail->pv_done[g], 1);
+      mbar_init(&tail->l_full[g], 4);
+      for (int b = 0; b < 2; ++b) {
+        mbar_init(&tail->p_full[g][b], 4);
+        mbar_init(&tail->a_empty[g][b], 4);  // one arrival per fold warp
+      }
     }
     tail->abort_flag = 0;
     fence_barrier_init();
@@ -248,120 +259,71 @@ attn_tok_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
         tma_load_2d(sk + TILE_BYTES, &tma_v, j * BKV, h * HD, &tail->kv_full[stage]);
         bulk_load(sk + 2 * TILE_BYTES, ksb_h + static_cast<int64_t>(j) * (2 * BKV), KSB_BYTES, &tail->kv_full[stage]);
       }
-    } else if (warp == 1) {
-      // ------------------------------ MMA issuer ------------------------------
+    } else if (warp == 1 || warp == 2) {
+      // ------------------------------ MMA issuers, one per query tile ------------------------------
       // The whole warp runs the loop converged (waits, counters, addresses are warp-uniform and can live in the
       // uniform datapath the MMA instruction reads its operands from); one elected lane issues MMAs and commits.
       constexpr uint32_t idesc_qk = make_idesc(2, 1, 1, BQ, BKV);  // s32 = s8 * s8
       constexpr uint32_t idesc_pv = make_idesc(2, 0, 1, BQ, HD);   // s32 = u8 * s8
-      auto all_ok = [](bool ok) { return __all_sync(0xffffffffu, ok) != 0; };
-      auto issue_qk = [&](int g, int j) {
-        const uint32_t q_addr = smem_u32(sQ + g * TILE_BYTES);
-        const uint32_t k_addr = smem_u32(sKV + (j % KV_STAGES) * STAGE_BYTES);
+      const int g = warp - 1;
+      const uint64_t q_desc = make_desc_k128(smem_u32(sQ + g * TILE_BYTES));
+      const uint64_t p_desc = make_desc_k128(smem_u32(sP + 2 * g * TILE_BYTES));
+      const uint64_t k_desc = make_desc_k128(smem_u32(sKV));
+      const uint64_t v_desc = make_desc_k128(smem_u32(sKV + TILE_BYTES));
+      const uint32_t s_tmem = tmem_base + g * 128, a_tmem = tmem_base + 256 + g * 128;
+      bool ok = warp_all(mbar_wait(&tail->q_full, 0, abort_flag, p.status, ST_TIMEOUT_TMA_FULL));
+      int st = 0, st_next = 0;          // ring stage of this step and of the one whose scores are asked for
+      uint32_t ph_next = 0;
+      auto issue_qk = [&](int j) {
+        // the softmax warps have read the scores of step j - 1
+        ok = ok && warp_all(mbar_wait_relaxed(&tail->kv_full[st_next], ph_next, abort_flag, p.status, ST_TIMEOUT_TMA_FULL, 32) &&
+                            mbar_wait_relaxed(&tail->s_empty[g], (j & 1) ^ 1, abort_flag, p.status, ST_TIMEOUT_ACC_EMPTY, 32));
+        if (!ok) return;
+        tc_fence_after();
         if (elect_one()) {
-          mma4_i8_ss(tmem_base + g * 128, make_desc_k128(q_addr), make_desc_k128(k_addr), idesc_qk, 1);  // onto the bias
+          mma4_i8_ss(s_tmem, q_desc, k_desc + st_next * (STAGE_BYTES / 16), idesc_qk, 0);
           mma_commit(&tail->s_full[g]);
         }
         __syncwarp();
+        if (++st_next == KV_STAGES) {
+          st_next = 0;
+          ph_next ^= 1;
+        }
       };
-      bool ok = all_ok(mbar_wait(&tail->q_full, 0, abort_flag, p.status, ST_TIMEOUT_TMA_FULL) &&
-                       mbar_wait(&tail->kv_full[0], 0, abort_flag, p.status, ST_TIMEOUT_TMA_FULL));
-      for (int g = 0; g < QG && ok; ++g) {
-        // completion 0 of s_empty: the softmax warps have biased both accumulators of this query tile
-        ok = all_ok(mbar_wait(&tail->s_empty[g], 0, abort_flag, p.status, ST_TIMEOUT_ACC_EMPTY));
-        if (ok) {
-          tc_fence_after();
-          issue_qk(g, 0);
-        }
-      }
+      issue_qk(0);
+#pragma unroll 1
       for (int j = 0; j < n_kv && ok; ++j) {
-        if (j + 1 < n_kv) {
-          const int ns = (j + 1) % KV_STAGES;
-          ok = all_ok(mbar_wait_relaxed(&tail->kv_full[ns], ((j + 1) / KV_STAGES) & 1, abort_flag, p.status, ST_TIMEOUT_TMA_FULL, 64));
-          for (int g = 0; g < QG && ok; ++g) {
-            // completion j+1 of s_empty: the softmax warps have read the scores of key tile j for the last time and
-            // put the bias back
-            ok = all_ok(mbar_wait_relaxed(&tail->s_empty[g], (j + 1) & 1, abort_flag, p.status, ST_TIMEOUT_ACC_EMPTY, 64));
-            if (ok) {
-              tc_fence_after();
-              issue_qk(g, j + 1);
-            }
-          }
-          if (!ok) break;
+        if (j + 1 < n_kv) issue_qk(j + 1);
+        // P of step j is in shared memory, and the accumulator of step j - 1 has been folded
+        ok = ok && warp_all(mbar_wait_relaxed(&tail->p_full[g][j & 1], (j >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_P_READY, 32) &&
+                            (j == 0 || mbar_wait_relaxed(&tail->a_empty[g][(j - 1) & 1], ((j - 1) >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_ACC_EMPTY, 32)));
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {
+          mma4_i8_ss(a_tmem, p_desc + (j & 1) * (TILE_BYTES / 16), v_desc + st * (STAGE_BYTES / 16), idesc_pv, 0);
+          mma_commit(&tail->pv_done[g]);
+          mma_commit(&tail->kv_empty[st]);
         }
-        const int stage = j % KV_STAGES;
-        const uint32_t v_addr = smem_u32(sKV + stage * STAGE_BYTES + TILE_BYTES);
-        for (int g = 0; g < QG && ok; ++g) {
-          // P of tile j is in shared memory, and the same threads have folded the accumulator of tile j-1
-          ok = all_ok(mbar_wait_relaxed(&tail->p_full[g], j & 1, abort_flag, p.status, ST_TIMEOUT_P_READY, 64));
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t p_addr = smem_u32(sP + (2 * g + (j & 1)) * TILE_BYTES);
-          if (elect_one()) {
-            mma4_i8_ss(tmem_base + 256 + g * 128, make_desc_k128(p_addr), make_desc_k128(v_addr), idesc_pv, 1);  // onto the bias
-            mma_commit(&tail->pv_done[g]);
-          }
-          __syncwarp();
-        }
-        if (ok) {
-          if (elect_one()) mma_commit(&tail->kv_empty[stage]);
-          __syncwarp();
-        }
+        __syncwarp();
+        if (++st == KV_STAGES) st = 0;
       }
     }
-  } else {
+  } else if (warp < 12) {
     // ============================ softmax warp groups ============================
-    reg_take_softmax();
+    reg_release_softmax();
     const int g = (warp >> 2) - 1;
     const int quad = warp & 3;
     const int row = quad * 32 + lane;
-    const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
-    const uint32_t t_row = tmem_base + g * 128 + lane_off;
-    const uint32_t a_row = tmem_base + 256 + g * 128 + lane_off;
+    const uint32_t t_row = tmem_base + g * 128 + (static_cast<uint32_t>(quad * 32) << 16);
     const int64_t q_row = static_cast<int64_t>(q_pair) * (QG * BQ) + g * BQ + row;
     const float c_row = __fmul_rn(p.qs[static_cast<int64_t>(h) * p.Lq_pad + q_row], p.sl2);
     uint8_t* p_row0 = sP + 2 * g * TILE_BYTES + row * 128;
     const int sw = row & 7;
-    uint64_t* s_full = &tail->s_full[g];
-    uint64_t* s_empty = &tail->s_empty[g];
-    uint64_t* p_full = &tail->p_full[g];
-    uint64_t* pv_done = &tail->pv_done[g];
-    float O[HD];   // the output row
-#pragma unroll
-    for (int i = 0; i < HD; ++i) O[i] = 0.f;
-    float m = -INFINITY, l = 0.f, a_prev = 0.f, ts_prev = 0.f;
+    float m = -INFINITY, l = 0.f;
     bool ok = true;
 
-    auto splat4 = [](uint32_t base) {
-      tmem_st32_splat(base, kMagicBits);
-      tmem_st32_splat(base + 32, kMagicBits);
-      tmem_st32_splat(base + 64, kMagicBits);
-      tmem_st32_splat(base + 96, kMagicBits);
-    };
-    // O = ts * A + a * O for the tile whose P.V has just finished; the accumulator gets its bias back
-    auto fold = [&](float a, float ts, bool rebias) {
-      tc_fence_after();
-      // two register sets: the load of the next 16 columns is in flight while these are folded
-      uint32_t ra[16], rb[16];
-      tmem_ld16_async(a_row, ra);
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        uint32_t* r = (c & 1) ? rb : ra;
-        tmem_ld_wait16(r);
-        if (c + 1 < 8) tmem_ld16_async(a_row + (c + 1) * 16, (c & 1) ? ra : rb);
-#pragma unroll
-        for (int i = 0; i < 16; ++i)
-          O[c * 16 + i] = fmaf(ts, __fsub_rn(__uint_as_float(r[i]), kMagic), __fmul_rn(O[c * 16 + i], a));
-      }
-      if (rebias) {
-        splat4(a_row);
-        tmem_st_wait();
-      }
-    };
-
     // two register sets: the load of the next 16 columns is in flight while these are worked on
-    auto pass1 = [&](auto bias, uint32_t ks_addr, uint32_t kb_addr) {
-      constexpr bool BIAS = decltype(bias)::value;
+    auto pass1 = [&](uint32_t ks_addr) {
       float tm = -INFINITY;
       uint32_t ra[16], rb[16];
       tmem_ld16_async(t_row, ra);
@@ -370,12 +332,17 @@ attn_tok_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
         uint32_t* r = (c & 1) ? rb : ra;
         tmem_ld_wait16(r);
         if (c + 1 < 8) tmem_ld16_async(t_row + (c + 1) * 16, (c & 1) ? ra : rb);
-        tm = chunk_tmax<BIAS>(r, ks_addr + c * 64, kb_addr + c * 64, tm);
+        tm = chunk_tmax<false>(r, ks_addr + c * 64, 0, tm);
+        tmem_st16(t_row + c * 16, r);
       }
       return tm;
     };
-    auto pass2 = [&](auto bias, uint32_t ks_addr, uint32_t kb_addr, float off, uint8_t* p_row, uint32_t& rs) {
-      constexpr bool BIAS = decltype(bias)::value;
+    auto hand_back = [&]() {
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tail->s_empty[g]);
+    };
+    auto pass2 = [&](float off, uint8_t* p_row, uint32_t& rs) {
       uint32_t ra[16], rb[16];
       tmem_ld16_async(t_row, ra);
 #pragma unroll
@@ -383,62 +350,113 @@ attn_tok_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
         uint32_t* r = (c & 1) ? rb : ra;
         tmem_ld_wait16(r);
         if (c + 1 < 8) tmem_ld16_async(t_row + (c + 1) * 16, (c & 1) ? ra : rb);
-        chunk_p<BIAS>(r, ks_addr + c * 64, kb_addr + c * 64, c_row, off, c, p_row, sw, rs);
+        else hand_back();   // the scores have been read for the last time
+        chunk_p(r, c_row, off, c, p_row, sw, rs);
       }
     };
-    // bias both accumulators of this query tile for key tile 0
-    splat4(t_row);
-    splat4(a_row);
-    tmem_st_wait();
-    tc_fence_before();
-    __syncwarp();
-    if (lane == 0) mbar_arrive(s_empty);
 
+    int stage = 0;
+    uint32_t phase = 0;
+#pragma unroll 1
     for (int j = 0; j < n_kv; ++j) {
-      const int stage = j % KV_STAGES;
       const uint32_t ks_addr = smem_u32(sKV + stage * STAGE_BYTES + 2 * TILE_BYTES), kb_addr = ks_addr + BKV * 4;
       const bool last = j == n_kv - 1;   // only the last key tile has padding keys (bias -inf)
       // the key scales of this stage came by bulk copy: observe its barrier before reading them
-      if (!mbar_wait_relaxed(&tail->kv_full[stage], (j / KV_STAGES) & 1, abort_flag, p.status, ST_TIMEOUT_TMA_FULL, 32)) { ok = false; break; }
-      if (!mbar_wait_relaxed(s_full, j & 1, abort_flag, p.status, ST_TIMEOUT_ACC_FULL, 32)) { ok = false; break; }
+      ok = warp_all(mbar_wait_relaxed(&tail->kv_full[stage], phase, abort_flag, p.status, ST_TIMEOUT_TMA_FULL, 32) &&
+                    mbar_wait_relaxed(&tail->s_full[g], j & 1, abort_flag, p.status, ST_TIMEOUT_ACC_FULL, 32));
+      if (!ok) break;
       tc_fence_after();
       // ---- pass 1: the tile's row maximum ----
-      const float tm = last ? pass1(std::true_type{}, ks_addr, kb_addr) : pass1(std::false_type{}, ks_addr, kb_addr);
+      float tm;
+      if (!last) {
+        tm = pass1(ks_addr);
+      } else {
+        tm = -INFINITY;
+#pragma unroll 1
+        for (int c = 0; c < 8; ++c) {
+          uint32_t r[16];
+          tmem_ld16_async(t_row + c * 16, r);
+          tmem_ld_wait16(r);
+          tm = chunk_tmax<true>(r, ks_addr + c * 64, kb_addr + c * 64, tm);
+          tmem_st16(t_row + c * 16, r);
+        }
+      }
+      tmem_st_wait();
       const float tmc = __fmul_rn(tm, c_row);
       const float m_new = fmaxf(m, tmc);
       const float a = ex2_approx(__fsub_rn(m, m_new)), ts = ex2_approx(__fsub_rn(tmc, m_new));
       const float off = __fsub_rn(kLog2_255, tmc);
       m = m_new;
+      // the fold of step j - 2 has read its factors (and s_full of this step says that its P.V has read its P)
+      ok = warp_all(j < 2 || mbar_wait_relaxed(&tail->a_empty[g][j & 1], ((j >> 1) & 1) ^ 1, abort_flag, p.status, ST_TIMEOUT_ACC_EMPTY, 32));
+      if (!ok) break;
+      tail->fold[g][j & 1][row] = make_float2(a, ts);
       // ---- pass 2: P into shared memory, integer row sum ----
-      // (this buffer was last read by P.V of tile j - 2, whose fold in the previous round waited for it)
       uint8_t* p_row = p_row0 + (j & 1) * TILE_BYTES;
       uint32_t rs = 0;
-      if (last) pass2(std::true_type{}, ks_addr, kb_addr, off, p_row, rs);
-      else pass2(std::false_type{}, ks_addr, kb_addr, off, p_row, rs);
-      // the scores have been read for the last time: bias the accumulator for the next Q.K^T and hand it back
-      splat4(t_row);
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(s_empty);
-      if (j > 0) {
-        // P.V of the previous tile has finished: fold its accumulator
-        if (!mbar_wait_relaxed(pv_done, (j - 1) & 1, abort_flag, p.status, ST_TIMEOUT_PV_DONE, 32)) { ok = false; break; }
-        fold(a_prev, ts_prev, true);
-      }
+      pass2(off, p_row, rs);
       l = fmaf(ts, static_cast<float>(rs), __fmul_rn(l, a));
-      a_prev = a;
-      ts_prev = ts;
       fence_proxy_async_smem();
-      tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(p_full);
+      if (lane == 0) mbar_arrive(&tail->p_full[g][j & 1]);
+      if (++stage == KV_STAGES) {
+        stage = 0;
+        phase ^= 1;
+      }
+    }
+    tail->row_sum[g][row] = l;
+    __syncwarp();
+    if (lane == 0 && ok) mbar_arrive(&tail->l_full[g]);
+  } else {
+    // ============================ fold warp groups ============================
+    // One query row per thread with its 128 fp32 outputs in registers: O = ts * A + a * O per key tile.
+    reg_take_fold();
+    const int g = (warp >> 2) - 3;
+    const int quad = warp & 3;
+    const int row = quad * 32 + lane;
+    const uint32_t a_row = tmem_base + 256 + g * 128 + (static_cast<uint32_t>(quad * 32) << 16);
+    const int64_t q_row = static_cast<int64_t>(q_pair) * (QG * BQ) + g * BQ + row;
+    float O[HD];   // the output row
+#pragma unroll
+    for (int i = 0; i < HD; ++i) O[i] = 0.f;
+    bool ok = true;
+#pragma unroll 1
+    for (int j = 0; j < n_kv; ++j) {
+      ok = warp_all(mbar_wait_relaxed(&tail->p_full[g][j & 1], (j >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_P_READY, 32) &&
+                    mbar_wait_relaxed(&tail->pv_done[g], j & 1, abort_flag, p.status, ST_TIMEOUT_PV_DONE, 32));
+      if (!ok) break;
+      tc_fence_after();
+      const float2 f = tail->fold[g][j & 1][row];
+      // two register sets: the load of the next 8 columns is in flight while these are folded
+      auto fold = [&](auto rescale) {
+        uint32_t ra[8], rb[8];
+        tmem_ld8_async(a_row, ra);
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+          uint32_t* r = (c & 1) ? rb : ra;
+          tmem_ld_wait8(r);
+          if (c + 1 < 16) {
+            tmem_ld8_async(a_row + (c + 1) * 8, (c & 1) ? ra : rb);
+          } else {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&tail->a_empty[g][j & 1]);
+          }
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            float& o = O[c * 8 + i];
+            o = fmaf(f.y, static_cast<float>(static_cast<int>(r[i])), decltype(rescale)::value ? __fmul_rn(o, f.x) : o);
+          }
+        }
+      };
+      // a is 1 in every row of the warp unless some row's maximum grew
+      if (__any_sync(0xffffffffu, f.x != 1.f)) fold(std::true_type{});
+      else fold(std::false_type{});
     }
     // ---- epilogue ----
-    if (ok && mbar_wait(pv_done, (n_kv - 1) & 1, abort_flag, p.status, ST_TIMEOUT_PV_DONE)) {
-      fold(a_prev, ts_prev, false);
+    if (ok && mbar_wait(&tail->l_full[g], 0, abort_flag, p.status, ST_TIMEOUT_P_READY)) {
       if (q_row < p.Lq) {
-        const float inv_l = __fdiv_rn(1.f, l);
+        const float inv_l = __fdiv_rn(1.f, tail->row_sum[g][row]);
         const float* vs = p.vscale + h * HD;
         const float* vm = p.vmean + h * HD;
         __nv_bfloat16* o = p.out + q_row * p.o_ss + static_cast<int64_t>(h) * p.o_sh;

@@ -88,6 +88,23 @@ def test_token_attention_matches_oracle(ops, shape):
     assert torch.equal(attn.attention(q.cuda(), k.cuda(), v.cuda(), rotate=True), out)
 
 
+@pytest.mark.parametrize("growing", [False, True])
+@pytest.mark.parametrize("shape", [(1, 1), (255, 127), (257, 128), (130, 129), (64, 1153)])
+def test_token_attention_maximum_early_or_late(ops, shape, growing):
+    """Edges of the query and key tiles with every row's maximum in the first key tile (the fold then never scales its
+    output row after the first step) or growing from tile to tile (it always does)."""
+    A, lib = ops
+    lq, lk = shape
+    q, k, v = (torch.randn(n, 2, 128, generator=inputs.gen(60 + i)) for i, n in enumerate((lq, lk, lk)))
+    q = q.abs() + 0.5
+    step = torch.arange(lk) // 128 + 1.0
+    k = k * 0.1 + (step if growing else 1.0 / step)[:, None, None]
+    q, k, v = (x.to(torch.bfloat16) for x in (q, k, v))
+    out = A.attention(q.cuda(), k.cuda(), v.cuda(), rotate=True)
+    lib.check_status()
+    assert rel_l2(out.cpu(), ot.attention(q, k, v)) <= TOL
+
+
 def test_token_attention_rr_and_strided_output(ops):
     attn, lib = ops
     s, h = 1500, 4
