@@ -319,6 +319,39 @@ int rh3_attn_int8_scatter(const void* q8, const float* qs, const void* k8, const
                           int64_t Lk_pad, int64_t H, float softmax_scale, void* const* dst, const int64_t* dst_start,
                           int64_t n_dst, int64_t o_ss, int64_t o_sh, cudaStream_t stream);
 
+/* ---- one fused DiT block ----
+ * The launches of a block's forward in the order of the reference's fused graph (custom_nodes/rapid_h3/__init__.py:253-320,
+ * with cross-attention to text when `cross` is 1), issued by one call: what the entry points above do one by one, on
+ * intermediate buffers inside the caller's workspace (256-byte aligned). x [S, d] is updated in place.
+ * The six fp32 tables are [R, d] views with one row stride; gate rows row0 / row1 serve the tokens before / from `split`;
+ * idx [S] names each token's table row, idx0 [S] is all zero; `zeros` fp32 [d] and `ones` bf16 [d] are constants; fc1 is in
+ * swiglu order (gate / up interleaved in groups of four); norm weights may be NULL. */
+typedef struct {
+  int64_t S, d, heads, mlp, text, text_dim;       /* tokens, widths, text tokens */
+  int64_t row0, row1, split, table_stride;
+  int64_t rotate, token_attn, cross;              /* H256 recipe, token-scaled attention, cross-attention */
+  double eps1, eps_qk, eps_c, eps_cqk, eps2;
+  void* x;
+  int64_t ldx;
+  const void* rope;                               /* bf16 [S, 48, 2, 2] */
+  const int32_t *idx, *idx0;
+  const float* zeros;
+  const void* ones;
+  const float *shift_msa, *scale_msa, *gate_msa, *shift_mlp, *scale_mlp, *gate_mlp;
+  const void *norm1, *q_norm, *k_norm, *norm_c, *cq_norm, *ck_norm, *norm2;   /* bf16 */
+  const void* ctx;                                /* bf16 [text, text_dim] */
+  int64_t ld_ctx;
+  const void* qkv;   const float* qkv_s;          /* int8 [3*heads*128, d] and its row scales; likewise below */
+  const void* out;   const float* out_s;
+  const void* cq;    const float* cq_s;
+  const void* ckv;   const float* ckv_s;
+  const void* co;    const float* co_s;
+  const void* fc1;   const float* fc1_s;
+  const void* fc2;   const float* fc2_s;
+} rh3_block_args;
+int64_t rh3_block_workspace_bytes(const rh3_block_args* b);
+int rh3_block_forward(const rh3_block_args* b, void* workspace, int64_t workspace_bytes, cudaStream_t stream);
+
 /* ---- fp16 ops of the VAE transformer decoder (the callers of the int8 path at fp16 activations) ----
  * rh3_vae_out_quant: o [B, H, S, D] fp16 head-major attention output -> q int8 [B*S, H*D], scales fp32 [B*S]:
  *   nan_to_num on load, H256 rotation in comfy-kitchen's stage order, int8 with value / scale / quotient rounded

@@ -72,10 +72,12 @@ SIGNATURES = {
     "rh3_gn_reduce": [_P, _I64, _I64, _P, _P],
     "rh3_gn_silu_apply": [_P, _P, _P, _P, _I64, _I64, _I64, _P, _P],
     "rh3_gn_silu_from_sums": [_P, _P, _D, _D, _P, _P, _I64, _I64, _I64, _P, _P],
+    "rh3_block_workspace_bytes": [_P],
+    "rh3_block_forward": [_P, _P, _I64, _P],
     "rh3_upsample_causal2x": [_P, _P, _I64, _I64, _I64, _I64, _I64, _P],
 }
 # entry points that return a value instead of a status
-RETURNS_I64 = ("rh3_attn_kv_stats_scratch_bytes", "rh3_conv3d_gn_part_rows")
+RETURNS_I64 = ("rh3_attn_kv_stats_scratch_bytes", "rh3_conv3d_gn_part_rows", "rh3_block_workspace_bytes")
 
 KIND_I8, KIND_F8 = 0, 1
 
@@ -83,7 +85,7 @@ _lib = None
 
 # kernels launched per entry point (for launch accounting in benchmarks)
 LAUNCHES = {"rh3_attn_kv_stats": 2, "rh3_attn_kv_stats_noalloc": 2, "rh3_attn_prepass": 3, "rh3_attn_tok_prepass": 5, "rh3_quant_tensor_fp8": 2, "rh3_te_gemm": 2, "rh3_version": 0, "rh3_gemm_use_pairs": 0, "rh3_sm_count": 0, "rh3_check_status": 0,
-            "rh3_attn_kv_stats_scratch_bytes": 0, "rh3_conv3d_gn_part_rows": 0}
+            "rh3_attn_kv_stats_scratch_bytes": 0, "rh3_conv3d_gn_part_rows": 0, "rh3_block_workspace_bytes": 0}
 launch_count = 0
 
 
@@ -128,11 +130,12 @@ def stream():
     return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
-def call(name, *args):
-    """Invoke an entry point; a non-zero return raises RuntimeError with the library's message."""
+def call(name, *args, launches=None):
+    """Invoke an entry point; a non-zero return raises RuntimeError with the library's message. `launches` is the number of
+    kernels behind this call where that depends on its arguments."""
     global launch_count
     rc = getattr(lib(), name)(*args)
-    launch_count += LAUNCHES.get(name, 1)
+    launch_count += LAUNCHES.get(name, 1) if launches is None else launches
     if rc != 0:
         raise RuntimeError(f"{name} failed ({rc}): {last_error()}")
 

@@ -9,14 +9,16 @@ stock path (non-bf16, CPU tensors, missing rope table) raise NotImplementedError
 no fallback path.
 """
 import re
+import struct
 
 import torch
 
-from . import attn_int8, kernels
+from . import _lib, attn_int8, kernels, timing
 from .timing import phase as _phase
 from . import gemm as cf
 from . import quantizers as tq
 
+_BLOCK_ARGS = struct.Struct("@13q5dPq5P6P7PPq14P")   # rh3_block_args
 NAME_RE = re.compile(r"^blocks\.(\d+)\.(attn|mlp|cross)\.(qkv_proj|out_proj|fc1|fc2|q_proj|kv_proj)$")
 
 _IDX_CACHE = {}   # (segment tuple, S, device) -> int32 [S]; a handful of entries at most
@@ -242,17 +244,87 @@ class FusedBlock:
                 cf.int8_gemm_gated_residual(xq[a:b], xs[a:b], qw.q, qw.scale, gates[int(row)], x[a:b])
         return x
 
+    def _native(self, x, tables, mod_segments, rope_freqs, ctx):
+        """The whole block in one call of the library (rh3_block_forward): the kernels of `forward` below on the same
+        operands, x updated in place. False, with nothing done, for anything that call does not take as it is: more than two
+        spans or per-token modulation rows, other layouts, widths or types. Those go on launch by launch."""
+        blk, a = self.block, self.block.attn
+        if type(self) is not FusedBlock or len(tables) != 6:
+            return False
+        s, d = x.shape
+        hd, two = a.heads * 128, self._two_gates(mod_segments, s, tables[2])
+        first = tables[0]
+        if (two is None or a.head_dim != 128 or x.stride(1) != 1 or a.q_norm.eps != a.k_norm.eps or x.requires_grad or type(x) is not torch.Tensor
+                or any(t.dtype != torch.float32 or t.shape != first.shape or t.stride() != first.stride() or t.device != x.device for t in tables)
+                or first.ndim != 2 or first.shape[1] != d or first.stride(1) != 1
+                or rope_freqs.dtype != torch.bfloat16 or rope_freqs.numel() != s * 192 or rope_freqs.device != x.device):
+            return False
+        linears = [self.qkv_q.qweight_for(), self.out_q.qweight_for(), self.fc2_q.qweight_for()]
+        w1q, w1s = self._fc1_swiglu_weight()
+        f = linears[2].q.shape[1]
+        shapes = [(3 * hd, d), (d, hd), (d, f)]
+        norms = [(self._norm_w(blk.norm1), d), (self._norm_w(a.q_norm), 128), (self._norm_w(a.k_norm), 128), (self._norm_w(blk.norm2), d)]
+        cross = self.cq_q is not None
+        if cross:
+            c = blk.cross
+            if (c.heads != a.heads or c.head_dim != 128 or c.q_norm.eps != c.k_norm.eps or type(ctx) is not torch.Tensor or ctx.ndim != 2
+                    or ctx.dtype != torch.bfloat16 or ctx.stride(1) != 1 or ctx.shape[0] == 0 or ctx.device != x.device):
+                return False
+            linears += [self.cq_q.qweight_for(), self.ckv_q.qweight_for(), self.co_q.qweight_for()]
+            shapes += [(hd, d), (2 * hd, ctx.shape[1]), (d, hd)]
+            norms += [(self._norm_w(blk.norm_c), d), (self._norm_w(c.q_norm), 128), (self._norm_w(c.k_norm), 128)]
+        linears.append(kernels.QWeight(w1q, w1s))
+        shapes.append((2 * f, d))
+        for qw, shape in zip(linears, shapes):
+            if (qw.q.dtype != torch.int8 or qw.q.shape != shape or not qw.q.is_contiguous() or qw.scale.dtype != torch.float32
+                    or qw.scale.numel() != shape[0] or not qw.scale.is_contiguous() or qw.q.device != x.device):
+                return False
+        if any(w is not None and (w.numel() != n or w.device != x.device) for w, n in norms) or norms[1][0] is None or norms[2][0] is None:
+            return False
+        if cross and (norms[5][0] is None or norms[6][0] is None):
+            return False
+        idx, tab, dev = _row_index(mod_segments, s, x.device), rope_freqs.contiguous(), x.device
+        if cross:
+            zeros, ones = self._zeros_tab(d, dev)
+            key0 = ("idx0", s, str(dev))
+            idx0 = self._const.get(key0)
+            if idx0 is None:
+                idx0 = self._const.setdefault(key0, torch.zeros(s, dtype=torch.int32, device=dev))
+            extra = (zeros.data_ptr(), ones.data_ptr(), idx0.data_ptr(), ctx.data_ptr(), ctx.stride(0), ctx.shape[0], ctx.shape[1])
+        else:
+            extra = (0,) * 7
+        n = [0 if w is None else w.data_ptr() for w, _ in norms] + [0] * (7 - len(norms))
+        p = [v for qw in linears for v in (qw.q.data_ptr(), qw.scale.data_ptr())]
+        qkv, out, fc2, fc1 = p[0:2], p[2:4], p[4:6], p[-2:]
+        cq, ckv, co = (p[6:8], p[8:10], p[10:12]) if cross else ((0, 0),) * 3
+        args = _BLOCK_ARGS.pack(s, d, a.heads, f, extra[5], extra[6], *two, first.stride(0), self.rotate, bool(ATTN_ROTATE), cross,
+                                self._eps(blk.norm1), a.q_norm.eps, self._eps(blk.norm_c) if cross else 0.0, c.q_norm.eps if cross else 0.0,
+                                self._eps(blk.norm2), x.data_ptr(), x.stride(0), tab.data_ptr(), idx.data_ptr(), extra[2], extra[0], extra[1],
+                                *(t.data_ptr() for t in tables), n[0], n[1], n[2], n[4], n[5], n[6], n[3], extra[3], extra[4],
+                                *qkv, *out, *cq, *ckv, *co, *fc1, *fc2)
+        work = torch.empty(_lib.lib().rh3_block_workspace_bytes(args), dtype=torch.uint8, device=dev)
+        attention = 6 if ATTN_ROTATE else 4
+        _lib.call("rh3_block_forward", args, work.data_ptr(), work.numel(), _lib.stream(),
+                  launches=attention + 8 + (attention + 6 if cross else 0))
+        return True
+
     # -- forward -----------------------------------------------------------------------------
     def forward(self, x, t_emb, mod_segments, rope_freqs, ctx=None, sp=None, trace=None):
         blk = self.block
         if rope_freqs is None or x.dtype != torch.bfloat16 or x.device.type != "cuda" or x.ndim != 2:
             raise NotImplementedError("FusedBlock: needs a 2-D CUDA bf16 packed sequence and a rope table")
+        if sp is None and trace is None and RR_CHECK is None and timing.PHASES is None:
+            tables = blk.adaln_proj(t_emb)
+            if self._native(x, tables, mod_segments, rope_freqs, ctx):
+                return x
+        else:
+            tables = None
         s, d = x.shape
         a = blk.attn
         hd = a.heads * a.head_dim
         f = blk.mlp.fc2.weight.shape[1] if blk.mlp.fc2.weight.numel() else self.fc2_q.qweight_for().q.shape[1]
         with _phase("adaln"):
-            shift_msa, scale_msa, gate_msa, shift_mlp, scale_mlp, gate_mlp = blk.adaln_proj(t_emb)
+            shift_msa, scale_msa, gate_msa, shift_mlp, scale_mlp, gate_mlp = blk.adaln_proj(t_emb) if tables is None else tables
             idx = _row_index(mod_segments, s, x.device)
             tab = rope_freqs.reshape(s, 48, 2, 2).contiguous()
         rot = self.rotate

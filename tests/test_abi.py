@@ -59,3 +59,21 @@ def test_argument_errors_at_the_edges_of_the_fused_entries():
     # no rows: nothing to do, and no count to set
     for fn, extra in ((lib.rh3_te_quant, ()), (lib.rh3_te_quant_counted, (None,))):
         assert fn(None, 256, 0, 256, 8.0, None, None, None, None, None, None, None, None, *extra, None) == 0
+
+
+def test_argument_errors_of_the_block_entry():
+    lib = _lib.lib()
+    err = lib.rh3_last_error_string
+    from rapid_h3_b200 import nodes
+    ints = [115, 256, 2, 512, 33, 256, 0, 1, 108, 1536, 0, 0, 1]   # tokens, widths, gate rows, recipe flags
+    pack = lambda v: nodes._BLOCK_ARGS.pack(*v, *[1e-6] * 5, 0, 256, *[0] * 18, 0, 256, *[0] * 14)  # noqa: E731
+    p = 4096  # an address that is never touched
+    need = lib.rh3_block_workspace_bytes(pack(ints))
+    assert need >= 115 * (256 + 2 * 768) + 2 * 256 * 128
+    assert lib.rh3_block_forward(None, p, need, None) < 0 and lib.rh3_block_forward(pack(ints), None, need, None) < 0
+    assert lib.rh3_block_forward(pack(ints), p, need - 1, None) < 0 and b"needed" in err()
+    assert lib.rh3_block_forward(pack(ints), p + 16, need, None) < 0 and b"aligned" in err()
+    for i in (0, 1, 2, 3, 4, 5):
+        bad = list(ints)
+        bad[i] = 0
+        assert lib.rh3_block_forward(pack(bad), p, need, None) < 0 and b"bad shape" in err()

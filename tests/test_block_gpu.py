@@ -349,3 +349,37 @@ def test_fused_rope_prepass_self_check(pkg, tmp_path, monkeypatch):
         r.nodes.RR_CHECK = None
     recs = [json.loads(line) for line in log.read_text().splitlines()]
     assert len(recs) == 2 and all(x["out_equal"] and x["operands_equal"] and x["max_abs_diff"] == 0.0 for x in recs)
+
+
+@pytest.mark.parametrize("mode,rotate", [("int8_rowwise", False), ("int8_rot", True)])
+@pytest.mark.parametrize("grid,audio,text,cross", [((1, 1, 1), 0, 1, True), ((3, 4, 11), 0, 300, True), ((5, 4, 5), 7, 48, True),
+                                                   ((4, 8, 8), 1, 130, False)])
+def test_block_in_one_call_has_the_bits_of_its_launches(pkg, mode, rotate, grid, audio, text, cross):
+    """The native block against the same block launch by launch (a trace asks for that), on one and two spans, text longer
+    and shorter than the sequence, padded and full tiles; a third span goes launch by launch and changes nothing."""
+    r = pkg
+    cfg = r.model.H3Config.tiny(cross_attention=cross, text_dim=256, mlp_hidden=768)
+    model = torch.nn.Module()
+    model.blocks = torch.nn.ModuleList([r.model.init_weights(r.model.DiTBlock(cfg), seed=1).cuda()])
+    fb = r.nodes.RapidH3LinearQuant().patch(model, mode)[0].block_forward[0]
+    _, _, t_emb, rope, ctx = r.step.make_inputs(cfg, grid, audio, 1, text, seed=3)
+    n = grid[0] * grid[1] * grid[2]
+    s = n + audio
+    segs = [(0, n, 0)] + ([(n, s, 1)] if audio else [])
+    x = torch.randn(s, cfg.d_model, generator=torch.Generator().manual_seed(5)).to(torch.bfloat16)
+    rest = (t_emb[0].cuda(), segs, rope.cuda(), ctx[0].cuda())
+    r.nodes.ATTN_ROTATE = rotate
+    try:
+        want = fb.forward(x.cuda(), *rest, trace={})
+        calls, r._lib.launch_count = r._lib.launch_count, 0
+        xd = x.cuda()
+        got = fb.forward(xd, *rest)
+        assert got.data_ptr() == xd.data_ptr() and torch.equal(got, want)
+        assert r._lib.launch_count == (12 if not rotate else 14) + ((10 if not rotate else 12) if cross else 0)
+        r._lib.launch_count = calls
+        if n > 2:
+            split = [(0, 1, 0), (1, n, 0)] + segs[1:]
+            assert torch.equal(fb.forward(x.cuda(), rest[0], split, *rest[2:]), want)
+    finally:
+        r.nodes.ATTN_ROTATE = False
+    r._lib.check_status()
