@@ -81,29 +81,50 @@ __device__ __forceinline__ TileCoord conv_tile(int tile, const ConvParams& p, in
 }
 
 // GroupNorm partials of a warp's 32 rows over one 32-column chunk: the GS channels of a group are summed per row
-// (in channel order), the 32 rows by an xor butterfly; lane 0 writes (sum, sum of squares) of every group the chunk
-// holds. GS is a template parameter so that every index into y[] is static (a run-time group width sends the array
-// to local memory, which made this loop the slowest part of the kernel).
+// (in channel order), the 32 rows by exchanges with the lanes 16, 8, 4, 2 and 1 away; (sum, sum of squares) of every
+// group the chunk holds are written. As long as a lane holds more than one of these values it hands half of them over
+// and keeps the other half, so the 16 values of 4-channel groups take 16 shuffles and not a butterfly of 5 for each (80,
+// which made this epilogue longer than the 54 K chunks of a 128-channel tile: 9 x 48 x 84 sites 32.6 us a layer, 28.8
+// now). Every sum has the same operands in the same order either way. GS is a template parameter so that every index into
+// y[] is static (a run-time group width sends the array to local memory).
 template <int GS>
 __device__ __forceinline__ void gn_partials_chunk(const float* y, float* part, int col0, int Cout, int lane) {
+  constexpr int NV = 2 * (32 / GS);   // values: (sum, sum of squares) of each group
+  float v[NV];
 #pragma unroll
-  for (int j0 = 0; j0 < 32; j0 += GS) {
+  for (int q = 0; q < 32 / GS; ++q) {
     float s1 = 0.f, s2 = 0.f;
 #pragma unroll
-    for (int j = j0; j < j0 + GS; ++j) {
+    for (int j = q * GS; j < (q + 1) * GS; ++j) {
       s1 += y[j];
       s2 += y[j] * y[j];
     }
+    v[2 * q] = s1;
+    v[2 * q + 1] = s2;
+  }
+  int at = 0;             // index of v[0] among the chunk's values
+  int rest = NV;          // values this lane still holds
+  int spare = 0;          // offsets at which both lanes hold the same single value: one of them stores it
 #pragma unroll
-    for (int o = 16; o; o >>= 1) {
-      s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-      s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+  for (int o = 16; o; o >>= 1) {
+    const bool upper = lane & o;
+    if (rest > 1) {
+      rest >>= 1;
+#pragma unroll
+      for (int i = 0; i < rest; ++i) {
+        const float send = upper ? v[i] : v[i + rest], keep = upper ? v[i + rest] : v[i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+      if (upper) at += rest;
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+      spare |= o;
     }
-    const int grp = (col0 + j0) / GS;
-    if (lane == 0 && col0 + j0 < Cout) {
-      part[grp * 2] = s1;
-      part[grp * 2 + 1] = s2;
-    }
+  }
+  if ((lane & spare) == 0) {
+#pragma unroll
+    for (int i = 0; i < rest; ++i)
+      if (col0 + (at + i) / 2 * GS < Cout) part[col0 / GS * 2 + at + i] = v[i];
   }
 }
 
@@ -272,8 +293,9 @@ conv3d_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__
           mbar_arrive_expect_tx(&tail->full[stage], (a_bytes + b_bytes) * KCH);
 #pragma unroll
           for (int q = 0; q < KCH; ++q) {
-            const int tap = (kb + q) / chunks, cc = kb + q - tap * chunks;
-            const int dt = tap / 9, dh = (tap / 3) % 3, dw = tap % 3;
+            // the three dh of a (dt, dw, 64 channels) follow each other, as in the pair kernel
+            const int dh = (kb + q) % 3, rest = (kb + q) / 3, cc = rest % chunks, dtw = rest / chunks;
+            const int dt = dtw / 3, dw = dtw % 3, tap = (dt * 3 + dh) * 3 + dw;
             uint8_t* sa = smem + stage * CSTAGE_BYTES + q * p.chunk_bytes;
             // out-of-range coordinates (negative or past the edge) read zeros: spatial and causal padding
             tma_load_5d(sa, &tma_x, cc * CBK, c.w0 + dw - 1, c.h0 + dh - 1, c.t + dt - 2 + p.halo, c.n, &tail->full[stage]);
@@ -364,11 +386,15 @@ conv3d_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__
 
 // ---------------------------------------------------------------------------------------------
 // The same convolution on CTA pairs (clusters of two, tcgen05 cta_group::2). A pair computes two neighbouring site
-// tiles (m = 2 * pair_m + rank) x BN output channels with MMAs of 256 rows: every CTA fetches the shifted input box of
-// its own site tile and HALF of the BN weight rows (rank r: rows [r * BN/2, (r+1) * BN/2) of the column tile), so an
-// SM takes in 16 KB + BN/2 * 128 B per K chunk instead of 16 KB + BN * 128 B: the single-CTA kernel is bound by that
-// ingest, not by the tensor pipe. Each CTA's TMEM receives its own 128 sites x BN channels and its own epilogue
-// warps drain them exactly as in the single-CTA kernel (same fp32 accumulation order: results are identical).
+// tiles (m = 2 * pair_m + rank) x BN output channels with MMAs of 256 rows: every CTA fetches the input box of its own site
+// tile and HALF of the BN weight rows (rank r: rows [r * BN/2, (r+1) * BN/2) of the column tile). Each CTA's TMEM receives its
+// own 128 sites x BN channels and its own epilogue warps drain them exactly as in the single-CTA kernel (same fp32
+// accumulation order: results are identical).
+// A ring stage is 64 channels of one (dt, dw): the tile's box with one more row of sites above and below it, which serves
+// all three dh, and the three taps' weight rows. What an SM has to take in and to write to its shared memory bounds tiles of
+// few output channels (the operand reads of the MMAs want the same bandwidth); a box per tap was 16 KB of it, a third of a
+// taller box is 6-9 KB. Before / after, us: 3 x 12 x 21 sites, 512 -> 512 channels 43.2 / 30.9, 5 x 24 x 42, 256 -> 256
+// 27.2 / 24.9, 141 x 96 x 168, 128 -> 128 1,792 / 1,748; full-width tiles are bound by the tensor pipe and measure the same.
 // When the number of site tiles is odd, the odd CTA of the last pair loads the last valid tile again and stores nothing.
 // Barriers as in the GEMM's pair kernel: both CTAs' loads count on the even CTA's `full`; stage release and
 // accumulator hand-over are one commit per CTA; every wait is bounded; the two cluster barriers are reached by all.
@@ -393,7 +419,6 @@ __device__ __forceinline__ void conv_pair_tile(int tile, int rank, int num_m, in
   if (!ok) m = num_m - 1;
 }
 
-template <int KCH>   // K chunks per ring stage
 __global__ void __launch_bounds__(CONV_THREADS, 1)
 conv3d_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUtensorMap tma_w,
                    const ConvParams p) {
@@ -411,9 +436,8 @@ conv3d_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_const
   const int num_m = p.N * p.T * p.tiles_h * p.tiles_w;
   const int num_tiles = ((num_m + 1) >> 1) * num_n;
   const int chunks = p.Cin / CBK;
-  const int num_kb = 27 * chunks;
   const int half_n = p.BN >> 1;
-  const uint32_t stage_tx = 2u * (static_cast<uint32_t>(p.bh * p.bw) * 128u + static_cast<uint32_t>(half_n) * 128u);
+  const uint32_t stage_tx = 2u * 128u * static_cast<uint32_t>((p.bh + 2) * p.bw + 3 * half_n);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < CP_STAGES; ++s) {
@@ -453,20 +477,20 @@ conv3d_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_const
       conv_pair_tile(tile, rank, num_m, num_n, m, n_blk, tile_ok);
       const TileCoord c = conv_tile(m * num_n + n_blk, p, num_n);
       const int wrow0 = n_blk * p.BN + rank * half_n;
-      for (int kb = 0; kb < num_kb; kb += KCH) {
+      for (int kb = 0; kb < 9 * chunks; ++kb) {
         ok = __all_sync(0xffffffffu, mbar_wait(&tail->empty[stage], phase ^ 1, abort_flag, p.status, ST_TIMEOUT_STAGE_EMPTY));
         if (!ok) break;
         const uint32_t leader_full = cluster_addr(&tail->full[stage], 0);
+        const int dtw = kb / chunks, cc = kb - dtw * chunks, dt = dtw / 3, dw = dtw - 3 * dt;
         if (elect_one()) {
-          if (rank == 0) mbar_arrive_expect_tx(&tail->full[stage], stage_tx * KCH);
+          if (rank == 0) mbar_arrive_expect_tx(&tail->full[stage], stage_tx);
+          uint8_t* sa = smem + stage * CP_STAGE_BYTES;
+          // the tile's rows and the one above and below them; out-of-range coordinates read zeros
+          tma_load_5d_pair(sa, &tma_x, cc * CBK, c.w0 + dw - 1, c.h0 - 1, c.t + dt - 2 + p.halo, c.n, leader_full);
 #pragma unroll
-          for (int q = 0; q < KCH; ++q) {
-            const int tap = (kb + q) / chunks, cc = kb + q - tap * chunks;
-            const int dt = tap / 9, dh = (tap / 3) % 3, dw = tap % 3;
-            uint8_t* sa = smem + stage * CP_STAGE_BYTES + q * p.chunk_bytes;
-            tma_load_5d_pair(sa, &tma_x, cc * CBK, c.w0 + dw - 1, c.h0 + dh - 1, c.t + dt - 2 + p.halo, c.n, leader_full);
-            tma_load_2d_pair(sa + CA_BYTES, &tma_w, tap * p.Cin + cc * CBK, wrow0, leader_full);
-          }
+          for (int dh = 0; dh < 3; ++dh)
+            tma_load_2d_pair(sa + p.chunk_bytes + dh * half_n * 128, &tma_w, ((dt * 3 + dh) * 3 + dw) * p.Cin + cc * CBK, wrow0,
+                             leader_full);
         }
         __syncwarp();
         if (++stage == CP_STAGES) { stage = 0; phase ^= 1; }
@@ -486,18 +510,19 @@ conv3d_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_const
         if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * 256;
-        for (int kb = 0; kb < num_kb; kb += KCH) {
+        for (int kb = 0; kb < 9 * chunks; ++kb) {
           ok = __all_sync(0xffffffffu, mbar_wait(&tail->full[stage], phase, abort_flag, p.status, ST_TIMEOUT_TMA_FULL));
           if (!ok) break;
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(smem + stage * CP_STAGE_BYTES);
+          const uint32_t a_addr = smem_u32(smem + stage * CP_STAGE_BYTES), b_addr = a_addr + p.chunk_bytes;
           const uint32_t empty0 = cluster_addr(&tail->empty[stage], 0), empty1 = cluster_addr(&tail->empty[stage], 1);
           if (elect_one()) {
-  #pragma unroll
-          for (int q = 0; q < KCH; ++q) {
-              const uint32_t aq = a_addr + q * p.chunk_bytes;
-              mma4_f16_pair(d_tmem, make_desc_k128(aq), make_desc_k128(aq + CA_BYTES), idesc, (kb + q) != 0);
-            }
+            // Tap row dh of a tile is the same box bw rows of shared memory further on. The swizzle goes by the address, and
+            // the box starts on a 1,024-byte boundary, so an operand may start at any of its 128-byte rows.
+#pragma unroll
+            for (int dh = 0; dh < 3; ++dh)
+              mma4_f16_pair(d_tmem, make_desc_k128(a_addr + dh * p.bw * 128), make_desc_k128(b_addr + dh * half_n * 128), idesc,
+                            (kb + dh) != 0);
             mma_commit_pair(empty0);   // the stage is free in both CTAs once these MMAs have read it
             mma_commit_pair(empty1);
           }
@@ -706,8 +731,8 @@ void choose_tile(int H, int W, int* bh, int* bw) {
 // cycles that a narrow tile's four MMAs per chunk (2 * BN tensor cycles) do not cover: narrow tiles put two or four
 // chunks behind one barrier; the pair kernel (32 KB per chunk at most) also does so for full-width tiles, where it
 // still gains 4-5 %. The count divides the 27 * chunks_per_tap chunks of a tile.
-int choose_kch(int bn, int chunks_per_tap, bool pair) {
-  int want = bn > 128 ? (pair ? 2 : 1) : (bn > 64 ? 2 : 4);
+int choose_kch(int bn, int chunks_per_tap) {
+  int want = bn > 128 ? 1 : (bn > 64 ? 2 : 4);
   while (want > 1 && chunks_per_tap % want != 0) want >>= 1;
   return want;
 }
@@ -787,41 +812,39 @@ extern "C" int rh3_conv3d_causal(const void* x, const void* w, const void* bias,
     if (int e = make_tmap_2d(&twp, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, w, 27 * Cin, Cout, 27 * Cin * 2, CBK, p.BN / 2,
                              CU_TENSOR_MAP_SWIZZLE_128B))
       return e;
-    p.chunk_bytes = CA_BYTES + p.BN / 2 * 128;
-    p.kch = choose_kch(p.BN, (int)(Cin / CBK), true);
-    p.stage_bytes = p.kch * p.chunk_bytes;
+    const uint32_t box_rows[5] = {CBK, (uint32_t)p.bw, (uint32_t)p.bh + 2, 1, 1};
+    if (int e = make_tmap_nd(&tx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x, 5, dims, strides, box_rows, CU_TENSOR_MAP_SWIZZLE_128B))
+      return e;
+    // a stage: the box (128 rows can be read from row 2 * bw on), then three taps' weight rows
+    p.chunk_bytes = (CBM + 2 * p.bw + 7) / 8 * 1024;
+    p.stage_bytes = p.chunk_bytes + 3 * (p.BN / 2) * 128;
     p.stages = CRING_MAX_BYTES / p.stage_bytes < CMAX_STAGES ? CRING_MAX_BYTES / p.stage_bytes : CMAX_STAGES;
     const int CONV_PAIR_SMEM_BYTES = 1024 + CTAIL_BYTES + p.stages * p.stage_bytes;
-    auto launch_pair = [&](auto kern) -> int {
-      if (int e = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, CONV_PAIR_SMEM_BYTES),
-                             "conv3d pair smem attribute"))
-        return e;
-      cudaLaunchConfig_t cfg{};
-      cudaLaunchAttribute attr{};
-      attr.id = cudaLaunchAttributeClusterDimension;
-      attr.val.clusterDim.x = 2;
-      attr.val.clusterDim.y = 1;
-      attr.val.clusterDim.z = 1;
-      cfg.blockDim = dim3(CONV_THREADS);
-      cfg.dynamicSmemBytes = CONV_PAIR_SMEM_BYTES;
-      cfg.stream = stream;
-      cfg.attrs = &attr;
-      cfg.numAttrs = 1;
-      cfg.gridDim = dim3(2 * (device_sm_count() / 2));
-      int max_clusters = 0;
-      if (cudaOccupancyMaxActiveClusters(&max_clusters, kern, &cfg) != cudaSuccess || max_clusters < 1)
-        return set_error(RH3_ARG_ERROR, "conv3d pair: no cluster of two CTAs can be resident");
-      const int64_t pair_tiles = (num_m + 1) / 2 * num_n;
-      cfg.gridDim = dim3(2 * static_cast<unsigned>(pair_tiles < max_clusters ? pair_tiles : max_clusters));
-      return check_cuda(cudaLaunchKernelEx(&cfg, kern, tx, twp, p), "conv3d pair launch");
-    };
-    if (int e = p.kch == 4 ? launch_pair(conv3d_pair_kernel<4>) : p.kch == 2 ? launch_pair(conv3d_pair_kernel<2>)
-                                                                            : launch_pair(conv3d_pair_kernel<1>))
+    auto kern = conv3d_pair_kernel;
+    if (int e = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, CONV_PAIR_SMEM_BYTES),
+                           "conv3d pair smem attribute"))
       return e;
-    return check_cuda(cudaGetLastError(), "conv3d pair launch");
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 2;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.blockDim = dim3(CONV_THREADS);
+    cfg.dynamicSmemBytes = CONV_PAIR_SMEM_BYTES;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cfg.gridDim = dim3(2 * (device_sm_count() / 2));
+    int max_clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&max_clusters, kern, &cfg) != cudaSuccess || max_clusters < 1)
+      return set_error(RH3_ARG_ERROR, "conv3d pair: no cluster of two CTAs can be resident");
+    const int64_t pair_tiles = (num_m + 1) / 2 * num_n;
+    cfg.gridDim = dim3(2 * static_cast<unsigned>(pair_tiles < max_clusters ? pair_tiles : max_clusters));
+    return check_cuda(cudaLaunchKernelEx(&cfg, kern, tx, twp, p), "conv3d pair launch");
   }
   p.chunk_bytes = CA_BYTES + p.BN * 128;
-  p.kch = choose_kch(p.BN, (int)(Cin / CBK), false);
+  p.kch = choose_kch(p.BN, (int)(Cin / CBK));
   p.stage_bytes = p.kch * p.chunk_bytes;
   p.stages = CRING_MAX_BYTES / p.stage_bytes < CMAX_STAGES ? CRING_MAX_BYTES / p.stage_bytes : CMAX_STAGES;
   const int CONV_SMEM_BYTES = 1024 + CTAIL_BYTES + p.stages * p.stage_bytes;
