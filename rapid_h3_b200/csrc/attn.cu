@@ -35,9 +35,11 @@
 //                 steps at 36,436 keys and in half of them at 4,500; done by the softmax threads the 128
 //                 columns cost them over 1,000 cycles each time.)
 // What bounds it: the serial chain of a softmax thread's step (wait, TMEM load, re-bias, maximum, exponentials,
-// hand-over) at two such warps per scheduler. Measured with H = 32: 16.8 ms at L = 36,436 and 0.340 ms at
-// L = 4,500 before the P buffers and the rescaling warps, 16.0 and 0.315 with them (0.306 with the wide epilogue); timing-only builds without
-// any MMA run 15.0 / 0.283, without the exponentials 14.2 / 0.276, with the barriers alone 7.3 / 0.155.
+// hand-over) at two such warps per scheduler, and, in seconds of it, the power cap: at 15.3 ms a chip draws 900-1,000 W, and
+// forms that need fewer cycles but execute more instructions end where they began. H = 32, ms at L = 36,436 / 4,500:
+// 16.8 / 0.340 before the P buffers and the rescaling warps, 16.0 / 0.305 with them and the wide epilogue, 15.8 / 0.298 with
+// rolled poll loops, 15.3 / 0.295 with narrow bias stores. Timing-only builds of the second form without any MMA ran
+// 15.0 / 0.283, without the exponentials 14.2 / 0.276, with the barriers alone 7.3 / 0.155.
 // TMEM (512 columns): S0 | S1 | O0 | O1, 128 columns each.
 // Tensor-core bound: 4 * Lq * Lk * 128 operations per head.
 #include <limits.h>

@@ -424,14 +424,13 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
       "r"(r[30]), "r"(r[31])
       : "memory");
 }
-// store the same 32-bit value to 32 lanes x 32 consecutive columns (one source register)
+// Store the same 32-bit value to 32 lanes x 32 consecutive columns, eight columns at a time: the instruction reads a run of
+// registers as long as it is wide, so one 32-wide store holds 32 registers of the caller's with copies of the value (in
+// attn_int8 that cost more than the three further instructions: 16.0 / 15.3 ms at L = 36,436, 0.298 / 0.295 at 4,500).
 __device__ __forceinline__ void tmem_st32_splat(uint32_t taddr, uint32_t v) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, "
-      "%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(taddr),
-      "r"(v)
-      : "memory");
+#pragma unroll
+  for (int c = 0; c < 32; c += 8)
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(taddr + c), "r"(v) : "memory");
 }
 // Same wait, tied to the 32 destination registers of an earlier tmem_ld32 so that the compiler cannot
 // move arithmetic on them above the wait (the load delivers its registers asynchronously).
