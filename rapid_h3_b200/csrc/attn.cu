@@ -269,6 +269,7 @@ attn_int8_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  grid_dependency_begin();
   const uint32_t tmem_base = tail->tmem_base;
 
   if (warp < 4) {
@@ -624,8 +625,7 @@ int attn_launch(const void* q8, const float* qs, const void* k8, const float* ks
   if (int e = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ATTN_SMEM_BYTES),
                          "attn smem attribute"))
     return e;
-  kern<<<grid, ATTN_THREADS, ATTN_SMEM_BYTES, stream>>>(tq, tk, tv, p);
-  return check_cuda(cudaGetLastError(), "attn_int8 launch");
+  return check_cuda(launch_chained(kern, grid, ATTN_THREADS, ATTN_SMEM_BYTES, stream, 1, tq, tk, tv, p), "attn_int8 launch");
 }
 }  // namespace
 

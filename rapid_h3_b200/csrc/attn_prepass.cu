@@ -283,6 +283,7 @@ struct RopeStatsParams {
 // kernel of its own, 114 registers)
 template <bool ROPE>
 __global__ void __launch_bounds__(256, 2) rope_stats_kernel(const RopeStatsParams p) {
+  grid_dependency_begin();
   __shared__ float sh[HW_PER_CTA * 4 * D];  // Q side: 16 block maxima; K/V side: per half-warp partials [hw][4][128]
   const int lane = threadIdx.x & 31, l16 = lane & 15, hw = threadIdx.x >> 4;
   const int n_first = p.kv_first ? p.kv_ctas : p.q_ctas;
@@ -409,6 +410,7 @@ __global__ void __launch_bounds__(256, 2) rope_stats_kernel(const RopeStatsParam
 __global__ void __launch_bounds__(128) kv_stats_final_kernel(const float* __restrict__ part, int nchunk, int64_t L,
                                                              float* __restrict__ kmean, float* __restrict__ vmean,
                                                              float* __restrict__ vscale, float v_qmax) {
+  grid_dependency_begin();
   const int h = blockIdx.x, c = threadIdx.x;
   const float* p = part + static_cast<int64_t>(h) * nchunk * 4 * D + c;
   float ksum = 0.f, vsum = 0.f, vhi = -INFINITY, vlo = INFINITY;
@@ -447,6 +449,7 @@ __global__ void __launch_bounds__(256, 3) quant_kv_kernel(const __nv_bfloat16* _
                                                        const float* __restrict__ vmean, const float* __restrict__ vscale,
                                                        int8_t* __restrict__ k8, float* __restrict__ kscale,
                                                        uint8_t* __restrict__ Vt) {
+  grid_dependency_begin();
   __shared__ __align__(16) uint8_t tile[DO_V ? 128 * D : 16];
   __shared__ float red[HW_PER_CTA];
   const int l16 = threadIdx.x & 15, hw = threadIdx.x >> 4;
@@ -587,6 +590,7 @@ __global__ void __launch_bounds__(256) quant_tok_kernel(const __nv_bfloat16* __r
                                                         __nv_bfloat16* __restrict__ x_out, int64_t xo_ss, int64_t xo_sh,
                                                         const float* __restrict__ mean, int8_t* __restrict__ q8,
                                                         float* __restrict__ scales) {
+  grid_dependency_begin();
   const int lane = threadIdx.x & 31, l = lane & 7;
   const int64_t row = static_cast<int64_t>(blockIdx.x) * TOK_ROWS + (threadIdx.x >> 3);
   const bool in_grid = row < Lpad * H;
@@ -673,8 +677,7 @@ int launch_rope_stats(RopeStatsParams p, int kv_ctas, cudaStream_t stream) {
   // keys (64) for 6,196 queries: 67.1 -> 58.6, for 36,436: 264 -> 258.
   p.kv_first = 5ll * kv_ctas <= 4ll * 2 * device_sm_count();
   auto kern = p.tab ? rope_stats_kernel<true> : rope_stats_kernel<false>;
-  kern<<<static_cast<unsigned>(ctas), 256, 0, stream>>>(p);
-  return check_cuda(cudaGetLastError(), "attention pre-pass (rope / statistics) launch");
+  return check_cuda(launch_chained(kern, dim3(static_cast<unsigned>(ctas)), 256, 0, stream, 1, p), "attention pre-pass (rope / statistics) launch");
 }
 
 int kv_stats_run(const void* k, int64_t k_ss, int64_t k_sh, const void* v, int64_t v_ss, int64_t v_sh, int64_t L,
@@ -687,9 +690,9 @@ int kv_stats_run(const void* k, int64_t k_ss, int64_t k_sh, const void* v, int64
   p.v = static_cast<const __nv_bfloat16*>(v); p.v_ss = v_ss; p.v_sh = v_sh;
   p.Lk = L; p.part = part; p.nchunk_k = static_cast<int>(nchunk); p.H = static_cast<int>(H);
   if (int e = launch_rope_stats(p, static_cast<int>(nchunk * H), stream)) return e;
-  kv_stats_final_kernel<<<static_cast<unsigned>(H), 128, 0, stream>>>(part, static_cast<int>(nchunk), L, kmean, vmean,
-                                                                      vscale, 448.f);
-  return check_cuda(cudaGetLastError(), "attention pre-pass (statistics) launch");
+  return check_cuda(launch_chained(kv_stats_final_kernel, dim3(static_cast<unsigned>(H)), 128, 0, stream, 1, part, static_cast<int>(nchunk), L,
+                                   kmean, vmean, vscale, 448.f),
+                    "attention pre-pass (statistics) launch");
 }
 
 }  // namespace
@@ -822,10 +825,10 @@ extern "C" int rh3_attn_quant_qk(const void* x, int64_t x_ss, int64_t x_sh, int6
   RH3_CHECK_ARG(aligned(x, 16) && aligned(codes, 16) && strides16(x_ss, x_sh) && (!mean || aligned(mean, 16)),
                 "attn_quant_qk: rows must be 16-byte aligned (strides multiples of 8 elements)");
   RH3_CHECK_ARG(Lpad / 128 < (1ll << 31), "attn_quant_qk: L too large");
-  quant_kv_kernel<true, false><<<dim3(static_cast<unsigned>(Lpad / 128), static_cast<unsigned>(H)), 256, 0, stream>>>(
+  const cudaError_t launched = launch_chained(quant_kv_kernel<true, false>, dim3(static_cast<unsigned>(Lpad / 128), static_cast<unsigned>(H)), 256, 0, stream, 1,
       static_cast<const __nv_bfloat16*>(x), x_ss, x_sh, nullptr, 0, 0, L, Lpad, mean, nullptr, nullptr,
       static_cast<int8_t*>(codes), scales, nullptr);
-  return check_cuda(cudaGetLastError(), "attn_quant_qk launch");
+  return check_cuda(launched, "attn_quant_qk launch");
 }
 
 extern "C" int rh3_attn_quant_v(const void* v, int64_t v_ss, int64_t v_sh, int64_t L, int64_t Lpad, int64_t H,
@@ -836,10 +839,10 @@ extern "C" int rh3_attn_quant_v(const void* v, int64_t v_ss, int64_t v_sh, int64
   RH3_CHECK_ARG(v && vmean && vscale && vt, "attn_quant_v: null pointer");
   RH3_CHECK_ARG(aligned(v, 16) && aligned(vt, 16) && aligned(vmean, 16) && aligned(vscale, 16) && strides16(v_ss, v_sh),
                 "attn_quant_v: rows must be 16-byte aligned (strides multiples of 8 elements)");
-  quant_kv_kernel<false, true><<<dim3(static_cast<unsigned>(Lpad / 128), static_cast<unsigned>(H)), 256, 0, stream>>>(
+  const cudaError_t launched = launch_chained(quant_kv_kernel<false, true>, dim3(static_cast<unsigned>(Lpad / 128), static_cast<unsigned>(H)), 256, 0, stream, 1,
       nullptr, 0, 0, static_cast<const __nv_bfloat16*>(v), v_ss, v_sh, L, Lpad, nullptr, vmean, vscale, nullptr, nullptr,
       static_cast<uint8_t*>(vt));
-  return check_cuda(cudaGetLastError(), "attn_quant_v launch");
+  return check_cuda(launched, "attn_quant_v launch");
 }
 
 // The whole pre-pass of one attention call (see the head of this file): three launches.
@@ -885,15 +888,18 @@ extern "C" int rh3_attn_prepass(const void* q, int64_t q_ss, int64_t q_sh, int64
   p.tab = static_cast<const __nv_bfloat16*>(rope_table); p.eps = eps; p.H = static_cast<int>(H);
   p.q_ctas = static_cast<int>(nchunk_q * H);
   if (int e = launch_rope_stats(p, static_cast<int>(nchunk_k * H), stream)) return e;
-  kv_stats_final_kernel<<<static_cast<unsigned>(H), 128, 0, stream>>>(p.part, p.nchunk_k, Lk, kmean, vmean, vscale, 448.f);
-  if (int e = check_cuda(cudaGetLastError(), "attn_prepass statistics launch")) return e;
+  if (int e = check_cuda(launch_chained(kv_stats_final_kernel, dim3(static_cast<unsigned>(H)), 128, 0, stream, 1, p.part, p.nchunk_k, Lk, kmean,
+                                        vmean, vscale, 448.f),
+                         "attn_prepass statistics launch"))
+    return e;
   // K is read where the first launch left it: the normalised copy when there is one
   const __nv_bfloat16* kq = k_weight ? static_cast<const __nv_bfloat16*>(k_roped) : static_cast<const __nv_bfloat16*>(k);
   const int64_t kq_ss = k_weight ? kr_ss : k_ss, kq_sh = k_weight ? kr_sh : k_sh;
-  quant_kv_kernel<true, true><<<dim3(static_cast<unsigned>(Lk_pad / 128), static_cast<unsigned>(H)), 256, 0, stream>>>(
-      kq, kq_ss, kq_sh, static_cast<const __nv_bfloat16*>(v), v_ss, v_sh, Lk, Lk_pad, kmean, vmean, vscale,
-      static_cast<int8_t*>(k8), ks, static_cast<uint8_t*>(vt));
-  return check_cuda(cudaGetLastError(), "attn_prepass quantizer launch");
+  const dim3 kv_grid(static_cast<unsigned>(Lk_pad / 128), static_cast<unsigned>(H));
+  return check_cuda(launch_chained(quant_kv_kernel<true, true>, kv_grid, 256, 0, stream, 1, kq, kq_ss, kq_sh,
+                                   static_cast<const __nv_bfloat16*>(v), v_ss, v_sh, Lk, Lk_pad, kmean, vmean, vscale,
+                                   static_cast<int8_t*>(k8), ks, static_cast<uint8_t*>(vt)),
+                    "attn_prepass quantizer launch");
 }
 
 // The pre-pass of the token-scaled attention kernel (rh3_attn_int8_tok): K/V statistics (the K side also applies and
@@ -939,22 +945,26 @@ extern "C" int rh3_attn_tok_prepass(const void* q, int64_t q_ss, int64_t q_sh, i
   p.Lk = Lk; p.part = static_cast<float*>(scratch); p.nchunk_k = static_cast<int>(nchunk_k);
   p.tab = static_cast<const __nv_bfloat16*>(rope_table); p.eps = eps; p.H = static_cast<int>(H);
   if (int e = launch_rope_stats(p, static_cast<int>(nchunk_k * H), stream)) return e;
-  kv_stats_final_kernel<<<static_cast<unsigned>(H), 128, 0, stream>>>(p.part, p.nchunk_k, Lk, kmean, vmean, vscale, 127.f);
-  if (int e = check_cuda(cudaGetLastError(), "attn_tok_prepass statistics launch")) return e;
+  if (int e = check_cuda(launch_chained(kv_stats_final_kernel, dim3(static_cast<unsigned>(H)), 128, 0, stream, 1, p.part, p.nchunk_k, Lk, kmean,
+                                        vmean, vscale, 127.f),
+                         "attn_tok_prepass statistics launch"))
+    return e;
   // 3: Q rows (norm + rope fused), 4: K rows from the normalised copy, 5: V
-  quant_tok_kernel<false><<<static_cast<unsigned>(q_ctas), 256, 0, stream>>>(
-      static_cast<const __nv_bfloat16*>(q), q_ss, q_sh, Lq, Lq_pad, static_cast<int>(H),
-      static_cast<const __nv_bfloat16*>(q_weight), eps, static_cast<const __nv_bfloat16*>(rope_table),
-      static_cast<__nv_bfloat16*>(q_roped), qr_ss, qr_sh, nullptr, static_cast<int8_t*>(q8), qs);
-  if (int e = check_cuda(cudaGetLastError(), "attn_tok_prepass Q launch")) return e;
+  if (int e = check_cuda(
+          launch_chained(quant_tok_kernel<false>, dim3(static_cast<unsigned>(q_ctas)), 256, 0, stream, 1,
+                         static_cast<const __nv_bfloat16*>(q), q_ss, q_sh, Lq, Lq_pad, static_cast<int>(H),
+                         static_cast<const __nv_bfloat16*>(q_weight), eps, static_cast<const __nv_bfloat16*>(rope_table),
+                         static_cast<__nv_bfloat16*>(q_roped), qr_ss, qr_sh, nullptr, static_cast<int8_t*>(q8), qs),
+          "attn_tok_prepass Q launch"))
+    return e;
   const __nv_bfloat16* kq = k_weight ? static_cast<const __nv_bfloat16*>(k_roped) : static_cast<const __nv_bfloat16*>(k);
   const int64_t kq_ss = k_weight ? kr_ss : k_ss, kq_sh = k_weight ? kr_sh : k_sh;
-  quant_tok_kernel<true><<<static_cast<unsigned>(k_ctas), 256, 0, stream>>>(
-      kq, kq_ss, kq_sh, Lk, Lk_pad, static_cast<int>(H), nullptr, eps, nullptr, nullptr, 0, 0, kmean,
-      static_cast<int8_t*>(k8), ksb);
-  if (int e = check_cuda(cudaGetLastError(), "attn_tok_prepass K launch")) return e;
-  quant_kv_kernel<false, true, true><<<dim3(static_cast<unsigned>(Lk_pad / 128), static_cast<unsigned>(H)), 256, 0, stream>>>(
-      nullptr, 0, 0, static_cast<const __nv_bfloat16*>(v), v_ss, v_sh, Lk, Lk_pad, nullptr, vmean, vscale, nullptr, nullptr,
-      static_cast<uint8_t*>(vt));
-  return check_cuda(cudaGetLastError(), "attn_tok_prepass V launch");
+  if (int e = check_cuda(launch_chained(quant_tok_kernel<true>, dim3(static_cast<unsigned>(k_ctas)), 256, 0, stream, 1, kq, kq_ss, kq_sh, Lk, Lk_pad,
+                                        static_cast<int>(H), nullptr, eps, nullptr, nullptr, 0, 0, kmean, static_cast<int8_t*>(k8), ksb),
+                         "attn_tok_prepass K launch"))
+    return e;
+  const dim3 kv_grid(static_cast<unsigned>(Lk_pad / 128), static_cast<unsigned>(H));
+  return check_cuda(launch_chained(quant_kv_kernel<false, true, true>, kv_grid, 256, 0, stream, 1, nullptr, 0, 0, static_cast<const __nv_bfloat16*>(v),
+                                   v_ss, v_sh, Lk, Lk_pad, nullptr, vmean, vscale, nullptr, nullptr, static_cast<uint8_t*>(vt)),
+                    "attn_tok_prepass V launch");
 }

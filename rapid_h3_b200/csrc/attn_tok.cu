@@ -237,6 +237,7 @@ attn_tok_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  grid_dependency_begin();
   const uint32_t tmem_base = tail->tmem_base;
 
   if (warp < 4) {
@@ -528,6 +529,5 @@ extern "C" int rh3_attn_int8_tok(const void* q8, const float* qs, const void* k8
   if (int e = check_cuda(cudaFuncSetAttribute(attn_tok_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TOK_SMEM_BYTES),
                          "attn_tok smem attribute"))
     return e;
-  attn_tok_kernel<<<grid, TOK_THREADS, TOK_SMEM_BYTES, stream>>>(tq, tk, tv, p);
-  return check_cuda(cudaGetLastError(), "attn_int8_tok launch");
+  return check_cuda(launch_chained(attn_tok_kernel, grid, TOK_THREADS, TOK_SMEM_BYTES, stream, 1, tq, tk, tv, p), "attn_int8_tok launch");
 }

@@ -37,6 +37,16 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// For kernels launched with launch_chained. All threads wait before the first access to global memory: what the kernels before
+// this one in the stream wrote is visible then, and what they read may be overwritten. The trigger only allows the next kernel's
+// CTAs to start (it waits for all of this one in its turn).
+__device__ __forceinline__ void grid_dependency_wait() { cudaGridDependencySynchronize(); }
+__device__ __forceinline__ void grid_dependency_trigger() { cudaTriggerProgrammaticLaunchCompletion(); }
+__device__ __forceinline__ void grid_dependency_begin() {
+  grid_dependency_trigger();
+  grid_dependency_wait();
+}
+
 // ---------------------------------------------------------------------------------------------
 // mbarrier
 // ---------------------------------------------------------------------------------------------
@@ -620,6 +630,33 @@ int read_and_clear_status(cudaStream_t stream, int* out);
 }  // namespace rh3
 
 #define RH3_ARG_ERROR (-1)
+
+namespace rh3 {
+// Launches `kern` so that its CTAs may start while the kernel before it in the stream still drains (programmatic stream
+// serialisation): every kernel launched this way calls grid_dependency_wait() before it touches global memory, and one that
+// says grid_dependency_trigger() lets the next one start as soon as its own CTAs have all started. What overlaps is the launch
+// latency, the set-up of barriers and tensor memory and the ramp-up of a kernel with the tail of the one before: 1-2 us for each
+// launch of a chain of short kernels. `cluster` > 1 launches clusters of that many CTAs.
+template <class... Params, class... Args>
+cudaError_t launch_chained(void (*kern)(Params...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, unsigned cluster,
+                           Args&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[2]{};
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kern, Params(args)...);
+}
+}  // namespace rh3
 #define RH3_CHECK_ARG(cond, ...)                          \
   do {                                                    \
     if (!(cond)) return rh3::set_error(RH3_ARG_ERROR, __VA_ARGS__); \

@@ -273,6 +273,7 @@ conv3d_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  grid_dependency_begin();
   const uint32_t tmem_base = tail->tmem_base;
 
   if (warp == 0) {
@@ -459,6 +460,7 @@ conv3d_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_const
   __syncthreads();
   cluster_sync_all();   // both CTAs' barriers exist before anything arrives on them from the other side
   tc_fence_after();
+  grid_dependency_begin();
   const uint32_t tmem_base = tail->tmem_base;
 
   if (warp == 0) {
@@ -591,6 +593,7 @@ conv3d_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_const
 // sums[n][g] = (sum, sum of squares) over all row blocks of sample n, added in a fixed order in fp64.
 __global__ void __launch_bounds__(256) gn_reduce_kernel(const float* __restrict__ part, int64_t rows_per_sample,
                                                         double* __restrict__ sums) {
+  grid_dependency_begin();
   __shared__ double red[2][256];
   const int n = blockIdx.x / GN_GROUPS, g = blockIdx.x % GN_GROUPS;
   const float* p = part + (static_cast<int64_t>(n) * rows_per_sample * GN_GROUPS + g) * 2;
@@ -640,6 +643,7 @@ __global__ void __launch_bounds__(256) gn_silu_kernel(const __nv_bfloat16* __res
                                                       const __nv_bfloat16* __restrict__ gamma,
                                                       const __nv_bfloat16* __restrict__ beta, int64_t sites_per_sample,
                                                       int C, __nv_bfloat16* __restrict__ y) {
+  grid_dependency_begin();
   __shared__ float2 mr_s[GN_GROUPS];
   if (FROM_SUMS) {
     if (threadIdx.x < GN_GROUPS) {
@@ -695,6 +699,7 @@ __global__ void __launch_bounds__(256) gn_silu_kernel(const __nv_bfloat16* __res
 // (the first frame is not repeated: T frames become 2T - 1).
 __global__ void __launch_bounds__(256) upsample_kernel(const __nv_bfloat16* __restrict__ x, int T, int H, int W, int C,
                                                        int64_t total_vec, __nv_bfloat16* __restrict__ y) {
+  grid_dependency_begin();
   const int64_t v = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x;
   if (v >= total_vec) return;
   const int vec_per_site = C >> 3;
@@ -840,8 +845,8 @@ extern "C" int rh3_conv3d_causal(const void* x, const void* w, const void* bias,
     if (cudaOccupancyMaxActiveClusters(&max_clusters, kern, &cfg) != cudaSuccess || max_clusters < 1)
       return set_error(RH3_ARG_ERROR, "conv3d pair: no cluster of two CTAs can be resident");
     const int64_t pair_tiles = (num_m + 1) / 2 * num_n;
-    cfg.gridDim = dim3(2 * static_cast<unsigned>(pair_tiles < max_clusters ? pair_tiles : max_clusters));
-    return check_cuda(cudaLaunchKernelEx(&cfg, kern, tx, twp, p), "conv3d pair launch");
+    const unsigned ctas = 2 * static_cast<unsigned>(pair_tiles < max_clusters ? pair_tiles : max_clusters);
+    return check_cuda(launch_chained(kern, dim3(ctas), CONV_THREADS, CONV_PAIR_SMEM_BYTES, stream, 2, tx, twp, p), "conv3d pair launch");
   }
   p.chunk_bytes = CA_BYTES + p.BN * 128;
   p.kch = choose_kch(p.BN, (int)(Cin / CBK));
@@ -854,8 +859,7 @@ extern "C" int rh3_conv3d_causal(const void* x, const void* w, const void* bias,
     if (int e = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, CONV_SMEM_BYTES),
                            "conv3d smem attribute"))
       return e;
-    kern<<<grid, CONV_THREADS, CONV_SMEM_BYTES, stream>>>(tx, tw, p);
-    return 0;
+    return check_cuda(launch_chained(kern, dim3(grid), CONV_THREADS, CONV_SMEM_BYTES, stream, 1, tx, tw, p), "conv3d launch");
   };
   if (int e = p.kch == 4 ? launch_single(conv3d_kernel<4>) : p.kch == 2 ? launch_single(conv3d_kernel<2>)
                                                                         : launch_single(conv3d_kernel<1>))
@@ -866,8 +870,8 @@ extern "C" int rh3_conv3d_causal(const void* x, const void* w, const void* bias,
 extern "C" int rh3_gn_reduce(const float* gn_part, int64_t rows_per_sample, int64_t N, double* sums,
                              cudaStream_t stream) {
   RH3_CHECK_ARG(gn_part && sums && rows_per_sample > 0 && N > 0 && N * GN_GROUPS < (1ll << 31), "gn_reduce: bad argument");
-  gn_reduce_kernel<<<static_cast<unsigned>(N * GN_GROUPS), 256, 0, stream>>>(gn_part, rows_per_sample, sums);
-  return check_cuda(cudaGetLastError(), "gn_reduce launch");
+  return check_cuda(launch_chained(gn_reduce_kernel, dim3(static_cast<unsigned>(N * GN_GROUPS)), 256, 0, stream, 1, gn_part, rows_per_sample, sums),
+                    "gn_reduce launch");
 }
 
 namespace {
@@ -883,10 +887,10 @@ int gn_silu_launch(const void* x, const float* mean_rstd, const double* sums, do
   const int64_t cap = static_cast<int64_t>(device_sm_count()) * 16;  // a few waves of resident blocks, grid-stride beyond
   const dim3 grid(static_cast<unsigned>(want < cap ? want : cap), static_cast<unsigned>(N));
   auto kern = sums ? gn_silu_kernel<true> : gn_silu_kernel<false>;
-  kern<<<grid, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(x), mean_rstd, sums, 1.0 / count, eps,
-                                 static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta),
-                                 sites_per_sample, (int)C, static_cast<__nv_bfloat16*>(y));
-  return check_cuda(cudaGetLastError(), "gn_silu_apply launch");
+  return check_cuda(launch_chained(kern, grid, 256, 0, stream, 1, static_cast<const __nv_bfloat16*>(x), mean_rstd, sums, 1.0 / count, eps,
+                                   static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta),
+                                   sites_per_sample, (int)C, static_cast<__nv_bfloat16*>(y)),
+                    "gn_silu_apply launch");
 }
 }  // namespace
 
@@ -930,9 +934,10 @@ extern "C" int rh3_upsample_causal2x(const void* x, void* y, int64_t N, int64_t 
                 "upsample_causal2x: bad argument");
   const int64_t total_vec = N * (2 * T - 1) * 2 * H * 2 * W * (C / 8);
   RH3_CHECK_ARG((total_vec + 255) / 256 < (1ll << 31), "upsample_causal2x: tensor too large");
-  upsample_kernel<<<static_cast<unsigned>((total_vec + 255) / 256), 256, 0, stream>>>(
-      static_cast<const __nv_bfloat16*>(x), (int)T, (int)H, (int)W, (int)C, total_vec, static_cast<__nv_bfloat16*>(y));
-  return check_cuda(cudaGetLastError(), "upsample_causal2x launch");
+  return check_cuda(launch_chained(upsample_kernel, dim3(static_cast<unsigned>((total_vec + 255) / 256)), 256, 0, stream, 1,
+                                   static_cast<const __nv_bfloat16*>(x), (int)T, (int)H, (int)W, (int)C, total_vec,
+                                   static_cast<__nv_bfloat16*>(y)),
+                    "upsample_causal2x launch");
 }
 
 extern "C" int rh3_depth_to_space8(const void* y, void* rgb, int64_t N, int64_t T, int64_t H, int64_t W,

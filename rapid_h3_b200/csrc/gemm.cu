@@ -382,6 +382,7 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   volatile int* abort_flag = &tail->abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (EPI == EPI_F32_ADD) grid_dependency_begin();   // its row count is read on the device
   const int M = gemm_rows<EPI>(p);
   const int num_m = (M + BM - 1) / BM, num_n = (p.N + BN - 1) / BN;
   const int num_tiles = num_m * num_n;
@@ -406,6 +407,7 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if (EPI != EPI_F32_ADD) grid_dependency_begin();
   const uint32_t tmem_base = tail->tmem_base;
 
   if (warp == 0) {
@@ -575,6 +577,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_cta_rank();          // 0 = the even CTA of the pair: it issues the MMAs
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
+  if (EPI == EPI_F32_ADD) grid_dependency_begin();   // its row count is read on the device
   const int M = gemm_rows<EPI>(p);
   const int num_m = (M + 2 * BM - 1) / (2 * BM), num_n = (p.N + BN - 1) / BN;
   const int num_tiles = num_m * num_n;
@@ -600,6 +603,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   __syncthreads();
   cluster_sync_all();   // both CTAs' barriers exist before anything arrives on them from the other side
   tc_fence_after();
+  if (EPI != EPI_F32_ADD) grid_dependency_begin();
   const uint32_t tmem_base = tail->tmem_base;
 
   if (warp == 0) {
@@ -760,9 +764,7 @@ int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmPar
   if (cudaOccupancyMaxActiveClusters(&max_clusters, kern, &cfg) != cudaSuccess || max_clusters < 1)
     return set_error(RH3_ARG_ERROR, "gemm pair: no cluster of two CTAs can be resident");
   const int pairs = num_tiles < max_clusters ? num_tiles : max_clusters;
-  cfg.gridDim = dim3(2 * pairs);
-  if (int e = check_cuda(cudaLaunchKernelEx(&cfg, kern, ta, tb, p), "gemm pair launch")) return e;
-  return check_cuda(cudaGetLastError(), "gemm pair launch");
+  return check_cuda(launch_chained(kern, dim3(2 * pairs), GEMM_THREADS, PAIR_SMEM_BYTES, stream, 2, ta, tb, p), "gemm pair launch");
 }
 
 template <int KIND_F8, int EPI>
@@ -777,8 +779,7 @@ int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
     return e;
   const int num_tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
   const int grid = num_tiles < device_sm_count() ? num_tiles : device_sm_count();
-  kern<<<grid, GEMM_THREADS, GEMM_SMEM_BYTES, stream>>>(ta, tb, p);
-  return check_cuda(cudaGetLastError(), "gemm launch");
+  return check_cuda(launch_chained(kern, dim3(grid), GEMM_THREADS, GEMM_SMEM_BYTES, stream, 1, ta, tb, p), "gemm launch");
 }
 
 int gemm_common(const void* xq, int64_t lda, const void* wq, const float* xs, const float* ws, int64_t M, int64_t N,

@@ -146,6 +146,7 @@ __device__ __forceinline__ void load_row(const QuantParams& p, int64_t row, int 
 // are issued before the current row is reduced and stored, so every CTA always has a row in flight.
 template <int KIND, int OUT_FP8, int T, int CPT, int ROT>
 __global__ void __launch_bounds__(T) quant_rows_kernel(const QuantParams p) {
+  grid_dependency_begin();
   __shared__ float red[T / 32];
   const int tid = threadIdx.x;
   const int nchunk = static_cast<int>(p.K >> 3);
@@ -252,6 +253,7 @@ template <int T, int CPT>
 __global__ void __launch_bounds__(T) rms_norm_rows_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx,
                                                           const __nv_bfloat16* __restrict__ w, float eps, int64_t M, int K,
                                                           __nv_bfloat16* __restrict__ out, int64_t ldo) {
+  grid_dependency_begin();
   __shared__ float red[T / 32];
   const int tid = threadIdx.x, nchunk = K >> 3;
   QuantParams p{};
@@ -436,6 +438,7 @@ template <int KIND, int OUT_FP8, int ROT = 0>
 int launch_quant(const QuantParams& p, cudaStream_t stream) {
   const int64_t nchunk = p.K >> 3;
   if (p.M == 0) return 0;
+  cudaError_t launched = cudaSuccess;
   // as many CTAs as are resident at once (a multiple of the SM count), each looping over its rows
 #define RH3_Q(T_, CPT_)                                                                                \
   do {                                                                                                 \
@@ -443,7 +446,7 @@ int launch_quant(const QuantParams& p, cudaStream_t stream) {
     int occ = 1;                                                                                       \
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, T_, 0) != cudaSuccess || occ < 1) occ = 1; \
     const int64_t resident = static_cast<int64_t>(device_sm_count()) * occ;                           \
-    kern<<<static_cast<unsigned>(p.M < resident ? p.M : resident), T_, 0, stream>>>(p);               \
+    launched = launch_chained(kern, dim3(static_cast<unsigned>(p.M < resident ? p.M : resident)), T_, 0, stream, 1, p); \
   } while (0)
   if (nchunk <= 128) RH3_Q(128, 1);
   else if (nchunk <= 256) RH3_Q(128, 2);
@@ -454,7 +457,7 @@ int launch_quant(const QuantParams& p, cudaStream_t stream) {
   else if (nchunk <= 8192) RH3_Q(1024, 8);
   else return set_error(RH3_ARG_ERROR, "quant_rows: K=%lld is larger than 65536", (long long)p.K);
 #undef RH3_Q
-  return check_cuda(cudaGetLastError(), "quant_rows launch");
+  return check_cuda(launched, "quant_rows launch");
 }
 
 int check_common(const void* x, int64_t ldx, int64_t M, int64_t K, const void* q, int64_t ldq, const float* s) {
@@ -639,13 +642,14 @@ extern "C" int rh3_rms_norm_rows(const void* x, int64_t ldx, const void* w, floa
   RH3_CHECK_ARG(K <= 16384, "rms_norm_rows: K=%lld is larger than 16384", (long long)K);
   if (M == 0) return 0;
   const int64_t nchunk = K >> 3;
+  cudaError_t launched = cudaSuccess;
 #define RH3_RN(T_, CPT_)                                                                                          \
   do {                                                                                                            \
     auto kern = rms_norm_rows_kernel<T_, CPT_>;                                                                   \
     const int64_t resident = static_cast<int64_t>(device_sm_count()) * (2048 / T_ < 8 ? 2048 / T_ : 8);           \
-    kern<<<static_cast<unsigned>(M < resident ? M : resident), T_, 0, stream>>>(                                  \
-        static_cast<const __nv_bfloat16*>(x), ldx, static_cast<const __nv_bfloat16*>(w), eps, M, (int)K,          \
-        static_cast<__nv_bfloat16*>(out), ldo);                                                                   \
+    launched = launch_chained(kern, dim3(static_cast<unsigned>(M < resident ? M : resident)), T_, 0, stream, 1,   \
+                              static_cast<const __nv_bfloat16*>(x), ldx, static_cast<const __nv_bfloat16*>(w),    \
+                              eps, M, (int)K, static_cast<__nv_bfloat16*>(out), ldo);                             \
   } while (0)
   if (nchunk <= 128) RH3_RN(128, 1);
   else if (nchunk <= 256) RH3_RN(128, 2);
@@ -653,7 +657,7 @@ extern "C" int rh3_rms_norm_rows(const void* x, int64_t ldx, const void* w, floa
   else if (nchunk <= 1024) RH3_RN(256, 4);
   else RH3_RN(512, 4);
 #undef RH3_RN
-  return check_cuda(cudaGetLastError(), "rms_norm_rows launch");
+  return check_cuda(launched, "rms_norm_rows launch");
 }
 
 extern "C" int rh3_te_quant_counted(const float* x, int64_t ldx, int64_t M, int64_t K, float ratio, void* q1, float* s1,

@@ -97,6 +97,7 @@ __device__ __forceinline__ void unpack16h(const uint4* raw, float* v) {
 
 template <int T, int ACT>
 __global__ void __launch_bounds__(T) vae_out_quant_kernel(const OutQuantParams p) {
+  grid_dependency_begin();
   __shared__ __align__(16) float patch[T / 16][PATCH_F];
   __shared__ float red[2][T / 16], red_ss[2][T / 16];  // two sets: one barrier per reduction and row is enough
   const int tid = threadIdx.x, grp = tid >> 4, t = tid & 15;
@@ -251,8 +252,8 @@ int launch_out_quant(const OutQuantParams& p, cudaStream_t stream) {
   int occ = 1;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, T, 0) != cudaSuccess || occ < 1) occ = 1;
   const int64_t resident = static_cast<int64_t>(device_sm_count()) * occ;
-  kern<<<static_cast<unsigned>(p.rows < resident ? p.rows : resident), T, 0, stream>>>(p);
-  return check_cuda(cudaGetLastError(), "vae_out_quant launch");
+  return check_cuda(launch_chained(kern, dim3(static_cast<unsigned>(p.rows < resident ? p.rows : resident)), T, 0, stream, 1, p),
+                    "vae_out_quant launch");
 }
 template <int ACT>
 int launch_out_quant_act(const OutQuantParams& p, cudaStream_t stream) {
