@@ -14,10 +14,10 @@
 // (reference: custom_nodes/rapid_h3/csrc/fp8_rowwise.cu:294-304 plain epilogue, :333-336 gated
 //  residual, :74-93 SwiGLU store; PyTorch emulation custom_nodes/rapid_h3/kernels.py:129-137).
 //
-// Structure (one persistent CTA per SM, 320 threads):
-//   warp 0      TMA producer: 128x128-byte A tile + 256x128-byte B tile per stage, 4-stage ring
-//   warp 1      MMA issuer: 4 x tcgen05.mma (M128 N256 K32) per stage into a TMEM accumulator;
-//               two 256-column accumulators so the epilogue of tile i overlaps the main loop of i+1
+// Structure (one persistent CTA per SM, 320 threads), tiles of 128 rows (256 on CTA pairs) x 256, 128 or 64 columns:
+//   warp 0      TMA producer: A rows and B rows of one to four 128-byte K slabs per stage, a 192 KB ring
+//   warp 1      MMA issuer: 4 x tcgen05.mma (K32) per slab into a TMEM accumulator;
+//               two accumulators so the epilogue of tile i overlaps the main loop of i+1
 //   warps 2..9  epilogue: tcgen05.ld 32 columns at a time, dequantize, fused epilogue, 64-byte
 //               contiguous bf16 stores per thread-row
 // Tensor-core bound: 2*M*N*K operations per call.
@@ -33,16 +33,25 @@ namespace {
 constexpr int BM = 128;
 constexpr int BN = 256;
 constexpr int BK = 128;  // bytes (= elements for 8-bit operands) along K per stage
-constexpr int STAGES = 4;
 constexpr int A_BYTES = BM * BK;
-constexpr int B_BYTES = BN * BK;
-constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+constexpr int RING_BYTES = 4 * (A_BYTES + BN * BK);   // what a ring may take: 192 KB
+constexpr int MAX_STAGES = 10;
+// Ring of a kernel whose CTAs load `brows` rows of B per stage: as many stages as fit, so that narrow tiles, whose stages
+// hold less, still have enough bytes in flight to cover the latency of L2.
+__host__ __device__ constexpr int slab_bytes(int brows) { return A_BYTES + brows * BK; }
+// K slabs behind one barrier: the round trip of a stage (wait, four MMAs, commit) is a few hundred cycles in the issuing warp,
+// which the 128 or 256 tensor cycles of a narrow slab do not cover. us at N = K = 4,096 with one, two and four slabs: 37 rows,
+// 64-column tiles 10.8 / 8.7 / 7.5, 200 rows, 64-column pair tiles 11.3 / 8.4 / 8.9, 512 rows, 128-column pair tiles
+// 12.7 / 10.3; two of 256 columns measure the same as one or worse (12.5 / 14.1 at 37 rows).
+__host__ __device__ constexpr int slabs_per_stage(int tn, bool pair) { return tn == 64 && !pair ? 4 : tn < BN ? 2 : 1; }
+__host__ __device__ constexpr int ring_stages(int brows, int slabs) {
+  return RING_BYTES / (slabs * slab_bytes(brows)) < MAX_STAGES ? RING_BYTES / (slabs * slab_bytes(brows)) : MAX_STAGES;
+}
 // Two warps per TMEM lane quadrant, each draining half of the accumulator's columns: with one, the epilogue of a short K
 // outlasts the main loop of the next tile (w1 + SwiGLU in fp16, 3,594 x 16,384 x 2,048: 187 us with four warps and the
 // division routine, 85 with eight and silu_div; fp16 with residual, N = 2,048, K = 8,192: 61 -> 56; long-K bf16 shapes
 // measure the same). The price is registers: 168 a thread at 320 threads, which every epilogue has to fit.
 constexpr int EPI_WARPS = 8;
-constexpr int EPI_COLS = BN / (EPI_WARPS / 4);
 constexpr int EPI_THREADS = 32 * EPI_WARPS;
 constexpr int GEMM_THREADS = 64 + EPI_THREADS;
 #ifndef RH3_GEMM_GROUP_M
@@ -55,6 +64,7 @@ __host__ __device__ constexpr bool is_gated(int epi) { return epi == EPI_GATED |
 
 struct GemmParams {
   int M, N, K;
+  int a_rows;                 // rows of A that a load brings in: 128, or fewer where the call has fewer (the rest of the tile is not read out)
   const float* xs;
   const float* ws;
   const __nv_bfloat16* bias;  // EPI_PLAIN (optional), EPI_BIAS2
@@ -82,8 +92,8 @@ struct GemmParams {
 };
 
 struct __align__(8) GemmSmemTail {
-  uint64_t full[STAGES];
-  uint64_t empty[STAGES];
+  uint64_t full[MAX_STAGES];
+  uint64_t empty[MAX_STAGES];
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
   uint32_t tmem_base;
@@ -93,7 +103,7 @@ struct __align__(8) GemmSmemTail {
   float aux2[BN];  // residual scale (EPI_F16) or second gate (EPI_GATED2) as fp32
 };
 
-constexpr int GEMM_SMEM_BYTES = STAGES * STAGE_BYTES + sizeof(GemmSmemTail) + 1024;  // +1024 alignment slack
+constexpr int GEMM_SMEM_BYTES = RING_BYTES + sizeof(GemmSmemTail) + 1024;  // +1024 alignment slack
 
 __device__ __forceinline__ void tile_coords(int tile, int num_m, int num_n, int& m_blk, int& n_blk) {
   const int per_group = GROUP_M * num_n;
@@ -111,7 +121,7 @@ __device__ __forceinline__ void tile_coords(int tile, int num_m, int num_n, int&
 // The residual row of an epilogue that adds one (gated residual, fp16 residual): its EPI_COLS columns are asked into L2
 // while the tile's MMAs still run, so the epilogue's loads do not wait on HBM (the residual of a step is far
 // larger than L2 and cold by the time its tile comes up).
-template <int EPI>
+template <int EPI, int EPI_COLS>
 __device__ __forceinline__ void prefetch_residual(const GemmParams& p, int row, bool row_ok, int n0) {  // n0: first of EPI_COLS columns
   if (!row_ok) return;
   if (is_gated(EPI)) {
@@ -179,7 +189,7 @@ __device__ __forceinline__ int gemm_rows(const GemmParams& p) {
   return EPI == EPI_F32_ADD ? min(p.M, *p.m_dev) : p.M;
 }
 
-template <int KIND_F8, int EPI>
+template <int KIND_F8, int EPI, int EPI_COLS>
 __device__ __forceinline__ void epilogue_row(const GemmParams& p, const GemmSmemTail* tail, uint32_t t_row, int row,
                                              bool row_ok, float xs, int n0, int c_first, const uint4* res0) {
   // `c_first`: first 32-column chunk of this warp's EPI_COLS columns
@@ -360,6 +370,13 @@ __device__ __forceinline__ void epilogue_row(const GemmParams& p, const GemmSmem
     }
     return;
   }
+  if (EPI_COLS == 32) {
+    uint32_t r[32];
+    tmem_ld32(t_row + c_first * 32, r);
+    tmem_ld_wait_regs(r);
+    chunk(r, c_first, nullptr);
+    return;
+  }
 #pragma unroll 1
   for (int c = c_first; c < c_first + EPI_COLS / 32; c += 2) {
     uint32_t ra[32], rb[32];
@@ -372,19 +389,20 @@ __device__ __forceinline__ void epilogue_row(const GemmParams& p, const GemmSmem
   }
 }
 
-template <int KIND_F8, int EPI>
+template <int KIND_F8, int EPI, int TN>   // TN: columns of a tile
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_w8a8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                  const GemmParams p) {
+  constexpr int KS = slabs_per_stage(TN, false), STAGES = ring_stages(TN, KS), STAGE_BYTES = KS * slab_bytes(TN), EPI_COLS = TN / (EPI_WARPS / 4);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  GemmSmemTail* tail = reinterpret_cast<GemmSmemTail*>(smem + STAGES * STAGE_BYTES);
+  GemmSmemTail* tail = reinterpret_cast<GemmSmemTail*>(smem + RING_BYTES);
   volatile int* abort_flag = &tail->abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (EPI == EPI_F32_ADD) grid_dependency_begin();   // its row count is read on the device
   const int M = gemm_rows<EPI>(p);
-  const int num_m = (M + BM - 1) / BM, num_n = (p.N + BN - 1) / BN;
+  const int num_m = (M + BM - 1) / BM, num_n = (p.N + TN - 1) / TN;
   const int num_tiles = num_m * num_n;
   const int num_kb = (p.K + BK - 1) / BK;
 
@@ -421,16 +439,18 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
         int m_blk, n_blk;
         tile_coords(tile, num_m, num_n, m_blk, n_blk);
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = 0; kb < num_kb; kb += KS) {   // a slab past K reads zeros
           if (!mbar_wait(&tail->empty[stage], phase ^ 1, abort_flag, p.status, ST_TIMEOUT_STAGE_EMPTY)) {
             ok = false;
             break;
           }
           uint8_t* sa = smem + stage * STAGE_BYTES;
-          uint8_t* sb = sa + A_BYTES;
-          mbar_arrive_expect_tx(&tail->full[stage], STAGE_BYTES);
-          tma_load_2d(sa, &tma_a, kb * BK, m_blk * BM, &tail->full[stage]);
-          tma_load_2d(sb, &tma_b, kb * BK, n_blk * BN, &tail->full[stage]);
+          mbar_arrive_expect_tx(&tail->full[stage], KS * (p.a_rows + TN) * BK);
+#pragma unroll
+          for (int q = 0; q < KS; ++q, sa += slab_bytes(TN)) {
+            tma_load_2d(sa, &tma_a, (kb + q) * BK, m_blk * BM, &tail->full[stage]);
+            tma_load_2d(sa + A_BYTES, &tma_b, (kb + q) * BK, n_blk * TN, &tail->full[stage]);
+          }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
       }
@@ -443,7 +463,7 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     // (rh3_selftest_mma_rate, patterns 1 and 3) a single lane in the loop reaches 3.2 POP/s and the converged warp
     // 4.5; in this kernel the two forms measure the same (2.7 POP/s at K = 4096), so the issuing thread is not what
     // holds the tensor pipe at 70 % here.
-    constexpr uint32_t idesc = KIND_F8 ? make_idesc(1, 0, 0, BM, BN) : make_idesc(2, 1, 1, BM, BN);
+    constexpr uint32_t idesc = KIND_F8 ? make_idesc(1, 0, 0, BM, TN) : make_idesc(2, 1, 1, BM, TN);
     int stage = 0;
     uint32_t phase = 0;
     int acc = 0;
@@ -454,15 +474,18 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       if (!ok) break;
       tc_fence_after();
       const uint32_t d_tmem = tmem_base + acc * BN;
-      for (int kb = 0; kb < num_kb; ++kb) {
+      for (int kb = 0; kb < num_kb; kb += KS) {   // a slab past K reads zeros
         ok = __all_sync(0xffffffffu, mbar_wait(&tail->full[stage], phase, abort_flag, p.status, ST_TIMEOUT_TMA_FULL));
         if (!ok) break;
         tc_fence_after();
         const uint32_t a_addr = smem_u32(smem + stage * STAGE_BYTES);
-        const uint32_t b_addr = a_addr + A_BYTES;
         if (elect_one()) {
-          if (KIND_F8) mma4_f8_ss(d_tmem, make_desc_k128(a_addr), make_desc_k128(b_addr), idesc, kb != 0);
-          else mma4_i8_ss(d_tmem, make_desc_k128(a_addr), make_desc_k128(b_addr), idesc, kb != 0);
+#pragma unroll
+          for (int q = 0; q < KS; ++q) {
+            const uint32_t aq = a_addr + q * slab_bytes(TN);
+            if (KIND_F8) mma4_f8_ss(d_tmem, make_desc_k128(aq), make_desc_k128(aq + A_BYTES), idesc, (kb + q) != 0);
+            else mma4_i8_ss(d_tmem, make_desc_k128(aq), make_desc_k128(aq + A_BYTES), idesc, (kb + q) != 0);
+          }
           mma_commit(&tail->empty[stage]);  // the stage is free once these MMAs have read it
         }
         __syncwarp();
@@ -483,10 +506,10 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
       int m_blk, n_blk;
       tile_coords(tile, num_m, num_n, m_blk, n_blk);
-      const int n0 = n_blk * BN;
+      const int n0 = n_blk * TN;
       // stage the per-column scale (and bias / gate) of this tile in shared memory
       asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory");  // previous tile's readers are done
-      for (int c = et; c < BN; c += EPI_THREADS) {
+      for (int c = et; c < TN; c += EPI_THREADS) {
         const int n = n0 + c;
         tail->ws[c] = n < p.N ? p.ws[n] : 0.f;
         if (EPI == EPI_PLAIN || EPI == EPI_BIAS2) tail->aux[c] = (p.bias && n < p.N) ? __bfloat162float(p.bias[n]) : 0.f;
@@ -501,12 +524,12 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       }
       const int row = m_blk * BM + quad * 32 + lane;
       const bool row_ok = row < M;
-      if (tile == static_cast<int>(blockIdx.x)) prefetch_residual<EPI>(p, row, row_ok, n0 + c_first * 32);
+      if (tile == static_cast<int>(blockIdx.x)) prefetch_residual<EPI, EPI_COLS>(p, row, row_ok, n0 + c_first * 32);
       if (tile + static_cast<int>(gridDim.x) < num_tiles) {   // the next tile's residual, a whole epilogue ahead
         int m2, n2;
         tile_coords(tile + gridDim.x, num_m, num_n, m2, n2);
         const int row2 = m2 * BM + quad * 32 + lane;
-        prefetch_residual<EPI>(p, row2, row2 < M, n2 * BN + c_first * 32);
+        prefetch_residual<EPI, EPI_COLS>(p, row2, row2 < M, n2 * TN + c_first * 32);
       }
       uint4 res0[4];
       if (is_gated(EPI)) load_gated_residual(p, row, row_ok, n0, c_first, res0);
@@ -517,7 +540,7 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       tc_fence_after();
       const float xs = row_ok ? p.xs[row] : 0.f;
       const uint32_t t_row = tmem_base + acc * BN + (static_cast<uint32_t>(quad * 32) << 16);
-      epilogue_row<KIND_F8, EPI>(p, tail, t_row, row, row_ok, xs, n0, c_first, res0);
+      epilogue_row<KIND_F8, EPI, EPI_COLS>(p, tail, t_row, row, row_ok, xs, n0, c_first, res0);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tail->acc_empty[acc]);
@@ -550,28 +573,26 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 // CTAs arrive on the even CTA's `acc_empty`. Every wait is bounded as in the single-CTA kernel; the two cluster-wide
 // barriers (after set-up, before tear-down) are reached by every thread on every path.
 // ---------------------------------------------------------------------------------------------
-constexpr int P_STAGES = 6;
-constexpr int P_B_BYTES = 128 * BK;                 // this CTA's half of B
-constexpr int P_STAGE_BYTES = A_BYTES + P_B_BYTES;  // 32 KB
 
 struct __align__(8) PairSmemTail {
-  uint64_t full[P_STAGES];
-  uint64_t empty[P_STAGES];
+  uint64_t full[MAX_STAGES];
+  uint64_t empty[MAX_STAGES];
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
   uint32_t tmem_base;
   int abort_flag;
   GemmSmemTail cols;   // ws / aux / aux2 staging of the epilogue (its barrier fields are unused here)
 };
-constexpr int PAIR_SMEM_BYTES = P_STAGES * P_STAGE_BYTES + sizeof(PairSmemTail) + 1024;
+constexpr int PAIR_SMEM_BYTES = RING_BYTES + sizeof(PairSmemTail) + 1024;
 
-template <int KIND_F8, int EPI>
+template <int KIND_F8, int EPI, int TN>   // TN: columns of a tile, half of whose B rows each CTA loads
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                  const GemmParams p) {
+  constexpr int KS = slabs_per_stage(TN, true), P_STAGES = ring_stages(TN / 2, KS), P_STAGE_BYTES = KS * slab_bytes(TN / 2), EPI_COLS = TN / (EPI_WARPS / 4);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  PairSmemTail* tail = reinterpret_cast<PairSmemTail*>(smem + P_STAGES * P_STAGE_BYTES);
+  PairSmemTail* tail = reinterpret_cast<PairSmemTail*>(smem + RING_BYTES);
   volatile int* abort_flag = &tail->abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -579,7 +600,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
   if (EPI == EPI_F32_ADD) grid_dependency_begin();   // its row count is read on the device
   const int M = gemm_rows<EPI>(p);
-  const int num_m = (M + 2 * BM - 1) / (2 * BM), num_n = (p.N + BN - 1) / BN;
+  const int num_m = (M + 2 * BM - 1) / (2 * BM), num_n = (p.N + TN - 1) / TN;
   const int num_tiles = num_m * num_n;
   const int num_kb = (p.K + BK - 1) / BK;
 
@@ -619,16 +640,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
       int m_blk, n_blk;
       tile_coords(tile, num_m, num_n, m_blk, n_blk);
-      const int row0 = m_blk * 2 * BM + static_cast<int>(rank) * BM, col0 = n_blk * BN + static_cast<int>(rank) * 128;
-      for (int kb = 0; kb < num_kb; ++kb) {
+      const int row0 = m_blk * 2 * BM + static_cast<int>(rank) * BM, col0 = n_blk * TN + static_cast<int>(rank) * (TN / 2);
+      for (int kb = 0; kb < num_kb; kb += KS) {
         ok = __all_sync(0xffffffffu, mbar_wait(&tail->empty[stage], phase ^ 1, abort_flag, p.status, ST_TIMEOUT_STAGE_EMPTY));
         if (!ok) break;
         uint8_t* sa = smem + stage * P_STAGE_BYTES;
         const uint32_t leader_full = cluster_addr(&tail->full[stage], 0);
         if (elect_one()) {
           if (rank == 0) mbar_arrive_expect_tx(&tail->full[stage], 2 * P_STAGE_BYTES);
-          tma_load_2d_pair(sa, &tma_a, kb * BK, row0, leader_full);
-          tma_load_2d_pair(sa + A_BYTES, &tma_b, kb * BK, col0, leader_full);
+#pragma unroll
+          for (int q = 0; q < KS; ++q, sa += slab_bytes(TN / 2)) {
+            tma_load_2d_pair(sa, &tma_a, (kb + q) * BK, row0, leader_full);
+            tma_load_2d_pair(sa + A_BYTES, &tma_b, (kb + q) * BK, col0, leader_full);
+          }
         }
         __syncwarp();
         if (++stage == P_STAGES) { stage = 0; phase ^= 1; }
@@ -637,7 +661,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (even CTA only; converged warp, one elected lane) ------------------------------
     if (rank == 0) {
-      constexpr uint32_t idesc = KIND_F8 ? make_idesc(1, 0, 0, 2 * BM, BN) : make_idesc(2, 1, 1, 2 * BM, BN);
+      constexpr uint32_t idesc = KIND_F8 ? make_idesc(1, 0, 0, 2 * BM, TN) : make_idesc(2, 1, 1, 2 * BM, TN);
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
@@ -648,16 +672,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = 0; kb < num_kb; kb += KS) {
           ok = __all_sync(0xffffffffu, mbar_wait(&tail->full[stage], phase, abort_flag, p.status, ST_TIMEOUT_TMA_FULL));
           if (!ok) break;
           tc_fence_after();
           const uint32_t a_addr = smem_u32(smem + stage * P_STAGE_BYTES);
-          const uint32_t b_addr = a_addr + A_BYTES;
           const uint32_t empty0 = cluster_addr(&tail->empty[stage], 0), empty1 = cluster_addr(&tail->empty[stage], 1);
           if (elect_one()) {
-            if (KIND_F8) mma4_f8_pair(d_tmem, make_desc_k128(a_addr), make_desc_k128(b_addr), idesc, kb != 0);
-            else mma4_i8_pair(d_tmem, make_desc_k128(a_addr), make_desc_k128(b_addr), idesc, kb != 0);
+#pragma unroll
+            for (int q = 0; q < KS; ++q) {
+              const uint32_t aq = a_addr + q * slab_bytes(TN / 2);
+              if (KIND_F8) mma4_f8_pair(d_tmem, make_desc_k128(aq), make_desc_k128(aq + A_BYTES), idesc, (kb + q) != 0);
+              else mma4_i8_pair(d_tmem, make_desc_k128(aq), make_desc_k128(aq + A_BYTES), idesc, (kb + q) != 0);
+            }
             mma_commit_pair(empty0);   // the stage is free in both CTAs once these MMAs have read it
             mma_commit_pair(empty1);
           }
@@ -685,9 +712,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     for (int tile = pair; tile < num_tiles; tile += num_pairs) {
       int m_blk, n_blk;
       tile_coords(tile, num_m, num_n, m_blk, n_blk);
-      const int n0 = n_blk * BN;
+      const int n0 = n_blk * TN;
       asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory");  // previous tile's readers are done
-      for (int c = et; c < BN; c += EPI_THREADS) {
+      for (int c = et; c < TN; c += EPI_THREADS) {
         const int n = n0 + c;
         cols->ws[c] = n < p.N ? p.ws[n] : 0.f;
         if (EPI == EPI_PLAIN || EPI == EPI_BIAS2) cols->aux[c] = (p.bias && n < p.N) ? __bfloat162float(p.bias[n]) : 0.f;
@@ -702,12 +729,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       }
       const int row = m_blk * 2 * BM + static_cast<int>(rank) * BM + quad * 32 + lane;
       const bool row_ok = row < M;
-      if (tile == pair) prefetch_residual<EPI>(p, row, row_ok, n0 + c_first * 32);
+      if (tile == pair) prefetch_residual<EPI, EPI_COLS>(p, row, row_ok, n0 + c_first * 32);
       if (tile + num_pairs < num_tiles) {   // the next tile's residual, a whole epilogue ahead
         int m2, n2;
         tile_coords(tile + num_pairs, num_m, num_n, m2, n2);
         const int row2 = m2 * 2 * BM + static_cast<int>(rank) * BM + quad * 32 + lane;
-        prefetch_residual<EPI>(p, row2, row2 < M, n2 * BN + c_first * 32);
+        prefetch_residual<EPI, EPI_COLS>(p, row2, row2 < M, n2 * TN + c_first * 32);
       }
       uint4 res0[4];
       if (is_gated(EPI)) load_gated_residual(p, row, row_ok, n0, c_first, res0);
@@ -716,7 +743,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       tc_fence_after();
       const float xs = row_ok ? p.xs[row] : 0.f;
       const uint32_t t_row = tmem_base + acc * BN + (static_cast<uint32_t>(quad * 32) << 16);
-      epilogue_row<KIND_F8, EPI>(p, cols, t_row, row, row_ok, xs, n0, c_first, res0);
+      epilogue_row<KIND_F8, EPI, EPI_COLS>(p, cols, t_row, row, row_ok, xs, n0, c_first, res0);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_remote(&tail->acc_empty[acc], 0);
@@ -740,26 +767,40 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 
 std::atomic<int> g_use_pairs{1};
 
-template <int KIND_F8, int EPI>
+// Rows of A per load: a multiple of the swizzle's eight. Rows past the end of A are not free: a box that asks for 128 rows of a
+// 16 x 4,096 operand took 15 us on 64 CTAs where one of 16 rows takes 10.9.
+int box_rows(int64_t M) { return M < BM ? static_cast<int>((M + 7) / 8 * 8) : BM; }
+
+// the tensor map of a call's activations, and what the one of its weights is made from once the tile is chosen
+struct GemmMaps {
+  CUtensorMap a;
+  const void* wq;
+  int64_t N, K;
+  int weights(CUtensorMap* b, int rows) const {
+    return make_tmap_2d(b, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, wq, K, N, K, BK, rows, CU_TENSOR_MAP_SWIZZLE_128B);
+  }
+};
+
+template <int KIND_F8, int EPI, int TN>
 int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, cudaStream_t stream) {
-  auto kern = gemm_pair_kernel<KIND_F8, EPI>;
+  auto kern = gemm_pair_kernel<KIND_F8, EPI, TN>;
   if (int e = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM_BYTES),
                          "gemm pair smem attribute"))
     return e;
-  const int num_tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN);
+  const int num_tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + TN - 1) / TN);
+  // as many pairs as can be resident at once (one CTA per SM), never more than there are tiles
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeClusterDimension;
   attr.val.clusterDim.x = 2;
   attr.val.clusterDim.y = 1;
   attr.val.clusterDim.z = 1;
+  cfg.gridDim = dim3(2 * (device_sm_count() / 2));
   cfg.blockDim = dim3(GEMM_THREADS);
   cfg.dynamicSmemBytes = PAIR_SMEM_BYTES;
   cfg.stream = stream;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  // as many pairs as can be resident at once (one CTA per SM), never more than there are tiles
-  cfg.gridDim = dim3(2 * (device_sm_count() / 2));
   int max_clusters = 0;
   if (cudaOccupancyMaxActiveClusters(&max_clusters, kern, &cfg) != cudaSuccess || max_clusters < 1)
     return set_error(RH3_ARG_ERROR, "gemm pair: no cluster of two CTAs can be resident");
@@ -767,23 +808,62 @@ int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmPar
   return check_cuda(launch_chained(kern, dim3(2 * pairs), GEMM_THREADS, PAIR_SMEM_BYTES, stream, 2, ta, tb, p), "gemm pair launch");
 }
 
-template <int KIND_F8, int EPI>
-int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tb_pair, const GemmParams& p,
-                cudaStream_t stream) {
-  // pairs need more than one 128-row tile to be worth their 256-row tiles
-  if (g_use_pairs.load(std::memory_order_relaxed) && p.M > BM && p.N > 128)
-    return launch_gemm_pair<KIND_F8, EPI>(ta, tb_pair, p, stream);
-  auto kern = gemm_w8a8_kernel<KIND_F8, EPI>;
+template <int KIND_F8, int EPI, int TN>
+int launch_gemm_single(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, cudaStream_t stream) {
+  auto kern = gemm_w8a8_kernel<KIND_F8, EPI, TN>;
   if (int e = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_BYTES),
                          "gemm smem attribute"))
     return e;
-  const int num_tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
+  const int num_tiles = ((p.M + BM - 1) / BM) * ((p.N + TN - 1) / TN);
   const int grid = num_tiles < device_sm_count() ? num_tiles : device_sm_count();
   return check_cuda(launch_chained(kern, dim3(grid), GEMM_THREADS, GEMM_SMEM_BYTES, stream, 1, ta, tb, p), "gemm launch");
 }
 
+// Columns of a tile. A K slab of a tile takes as long as the SM needs to take its operands in (about 72 bytes per clock) or the
+// tensor pipe to multiply them; a narrower tile loads the same A rows for fewer columns, so it pays where the full width leaves
+// SMs idle in its only or its last wave: the width with the smallest waves x time of a slab. `tile_rows` by `ctas` CTAs that
+// share a tile (each loads its rows of A and its part of B). Against every fixed width at six N x K and fifteen M from 1 to
+// 17,896 the rule is within 8 % of the best one. Time at 256 columns for everything / now, us: N = K = 4,096: 37 rows 13.2 / 7.5,
+// 200 rows 15.6 / 8.4, 512 rows 15.9 / 10.3, 1,500 rows 25.3 / 20.9; N = 4,096, K = 16,384: 37 rows 43 / 25, 512 rows 42 / 29;
+// N = 12,288, K = 4,096: 37 rows 13.4 / 10.0, 512 rows 25.4 / 21.2.
+int tile_columns(const GemmParams& p, int tile_rows, int ctas) {
+  const long long resident = device_sm_count() / ctas, m_tiles = (p.M + tile_rows - 1) / tile_rows;
+  const long long kb = (p.K + BK - 1) / BK;
+  long long best = 0;
+  int width = 0;
+  for (int tn = BN; tn >= 64; tn >>= 1) {
+    const long long waves = (m_tiles * ((p.N + tn - 1) / tn) + resident - 1) / resident;
+    const long long feed = BK * (p.a_rows + tn / ctas) / 72, mma = 2 * tn + 50;
+    const long long cost = waves * kb * (feed > mma ? feed : mma) + 8 * tn;   // + draining the last accumulator
+    if (!width || cost < best) {
+      best = cost;
+      width = tn;
+    }
+  }
+  return width;
+}
+
+template <int KIND_F8, int EPI>
+int launch_gemm(const GemmMaps& maps, GemmParams p, cudaStream_t stream) {
+  CUtensorMap tb;
+  p.a_rows = box_rows(p.M);
+  // pairs need more than one 128-row tile to be worth their 256-row tiles
+  if (g_use_pairs.load(std::memory_order_relaxed) && p.M > BM && p.N > 128) {
+    const int tn = tile_columns(p, 2 * BM, 2);
+    if (int e = maps.weights(&tb, tn / 2)) return e;   // a CTA loads half of a tile's B rows
+    return tn == 256   ? launch_gemm_pair<KIND_F8, EPI, 256>(maps.a, tb, p, stream)
+           : tn == 128 ? launch_gemm_pair<KIND_F8, EPI, 128>(maps.a, tb, p, stream)
+                       : launch_gemm_pair<KIND_F8, EPI, 64>(maps.a, tb, p, stream);
+  }
+  const int tn = tile_columns(p, BM, 1);
+  if (int e = maps.weights(&tb, tn)) return e;
+  return tn == 256   ? launch_gemm_single<KIND_F8, EPI, 256>(maps.a, tb, p, stream)
+         : tn == 128 ? launch_gemm_single<KIND_F8, EPI, 128>(maps.a, tb, p, stream)
+                     : launch_gemm_single<KIND_F8, EPI, 64>(maps.a, tb, p, stream);
+}
+
 int gemm_common(const void* xq, int64_t lda, const void* wq, const float* xs, const float* ws, int64_t M, int64_t N,
-                int64_t K, int kind, CUtensorMap* ta, CUtensorMap* tb, CUtensorMap* tb_pair) {
+                int64_t K, int kind, GemmMaps* maps) {
   RH3_CHECK_ARG(kind == RH3_KIND_I8 || kind == RH3_KIND_F8, "gemm_w8a8: kind must be RH3_KIND_I8 or RH3_KIND_F8");
   RH3_CHECK_ARG(M >= 0 && N > 0 && K > 0 && M < (1ll << 31) && N < (1ll << 31) && K < (1ll << 31),
                 "gemm_w8a8: bad shape M=%lld N=%lld K=%lld", (long long)M, (long long)N, (long long)K);
@@ -794,14 +874,8 @@ int gemm_common(const void* xq, int64_t lda, const void* wq, const float* xs, co
   RH3_CHECK_ARG(xq && wq && xs && ws, "gemm_w8a8: null pointer");
   RH3_CHECK_ARG((reinterpret_cast<uintptr_t>(xq) & 15) == 0 && (reinterpret_cast<uintptr_t>(wq) & 15) == 0,
                 "gemm_w8a8: xq and wq must be 16-byte aligned");
-  if (int e = make_tmap_2d(ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, xq, K, M, lda, BK, BM, CU_TENSOR_MAP_SWIZZLE_128B))
-    return e;
-  if (int e = make_tmap_2d(tb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, wq, K, N, K, BK, BN, CU_TENSOR_MAP_SWIZZLE_128B))
-    return e;
-  // the CTA-pair kernel loads B in halves of 128 rows
-  if (int e = make_tmap_2d(tb_pair, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, wq, K, N, K, BK, 128, CU_TENSOR_MAP_SWIZZLE_128B))
-    return e;
-  return 0;
+  maps->wq = wq, maps->N = N, maps->K = K;
+  return make_tmap_2d(&maps->a, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, xq, K, M, lda, BK, box_rows(M), CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 }  // namespace
@@ -819,8 +893,8 @@ extern "C" int rh3_gemm_use_pairs(int on) { return g_use_pairs.exchange(on ? 1 :
 extern "C" int rh3_gemm_w8a8(const void* xq, int64_t lda, const void* wq, const float* xs, const float* ws,
                              const void* bias, int64_t M, int64_t N, int64_t K, int kind, void* out, int64_t ldo,
                              int32_t* acc_dump, cudaStream_t stream) {
-  CUtensorMap ta, tb, tbp;
-  if (int e = gemm_common(xq, lda, wq, xs, ws, M, N, K, kind, &ta, &tb, &tbp)) return e;
+  GemmMaps maps;
+  if (int e = gemm_common(xq, lda, wq, xs, ws, M, N, K, kind, &maps)) return e;
   if (M == 0) return 0;
   RH3_CHECK_ARG(out && ldo >= N && ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0,
                 "gemm_w8a8: out must be 16-byte aligned with a row stride >= N that is a multiple of 8");
@@ -830,7 +904,7 @@ extern "C" int rh3_gemm_w8a8(const void* xq, int64_t lda, const void* wq, const 
   p.bias = static_cast<const __nv_bfloat16*>(bias);
   p.out = static_cast<__nv_bfloat16*>(out); p.ldo = ldo; p.acc_dump = acc_dump; p.status = device_status_word();
   p.wide = (reinterpret_cast<uintptr_t>(out) & 31) == 0 && ldo % 16 == 0;
-  return kind == RH3_KIND_F8 ? launch_gemm<1, EPI_PLAIN>(ta, tb, tbp, p, stream) : launch_gemm<0, EPI_PLAIN>(ta, tb, tbp, p, stream);
+  return kind == RH3_KIND_F8 ? launch_gemm<1, EPI_PLAIN>(maps, p, stream) : launch_gemm<0, EPI_PLAIN>(maps, p, stream);
 }
 
 // The bias lands on the rounded product (two roundings), so the result is bit for bit that of rh3_gemm_w8a8 without a
@@ -839,8 +913,8 @@ extern "C" int rh3_gemm_w8a8(const void* xq, int64_t lda, const void* wq, const 
 extern "C" int rh3_gemm_w8a8_bias_after(const void* xq, int64_t lda, const void* wq, const float* xs, const float* ws,
                                         const void* bias, int64_t M, int64_t N, int64_t K, int kind, void* out,
                                         int64_t ldo, cudaStream_t stream) {
-  CUtensorMap ta, tb, tbp;
-  if (int e = gemm_common(xq, lda, wq, xs, ws, M, N, K, kind, &ta, &tb, &tbp)) return e;
+  GemmMaps maps;
+  if (int e = gemm_common(xq, lda, wq, xs, ws, M, N, K, kind, &maps)) return e;
   if (M == 0) return 0;
   RH3_CHECK_ARG(bias, "gemm_w8a8_bias_after: bias is required");
   RH3_CHECK_ARG(out && ldo >= N && ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0,
@@ -850,14 +924,14 @@ extern "C" int rh3_gemm_w8a8_bias_after(const void* xq, int64_t lda, const void*
   p.bias = static_cast<const __nv_bfloat16*>(bias);
   p.out = static_cast<__nv_bfloat16*>(out); p.ldo = ldo; p.status = device_status_word();
   p.wide = (reinterpret_cast<uintptr_t>(out) & 31) == 0 && ldo % 16 == 0;
-  return kind == RH3_KIND_F8 ? launch_gemm<1, EPI_BIAS2>(ta, tb, tbp, p, stream) : launch_gemm<0, EPI_BIAS2>(ta, tb, tbp, p, stream);
+  return kind == RH3_KIND_F8 ? launch_gemm<1, EPI_BIAS2>(maps, p, stream) : launch_gemm<0, EPI_BIAS2>(maps, p, stream);
 }
 
 extern "C" int rh3_gemm_w8a8_gated_residual(const void* xq, int64_t lda, const void* wq, const float* xs,
                                             const float* ws, const void* gate, void* resid, int64_t ldr, int64_t M,
                                             int64_t N, int64_t K, int kind, cudaStream_t stream) {
-  CUtensorMap ta, tb, tbp;
-  if (int e = gemm_common(xq, lda, wq, xs, ws, M, N, K, kind, &ta, &tb, &tbp)) return e;
+  GemmMaps maps;
+  if (int e = gemm_common(xq, lda, wq, xs, ws, M, N, K, kind, &maps)) return e;
   if (M == 0) return 0;
   RH3_CHECK_ARG(gate && resid && ldr >= N && ldr % 8 == 0 && (reinterpret_cast<uintptr_t>(resid) & 15) == 0,
                 "gemm_w8a8_gated_residual: resid must be 16-byte aligned with a row stride >= N, multiple of 8");
@@ -866,7 +940,7 @@ extern "C" int rh3_gemm_w8a8_gated_residual(const void* xq, int64_t lda, const v
   p.gate = static_cast<const __nv_bfloat16*>(gate);
   p.resid = static_cast<__nv_bfloat16*>(resid); p.ldr = ldr; p.status = device_status_word();
   p.wide = (reinterpret_cast<uintptr_t>(resid) & 31) == 0 && ldr % 16 == 0;
-  return kind == RH3_KIND_F8 ? launch_gemm<1, EPI_GATED>(ta, tb, tbp, p, stream) : launch_gemm<0, EPI_GATED>(ta, tb, tbp, p, stream);
+  return kind == RH3_KIND_F8 ? launch_gemm<1, EPI_GATED>(maps, p, stream) : launch_gemm<0, EPI_GATED>(maps, p, stream);
 }
 
 // The gated residual over a packed sequence of two modalities in one launch: a launch per modality ran the 148 audio rows
@@ -874,8 +948,8 @@ extern "C" int rh3_gemm_w8a8_gated_residual(const void* xq, int64_t lda, const v
 extern "C" int rh3_gemm_w8a8_gated_residual2(const void* xq, int64_t lda, const void* wq, const float* xs, const float* ws,
                                              const float* gate0, const float* gate1, int64_t split, void* resid,
                                              int64_t ldr, int64_t M, int64_t N, int64_t K, int kind, cudaStream_t stream) {
-  CUtensorMap ta, tb, tbp;
-  if (int e = gemm_common(xq, lda, wq, xs, ws, M, N, K, kind, &ta, &tb, &tbp)) return e;
+  GemmMaps maps;
+  if (int e = gemm_common(xq, lda, wq, xs, ws, M, N, K, kind, &maps)) return e;
   if (M == 0) return 0;
   RH3_CHECK_ARG(gate0 && gate1 && split >= 0, "gemm_w8a8_gated_residual2: two gate rows and a split >= 0 are required");
   RH3_CHECK_ARG(resid && ldr >= N && ldr % 8 == 0 && (reinterpret_cast<uintptr_t>(resid) & 15) == 0,
@@ -885,14 +959,14 @@ extern "C" int rh3_gemm_w8a8_gated_residual2(const void* xq, int64_t lda, const 
   p.gate_f[0] = gate0; p.gate_f[1] = gate1; p.gate_split = (int)(split < M ? split : M);
   p.resid = static_cast<__nv_bfloat16*>(resid); p.ldr = ldr; p.status = device_status_word();
   p.wide = (reinterpret_cast<uintptr_t>(resid) & 31) == 0 && ldr % 16 == 0;
-  return kind == RH3_KIND_F8 ? launch_gemm<1, EPI_GATED2>(ta, tb, tbp, p, stream) : launch_gemm<0, EPI_GATED2>(ta, tb, tbp, p, stream);
+  return kind == RH3_KIND_F8 ? launch_gemm<1, EPI_GATED2>(maps, p, stream) : launch_gemm<0, EPI_GATED2>(maps, p, stream);
 }
 
 extern "C" int rh3_gemm_w8a8_swiglu(const void* xq, int64_t lda, const void* wq, const float* xs, const float* ws,
                                     int64_t M, int64_t N, int64_t K, int kind, void* out, int64_t ldo,
                                     cudaStream_t stream) {
-  CUtensorMap ta, tb, tbp;
-  if (int e = gemm_common(xq, lda, wq, xs, ws, M, N, K, kind, &ta, &tb, &tbp)) return e;
+  GemmMaps maps;
+  if (int e = gemm_common(xq, lda, wq, xs, ws, M, N, K, kind, &maps)) return e;
   RH3_CHECK_ARG(N % 16 == 0, "gemm_w8a8_swiglu: N=%lld must be a multiple of 16", (long long)N);
   if (M == 0) return 0;
   RH3_CHECK_ARG(out && ldo >= N / 2 && ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0,
@@ -901,7 +975,7 @@ extern "C" int rh3_gemm_w8a8_swiglu(const void* xq, int64_t lda, const void* wq,
   p.M = (int)M; p.N = (int)N; p.K = (int)K; p.xs = xs; p.ws = ws;
   p.out = static_cast<__nv_bfloat16*>(out); p.ldo = ldo; p.status = device_status_word();
   p.wide = (reinterpret_cast<uintptr_t>(out) & 31) == 0 && ldo % 16 == 0;
-  return kind == RH3_KIND_F8 ? launch_gemm<1, EPI_SWIGLU>(ta, tb, tbp, p, stream) : launch_gemm<0, EPI_SWIGLU>(ta, tb, tbp, p, stream);
+  return kind == RH3_KIND_F8 ? launch_gemm<1, EPI_SWIGLU>(maps, p, stream) : launch_gemm<0, EPI_SWIGLU>(maps, p, stream);
 }
 
 // ---- fp32 epilogues: the text encoder's linears (fp32 in and out, custom_nodes/rapid_h3/te_quant.py:90-115) ----
@@ -911,8 +985,8 @@ extern "C" int rh3_gemm_w8a8_swiglu(const void* xq, int64_t lda, const void* wq,
 extern "C" int rh3_te_gemm(const void* q1, const float* s1, const void* wq, const float* ws, const float* bias, int64_t M,
                            int64_t N, int64_t K, const void* flags, const int32_t* count, const int32_t* rows,
                            const void* q2, const float* s2, float* out, int64_t ldo, cudaStream_t stream) {
-  CUtensorMap ta, tb, tbp;
-  if (int e = gemm_common(q1, K, wq, s1, ws, M, N, K, RH3_KIND_I8, &ta, &tb, &tbp)) return e;
+  GemmMaps maps;
+  if (int e = gemm_common(q1, K, wq, s1, ws, M, N, K, RH3_KIND_I8, &maps)) return e;
   if (M == 0) return 0;
   RH3_CHECK_ARG(out && ldo >= N && ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(out) & 31) == 0,
                 "te_gemm: out must be 32-byte aligned with a row stride >= N that is a multiple of 8");
@@ -921,11 +995,11 @@ extern "C" int rh3_te_gemm(const void* q1, const float* s1, const void* wq, cons
   p.M = (int)M; p.N = (int)N; p.K = (int)K; p.xs = s1; p.ws = ws; p.bias_f = bias;
   p.out_f = out; p.ldo = ldo; p.status = device_status_word();
   p.flags = rows ? static_cast<const uint8_t*>(flags) : nullptr;
-  if (int e = launch_gemm<0, EPI_F32>(ta, tb, tbp, p, stream)) return e;
+  if (int e = launch_gemm<0, EPI_F32>(maps, p, stream)) return e;
   if (!rows) return 0;
-  if (int e = gemm_common(q2, K, wq, s2, ws, M, N, K, RH3_KIND_I8, &ta, &tb, &tbp)) return e;
+  if (int e = gemm_common(q2, K, wq, s2, ws, M, N, K, RH3_KIND_I8, &maps)) return e;
   p.xs = s2; p.flags = nullptr; p.rows = rows; p.m_dev = count;
-  return launch_gemm<0, EPI_F32_ADD>(ta, tb, tbp, p, stream);
+  return launch_gemm<0, EPI_F32_ADD>(maps, p, stream);
 }
 
 // ---- fp16 epilogues: the reference's VAE transformer-decoder GEMMs (custom_nodes/rapid_h3/csrc/vae_ops.cu:150-227
@@ -933,8 +1007,8 @@ extern "C" int rh3_te_gemm(const void* q1, const float* s1, const void* wq, cons
 extern "C" int rh3_vae_gemm(const void* xq, int64_t lda, const void* wq, const float* xs, const float* ws,
                             const void* bias_f16, const void* rscale_f16, const void* resid_f16, int64_t ldr,
                             int64_t M, int64_t N, int64_t K, void* out_f16, int64_t ldo, cudaStream_t stream) {
-  CUtensorMap ta, tb, tbp;
-  if (int e = gemm_common(xq, lda, wq, xs, ws, M, N, K, RH3_KIND_I8, &ta, &tb, &tbp)) return e;
+  GemmMaps maps;
+  if (int e = gemm_common(xq, lda, wq, xs, ws, M, N, K, RH3_KIND_I8, &maps)) return e;
   if (M == 0) return 0;
   RH3_CHECK_ARG(bias_f16, "vae_gemm: bias is required (pass zeros for none)");
   RH3_CHECK_ARG(out_f16 && ldo >= N && ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(out_f16) & 15) == 0,
@@ -947,14 +1021,14 @@ extern "C" int rh3_vae_gemm(const void* xq, int64_t lda, const void* wq, const f
   p.bias_h = static_cast<const __half*>(bias_f16); p.rscale_h = static_cast<const __half*>(rscale_f16);
   p.resid_h = static_cast<const __half*>(resid_f16); p.ldr = ldr;
   p.out_h = static_cast<__half*>(out_f16); p.ldo = ldo; p.status = device_status_word();
-  return launch_gemm<0, EPI_F16>(ta, tb, tbp, p, stream);
+  return launch_gemm<0, EPI_F16>(maps, p, stream);
 }
 
 extern "C" int rh3_vae_gemm_swiglu(const void* xq, int64_t lda, const void* wq, const float* xs, const float* ws,
                                    const void* bias_f16, int64_t M, int64_t N, int64_t K, void* out_f16, int64_t ldo,
                                    cudaStream_t stream) {
-  CUtensorMap ta, tb, tbp;
-  if (int e = gemm_common(xq, lda, wq, xs, ws, M, N, K, RH3_KIND_I8, &ta, &tb, &tbp)) return e;
+  GemmMaps maps;
+  if (int e = gemm_common(xq, lda, wq, xs, ws, M, N, K, RH3_KIND_I8, &maps)) return e;
   RH3_CHECK_ARG(N % 16 == 0, "vae_gemm_swiglu: N=%lld must be a multiple of 16", (long long)N);
   if (M == 0) return 0;
   RH3_CHECK_ARG(bias_f16, "vae_gemm_swiglu: bias is required (pass zeros for none)");
@@ -964,5 +1038,5 @@ extern "C" int rh3_vae_gemm_swiglu(const void* xq, int64_t lda, const void* wq, 
   p.M = (int)M; p.N = (int)N; p.K = (int)K; p.xs = xs; p.ws = ws;
   p.bias_h = static_cast<const __half*>(bias_f16);
   p.out_h = static_cast<__half*>(out_f16); p.ldo = ldo; p.status = device_status_word();
-  return launch_gemm<0, EPI_SWIGLU_F16>(ta, tb, tbp, p, stream);
+  return launch_gemm<0, EPI_SWIGLU_F16>(maps, p, stream);
 }

@@ -281,3 +281,25 @@ def test_gated_residual_with_two_gates(ops, m, split, n):
     got = gemm.int8_gemm_gated_residual2(*dev, gates[2], gates[0], split, res)
     lib.check_status()
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("kind", ["i8", "f8"])
+@pytest.mark.parametrize("m,n,k", [(1, 8, 16), (9, 72, 144), (37, 4104, 1168), (100, 12288, 400), (128, 4096, 640), (129, 1032, 656),
+                                   (200, 4096, 1168), (300, 4136, 1296), (513, 4096, 272), (1500, 4096, 144)])
+def test_gemm_tile_widths(m, n, k, kind):
+    """The rule for the tile's width at rows, columns and K slabs that fill no tile: narrow and full tiles, single CTAs and pairs, one
+    to four K slabs per stage with the last stage partly past K, and A boxes of fewer than 128 rows. The accumulators of int8
+    are exact; e4m3 codes are small integers here, so theirs are as well."""
+    from rapid_h3_b200 import _lib, gemm
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    top = 127 if kind == "i8" else 8
+    a, b = (torch.randint(-top, top + 1, (r, k), device="cuda", generator=g) for r in (m, n))
+    dtype = torch.int8 if kind == "i8" else torch.float8_e4m3fn
+    xq, wq = (t.to(torch.float32).to(dtype) for t in (a, b))
+    xs, ws = torch.rand(m, device="cuda", generator=g), torch.rand(n, device="cuda", generator=g)
+    acc = torch.zeros(m, n, device="cuda", dtype=torch.int32)
+    out = (gemm.int8_gemm if kind == "i8" else gemm.fp8_gemm)(xq, xs, wq, ws, acc_dump=acc)
+    _lib.check_status()
+    ref = a.double() @ b.double().t()   # sums below 2^53: exact in fp64
+    assert torch.equal((acc if kind == "i8" else acc.view(torch.float32)).double(), ref)
+    assert torch.equal(out, ((ref.float() * xs[:, None]) * ws[None]).bfloat16())
