@@ -262,3 +262,30 @@ def test_tiled_decode_batches_tiles_across_rows(vae):
     first = torch.cat([latent[..., 0:3, 0:3], latent[..., 0:3, 2:5], latent[..., 0:3, 4:7]])[: calls[0]]
     alone = plain_decode(first.contiguous())[0:1]
     assert torch.equal(rgb[..., :64, :64], alone[..., :64, :64])
+
+
+@pytest.mark.parametrize("rows,n,shift", [(1, 1, 0), (31, 2, 0), (257, 3, 1), (1025, 1, 2), (9000, 2, 0)])
+def test_group_norm_sums_of_any_number_of_rows(vae, rows, n, shift):
+    """The fp64 sums of the partials at row counts that fill no pass of the cluster, and from partials that start off a
+    16-byte boundary. Against torch's fp64 sum in another order: at most rows additions of values below 8, 2^-53 each."""
+    v, lib = vae
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    buf = torch.randn(n * rows * 64 + 4, device="cuda", generator=g).clamp(-8, 8)
+    part = buf[shift:shift + n * rows * 64]
+    sums = torch.full((n, 32, 2), float("nan"), device="cuda", dtype=torch.float64)
+    lib.call("rh3_gn_reduce", part.data_ptr(), rows, n, sums.data_ptr(), lib.stream())
+    lib.check_status()
+    assert (sums - part.view(n, rows, 32, 2).double().sum(1)).abs().max().item() <= 2 * 8 * rows * rows * 2.0 ** -53
+
+
+@pytest.mark.parametrize("t,h,w", [(1, 1, 1), (1, 3, 32), (2, 2, 33), (3, 5, 65)])
+def test_upsampling_and_depth_to_space_at_the_edges_of_their_blocks(vae, t, h, w):
+    v, lib = vae
+    g = torch.Generator(device="cuda").manual_seed(t + h + w)
+    x = torch.randn(2, t, h, w, 72, device="cuda", generator=g).bfloat16()
+    frames = torch.tensor([0] + [i for i in range(1, t) for _ in range(2)], device="cuda")
+    assert torch.equal(v.upsample(x), x[:, frames].repeat_interleave(2, 2).repeat_interleave(2, 3))
+    y = torch.randn(2, t, h, w, 192, device="cuda", generator=g).bfloat16()
+    ref = y.view(2, t, h, w, 3, 8, 8).permute(0, 4, 1, 2, 5, 3, 6).reshape(2, 3, t, 8 * h, 8 * w)
+    assert torch.equal(v.depth_to_space8(y), ref)
+    lib.check_status()
