@@ -46,7 +46,7 @@ def peaks():
 # dram__bytes_read.sum + dram__bytes_write.sum of the launch at Lq = Lk = 36,436, H = 32, and the first 16 hex digits of
 # the SHA-256 of the kernel source the capture was made with. A different source means the figure is stale: the
 # bench then reports traffic null instead of a number that no longer belongs to the kernel it times.
-ATTN_TRAFFIC = {"bytes": 725.26e6, "lq": 36436, "lk": 36436, "heads": 32, "attn_cu_sha16": "f6e2dcdd3c87ef6b"}
+ATTN_TRAFFIC = {"bytes": 722.47e6, "lq": 36436, "lk": 36436, "heads": 32, "attn_cu_sha16": "e8bacba757432c89"}
 
 
 def attn_traffic(alg_bytes_this_launch):
