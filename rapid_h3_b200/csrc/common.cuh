@@ -39,7 +39,8 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 
 // For kernels launched with launch_chained. All threads wait before the first access to global memory: what the kernels before
 // this one in the stream wrote is visible then, and what they read may be overwritten. The trigger only allows the next kernel's
-// CTAs to start (it waits for all of this one in its turn).
+// CTAs to start (it waits for all of this one in its turn); a kernel that uses tensor memory triggers after it has allocated it,
+// so that the next kernel cannot hold columns that this one, which it waits for, still needs.
 __device__ __forceinline__ void grid_dependency_wait() { cudaGridDependencySynchronize(); }
 __device__ __forceinline__ void grid_dependency_trigger() { cudaTriggerProgrammaticLaunchCompletion(); }
 __device__ __forceinline__ void grid_dependency_begin() {

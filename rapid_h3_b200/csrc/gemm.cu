@@ -400,7 +400,7 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   volatile int* abort_flag = &tail->abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (EPI == EPI_F32_ADD) grid_dependency_begin();   // its row count is read on the device
+  if (EPI == EPI_F32_ADD) grid_dependency_wait();   // its row count is read on the device
   const int M = gemm_rows<EPI>(p);
   const int num_m = (M + BM - 1) / BM, num_n = (p.N + TN - 1) / TN;
   const int num_tiles = num_m * num_n;
@@ -425,7 +425,8 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (EPI != EPI_F32_ADD) grid_dependency_begin();
+  grid_dependency_trigger();
+  if (EPI != EPI_F32_ADD) grid_dependency_wait();
   const uint32_t tmem_base = tail->tmem_base;
 
   if (warp == 0) {
@@ -598,7 +599,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_cta_rank();          // 0 = the even CTA of the pair: it issues the MMAs
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
-  if (EPI == EPI_F32_ADD) grid_dependency_begin();   // its row count is read on the device
+  if (EPI == EPI_F32_ADD) grid_dependency_wait();   // its row count is read on the device
   const int M = gemm_rows<EPI>(p);
   const int num_m = (M + 2 * BM - 1) / (2 * BM), num_n = (p.N + TN - 1) / TN;
   const int num_tiles = num_m * num_n;
@@ -624,7 +625,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   __syncthreads();
   cluster_sync_all();   // both CTAs' barriers exist before anything arrives on them from the other side
   tc_fence_after();
-  if (EPI != EPI_F32_ADD) grid_dependency_begin();
+  grid_dependency_trigger();
+  if (EPI != EPI_F32_ADD) grid_dependency_wait();
   const uint32_t tmem_base = tail->tmem_base;
 
   if (warp == 0) {

@@ -1,0 +1,44 @@
+"""Rules of the kernels that may start under the tail of the one before them (launch_chained), read off their sources."""
+import os
+import re
+
+import pytest
+
+from rapid_h3_b200 import _build
+
+
+def kernels(name):
+    """{kernel name: (parameter list, body)} of every __global__ function of csrc/<name>, comments left out."""
+    text = open(os.path.join(_build.CSRC, name)).read()
+    text = re.sub(r"//[^\n]*", "", text)
+    out = {}
+    for m in re.finditer(r"__global__[^;{]*?\b(\w+_kernel)\s*\(", text):
+        at, depth = m.end(), 1
+        while depth:
+            depth += {"(": 1, ")": -1}.get(text[at], 0)
+            at += 1
+        params, start = text[m.end():at - 1], text.index("{", at)
+        at, depth = start + 1, 1
+        while depth:
+            depth += {"{": 1, "}": -1}.get(text[at], 0)
+            at += 1
+        out[m.group(1)] = (params, text[start:at])
+    return out
+
+
+CHAINED = [(f, k) for f in _build.sources() for k, (_, body) in kernels(f).items() if "grid_dependency_" in body]
+
+
+def test_the_chained_kernels_are_found():
+    launched = sum(open(os.path.join(_build.CSRC, f)).read().count("launch_chained(") for f in _build.sources())
+    assert len(CHAINED) >= 15 and launched >= len(CHAINED)
+
+
+@pytest.mark.parametrize("source,kernel", CHAINED)
+def test_tensor_memory_is_allocated_before_the_next_kernel_may_start(source, kernel):
+    """A kernel that lets the next one start and allocates afterwards could find the tensor memory of its SM taken by a kernel
+    that waits for it in its turn."""
+    body = kernels(source)[kernel][1]
+    if "tmem_alloc" in body:
+        triggers = [m.start() for m in re.finditer(r"grid_dependency_(begin|trigger)\(", body)]
+        assert triggers and body.index("tmem_alloc") < min(triggers)
