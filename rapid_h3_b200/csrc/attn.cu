@@ -511,7 +511,7 @@ attn_int8_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constan
       // the caller's arrays are aligned for them, L1). Eight channels at a time with scalar loads and 16-byte stores cost
       // a cross-attention CTA as much as one of its four key tiles: 36,436 x 512 keys 0.547 ms then, 0.474 now.
       auto load4 = [&](const float* q) {
-        return p.vec_scales ? __ldg(reinterpret_cast<const float4*>(q)) : make_float4(q[0], q[1], q[2], q[3]);
+        return p.vec_scales ? *reinterpret_cast<const float4*>(q) : make_float4(q[0], q[1], q[2], q[3]);
       };
       const bool wide = (reinterpret_cast<uintptr_t>(o) & 31) == 0;
 #pragma unroll 1

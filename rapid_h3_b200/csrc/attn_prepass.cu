@@ -52,7 +52,7 @@ __device__ __forceinline__ void unpack8(const uint4 raw, float* x) {
   x[4] = bf16_lo(raw.z); x[5] = bf16_hi(raw.z); x[6] = bf16_lo(raw.w); x[7] = bf16_hi(raw.w);
 }
 __device__ __forceinline__ uint4 load_row16(const __nv_bfloat16* row, int l16) {
-  return __ldg(reinterpret_cast<const uint4*>(row + l16 * 8));
+  return ld_global_16(row + l16 * 8);
 }
 // sum over the 16 lanes of a half-warp, same value in every lane, fixed order (xor 8, 4, 2, 1)
 __device__ __forceinline__ float half_warp_max(float v) {
@@ -92,11 +92,11 @@ template <int CH, bool PACKED>
 __device__ __forceinline__ void load_rope_row(const __nv_bfloat16* __restrict__ tab_row, int l, NormRope<CH, PACKED>& nr) {
   constexpr int HALF = 48 / CH;  // lanes per half
   if (l < 2 * HALF) {
-    const uint4* p = reinterpret_cast<const uint4*>(tab_row + (l < HALF ? l : l - HALF) * CH * 4);
+    const uint4* tab_words = reinterpret_cast<const uint4*>(tab_row + (l < HALF ? l : l - HALF) * CH * 4);
     const uint32_t pick = l < HALF ? 0x3210u : 0x5476u;  // the first word, or the second one with its halves swapped
 #pragma unroll
     for (int i = 0; i < CH / 2; ++i) {
-      const uint4 q = __ldg(p + i);
+      const uint4 q = __ldg(tab_words + i);
       if constexpr (PACKED) {
         nr.t[2 * i] = __byte_perm(q.x, q.y, pick);
         nr.t[2 * i + 1] = __byte_perm(q.z, q.w, pick);
@@ -407,7 +407,7 @@ __global__ void __launch_bounds__(256, 2) rope_stats_kernel(const RopeStatsParam
 // ---------------------------------------------------------------------------------------------
 // Launch 2: chunk partials -> K mean, V mean, V scale. A thread per (head, channel) walks the chunks in order.
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) kv_stats_final_kernel(const float* __restrict__ part, int nchunk, int64_t L,
+__global__ void __launch_bounds__(128) kv_stats_final_kernel(const float* part, int nchunk, int64_t L,
                                                              float* __restrict__ kmean, float* __restrict__ vmean,
                                                              float* __restrict__ vscale, float v_qmax) {
   grid_dependency_begin();
@@ -443,10 +443,10 @@ __device__ __forceinline__ uint2 quant8_i8_per_channel(const float* y, const flo
 }
 
 template <bool DO_K, bool DO_V, bool V_I8 = false>
-__global__ void __launch_bounds__(256, 3) quant_kv_kernel(const __nv_bfloat16* __restrict__ K, int64_t k_ss, int64_t k_sh,
-                                                       const __nv_bfloat16* __restrict__ V, int64_t v_ss, int64_t v_sh,
-                                                       int64_t L, int64_t Lpad, const float* __restrict__ kmean,
-                                                       const float* __restrict__ vmean, const float* __restrict__ vscale,
+__global__ void __launch_bounds__(256, 3) quant_kv_kernel(const __nv_bfloat16* K, int64_t k_ss, int64_t k_sh,
+                                                       const __nv_bfloat16* V, int64_t v_ss, int64_t v_sh,
+                                                       int64_t L, int64_t Lpad, const float* kmean,
+                                                       const float* vmean, const float* vscale,
                                                        int8_t* __restrict__ k8, float* __restrict__ kscale,
                                                        uint8_t* __restrict__ Vt) {
   grid_dependency_begin();
@@ -580,15 +580,16 @@ constexpr int TOK_ROWS = 32;  // rows of a 256-thread CTA, eight lanes each
 
 // Eight lanes per row, 16 channels each. With sixteen lanes per row (and 64-bit index divisions) this took, with the norm
 // and the rotation, 70 us for the Q rows of 6,196 tokens x 32 heads and 47 us for their K rows without them, now 60 and 40
-// (38 for 55 where Q is normalised but not rotated); 11 us is what their bytes take. A persistent form with the next
+// (38 for 55 where Q is normalised but not rotated); 11 us is what their bytes take. Four CTAs per SM: with the 66 and 70
+// registers that the compiler takes by itself three fit, and the five launches of that call take 204 us, 196 with four. A persistent form with the next
 // row's loads in flight measures the same: instruction issue is the bound.
 template <bool IS_K>
-__global__ void __launch_bounds__(256) quant_tok_kernel(const __nv_bfloat16* __restrict__ x, int64_t x_ss, int64_t x_sh,
+__global__ void __launch_bounds__(256, 4) quant_tok_kernel(const __nv_bfloat16* x, int64_t x_ss, int64_t x_sh,
                                                         int64_t L, int64_t Lpad, int H,
                                                         const __nv_bfloat16* __restrict__ w, float eps,
                                                         const __nv_bfloat16* __restrict__ tab,
-                                                        __nv_bfloat16* __restrict__ x_out, int64_t xo_ss, int64_t xo_sh,
-                                                        const float* __restrict__ mean, int8_t* __restrict__ q8,
+                                                        __nv_bfloat16* x_out, int64_t xo_ss, int64_t xo_sh,
+                                                        const float* mean, int8_t* __restrict__ q8,
                                                         float* __restrict__ scales) {
   grid_dependency_begin();
   const int lane = threadIdx.x & 31, l = lane & 7;
@@ -608,7 +609,7 @@ __global__ void __launch_bounds__(256) quant_tok_kernel(const __nv_bfloat16* __r
   }
   const bool live = in_grid && s < L;
   const __nv_bfloat16* src = x + (live ? s : 0) * x_ss + h * x_sh + l * 16;
-  const uint4 r0 = __ldg(reinterpret_cast<const uint4*>(src)), r1 = __ldg(reinterpret_cast<const uint4*>(src + 8));
+  const uint4 r0 = ld_global_16(src), r1 = ld_global_16(src + 8);
   float v[16];
   unpack8(r0, v);
   unpack8(r1, v + 8);

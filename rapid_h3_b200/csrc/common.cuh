@@ -41,6 +41,9 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 // this one in the stream wrote is visible then, and what they read may be overwritten. The trigger only allows the next kernel's
 // CTAs to start (it waits for all of this one in its turn); a kernel that uses tensor memory triggers after it has allocated it,
 // so that the next kernel cannot hold columns that this one, which it waits for, still needs.
+// What an earlier kernel may have written (activations, codes, scales, partials, modulation tables) is read by ordinary loads (ld_global_16 or plain ones): __ldg
+// and `const __restrict__` promise data that do not change during the kernel's lifetime, and that begins before the wait. They stay
+// for norm weights, affine parameters and rope tables.
 __device__ __forceinline__ void grid_dependency_wait() { cudaGridDependencySynchronize(); }
 __device__ __forceinline__ void grid_dependency_trigger() { cudaTriggerProgrammaticLaunchCompletion(); }
 __device__ __forceinline__ void grid_dependency_begin() {
@@ -190,6 +193,14 @@ __device__ __forceinline__ void ld_global_32(const void* p, uint4& a, uint4& b) 
                : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
                : "l"(p)
                : "memory");
+}
+// 16 bytes by an ordinary load. Like __ldg it may move among the kernel's other accesses (a load of the next row, of a lane's
+// channels), so what it reads is not written earlier by the same kernel; unlike __ldg it is coherent and stays behind
+// grid_dependency_wait().
+__device__ __forceinline__ uint4 ld_global_16(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
 }
 // asks L2 for the 128-byte line that holds `p` (no register, no wait): an epilogue that will read a residual row
 // issues these before it waits for its accumulator, so the reads that follow hit L2 instead of HBM

@@ -597,7 +597,7 @@ conv3d_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_const
 // and 1,152 rows 6.6; 30 and 5.6 now.
 constexpr int GNR_CTAS = 8, GNR_THREADS = 512, GNR_VEC = 2 * GN_GROUPS / 4, GNR_LANES = GNR_THREADS / GNR_VEC;
 template <bool ALIGNED>   // the partials start on a 16-byte boundary
-__global__ void __launch_bounds__(GNR_THREADS) gn_reduce_kernel(const float* __restrict__ part, int64_t rows_per_sample,
+__global__ void __launch_bounds__(GNR_THREADS) gn_reduce_kernel(const float* part, int64_t rows_per_sample,
                                                                 double* __restrict__ sums) {
   grid_dependency_begin();
   __shared__ double red[GNR_LANES][2 * GN_GROUPS];
@@ -606,7 +606,7 @@ __global__ void __launch_bounds__(GNR_THREADS) gn_reduce_kernel(const float* __r
   const float* p = part + n * rows_per_sample * (2 * GN_GROUPS) + col;
   auto load = [&](int64_t r) {
     const float* q = p + r * (2 * GN_GROUPS);
-    return ALIGNED ? __ldg(reinterpret_cast<const float4*>(q)) : make_float4(q[0], q[1], q[2], q[3]);
+    return ALIGNED ? *reinterpret_cast<const float4*>(q) : make_float4(q[0], q[1], q[2], q[3]);
   };
   constexpr int64_t STEP = GNR_CTAS * GNR_LANES;
   double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
@@ -667,16 +667,29 @@ __device__ __forceinline__ float silu_fast(float t) {
 // a chain of elementwise kernels would compute them (s * (1/count), E[x^2] - mean^2, clamped, + eps, rsqrt, all rounded
 // one by one in fp64), so the bits are the same and the chain's eight launches of one tiny block each are gone: a decode
 // runs 13 of these norms, 104 launches of about 3 us, which bounded small decodes on the host side.
+// Six CTAs per SM: the compiler's own 50 registers leave five (141 x 96 x 168 sites of 128 channels 213 us, 237 with five; 9 x 48 x 84
+// 8.6 and 9.0), and the first site is asked for ahead of the factors, whose barrier an ordinary load does not pass (8.6 for 9.6).
 template <bool FROM_SUMS>
-__global__ void __launch_bounds__(256) gn_silu_kernel(const __nv_bfloat16* __restrict__ x,
-                                                      const float* __restrict__ mean_rstd,  // [N][32][2]
-                                                      const double* __restrict__ sums,      // [N][32][2]
-                                                      double inv_count, double eps,
-                                                      const __nv_bfloat16* __restrict__ gamma,
-                                                      const __nv_bfloat16* __restrict__ beta, int64_t sites_per_sample,
-                                                      int C, __nv_bfloat16* __restrict__ y) {
+__global__ void __launch_bounds__(256, 6) gn_silu_kernel(const __nv_bfloat16* x,
+                                                         const float* mean_rstd,  // [N][32][2]
+                                                         const double* sums,      // [N][32][2]
+                                                         double inv_count, double eps,
+                                                         const __nv_bfloat16* __restrict__ gamma,
+                                                         const __nv_bfloat16* __restrict__ beta, int64_t sites_per_sample,
+                                                         int C, __nv_bfloat16* __restrict__ y) {
   grid_dependency_begin();
   __shared__ float2 mr_s[GN_GROUPS];
+  const int vps = C >> 3;                       // 16-byte vectors per site
+  const int lane_vec = threadIdx.x % vps;       // this thread's vector inside a site
+  const int site_in_block = threadIdx.x / vps;
+  const int sites_per_iter = 256 / vps;
+  const int n = blockIdx.y;
+  const int c0 = lane_vec << 3;
+  const __nv_bfloat16* xs = x + static_cast<int64_t>(n) * sites_per_sample * C;
+  const int64_t step = static_cast<int64_t>(gridDim.x) * sites_per_iter;
+  int64_t site = site_in_block < sites_per_iter ? static_cast<int64_t>(blockIdx.x) * sites_per_iter + site_in_block : sites_per_sample;
+  uint4 first;   // on its way while the factors are made
+  if (site < sites_per_sample) first = ld_global_16(xs + site * C + c0);
   if (FROM_SUMS) {
     if (threadIdx.x < GN_GROUPS) {
       const double* sg = sums + (static_cast<int64_t>(blockIdx.y) * GN_GROUPS + threadIdx.x) * 2;
@@ -687,13 +700,7 @@ __global__ void __launch_bounds__(256) gn_silu_kernel(const __nv_bfloat16* __res
     }
     __syncthreads();
   }
-  const int vps = C >> 3;                       // 16-byte vectors per site
-  const int lane_vec = threadIdx.x % vps;       // this thread's vector inside a site
-  const int site_in_block = threadIdx.x / vps;
-  const int sites_per_iter = 256 / vps;
-  if (site_in_block >= sites_per_iter) return;
-  const int n = blockIdx.y;
-  const int c0 = lane_vec << 3;
+  if (site >= sites_per_sample) return;
   const int gs = C / GN_GROUPS;
   float a[8], b[8];
   {
@@ -710,11 +717,8 @@ __global__ void __launch_bounds__(256) gn_silu_kernel(const __nv_bfloat16* __res
       b[j] = fmaf(-mr.x, a[j], bv);
     }
   }
-  const __nv_bfloat16* xs = x + static_cast<int64_t>(n) * sites_per_sample * C;
   __nv_bfloat16* ys = y + static_cast<int64_t>(n) * sites_per_sample * C;
-  for (int64_t site = static_cast<int64_t>(blockIdx.x) * sites_per_iter + site_in_block; site < sites_per_sample;
-       site += static_cast<int64_t>(gridDim.x) * sites_per_iter) {
-    const uint4 raw = __ldg(reinterpret_cast<const uint4*>(xs + site * C + c0));
+  auto apply = [&](const uint4& raw) {
     const uint32_t xw[4] = {raw.x, raw.y, raw.z, raw.w};
     uint32_t o[4];
 #pragma unroll
@@ -724,14 +728,16 @@ __global__ void __launch_bounds__(256) gn_silu_kernel(const __nv_bfloat16* __res
       o[j] = pack_bf16x2(silu_fast(t0), silu_fast(t1));
     }
     *reinterpret_cast<uint4*>(ys + site * C + c0) = make_uint4(o[0], o[1], o[2], o[3]);
-  }
+  };
+  apply(first);
+  for (site += step; site < sites_per_sample; site += step) apply(ld_global_16(xs + site * C + c0));
 }
 
 // out[n, u, yy, xx, :] = in[n, (u + 1) / 2, yy / 2, xx / 2, :]: nearest 2x in space, causal 2x in time
 // (the first frame is not repeated: T frames become 2T - 1). A CTA per input row: every 16 bytes are read once and stored to
 // their four places in one or two frames. Bound by the stores; a thread per output vector, with five 64-bit divisions each,
 // took 426 us for 71 x 48 x 84 sites of 256 channels (1.31 GB), 217 now (0.92 of the measured copy rate).
-__global__ void __launch_bounds__(256) upsample_kernel(const __nv_bfloat16* __restrict__ x, int T, int H, int W, int C,
+__global__ void __launch_bounds__(256) upsample_kernel(const __nv_bfloat16* x, int T, int H, int W, int C,
                                                        __nv_bfloat16* __restrict__ y) {
   grid_dependency_begin();
   const int vec = C >> 3;                              // 16-byte vectors per site
@@ -742,7 +748,7 @@ __global__ void __launch_bounds__(256) upsample_kernel(const __nv_bfloat16* __re
   uint4* dst = reinterpret_cast<uint4*>(y) + (static_cast<int64_t>(n) * (2 * T - 1) + u0) * frame + 2 * h * row;
   const int total = W * vec;
   for (int i = threadIdx.x; i < total; i += 256) {
-    const uint4 v = __ldg(src + i);
+    const uint4 v = ld_global_16(src + i);
     const int w = i / vec;
     uint4* d = dst + i + static_cast<int64_t>(w) * vec;   // site 2w: (2w) * vec + (i - w * vec)
     d[0] = v;
@@ -956,7 +962,7 @@ extern "C" int rh3_gn_silu_from_sums(const void* x, const double* sums, double c
 // lie, and each of the 24 output rows gets its 32 vectors as one contiguous run. With a thread per output vector, whose loads
 // were 384 bytes apart, 141 x 96 x 168 sites (1.75 GB) took 359 us, 253 now.
 constexpr int D2S_SITES = 32;
-__global__ void __launch_bounds__(256) depth_to_space8_kernel(const __nv_bfloat16* __restrict__ y, int T, int H, int W, int w_blocks,
+__global__ void __launch_bounds__(256) depth_to_space8_kernel(const __nv_bfloat16* y, int T, int H, int W, int w_blocks,
                                                               __nv_bfloat16* __restrict__ rgb) {
   grid_dependency_begin();
   __shared__ uint4 tile[D2S_SITES][25];   // one vector of padding: the column reads below meet no bank twice
@@ -966,7 +972,7 @@ __global__ void __launch_bounds__(256) depth_to_space8_kernel(const __nv_bfloat1
   const int64_t nt = site_row / H, n = nt / T, t = nt - n * T;
   const int sites = min(D2S_SITES, W - w0);
   const uint4* src = reinterpret_cast<const uint4*>(y) + (site_row * W + w0) * 24;
-  for (int i = threadIdx.x; i < sites * 24; i += 256) tile[i / 24][i % 24] = __ldg(src + i);
+  for (int i = threadIdx.x; i < sites * 24; i += 256) tile[i / 24][i % 24] = ld_global_16(src + i);
   __syncthreads();
   const int lane = threadIdx.x & 31;
   for (int k = threadIdx.x >> 5; k < 24; k += 8) {

@@ -136,16 +136,21 @@ __device__ __forceinline__ void load_row(const QuantParams& p, int64_t row, int 
       } else {
         src = p.x + row * p.ldx + (static_cast<int64_t>(c) << 3);
       }
-      raw[i] = __ldg(reinterpret_cast<const uint4*>(src));
-      if (KIND == KIND_SWIGLU) raw2[i] = __ldg(reinterpret_cast<const uint4*>(src + p.K));
+      raw[i] = ld_global_16(src);
+      if (KIND == KIND_SWIGLU) raw2[i] = ld_global_16(src + p.K);
     }
   }
 }
 
 // One CTA of T threads works on rows blockIdx.x, blockIdx.x + gridDim.x, ...; the loads of the next row
 // are issued before the current row is reduced and stored, so every CTA always has a row in flight.
+// CTAs that an SM has to hold, where the compiler by itself takes a few registers more than that leaves (0: its own choice).
+// Plain rows of 4,096 with seven (72 registers) or six (75): 36,436 rows 88.1 / 91.6 us, e4m3 97.1 / 100.6.
+__host__ __device__ constexpr int quant_min_ctas(int kind, int threads, int cpt, int rot) {
+  return kind == KIND_PLAIN && threads == 128 && cpt == 4 && !rot ? 7 : kind == KIND_SWIGLU && threads == 128 && cpt == 2 && rot ? 8 : 0;
+}
 template <int KIND, int OUT_FP8, int T, int CPT, int ROT>
-__global__ void __launch_bounds__(T) quant_rows_kernel(const QuantParams p) {
+__global__ void __launch_bounds__(T, quant_min_ctas(KIND, T, CPT, ROT)) quant_rows_kernel(const QuantParams p) {
   grid_dependency_begin();
   __shared__ float red[T / 32];
   const int tid = threadIdx.x;
@@ -195,10 +200,10 @@ __global__ void __launch_bounds__(T) quant_rows_kernel(const QuantParams p) {
         if (p.w) {
           unpack8(__ldg(reinterpret_cast<const uint4*>(p.w + col)), wv);
         }
-        const float4 sc0 = __ldg(reinterpret_cast<const float4*>(p.scale + trow + col));
-        const float4 sc1 = __ldg(reinterpret_cast<const float4*>(p.scale + trow + col + 4));
-        const float4 sh0 = __ldg(reinterpret_cast<const float4*>(p.shift + trow + col));
-        const float4 sh1 = __ldg(reinterpret_cast<const float4*>(p.shift + trow + col + 4));
+        const float4 sc0 = *reinterpret_cast<const float4*>(p.scale + trow + col);
+        const float4 sc1 = *reinterpret_cast<const float4*>(p.scale + trow + col + 4);
+        const float4 sh0 = *reinterpret_cast<const float4*>(p.shift + trow + col);
+        const float4 sh1 = *reinterpret_cast<const float4*>(p.shift + trow + col + 4);
         const float sc[8] = {sc0.x, sc0.y, sc0.z, sc0.w, sc1.x, sc1.y, sc1.z, sc1.w};
         const float sh[8] = {sh0.x, sh0.y, sh0.z, sh0.w, sh1.x, sh1.y, sh1.z, sh1.w};
 #pragma unroll
@@ -226,7 +231,7 @@ __global__ void __launch_bounds__(T) quant_rows_kernel(const QuantParams p) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) am = fmaxf(am, fabsf(v[i][j]));
   }
-  am = p.tensor_amax ? __ldg(p.tensor_amax) : block_max<T>(am, red);
+  am = p.tensor_amax ? *p.tensor_amax : block_max<T>(am, red);
   const float qmax = OUT_FP8 ? 448.f : 127.f;
   const float s = fmaxf(__fdiv_rn(am, qmax), 1e-12f);
   const float inv = __fdiv_rn(1.f, s);
@@ -250,9 +255,9 @@ __global__ void __launch_bounds__(T) quant_rows_kernel(const QuantParams p) {
 // elementwise kernels (fp32 copy, square, mean, rsqrt, two products, copy back) the same rows cost about 40 bytes per
 // element (2 + 4, 4 + 4, 4, 4 + 4, 4 + 4, 4 + 2), in part out of L2: 80 us for 1,008 x 4,096, 5.9 us here; 6,196 x 4,096 take 16 us (6.3 TB/s).
 template <int T, int CPT>
-__global__ void __launch_bounds__(T) rms_norm_rows_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx,
+__global__ void __launch_bounds__(T, T == 128 ? 0 : 1024 / T) rms_norm_rows_kernel(const __nv_bfloat16* x, int64_t ldx,
                                                           const __nv_bfloat16* __restrict__ w, float eps, int64_t M, int K,
-                                                          __nv_bfloat16* __restrict__ out, int64_t ldo) {
+                                                          __nv_bfloat16* out, int64_t ldo) {
   grid_dependency_begin();
   __shared__ float red[T / 32];
   const int tid = threadIdx.x, nchunk = K >> 3;

@@ -42,3 +42,23 @@ def test_tensor_memory_is_allocated_before_the_next_kernel_may_start(source, ker
     if "tmem_alloc" in body:
         triggers = [m.start() for m in re.finditer(r"grid_dependency_(begin|trigger)\(", body)]
         assert triggers and body.index("tmem_alloc") < min(triggers)
+
+
+# what a chained kernel may read as read-only data: norm weights and affine parameters, rope tables
+CONSTANTS = r"(?:w|p\.w|p\.act_w|gamma|beta|tab|tab_words)"
+
+
+@pytest.mark.parametrize("source", sorted({f for f, _ in CHAINED}))
+def test_what_the_kernel_before_wrote_is_read_by_ordinary_loads(source):
+    """__ldg and `const __restrict__` promise that the data stay as they are for the kernel's lifetime, which begins while the
+    kernel before it may still write them: chained kernels make that promise for constants only."""
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(_build.CSRC, source)).read())
+    for kernel, (params, body) in kernels(source).items():
+        if (source, kernel) in CHAINED:
+            promised = re.findall(r"const\s+\w+\s*\*\s*__restrict__\s+(\w+)", params)
+            assert all(re.fullmatch(CONSTANTS, n) for n in promised), (kernel, promised)
+        else:
+            text = text.replace(body, "")
+    for arg in re.findall(r"__ldg\((.*)", text):
+        name = re.match(r"(?:reinterpret_cast<[^>]*>\()?([\w.]+)", arg).group(1)
+        assert re.fullmatch(CONSTANTS, name), arg
