@@ -80,13 +80,35 @@ __device__ __forceinline__ TileCoord conv_tile(int tile, const ConvParams& p, in
   return c;
 }
 
+// Sums over the 32 lanes of the REST values v[0..REST) each of them holds, by exchanges with the lanes O, O / 2, ... 1 away. As
+// long as a lane holds more than one value it hands half of them over and keeps the other half (`at`: index of v[0] among all
+// values); from then on both lanes of an exchange hold the same single value. REST and O are template parameters so that every
+// index into v[] is static: with a run-time count in one unrolled loop the array went to local memory (256 bytes of stack in all
+// four convolution kernels).
+template <int REST, int O, int NV>
+__device__ __forceinline__ void gn_exchange(float (&v)[NV], int lane, int& at) {
+  if constexpr (O > 0) {
+    const bool upper = lane & O;
+    if constexpr (REST > 1) {
+#pragma unroll
+      for (int i = 0; i < REST / 2; ++i) {
+        const float send = upper ? v[i] : v[i + REST / 2], keep = upper ? v[i + REST / 2] : v[i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, O);
+      }
+      if (upper) at += REST / 2;
+      gn_exchange<REST / 2, O / 2>(v, lane, at);
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], O);
+      gn_exchange<1, O / 2>(v, lane, at);
+    }
+  }
+}
+
 // GroupNorm partials of a warp's 32 rows over one 32-column chunk: the GS channels of a group are summed per row
-// (in channel order), the 32 rows by exchanges with the lanes 16, 8, 4, 2 and 1 away; (sum, sum of squares) of every
-// group the chunk holds are written. As long as a lane holds more than one of these values it hands half of them over
-// and keeps the other half, so the 16 values of 4-channel groups take 16 shuffles and not a butterfly of 5 for each (80,
-// which made this epilogue longer than the 54 K chunks of a 128-channel tile: 9 x 48 x 84 sites 32.6 us a layer, 28.8
-// now). Every sum has the same operands in the same order either way. GS is a template parameter so that every index into
-// y[] is static (a run-time group width sends the array to local memory).
+// (in channel order), the 32 rows by gn_exchange; (sum, sum of squares) of every group the chunk holds are written. The
+// exchanges take 16 shuffles for the 16 values of 4-channel groups where a butterfly of 5 for each takes 80, which made
+// this epilogue longer than the 54 K chunks of a 128-channel tile: 9 x 48 x 84 sites 32.6 us a layer, @@A@@. Every sum has the
+// same operands in the same order either way.
 template <int GS>
 __device__ __forceinline__ void gn_partials_chunk(const float* y, float* part, int col0, int Cout, int lane) {
   constexpr int NV = 2 * (32 / GS);   // values: (sum, sum of squares) of each group
@@ -102,28 +124,12 @@ __device__ __forceinline__ void gn_partials_chunk(const float* y, float* part, i
     v[2 * q] = s1;
     v[2 * q + 1] = s2;
   }
-  int at = 0;             // index of v[0] among the chunk's values
-  int rest = NV;          // values this lane still holds
-  int spare = 0;          // offsets at which both lanes hold the same single value: one of them stores it
+  int at = 0;
+  gn_exchange<NV, 16>(v, lane, at);
+  constexpr int HELD = NV > 32 ? NV / 32 : 1, COPIES = NV > 32 ? 1 : 32 / NV;   // values a lane ends with, lanes that end with the same one
+  if ((lane & (COPIES - 1)) == 0) {
 #pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    const bool upper = lane & o;
-    if (rest > 1) {
-      rest >>= 1;
-#pragma unroll
-      for (int i = 0; i < rest; ++i) {
-        const float send = upper ? v[i] : v[i + rest], keep = upper ? v[i + rest] : v[i];
-        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-      }
-      if (upper) at += rest;
-    } else {
-      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
-      spare |= o;
-    }
-  }
-  if ((lane & spare) == 0) {
-#pragma unroll
-    for (int i = 0; i < rest; ++i)
+    for (int i = 0; i < HELD; ++i)
       if (col0 + (at + i) / 2 * GS < Cout) part[col0 / GS * 2 + at + i] = v[i];
   }
 }
