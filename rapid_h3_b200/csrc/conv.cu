@@ -740,33 +740,30 @@ __global__ void __launch_bounds__(256, 6) gn_silu_kernel(const __nv_bfloat16* x,
 }
 
 // out[n, u, yy, xx, :] = in[n, (u + 1) / 2, yy / 2, xx / 2, :]: nearest 2x in space, causal 2x in time
-// (the first frame is not repeated: T frames become 2T - 1). A CTA per input row: every 16 bytes are read once and stored to
-// their four places in one or two frames. Bound by the stores; a thread per output vector, with five 64-bit divisions each,
-// took 426 us for 71 x 48 x 84 sites of 256 channels (1.31 GB), 217 now (0.92 of the measured copy rate).
-__global__ void __launch_bounds__(256) upsample_kernel(const __nv_bfloat16* x, int T, int H, int W, int C,
-                                                       __nv_bfloat16* __restrict__ y) {
+// (the first frame is not repeated: T frames become 2T - 1). A thread per 16 bytes of the input, read once and stored to their
+// four places in one or two frames. Bound by the stores. us with a thread per output vector (five 64-bit divisions each) / a CTA
+// per input row / now: 71 x 48 x 84 sites of 256 channels (1.31 GB) 427 / 218 / 201 (of the measured copy rate 1.0), 36 x 24 x 42 of
+// 512 109 / 69.5 / 53, and where rows are few, 3 x 12 x 21 of 512 3.5 / 4.3 / 2.3, 1 x 24 x 42 of 512 3.0 / 4.2 / 2.2.
+__global__ void __launch_bounds__(256) upsample_kernel(const __nv_bfloat16* x, uint32_t total, uint32_t T, uint32_t H, uint32_t W,
+                                                       uint32_t vec, __nv_bfloat16* __restrict__ y) {   // vec: 16-byte vectors per site
   grid_dependency_begin();
-  const int vec = C >> 3;                              // 16-byte vectors per site
-  const int h = blockIdx.x % H, nt = blockIdx.x / H, t = nt % T, n = nt / T;
-  const uint4* src = reinterpret_cast<const uint4*>(x) + static_cast<int64_t>(blockIdx.x) * W * vec;
+  const uint32_t v = blockIdx.x * 256 + threadIdx.x;
+  if (v >= total) return;
+  const uint4 q = ld_global_16(reinterpret_cast<const uint4*>(x) + v);
+  const uint32_t site = v / vec, r = site / W, nt = r / H, n = nt / T;   // r: row of sites
+  const uint32_t w = site - r * W, h = r - nt * H, t = nt - n * T;
   const int64_t row = 2ll * W * vec, frame = 2ll * H * row;
-  const int64_t u0 = t == 0 ? 0 : 2 * t - 1;
-  uint4* dst = reinterpret_cast<uint4*>(y) + (static_cast<int64_t>(n) * (2 * T - 1) + u0) * frame + 2 * h * row;
-  const int total = W * vec;
-  for (int i = threadIdx.x; i < total; i += 256) {
-    const uint4 v = ld_global_16(src + i);
-    const int w = i / vec;
-    uint4* d = dst + i + static_cast<int64_t>(w) * vec;   // site 2w: (2w) * vec + (i - w * vec)
-    d[0] = v;
-    d[vec] = v;
-    d[row] = v;
-    d[row + vec] = v;
-    if (t) {
-      d[frame] = v;
-      d[frame + vec] = v;
-      d[frame + row] = v;
-      d[frame + row + vec] = v;
-    }
+  uint4* d = reinterpret_cast<uint4*>(y) + (static_cast<int64_t>(n) * (2 * T - 1) + (t == 0 ? 0 : 2 * t - 1)) * frame +
+             2ll * h * row + 2ll * w * vec + (v - site * vec);
+  d[0] = q;
+  d[vec] = q;
+  d[row] = q;
+  d[row + vec] = q;
+  if (t) {
+    d[frame] = q;
+    d[frame + vec] = q;
+    d[frame + row] = q;
+    d[frame + row + vec] = q;
   }
 }
 
@@ -992,10 +989,12 @@ extern "C" int rh3_upsample_causal2x(const void* x, void* y, int64_t N, int64_t 
                                      cudaStream_t stream) {
   RH3_CHECK_ARG(x && y && a16(x) && a16(y) && N > 0 && T > 0 && H > 0 && W > 0 && C > 0 && C % 8 == 0,
                 "upsample_causal2x: bad argument");
-  const int64_t total_vec = N * (2 * T - 1) * 2 * H * 2 * W * (C / 8);
-  RH3_CHECK_ARG((total_vec + 255) / 256 < (1ll << 31), "upsample_causal2x: tensor too large");
-  return check_cuda(launch_chained(upsample_kernel, dim3(static_cast<unsigned>(N * T * H)), 256, 0, stream, 1,
-                                   static_cast<const __nv_bfloat16*>(x), (int)T, (int)H, (int)W, (int)C,
+  // input vectors; one past 32 bits would need 64 GB of input and four to eight times that of output
+  const int64_t total = N * T * H * W * (C / 8);
+  RH3_CHECK_ARG(total <= 0xffffff00ll, "upsample_causal2x: tensor too large");
+  return check_cuda(launch_chained(upsample_kernel, dim3(static_cast<unsigned>((total + 255) / 256)), 256, 0, stream, 1,
+                                   static_cast<const __nv_bfloat16*>(x), static_cast<uint32_t>(total), static_cast<uint32_t>(T),
+                                   static_cast<uint32_t>(H), static_cast<uint32_t>(W), static_cast<uint32_t>(C / 8),
                                    static_cast<__nv_bfloat16*>(y)),
                     "upsample_causal2x launch");
 }

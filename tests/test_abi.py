@@ -77,3 +77,9 @@ def test_argument_errors_of_the_block_entry():
         bad = list(ints)
         bad[i] = 0
         assert lib.rh3_block_forward(pack(bad), p, need, None) < 0 and b"bad shape" in err()
+
+
+def test_upsampling_refuses_what_its_32_bit_indices_do_not_hold():
+    lib = _lib.lib()
+    p = 4096  # an address that is never touched
+    assert lib.rh3_upsample_causal2x(p, p, 1, 1, 1 << 20, 1 << 10, 64, None) < 0 and b"too large" in lib.rh3_last_error_string()
