@@ -292,6 +292,7 @@ conv3d_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
         const TileCoord c = conv_tile(tile, p, num_n);
+        int dh = 0, cc = 0, dw = 0, dt = 0;   // the three dh of a (dt, dw, 64 channels) follow each other, as in the pair kernel
         for (int kb = 0; kb < num_kb; kb += KCH) {
           if (!mbar_wait(&tail->empty[stage], phase ^ 1, abort_flag, p.status, ST_TIMEOUT_STAGE_EMPTY)) {
             ok = false;
@@ -300,13 +301,21 @@ conv3d_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__
           mbar_arrive_expect_tx(&tail->full[stage], (a_bytes + b_bytes) * KCH);
 #pragma unroll
           for (int q = 0; q < KCH; ++q) {
-            // the three dh of a (dt, dw, 64 channels) follow each other, as in the pair kernel
-            const int dh = (kb + q) % 3, rest = (kb + q) / 3, cc = rest % chunks, dtw = rest / chunks;
-            const int dt = dtw / 3, dw = dtw % 3, tap = (dt * 3 + dh) * 3 + dw;
+            const int tap = (dt * 3 + dh) * 3 + dw;
             uint8_t* sa = smem + stage * CSTAGE_BYTES + q * p.chunk_bytes;
             // out-of-range coordinates (negative or past the edge) read zeros: spatial and causal padding
             tma_load_5d(sa, &tma_x, cc * CBK, c.w0 + dw - 1, c.h0 + dh - 1, c.t + dt - 2 + p.halo, c.n, &tail->full[stage]);
             tma_load_2d(sa + CA_BYTES, &tma_w, tap * p.Cin + cc * CBK, c.n_blk * p.BN, &tail->full[stage]);
+            if (++dh == 3) {
+              dh = 0;
+              if (++cc == chunks) {
+                cc = 0;
+                if (++dw == 3) {
+                  dw = 0;
+                  ++dt;
+                }
+              }
+            }
           }
           if (++stage == CSTAGES) { stage = 0; phase ^= 1; }
         }
