@@ -249,8 +249,8 @@ class FusedBlock:
         operands, x updated in place. False, with nothing done, for anything that call does not take as it is: more than two
         spans or per-token modulation rows, other layouts, widths or types. Those go on launch by launch."""
         blk, a = self.block, self.block.attn
-        if type(self) is not FusedBlock or len(tables) != 6:
-            return False
+        if type(self) is not FusedBlock or len(tables) != 6 or not vars(FusedBlock).keys().isdisjoint(vars(self)):
+            return False   # a subclass, or a helper that was put in its place on this one block
         s, d = x.shape
         hd, two = a.heads * 128, self._two_gates(mod_segments, s, tables[2])
         first = tables[0]
@@ -314,7 +314,7 @@ class FusedBlock:
         if rope_freqs is None or x.dtype != torch.bfloat16 or x.device.type != "cuda" or x.ndim != 2:
             raise NotImplementedError("FusedBlock: needs a 2-D CUDA bf16 packed sequence and a rope table")
         if sp is None and trace is None and RR_CHECK is None and timing.PHASES is None:
-            tables = blk.adaln_proj(t_emb)
+            tables = tuple(blk.adaln_proj(t_emb))
             if self._native(x, tables, mod_segments, rope_freqs, ctx):
                 return x
         else:

@@ -383,3 +383,27 @@ def test_block_in_one_call_has_the_bits_of_its_launches(pkg, mode, rotate, grid,
     finally:
         r.nodes.ATTN_ROTATE = False
     r._lib.check_status()
+
+
+def test_block_in_one_call_leaves_replaced_parts_in_place(pkg):
+    """A modulation that yields its six tables one by one, and a helper put in its place on one block: both as before the block
+    went through one call of the library."""
+    r = pkg
+    cfg = r.model.H3Config.tiny(text_dim=256)
+    model = torch.nn.Module()
+    model.blocks = torch.nn.ModuleList([r.model.init_weights(r.model.DiTBlock(cfg), seed=1).cuda()])
+    fb = r.nodes.RapidH3LinearQuant().patch(model, "int8_rowwise")[0].block_forward[0]
+    _, _, t_emb, rope, ctx, segs, s = _case(r, cfg)
+    x = torch.randn(s, cfg.d_model, generator=torch.Generator().manual_seed(5)).to(torch.bfloat16)
+    args = (t_emb[0].cuda(), segs, rope.cuda(), ctx[0].cuda())
+    want = fb.forward(x.cuda(), *args)
+    tables = fb.block.adaln_proj.forward
+    fb.block.adaln_proj.forward = lambda t: (v for v in tables(t))
+    assert torch.equal(fb.forward(x.cuda(), *args), want)
+    del fb.block.adaln_proj.forward
+    seen = []
+    plain = fb._gemm_gated
+    fb._gemm_gated = lambda *a: (seen.append(a[0].shape), plain(*a))[1]
+    assert torch.equal(fb.forward(x.cuda(), *args), want)
+    assert len(seen) == 2
+    r._lib.check_status()
