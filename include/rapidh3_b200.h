@@ -134,6 +134,9 @@ int rh3_te_quant_counted(const float* x, int64_t ldx, int64_t M, int64_t K, floa
  * the weight rows, for calls with more than one site tile. Returns the previous setting; process-wide. Results are the same
  * bits either way. */
 int rh3_gemm_use_pairs(int on);
+/* The tile that the GEMM entries below compute a call of M x N x K on, on the current device and setting: 128 rows, or 256 on a
+ * CTA pair, by 64, 128 or 256 columns. Nothing is launched. */
+int rh3_gemm_tile(int64_t M, int64_t N, int64_t K, int64_t* rows, int64_t* columns);
 /* out[M,N] bf16 = ((acc * xs[m]) * ws[n]) + bias[n]; xq[M,K] (row stride lda), wq[N,K] contiguous.
  * bias may be NULL. acc_dump (optional, [M,N] int32 / fp32 bits) receives the raw accumulators.
  * Replaces int8_rowwise_gemm / fp8_rowwise_gemm (custom_nodes/rapid_h3/csrc/fp8_rowwise.cu:512-584)

@@ -828,14 +828,14 @@ int launch_gemm_single(const CUtensorMap& ta, const CUtensorMap& tb, const GemmP
 // 17,896 the rule is within 8 % of the best one. Time at 256 columns for everything / now, us: N = K = 4,096: 37 rows 13.2 / 7.5,
 // 200 rows 15.6 / 8.4, 512 rows 15.9 / 10.3, 1,500 rows 25.3 / 20.9; N = 4,096, K = 16,384: 37 rows 43 / 25, 512 rows 42 / 29;
 // N = 12,288, K = 4,096: 37 rows 13.4 / 10.0, 512 rows 25.4 / 21.2.
-int tile_columns(const GemmParams& p, int tile_rows, int ctas) {
-  const long long resident = device_sm_count() / ctas, m_tiles = (p.M + tile_rows - 1) / tile_rows;
-  const long long kb = (p.K + BK - 1) / BK;
+int tile_columns(long long M, long long N, long long K, int tile_rows, int ctas) {
+  const long long resident = device_sm_count() / ctas, m_tiles = (M + tile_rows - 1) / tile_rows;
+  const long long kb = (K + BK - 1) / BK;
   long long best = 0;
   int width = 0;
   for (int tn = BN; tn >= 64; tn >>= 1) {
-    const long long waves = (m_tiles * ((p.N + tn - 1) / tn) + resident - 1) / resident;
-    const long long feed = BK * (p.a_rows + tn / ctas) / 72, mma = 2 * tn + 50;
+    const long long waves = (m_tiles * ((N + tn - 1) / tn) + resident - 1) / resident;
+    const long long feed = BK * (box_rows(M) + tn / ctas) / 72, mma = 2 * tn + 50;
     const long long cost = waves * kb * (feed > mma ? feed : mma) + 8 * tn;   // + draining the last accumulator
     if (!width || cost < best) {
       best = cost;
@@ -845,19 +845,21 @@ int tile_columns(const GemmParams& p, int tile_rows, int ctas) {
   return width;
 }
 
+// pairs need more than one 128-row tile to be worth their 256-row tiles
+bool on_pairs(int64_t M, int64_t N) { return g_use_pairs.load(std::memory_order_relaxed) && M > BM && N > 128; }
+
 template <int KIND_F8, int EPI>
 int launch_gemm(const GemmMaps& maps, GemmParams p, cudaStream_t stream) {
   CUtensorMap tb;
   p.a_rows = box_rows(p.M);
-  // pairs need more than one 128-row tile to be worth their 256-row tiles
-  if (g_use_pairs.load(std::memory_order_relaxed) && p.M > BM && p.N > 128) {
-    const int tn = tile_columns(p, 2 * BM, 2);
+  if (on_pairs(p.M, p.N)) {
+    const int tn = tile_columns(p.M, p.N, p.K, 2 * BM, 2);
     if (int e = maps.weights(&tb, tn / 2)) return e;   // a CTA loads half of a tile's B rows
     return tn == 256   ? launch_gemm_pair<KIND_F8, EPI, 256>(maps.a, tb, p, stream)
            : tn == 128 ? launch_gemm_pair<KIND_F8, EPI, 128>(maps.a, tb, p, stream)
                        : launch_gemm_pair<KIND_F8, EPI, 64>(maps.a, tb, p, stream);
   }
-  const int tn = tile_columns(p, BM, 1);
+  const int tn = tile_columns(p.M, p.N, p.K, BM, 1);
   if (int e = maps.weights(&tb, tn)) return e;
   return tn == 256   ? launch_gemm_single<KIND_F8, EPI, 256>(maps.a, tb, p, stream)
          : tn == 128 ? launch_gemm_single<KIND_F8, EPI, 128>(maps.a, tb, p, stream)
@@ -891,6 +893,15 @@ using namespace rh3;
 // setting. Results are identical (int32 accumulators, same epilogue). The convolution follows the same switch
 // (conv3d_pair_kernel: fp32 accumulation in the same order, identical results).
 extern "C" int rh3_gemm_use_pairs(int on) { return g_use_pairs.exchange(on ? 1 : 0); }
+
+extern "C" int rh3_gemm_tile(int64_t M, int64_t N, int64_t K, int64_t* rows, int64_t* columns) {
+  RH3_CHECK_ARG(rows && columns && M > 0 && N > 0 && K > 0 && M < (1ll << 31) && N < (1ll << 31) && K < (1ll << 31),
+                "gemm_tile: bad shape or null pointer");
+  const bool pair = on_pairs(M, N);
+  *rows = pair ? 2 * BM : BM;
+  *columns = tile_columns(M, N, K, pair ? 2 * BM : BM, pair ? 2 : 1);
+  return 0;
+}
 
 extern "C" int rh3_gemm_w8a8(const void* xq, int64_t lda, const void* wq, const float* xs, const float* ws,
                              const void* bias, int64_t M, int64_t N, int64_t K, int kind, void* out, int64_t ldo,

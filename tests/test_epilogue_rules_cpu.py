@@ -42,3 +42,17 @@ def test_two_gates_takes_one_or_two_plain_spans_only():
         assert two(segs, 10, gpu) is None
     assert two([(0, 10, 0)], 10, tab) is None and two([(0, 10, 0)], 10, gpu.to(torch.bfloat16)) is None
     assert two([(0, 10, 0)], 10, torch.zeros(8, 2).t().as_subclass(OnGpu)) is None
+
+
+def test_the_shapes_of_the_tile_test_reach_every_tile():
+    from test_gemm_gpu import WIDTH_CASES, tile_of
+    from rapid_h3_b200 import _lib
+    assert {tile_of(_lib, *c) for c in WIDTH_CASES} == {(r, c) for r in (128, 256) for c in (64, 128, 256)}
+    # a call of the e4m3 recipe and one of a transformer block run at full width, a few rows on narrow tiles
+    assert tile_of(_lib, 5003, 12288, 4096) == (256, 256) and tile_of(_lib, 36436, 4096, 4096) == (256, 256)
+    assert tile_of(_lib, 37, 4096, 4096) == (128, 64)
+    prev = _lib.lib().rh3_gemm_use_pairs(0)
+    try:
+        assert tile_of(_lib, 5003, 12288, 4096) == (128, 256)
+    finally:
+        _lib.lib().rh3_gemm_use_pairs(prev)

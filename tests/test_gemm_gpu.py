@@ -283,9 +283,20 @@ def test_gated_residual_with_two_gates(ops, m, split, n):
     assert torch.equal(got, want)
 
 
+def tile_of(lib, m, n, k):
+    import ctypes
+    rows, columns = ctypes.c_int64(), ctypes.c_int64()
+    lib.call("rh3_gemm_tile", m, n, k, ctypes.addressof(rows), ctypes.addressof(columns))
+    return rows.value, columns.value
+
+
+# tests/test_epilogue_rules_cpu.py holds that these reach all six tiles
+WIDTH_CASES = [(1, 8, 16), (9, 72, 144), (37, 4104, 1168), (100, 12288, 400), (128, 4096, 640), (129, 1032, 656), (200, 4096, 1168),
+               (300, 4136, 1296), (513, 4096, 272), (1500, 4096, 144), (2049, 8192, 272), (100, 36864, 1168)]
+
+
 @pytest.mark.parametrize("kind", ["i8", "f8"])
-@pytest.mark.parametrize("m,n,k", [(1, 8, 16), (9, 72, 144), (37, 4104, 1168), (100, 12288, 400), (128, 4096, 640), (129, 1032, 656),
-                                   (200, 4096, 1168), (300, 4136, 1296), (513, 4096, 272), (1500, 4096, 144)])
+@pytest.mark.parametrize("m,n,k", WIDTH_CASES)
 def test_gemm_tile_widths(m, n, k, kind):
     """The rule for the tile's width at rows, columns and K slabs that fill no tile: narrow and full tiles, single CTAs and pairs, one
     to four K slabs per stage with the last stage partly past K, and A boxes of fewer than 128 rows. The accumulators of int8
@@ -303,3 +314,62 @@ def test_gemm_tile_widths(m, n, k, kind):
     ref = a.double() @ b.double().t()   # sums below 2^53: exact in fp64
     assert torch.equal((acc if kind == "i8" else acc.view(torch.float32)).double(), ref)
     assert torch.equal(out, ((ref.float() * xs[:, None]) * ws[None]).bfloat16())
+
+
+EPILOGUES = ["plain", "fp8", "bias", "bias_fp8", "gated", "gated2", "swiglu", "fp16", "fp16_resid", "fp16_swiglu", "fp32", "fp32_add"]
+
+
+@pytest.mark.parametrize("epilogue", EPILOGUES)
+def test_every_epilogue_has_the_same_bits_on_every_tile(ops, epilogue):
+    """2,049 x 8,192 outputs on 256-column tiles of CTA pairs and of single CTAs (pairs off) against slices of their rows, which run on
+    tiles of 64 and 128 columns: rows do not depend on one another, and every product here is exact (integers, or e4m3 codes that
+    are small integers), so a row's bits are the same whatever tile it is computed on."""
+    from rapid_h3_b200 import te_quant, vae_fast
+    gemm, kernels, lib = ops
+    m, n, k = 2049, 8192, 512
+    g = torch.Generator(device="cuda").manual_seed(EPILOGUES.index(epilogue))
+    f8 = epilogue.endswith("fp8")
+    xq, wq = (torch.randint(-8 if f8 else -127, 9 if f8 else 128, (r, k), device="cuda", generator=g).to(torch.int8) for r in (m, n))
+    if f8:
+        xq, wq = xq.to(torch.float8_e4m3fn), wq.to(torch.float8_e4m3fn)
+    xs, ws = (1e-3 * torch.rand(r, device="cuda", generator=g) + 1e-5 for r in (m, n))
+    vec = torch.randn(3, n, device="cuda", generator=g)
+    resid = torch.randn(m, n, device="cuda", generator=g)
+    x32 = torch.randn(m, k, device="cuda", generator=g)
+    x32[::7, 256:512] += 6.0 * (16.0 * ol.regular_hadamard(256)[5]).float().cuda()   # outlier rows: the second product adds to these
+    te = te_quant._TELinear(kernels.QWeight(wq, ws[None]), vec[0].contiguous(), "int8_rot" if epilogue == "fp32_add" else "int8_rot_plain") if not f8 else None
+
+    def run(a, b):
+        xa, sa = xq[a:b], xs[a:b].contiguous()
+        if epilogue in ("plain", "fp8"):
+            return (gemm.fp8_gemm if f8 else gemm.int8_gemm)(xa, sa, wq, ws)
+        if epilogue.startswith("bias"):
+            return gemm.gemm_bias_after(xa, sa, wq, ws, vec[0].to(torch.bfloat16))
+        if epilogue == "gated":
+            return gemm.int8_gemm_gated_residual(xa, sa, wq, ws, vec[0].to(torch.bfloat16), resid[a:b].to(torch.bfloat16))
+        if epilogue == "gated2":
+            return gemm.int8_gemm_gated_residual2(xa, sa, wq, ws, vec[0], vec[1], min(max(1000 - a, 0), b - a), resid[a:b].to(torch.bfloat16))
+        if epilogue == "swiglu":
+            return gemm.int8_gemm_swiglu(xa, sa, wq, ws)
+        if epilogue == "fp16":
+            return vae_fast.vae_gemm(xa, wq, sa, ws, vec[0].half())
+        if epilogue == "fp16_resid":
+            return vae_fast.vae_gemm(xa, wq, sa, ws, vec[0].half(), vec[1].half(), resid[a:b].half())
+        if epilogue == "fp16_swiglu":
+            return vae_fast.vae_gemm_swiglu(xa, wq, sa, ws, vec[0].half())
+        return te(x32[a:b])
+
+    assert tile_of(lib, m, n, k) == (256, 256) and tile_of(lib, 200, n, k) == (256, 128) and tile_of(lib, 100, n, k) == (128, 64)
+    full = run(0, m)
+    for a, b in ((0, 100), (100, 300), (995, 1195), (1949, 2049), (2048, 2049)):
+        assert torch.equal(run(a, b), full[a:b])
+    prev = lib.lib().rh3_gemm_use_pairs(0)
+    try:
+        assert tile_of(lib, m, n, k) == (128, 256) and tile_of(lib, 200, n, k) == (128, 128)
+        assert torch.equal(run(0, m), full) and torch.equal(run(100, 300), full[100:300])
+    finally:
+        lib.lib().rh3_gemm_use_pairs(prev)
+    lib.check_status()
+    if epilogue in ("plain", "fp8"):   # the anchor: these bits against the product in 64 bits
+        want = (xq.double() @ wq.double().t()).float()
+        assert torch.equal(full, ((want * xs[:, None]) * ws[None]).bfloat16())
