@@ -864,22 +864,16 @@ extern "C" int rh3_conv3d_causal(const void* x, const void* w, const void* bias,
   const uint64_t dims[5] = {(uint64_t)Cin, (uint64_t)W, (uint64_t)H, Tin, (uint64_t)N};
   const uint64_t strides[4] = {(uint64_t)Cin * 2, (uint64_t)W * Cin * 2, (uint64_t)H * W * Cin * 2,
                                Tin * H * W * Cin * 2};
-  const uint32_t box[5] = {CBK, (uint32_t)p.bw, (uint32_t)p.bh, 1, 1};
-  if (int e = make_tmap_nd(&tx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x, 5, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B))
-    return e;
-  if (int e = make_tmap_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, w, 27 * Cin, Cout, 27 * Cin * 2, CBK, p.BN,
-                           CU_TENSOR_MAP_SWIZZLE_128B))
-    return e;
   const int64_t num_m = N * T * p.tiles_h * p.tiles_w, num_n = (Cout + p.BN - 1) / p.BN;
   // CTA pairs: two site tiles per pair and BN/2 weight rows per CTA (a multiple of 16, so every MMA shape is legal)
-  if (pairs_enabled() && num_m >= 2 && p.BN % 32 == 0) {
-    CUtensorMap twp;
-    if (int e = make_tmap_2d(&twp, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, w, 27 * Cin, Cout, 27 * Cin * 2, CBK, p.BN / 2,
-                             CU_TENSOR_MAP_SWIZZLE_128B))
-      return e;
-    const uint32_t box_rows[5] = {CBK, (uint32_t)p.bw, (uint32_t)p.bh + 2, 1, 1};
-    if (int e = make_tmap_nd(&tx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x, 5, dims, strides, box_rows, CU_TENSOR_MAP_SWIZZLE_128B))
-      return e;
+  const bool pair = pairs_enabled() && num_m >= 2 && p.BN % 32 == 0;
+  const uint32_t box[5] = {CBK, (uint32_t)p.bw, (uint32_t)(pair ? p.bh + 2 : p.bh), 1, 1};
+  if (int e = make_tmap_nd(&tx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x, 5, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B))
+    return e;
+  if (int e = make_tmap_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, w, 27 * Cin, Cout, 27 * Cin * 2, CBK, pair ? p.BN / 2 : p.BN,
+                           CU_TENSOR_MAP_SWIZZLE_128B))
+    return e;
+  if (pair) {
     // a stage: the box (128 rows can be read from row 2 * bw on), then three taps' weight rows
     p.chunk_bytes = (CBM + 2 * p.bw + 7) / 8 * 1024;
     p.stage_bytes = p.chunk_bytes + 3 * (p.BN / 2) * 128;
@@ -906,7 +900,7 @@ extern "C" int rh3_conv3d_causal(const void* x, const void* w, const void* bias,
       return set_error(RH3_ARG_ERROR, "conv3d pair: no cluster of two CTAs can be resident");
     const int64_t pair_tiles = (num_m + 1) / 2 * num_n;
     const unsigned ctas = 2 * static_cast<unsigned>(pair_tiles < max_clusters ? pair_tiles : max_clusters);
-    return check_cuda(launch_chained(kern, dim3(ctas), CONV_THREADS, CONV_PAIR_SMEM_BYTES, stream, 2, tx, twp, p), "conv3d pair launch");
+    return check_cuda(launch_chained(kern, dim3(ctas), CONV_THREADS, CONV_PAIR_SMEM_BYTES, stream, 2, tx, tw, p), "conv3d pair launch");
   }
   p.chunk_bytes = CA_BYTES + p.BN * 128;
   p.kch = choose_kch(p.BN, (int)(Cin / CBK));
