@@ -842,13 +842,15 @@ extern "C" int rh3_conv3d_causal(const void* x, const void* w, const void* bias,
   };
   // Few sites leave most of the chip idle at full width (a 3 x 12 x 21 latent has 6 site tiles: 12 CTAs at 512 channels,
   // 79 us a layer), so the channels are split further while that lowers waves x time of a tile. A pair's tile takes as
-  // long as an SM needs to take in its K chunks, 16 KB of sites and 64 B per channel each, so a split is not free: half
-  // the width costs 3/4 of the time, and with enough site tiles for a whole wave full width stays the better one.
+  // long as an SM needs to take in its K chunks: a third of the box of bh + 2 rows, which serves three taps, and 64 B per channel
+  // each, so a split is not free. us a layer with the 16 KB of a box per tap in that place / with the box's third: 13 x 22 x 82
+  // sites of 256 channels 74.6 / 58.7, 36 x 24 x 11 of 512 137 / 113, 25 x 7 x 42 of 512 137 / 103 (full width in 1.03 to 1.5
+  // waves, half the width in 2.05 to 3).
   {
     const int64_t pairs = (N * T * p.tiles_h * p.tiles_w + 1) / 2, resident = device_sm_count() / 2;
     auto cost = [&](int n) {
       const int bn = tile_width(n);
-      return ((pairs * ((p.Cout + bn - 1) / bn) + resident - 1) / resident) * (16384 + 64ll * bn);
+      return ((pairs * ((p.Cout + bn - 1) / bn) + resident - 1) / resident) * ((p.bh + 2) * p.bw * 128ll / 3 + 64ll * bn);
     };
     for (int n = splits * 2; tile_width(n) >= 64 && cost(n) < cost(splits); n *= 2) splits = n;
   }
