@@ -129,7 +129,7 @@ int rh3_te_quant_counted(const float* x, int64_t ldx, int64_t M, int64_t K, floa
                          int32_t* count, int32_t* rows, void* q2, float* s2, void* total, void* seen, cudaStream_t stream);
 /* ---- W8A8 row-wise-scaled GEMMs (tensor-core bound) ---------------------------------------- */
 /* Kernel choice of the GEMM entries below and of rh3_conv3d_causal (no reference counterpart): 0 = one CTA per tile, 1 (the
- * default) = CTA pairs (clusters of two, tcgen05 cta_group::2): 256 x 256 GEMM tiles with each CTA loading its own half of
+ * default) = CTA pairs (clusters of two, tcgen05 cta_group::2): GEMM tiles of 256 rows with each CTA loading its own half of
  * B, for calls with more than 128 rows and columns; two site tiles of the convolution per pair with each CTA loading half of
  * the weight rows, for calls with more than one site tile. Returns the previous setting; process-wide. Results are the same
  * bits either way. */

@@ -29,7 +29,8 @@
 //                    registers: O = ts * A + a * O, from the factors the softmax threads leave in shared memory; where no
 //                    row of a warp has a new maximum (a = 1) the multiplication by a is left out
 // TMEM (512 columns): S0 | S1 | A0 | A1. 96 registers a thread are launched; the warp groups' shares add up to them.
-// What bounds it: issue slots (2,850 per scheduler and step of 4,880 cycles; an f32x2 instruction takes two) and the chain
+// What bounds it: issue slots (by the executed-instruction counter 2,900 warp instructions per scheduler and step, which takes
+// 4,700 cycles at L = 22,332; an f32x2 instruction takes two slots) and the chain
 // scores -> first pass -> second pass -> next scores, which the fold warps and the other query tile run under. H = 32, ms at
 // L = 22,332 / 6,196 / 1,000: 11.28 / 0.997 / 0.037 with the fold, the scores' second conversion and scaling, and a bias
 // stored into both accumulators in the softmax threads' own chain (384 threads); 10.20 / 0.910 / 0.036 with the fold in warp

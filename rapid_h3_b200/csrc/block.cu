@@ -1,6 +1,6 @@
 // One fused DiT block as a list of launches: the host side of the block in native code. Bound by the launches themselves:
 // driven from Python, the 16 calls of a block cost 440 us of interpreter, argument conversion and buffer allocation, which
-// is all of the time of a small step and most of that of one picture: two blocks on 115 tokens 1.26 -> 0.55 ms, two blocks
+// is all of the time of a small step and most of that of one picture: two blocks on 115 tokens 1.26 -> 0.57 ms, two blocks
 // on two samples of 1,008 tokens (width 4,096) 2.23 -> 2.01 ms.
 // The buffers of a block overlap where their lifetimes do not: codes | bf16 rows (q|k|v, then the attention output, then the
 // MLP's hidden rows) | attention operands, then the hidden rows' codes.

@@ -6,10 +6,14 @@
 //                                      + bias[co] (+ residual[n, t, h, w, co]) )
 //   zero padding: one pixel around H and W, two frames BEFORE t = 0 (causal: no frame after t is read).
 //
-// There is no im2col buffer: for every tap the A operand of the GEMM is a shifted box of the input,
-// fetched by a 5-D TMA tensor copy whose out-of-range coordinates are filled with zeros (that is the
-// padding). One output tile = bh x bw sites of one frame (bh * bw <= 128 rows of the MMA) x BN output
-// channels; the K loop runs over 27 taps x Cin/64 channel chunks (64 bf16 = one 128-byte swizzled row).
+// There is no im2col buffer: the A operand of the GEMM is a shifted box of the input, fetched by a 5-D TMA tensor copy
+// whose out-of-range coordinates are filled with zeros (that is the padding): a box per tap in the single-CTA kernel, one
+// box for the three dh of a (dt, dw) in the pair kernel. The K loop runs over (dt, dw, 64 channels, dh) in both, so their
+// results agree bit for bit; with the order (dt, dh, dw, channels) of a plain tap loop the same fp32 sums round differently
+// (whole decodes differ by 6.4e-3 to 7.8e-3 relative), equally far from the exact ones: over 93 M outputs of 13 layer shapes
+// 0.2636 % against 0.2632 % are not the rounded 64-bit value, and decodes lie 7.524e-3 and 7.527e-3 from one in 64 bits.
+// One output tile = bh x bw sites of one frame (bh * bw <= 128 rows of the MMA) x BN output
+// channels; a K chunk is 64 channels of a tap (64 bf16 = one 128-byte swizzled row).
 // Same warp roles and double-buffered TMEM accumulators as the W8A8 GEMM; the ring has as many stages as fit in
 // shared memory (4 of 48 KB at 256 output channels per tile, up to 12 for narrow tiles): a stage of a narrow tile
 // holds few tensor cycles of work, and the ring has to cover the L2 latency with them.
@@ -44,9 +48,11 @@ struct ConvParams {
   const __nv_bfloat16* residual;  // [N,T,H,W,Cout] or null
   __nv_bfloat16* out;
   float* gn_part;      // [num_m_tiles * 4][32][2] partial (sum, sumsq) per GroupNorm group, or null
-  int stages, stage_bytes;   // ring: stage_bytes = kch * chunk_bytes
+  int stages, stage_bytes;   // ring
   int wide;                  // out (and residual) rows are 32-byte aligned: 32-byte accesses in the epilogue
-  int kch, chunk_bytes;      // K chunks per stage (one barrier round trip each), CA_BYTES + (weight rows a CTA loads) * 128
+  // single CTA: K chunks per stage (one barrier round trip each) of CA_BYTES + BN * 128 bytes. Pair: a stage is the box, of
+  // chunk_bytes, and the weight rows of its three taps
+  int kch, chunk_bytes;
   int* status;
 };
 
@@ -411,6 +417,8 @@ conv3d_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__
 // few output channels (the operand reads of the MMAs want the same bandwidth); a box per tap was 16 KB of it, a third of a
 // taller box is 6-9 KB. Before / after, us: 3 x 12 x 21 sites, 512 -> 512 channels 43.2 / 30.9, 5 x 24 x 42, 256 -> 256
 // 27.2 / 24.9, 141 x 96 x 168, 128 -> 128 1,792 / 1,748; full-width tiles are bound by the tensor pipe and measure the same.
+// Where a tile is one or two rows high (frames 56 to 64 or more than 112 sites wide) the box saves little and a stage of 256
+// channels leaves room for two only: 7 x 26 x 62 of 256 channels 59.1 / 61.6, 8 x 23 x 128 76.0 / 79.0, but 4 x 9 x 125 28.1 / 18.5.
 // When the number of site tiles is odd, the odd CTA of the last pair loads the last valid tile again and stores nothing.
 // Barriers as in the GEMM's pair kernel: both CTAs' loads count on the even CTA's `full`; stage release and
 // accumulator hand-over are one commit per CTA; every wait is bounded; the two cluster barriers are reached by all.
@@ -608,8 +616,8 @@ conv3d_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_const
 // sums[n][g] = (sum, sum of squares) over all row blocks of sample n, added in a fixed order in fp64. A cluster of eight CTAs
 // per sample: a row of partials is 64 consecutive floats, so 16 threads read one coalesced and a CTA 32 at a time, four such
 // in flight; the CTAs' sums meet in the first one's through distributed shared memory. With a CTA per group, each reading 8
-// of a row's 256 bytes, the 71,064 rows of 141 x 96 x 168 sites took 76 us (of 1.68 ms for the convolution they come from)
-// and 1,152 rows 6.6; 30 and 5.6 now.
+// of a row's 256 bytes, the 71,064 rows of 141 x 96 x 168 sites took 76 us (of 1.3 ms for the convolution they come from);
+// 28 now, 8,946 rows 5.5, 1,134 rows 2.5 in a chain.
 constexpr int GNR_CTAS = 8, GNR_THREADS = 512, GNR_VEC = 2 * GN_GROUPS / 4, GNR_LANES = GNR_THREADS / GNR_VEC;
 template <bool ALIGNED>   // the partials start on a 16-byte boundary
 __global__ void __launch_bounds__(GNR_THREADS) gn_reduce_kernel(const float* part, int64_t rows_per_sample,
@@ -792,10 +800,9 @@ void choose_tile(int H, int W, int* bh, int* bw) {
   }
 }
 
-// K chunks per ring stage. A stage costs one barrier round trip in the producer and in the MMA issuer, a few hundred
-// cycles that a narrow tile's four MMAs per chunk (2 * BN tensor cycles) do not cover: narrow tiles put two or four
-// chunks behind one barrier; the pair kernel (32 KB per chunk at most) also does so for full-width tiles, where it
-// still gains 4-5 %. The count divides the 27 * chunks_per_tap chunks of a tile.
+// K chunks per ring stage of the single-CTA kernel. A stage costs one barrier round trip in the producer and in the MMA
+// issuer, a few hundred cycles that a narrow tile's four MMAs per chunk (2 * BN tensor cycles) do not cover: narrow tiles put two
+// or four chunks behind one barrier. The count divides the 27 * chunks_per_tap chunks of a tile.
 int choose_kch(int bn, int chunks_per_tap) {
   int want = bn > 128 ? 1 : (bn > 64 ? 2 : 4);
   while (want > 1 && chunks_per_tap % want != 0) want >>= 1;
@@ -968,7 +975,7 @@ extern "C" int rh3_gn_silu_from_sums(const void* x, const double* sums, double c
 // Depth-to-space by 8 of the decoder head: y [N, T, H, W, 3*8*8] (channel = (ch*8 + dy)*8 + dx) ->
 // rgb [N, 3, T, 8H, 8W]. A CTA moves 32 sites of a row through shared memory: 24 vectors of 16 bytes per site come in as they
 // lie, and each of the 24 output rows gets its 32 vectors as one contiguous run. With a thread per output vector, whose loads
-// were 384 bytes apart, 141 x 96 x 168 sites (1.75 GB) took 359 us, 253 now.
+// were 384 bytes apart, 141 x 96 x 168 sites (1.75 GB) took 359 us, 254 now.
 constexpr int D2S_SITES = 32;
 __global__ void __launch_bounds__(256) depth_to_space8_kernel(const __nv_bfloat16* y, int T, int H, int W, int w_blocks,
                                                               __nv_bfloat16* __restrict__ rgb) {

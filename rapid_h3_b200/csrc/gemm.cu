@@ -564,11 +564,11 @@ gemm_w8a8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 }
 
 // ---------------------------------------------------------------------------------------------
-// The same GEMM on CTA pairs (thread-block clusters of two, tcgen05 cta_group::2): a pair computes a 256 x 256 tile.
-// CTA r of the pair loads A rows [128 r, 128 r + 128) and B rows (output columns) [128 r, 128 r + 128) of the tile
-// into its own shared memory (32 KB per stage instead of 48: what an SM has to take in per 512 tensor cycles is
-// what bounds the single-CTA kernel), one thread of the even CTA issues MMAs of 256 x 256 x 32 that read both CTAs'
-// tiles, and each CTA's TMEM receives its 128 rows x 256 columns, which its own epilogue warps drain as before.
+// The same GEMM on CTA pairs (thread-block clusters of two, tcgen05 cta_group::2): a pair computes a tile of 256 rows x TN
+// columns. CTA r of the pair loads A rows [128 r, 128 r + 128) and B rows (output columns) [TN/2 r, TN/2 r + TN/2) of the tile
+// into its own shared memory (at TN = 256 32 KB per K slab instead of 48: what an SM has to take in per 512 tensor cycles is
+// what bounds the single-CTA kernel), one thread of the even CTA issues MMAs of 256 x TN x 32 that read both CTAs'
+// tiles, and each CTA's TMEM receives its 128 rows x TN columns, which its own epilogue warps drain as before.
 // Barriers: the TMA loads of both CTAs count their bytes on the even CTA's `full`; stage release and accumulator
 // hand-over are commits to the barrier of each CTA in turn (no multicast form anywhere); the epilogue warps of both
 // CTAs arrive on the even CTA's `acc_empty`. Every wait is bounded as in the single-CTA kernel; the two cluster-wide
@@ -821,11 +821,12 @@ int launch_gemm_single(const CUtensorMap& ta, const CUtensorMap& tb, const GemmP
   return check_cuda(launch_chained(kern, dim3(grid), GEMM_THREADS, GEMM_SMEM_BYTES, stream, 1, ta, tb, p), "gemm launch");
 }
 
-// Columns of a tile. A K slab of a tile takes as long as the SM needs to take its operands in (about 72 bytes per clock) or the
-// tensor pipe to multiply them; a narrower tile loads the same A rows for fewer columns, so it pays where the full width leaves
-// SMs idle in its only or its last wave: the width with the smallest waves x time of a slab. `tile_rows` by `ctas` CTAs that
-// share a tile (each loads its rows of A and its part of B). Against every fixed width at six N x K and fifteen M from 1 to
-// 17,896 the rule is within 8 % of the best one. Time at 256 columns for everything / now, us: N = K = 4,096: 37 rows 13.2 / 7.5,
+// Columns of a tile. A K slab of a tile takes as long as the SM needs to take its operands in or the tensor pipe to multiply them; a
+// narrower tile loads the same A rows for fewer columns, so it pays where the full width leaves SMs idle in its only or its last
+// wave: the width with the smallest waves x time of a slab. `tile_rows` by `ctas` CTAs that share a tile (each loads its rows of A and
+// its part of B). The 72 bytes per clock are the model's, no measured rate (a ring filled by bulk copies alone, with all SMs at it,
+// reaches 61): what they are held against is every fixed width at six N x K and fifteen M from 1 to 17,896, where the rule is
+// within 8 % of the best one. Time at 256 columns for everything / now, us: N = K = 4,096: 37 rows 13.2 / 7.5,
 // 200 rows 15.6 / 8.4, 512 rows 15.9 / 10.3, 1,500 rows 25.3 / 20.9; N = 4,096, K = 16,384: 37 rows 43 / 25, 512 rows 42 / 29;
 // N = 12,288, K = 4,096: 37 rows 13.4 / 10.0, 512 rows 25.4 / 21.2.
 int tile_columns(long long M, long long N, long long K, int tile_rows, int ctas) {
@@ -888,8 +889,8 @@ int pairs_enabled() { return g_use_pairs.load(std::memory_order_relaxed); }
 
 using namespace rh3;
 
-// Selects the kernel the GEMM entries launch: 0 = one CTA per 128 x 256 tile, 1 (default) = CTA pairs on 256 x 256
-// tiles (gemm_pair_kernel) for every call with more than 128 rows and more than 128 columns. Returns the previous
+// Selects the kernel the GEMM entries launch: 0 = one CTA per tile of 128 rows, 1 (default) = CTA pairs on tiles of 256
+// rows (gemm_pair_kernel) for every call with more than 128 rows and more than 128 columns. Returns the previous
 // setting. Results are identical (int32 accumulators, same epilogue). The convolution follows the same switch
 // (conv3d_pair_kernel: fp32 accumulation in the same order, identical results).
 extern "C" int rh3_gemm_use_pairs(int on) { return g_use_pairs.exchange(on ? 1 : 0); }
