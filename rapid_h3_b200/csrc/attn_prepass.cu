@@ -664,6 +664,12 @@ __global__ void __launch_bounds__(256, 4) quant_tok_kernel(const __nv_bfloat16* 
 bool aligned(const void* p, uintptr_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }
 bool strides16(int64_t a, int64_t b) { return a % 8 == 0 && b % 8 == 0; }  // rows start on 16-byte boundaries
 
+// Launch 1 starts under the kernel before it (launch_kernel) up to 2^17 rows of Q, K on a stream, the launches behind it at every size;
+// in a graph only launch 2, one CTA per head. us with launch 1 chained / not on a stream: block of 1,008 tokens 465 / 468, of 2,024 753 /
+// 757, of 9,108 3,724 / 3,704, of 36,436 26.59 / 26.45 ms; attention of 6,196 tokens 711 / 701. All chained / launch 2 alone in a graph:
+// 512 x 512 x 32 41.3 / 33.1, 2,016 120.5 / 119.2.
+constexpr int64_t ROPE_CHAINED_ROWS = 1 << 17;
+
 int launch_rope_stats(RopeStatsParams p, int kv_ctas, cudaStream_t stream) {
   p.kv_ctas = kv_ctas;
   const int64_t ctas = static_cast<int64_t>(p.q_ctas) + kv_ctas;
@@ -678,7 +684,7 @@ int launch_rope_stats(RopeStatsParams p, int kv_ctas, cudaStream_t stream) {
   // keys (64) for 6,196 queries: 67.1 -> 58.6, for 36,436: 264 -> 258.
   p.kv_first = 5ll * kv_ctas <= 4ll * 2 * device_sm_count();
   auto kern = p.tab ? rope_stats_kernel<true> : rope_stats_kernel<false>;
-  return check_cuda(launch_kernel(false, kern, dim3(static_cast<unsigned>(ctas)), 256, 0, stream, 1, p), "attention pre-pass (rope / statistics) launch");
+  return check_cuda(launch_kernel(!in_capture(stream) && (p.Lq + p.Lk) * p.H <= ROPE_CHAINED_ROWS, kern, dim3(static_cast<unsigned>(ctas)), 256, 0, stream, 1, p), "attention pre-pass (rope / statistics) launch");
 }
 
 int kv_stats_run(const void* k, int64_t k_ss, int64_t k_sh, const void* v, int64_t v_ss, int64_t v_sh, int64_t L,
@@ -826,7 +832,7 @@ extern "C" int rh3_attn_quant_qk(const void* x, int64_t x_ss, int64_t x_sh, int6
   RH3_CHECK_ARG(aligned(x, 16) && aligned(codes, 16) && strides16(x_ss, x_sh) && (!mean || aligned(mean, 16)),
                 "attn_quant_qk: rows must be 16-byte aligned (strides multiples of 8 elements)");
   RH3_CHECK_ARG(Lpad / 128 < (1ll << 31), "attn_quant_qk: L too large");
-  const cudaError_t launched = launch_kernel(false, quant_kv_kernel<true, false>, dim3(static_cast<unsigned>(Lpad / 128), static_cast<unsigned>(H)), 256, 0, stream, 1,
+  const cudaError_t launched = launch_kernel(!in_capture(stream), quant_kv_kernel<true, false>, dim3(static_cast<unsigned>(Lpad / 128), static_cast<unsigned>(H)), 256, 0, stream, 1,
       static_cast<const __nv_bfloat16*>(x), x_ss, x_sh, nullptr, 0, 0, L, Lpad, mean, nullptr, nullptr,
       static_cast<int8_t*>(codes), scales, nullptr);
   return check_cuda(launched, "attn_quant_qk launch");
@@ -840,7 +846,7 @@ extern "C" int rh3_attn_quant_v(const void* v, int64_t v_ss, int64_t v_sh, int64
   RH3_CHECK_ARG(v && vmean && vscale && vt, "attn_quant_v: null pointer");
   RH3_CHECK_ARG(aligned(v, 16) && aligned(vt, 16) && aligned(vmean, 16) && aligned(vscale, 16) && strides16(v_ss, v_sh),
                 "attn_quant_v: rows must be 16-byte aligned (strides multiples of 8 elements)");
-  const cudaError_t launched = launch_kernel(false, quant_kv_kernel<false, true>, dim3(static_cast<unsigned>(Lpad / 128), static_cast<unsigned>(H)), 256, 0, stream, 1,
+  const cudaError_t launched = launch_kernel(!in_capture(stream), quant_kv_kernel<false, true>, dim3(static_cast<unsigned>(Lpad / 128), static_cast<unsigned>(H)), 256, 0, stream, 1,
       nullptr, 0, 0, static_cast<const __nv_bfloat16*>(v), v_ss, v_sh, L, Lpad, nullptr, vmean, vscale, nullptr, nullptr,
       static_cast<uint8_t*>(vt));
   return check_cuda(launched, "attn_quant_v launch");
@@ -897,7 +903,7 @@ extern "C" int rh3_attn_prepass(const void* q, int64_t q_ss, int64_t q_sh, int64
   const __nv_bfloat16* kq = k_weight ? static_cast<const __nv_bfloat16*>(k_roped) : static_cast<const __nv_bfloat16*>(k);
   const int64_t kq_ss = k_weight ? kr_ss : k_ss, kq_sh = k_weight ? kr_sh : k_sh;
   const dim3 kv_grid(static_cast<unsigned>(Lk_pad / 128), static_cast<unsigned>(H));
-  return check_cuda(launch_kernel(false, quant_kv_kernel<true, true>, kv_grid, 256, 0, stream, 1, kq, kq_ss, kq_sh,
+  return check_cuda(launch_kernel(!in_capture(stream), quant_kv_kernel<true, true>, kv_grid, 256, 0, stream, 1, kq, kq_ss, kq_sh,
                                    static_cast<const __nv_bfloat16*>(v), v_ss, v_sh, Lk, Lk_pad, kmean, vmean, vscale,
                                    static_cast<int8_t*>(k8), ks, static_cast<uint8_t*>(vt)),
                     "attn_prepass quantizer launch");
@@ -952,7 +958,7 @@ extern "C" int rh3_attn_tok_prepass(const void* q, int64_t q_ss, int64_t q_sh, i
     return e;
   // 3: Q rows (norm + rope fused), 4: K rows from the normalised copy, 5: V
   if (int e = check_cuda(
-          launch_kernel(false, quant_tok_kernel<false>, dim3(static_cast<unsigned>(q_ctas)), 256, 0, stream, 1,
+          launch_kernel(!in_capture(stream), quant_tok_kernel<false>, dim3(static_cast<unsigned>(q_ctas)), 256, 0, stream, 1,
                          static_cast<const __nv_bfloat16*>(q), q_ss, q_sh, Lq, Lq_pad, static_cast<int>(H),
                          static_cast<const __nv_bfloat16*>(q_weight), eps, static_cast<const __nv_bfloat16*>(rope_table),
                          static_cast<__nv_bfloat16*>(q_roped), qr_ss, qr_sh, nullptr, static_cast<int8_t*>(q8), qs),
@@ -960,12 +966,12 @@ extern "C" int rh3_attn_tok_prepass(const void* q, int64_t q_ss, int64_t q_sh, i
     return e;
   const __nv_bfloat16* kq = k_weight ? static_cast<const __nv_bfloat16*>(k_roped) : static_cast<const __nv_bfloat16*>(k);
   const int64_t kq_ss = k_weight ? kr_ss : k_ss, kq_sh = k_weight ? kr_sh : k_sh;
-  if (int e = check_cuda(launch_kernel(false, quant_tok_kernel<true>, dim3(static_cast<unsigned>(k_ctas)), 256, 0, stream, 1, kq, kq_ss, kq_sh, Lk, Lk_pad,
+  if (int e = check_cuda(launch_kernel(!in_capture(stream), quant_tok_kernel<true>, dim3(static_cast<unsigned>(k_ctas)), 256, 0, stream, 1, kq, kq_ss, kq_sh, Lk, Lk_pad,
                                         static_cast<int>(H), nullptr, eps, nullptr, nullptr, 0, 0, kmean, static_cast<int8_t*>(k8), ksb),
                          "attn_tok_prepass K launch"))
     return e;
   const dim3 kv_grid(static_cast<unsigned>(Lk_pad / 128), static_cast<unsigned>(H));
-  return check_cuda(launch_kernel(false, quant_kv_kernel<false, true, true>, kv_grid, 256, 0, stream, 1, nullptr, 0, 0, static_cast<const __nv_bfloat16*>(v),
+  return check_cuda(launch_kernel(!in_capture(stream), quant_kv_kernel<false, true, true>, kv_grid, 256, 0, stream, 1, nullptr, 0, 0, static_cast<const __nv_bfloat16*>(v),
                                    v_ss, v_sh, Lk, Lk_pad, nullptr, vmean, vscale, nullptr, nullptr, static_cast<uint8_t*>(vt)),
                     "attn_tok_prepass V launch");
 }

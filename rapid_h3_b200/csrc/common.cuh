@@ -649,11 +649,17 @@ namespace rh3 {
 // says grid_dependency_trigger() lets the next one start as soon as its own CTAs have all started. What overlaps is the launch
 // latency, the set-up of barriers and tensor memory and the ramp-up of a kernel with the tail of the one before: 1-2 us for each
 // launch of a chain of short kernels. `cluster` > 1 launches clusters of that many CTAs.
-// Chained are kernels of one CTA per SM (GEMM, attention, convolution), what runs between convolutions, and small grids. A kernel of
-// many CTAs that starts early is packed onto the SMs that are free by then, as many CTAs as fit on each, and stays distributed that
-// way. us chained / not: pre-pass of an attention call, 512 x 512 tokens x 32 heads 41.3 / 33.1 (the whole call), 1,008 x 512 keys 40.6 /
-// 34.3, 36,436 x 512 644 / 622; row quantizer of a linear, 256 x 4,096 11.7 / 11.2, 5,003 x 4,096 78.5 / 74.2, 3,024 x 16,384 191 / 176,
-// but 37 x 4,096 10.1 / 10.4; norms and upsampling of a 3 x 12 x 21 latent's decode 546 / 565.
+// Chained are kernels of one CTA per SM (GEMM, attention, convolution) and what runs between convolutions. A kernel of many CTAs that
+// starts early is packed onto the SMs that are free by then, as many CTAs as fit on each, and stays distributed that way: the row
+// kernels and the attention pre-pass are chained while they are small. Where that ends depends on what a plain launch costs: on a
+// stream some 2 us behind a kernel that it waits for, between two nodes of a graph hardly anything. us all chained / all plain,
+// calls queued on a stream: attention of 1,008 x 1,008 tokens x 32 heads 52.4 / 56.2, of 36,436 x 512 keys 652 / 639; a linear of
+// 512 x 4,096 15.5 / 16.5 with its row quantizer plain, of 5,003 80.4 / 79.4; the same from graphs: 50.0 / 47.6, 644 / 623, 13.6 / 13.4, 78.5 / 74.2.
+inline bool in_capture(cudaStream_t stream) {   // the legacy stream cannot be captured
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  return stream && stream != cudaStreamLegacy && cudaStreamIsCapturing(stream, &status) == cudaSuccess &&
+         status == cudaStreamCaptureStatusActive;
+}
 template <class... Params, class... Args>
 cudaError_t launch_kernel(bool chained, void (*kern)(Params...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream,
                           unsigned cluster, Args&&... args) {

@@ -439,10 +439,10 @@ __global__ void __launch_bounds__(256) tensor_absmax_kernel(const __nv_bfloat16*
   if (threadIdx.x == 0) atomicMax(reinterpret_cast<unsigned int*>(out), __float_as_uint(am));
 }
 
-// Row kernels start under the kernel before them (launch_kernel) while they are small: us of a linear with its quantizer chained / not,
-// N = 4,096: 128 x 4,096 rows 11.2 / 11.5, 148 11.3 / 10.8, 400 13.5 / 12.8; 200 x 2,048 8.55 / 8.35 at N = 4,096 and 9.06 / 9.43 at 5,376;
-// 400 x 1,024 6.5 / 7.0, 2,016 10.2 / 9.8; 37 x 16,384 28.9 / 26.1.
-bool chain_rows(int64_t M, int64_t K) { return M * K <= (1ll << 19); }
+// Row kernels start under the kernel before them (launch_kernel) while they are small. us chained / not on a stream, a linear with
+// its quantizer: 37 x 4,096 rows 11.1 / 12.4, 512 15.5 / 16.5, 2,016 34.4 / 35.2, 5,003 80.4 / 79.4; 512 x 16,384 42.2 / 42.8, 3,024 172 / 170; one
+// block of 2,024 tokens 746 / 753. From graphs: 128 x 4,096 11.2 / 11.5, 148 11.3 / 10.8, 400 13.5 / 12.8, 400 x 1,024 6.5 / 7.0.
+bool chain_rows(int64_t M, int64_t K, cudaStream_t stream) { return M * K <= (in_capture(stream) ? 1ll << 19 : 1ll << 23); }
 
 template <int KIND, int OUT_FP8, int ROT = 0>
 int launch_quant(const QuantParams& p, cudaStream_t stream) {
@@ -456,7 +456,7 @@ int launch_quant(const QuantParams& p, cudaStream_t stream) {
     int occ = 1;                                                                                       \
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, T_, 0) != cudaSuccess || occ < 1) occ = 1; \
     const int64_t resident = static_cast<int64_t>(device_sm_count()) * occ;                           \
-    launched = launch_kernel(chain_rows(p.M, p.K), kern, dim3(static_cast<unsigned>(p.M < resident ? p.M : resident)), T_, 0, stream, 1, p); \
+    launched = launch_kernel(chain_rows(p.M, p.K, stream), kern, dim3(static_cast<unsigned>(p.M < resident ? p.M : resident)), T_, 0, stream, 1, p); \
   } while (0)
   if (nchunk <= 128) RH3_Q(128, 1);
   else if (nchunk <= 256) RH3_Q(128, 2);
@@ -657,7 +657,7 @@ extern "C" int rh3_rms_norm_rows(const void* x, int64_t ldx, const void* w, floa
   do {                                                                                                            \
     auto kern = rms_norm_rows_kernel<T_, CPT_>;                                                                   \
     const int64_t resident = static_cast<int64_t>(device_sm_count()) * (2048 / T_ < 8 ? 2048 / T_ : 8);           \
-    launched = launch_kernel(chain_rows(M, K), kern, dim3(static_cast<unsigned>(M < resident ? M : resident)), T_, 0, stream, 1, \
+    launched = launch_kernel(chain_rows(M, K, stream), kern, dim3(static_cast<unsigned>(M < resident ? M : resident)), T_, 0, stream, 1, \
                              static_cast<const __nv_bfloat16*>(x), ldx, static_cast<const __nv_bfloat16*>(w),     \
                              eps, M, (int)K, static_cast<__nv_bfloat16*>(out), ldo);                              \
   } while (0)

@@ -254,8 +254,9 @@ int launch_out_quant(const OutQuantParams& p, cudaStream_t stream) {
   int occ = 1;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, T, 0) != cudaSuccess || occ < 1) occ = 1;
   const int64_t resident = static_cast<int64_t>(device_sm_count()) * occ;
-  // not chained at any size (launch_kernel): feed-forward of 64 rows 28.2 us, 28.8 chained, of 3,594 rows 218 and 225
-  return check_cuda(launch_kernel(false, kern, dim3(static_cast<unsigned>(p.rows < resident ? p.rows : resident)), T, 0, stream, 1, p),
+  // chained (launch_kernel) while small, and not in a graph. Feed-forward, us with both quantizers chained / not, on a stream: 64 rows
+  // 30.7 / 32.5, 1,000 75.2 / 78.9, 3,594 208.0 / 206.7; from graphs 28.8 / 28.2, 70.8 / 71.5, 224 / 218
+  return check_cuda(launch_kernel(!in_capture(stream) && p.rows * p.K <= (1ll << 23), kern, dim3(static_cast<unsigned>(p.rows < resident ? p.rows : resident)), T, 0, stream, 1, p),
                     "vae_out_quant launch");
 }
 template <int ACT>
