@@ -249,8 +249,8 @@ class FusedBlock:
         operands, x updated in place. False, with nothing done, for anything that call does not take as it is: more than two
         spans or per-token modulation rows, other layouts, widths or types. Those go on launch by launch."""
         blk, a = self.block, self.block.attn
-        if type(self) is not FusedBlock or len(tables) != 6 or not vars(FusedBlock).keys().isdisjoint(vars(self)):
-            return False   # a subclass, or a helper that was put in its place on this one block
+        if type(self) is not FusedBlock or len(tables) != 6 or "_gemm_gated" in vars(self):
+            return False   # a subclass, or the one helper that the call passes by put in its place on this block
         s, d = x.shape
         hd, two = a.heads * 128, self._two_gates(mod_segments, s, tables[2])
         first = tables[0]
